@@ -8,18 +8,32 @@
 //   MMA warp         S^T[row, head] = K_block . Q^T      (K panels as the K-major A operand)
 //                    O^T[dim, head] += V^T . P           (the same panels as the MN-major A operand:
 //                                                         K = V = the latent row, stored once)
-//   softmax warps    read S^T from TMEM (one row per thread), online softmax with a per-head running
-//                    maximum (cross-row maximum by warp shuffles), write P as the K-major B operand,
-//                    rescale O in TMEM only when a head's maximum moved
+//   softmax warps    read S^T from TMEM (one row and half of the heads per thread), write P as the K-major B
+//                    operand, rescale O in TMEM only when some score outgrew its head's maximum by 2^8
+//
+// What bounds it: the key block (128 KB in bf16) and Q (64 KB) fill shared memory, so there is one key buffer, and a block is
+// scores -> softmax -> values in turn.  Everything else is taken off that chain:
+//   * panels change hands one by one: scores start on the first panel that has landed, and a pair of panels goes back to the
+//     producers as soon as its 128 output dims are accumulated, so the next block is written under the value products;
+//   * sixteen producer warps hold the codes of the whole next block in registers, so no gather latency is on the chain (eight
+//     warps with twice the rows each left the conversions waiting for their own results); a load instruction takes 64 contiguous
+//     bytes of eight rows, and its two stores per lane hit every bank once.  The rotated part needs no conversion: it is copied
+//     asynchronously into the panel that is freed first and scored last;
+//   * the softmax works with a maximum that may be stale by up to 2^8 (weights keep their relative precision, only their common
+//     factor moves), so the reductions over the 128 rows that a maximum needs run for a token's first block and rarely after;
+//     the row sums of P stay in registers (one per head and row) and are reduced once per CTA.
+// Measured (4096 tokens, 64 heads, 128 + 2048 rows): 5166 us with one thread block of thirteen warps working through
+// load -> scores -> softmax -> values without overlap, 2524 us now (8400 cycles per block, 3100 of them on the tensor cores).
 //
 // Accumulators live in TMEM: S (NH columns) and four O^T tiles of [128 dims x NH heads].
-// The CTA writes an un-normalised partial (o, m, l) that `sparse_mla_combine` merges with the sink.
+// A CTA of a split writes an un-normalised partial (o, m, l) that `sparse_mla_combine` merges with the sink.
 // Every mbarrier wait is bounded; on expiry the status word is set and the CTA drains and exits.
 //
 // Replaces the reference's FlashInfer sparse-MLA decode/prefill kernels
 // (overlay/flashinfer_sparse.py:323-541).
 #define STK_PDL_CLASS 128      // bit of this file's kernels in the PDL mask (STK_PDL, stk_set_pdl_mask)
 #include "common.cuh"
+#include "pairs.cuh"
 #include "warp_reduce.cuh"
 
 namespace stk {
@@ -53,26 +67,49 @@ __device__ __forceinline__ unsigned long long global_ns() {
 
 constexpr int kD = 512, kR = 64, kNope = 448, kDataBytes = 576, kPanels = 8, kRows = 128;
 constexpr int kPanelBytes = kRows * 128;                 // 16 KB
-constexpr int kProducerWarps = 8, kSoftmaxWarps = 4;
-constexpr int kThreads = 32 * (1 + kSoftmaxWarps + kProducerWarps);
+constexpr int kProducerWarps = 16;
+constexpr float kStale = 8.f;                            // how far (in powers of two) a score may pass the maximum in use
 
-struct alignas(8) MlaBars {
-  uint64_t k_full, s_full, p_full, pv_done;
-  uint32_t tmem_base;
-  int abort_flag;
+// Warpgroups: the first issues products (one warp of it), then the softmax warps, then the producers.  From 32 heads on two
+// softmax warps share a lane quarter of TMEM and take half of the heads each.  Registers follow the roles: what the first
+// warpgroup gives back (launch total 640 x 96) pays for the sums that the softmax warps hold.
+template <int NH>
+struct MlaCfg {
+  static constexpr int kHalves = NH >= 32 ? 2 : 1;
+  static constexpr int kHeads = NH / kHalves;            // heads per softmax thread
+  static constexpr int kSoftmaxWarps = 4 * kHalves;
+  static constexpr int kThreads = 32 * (4 + kSoftmaxWarps + kProducerWarps);
+  static constexpr int kLaunchRegs = kThreads > 768 ? 72 : 80;
+  static constexpr int kIssueRegs = 24, kSoftmaxRegs = kHalves == 2 ? 96 : 128, kProducerRegs = 72;
+  static_assert(128 * kIssueRegs + 32 * kSoftmaxWarps * kSoftmaxRegs + 32 * kProducerWarps * kProducerRegs <= kThreads * kLaunchRegs,
+                "register split");
+  static constexpr int kTmemCols = (5 * NH <= 128) ? 128 : (5 * NH <= 256) ? 256 : 512;
 };
 
-__device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
-      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-      "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]),
-      "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]),
-      "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-      : "memory");
+constexpr int kBarBytes = 192;
+// Order in which panels are written and scored, and in which pairs of them are summed and freed: the rotated part (panel 7)
+// is freed first and needed last.
+__device__ __forceinline__ constexpr int panel_at(int i) { return i == 0 ? 6 : i == 7 ? 7 : i - 1; }
+__device__ __forceinline__ constexpr int pair_at(int i) { return i == 0 ? 3 : i - 1; }
+
+__device__ __forceinline__ void copy16_async(void* smem_dst, const void* src, bool valid) {     // zeros where there is no row
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(smem_dst)), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
+
+template <int N>
+__device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+
+struct alignas(8) MlaBars {
+  uint64_t k_full[5];              // panels 0 + 1, 2 + 3, 4 + 5, 6, 7 of the block are in shared memory
+  uint64_t k_free[kPanels / 2];    // the value products of a pair of panels are done
+  uint64_t s_full, p_full, pv_done;
+  uint32_t tmem_base;
+  int grow[2];                     // by block parity: some score outgrew its head's maximum
+};
+static_assert(sizeof(MlaBars) <= kBarBytes, "barrier block");
+
 __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
@@ -83,44 +120,40 @@ __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// MN-major operand, 128-byte swizzle: 128-byte column blocks are `lbo` bytes apart along M/N,
-// 8-row groups are 1024 bytes apart along K.
-__device__ __forceinline__ uint64_t umma_desc_mn_sw128(uint32_t smem_addr, uint32_t lbo_bytes) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((smem_addr & 0x3FFFF) >> 4);
-  d |= static_cast<uint64_t>(lbo_bytes >> 4) << 16;
-  d |= static_cast<uint64_t>(1024 >> 4) << 32;
-  d |= static_cast<uint64_t>(1) << 46;
-  d |= static_cast<uint64_t>(2) << 61;
-  return d;
-}
-
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
 
+__device__ __forceinline__ void put16(uint32_t smem_addr, uint32_t v) {
+  asm volatile("st.shared.b16 [%0], %1;" ::"r"(smem_addr), "h"(static_cast<unsigned short>(v)) : "memory");
+}
+
 __device__ __forceinline__ void named_bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 
-// fp8 e4m3 x4 (one 32-bit word) times a power-of-two scale -> four bf16 (two packed words)
-__device__ __forceinline__ void fp8x4_to_bf16x4(uint32_t w, float sc, uint32_t& lo, uint32_t& hi) {
-  const __half2_raw h01 = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(w & 0xffff), __NV_E4M3);
-  const __half2_raw h23 = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(w >> 16), __NV_E4M3);
-  const float2 f01 = __half22float2(*reinterpret_cast<const __half2*>(&h01));
-  const float2 f23 = __half22float2(*reinterpret_cast<const __half2*>(&h23));
-  const __nv_bfloat162 b01 = __floats2bfloat162_rn(f01.x * sc, f01.y * sc);
-  const __nv_bfloat162 b23 = __floats2bfloat162_rn(f23.x * sc, f23.y * sc);
-  lo = *reinterpret_cast<const uint32_t*>(&b01);
-  hi = *reinterpret_cast<const uint32_t*>(&b23);
+// Four e4m3 codes (one word) times a power of two -> four bf16.  (Moving the codes' bits into place and one product per pair
+// measured half this rate: shifts and logic share one pipe, which these conversions mostly leave alone.)
+__device__ __forceinline__ void e4m3x4_to_bf16(uint32_t w, uint64_t scale2, uint32_t& lo, uint32_t& hi) {
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(i ? w >> 16 : w & 0xffff), __NV_E4M3);
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
+    float x, y;
+    unpack2(mul2(pack2(f.x, f.y), scale2), x, y);
+    const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
+    (i ? hi : lo) = *reinterpret_cast<const uint32_t*>(&v);
+  }
 }
 
 template <int NH>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(MlaCfg<NH>::kThreads, 1)
 sparse_mla_tc_kernel(const MlaTcArgs a) {
   pdl_wait();
   pdl_trigger();
-  constexpr int kTmemCols = (5 * NH <= 128) ? 128 : (5 * NH <= 256) ? 256 : 512;
+  using Cfg = MlaCfg<NH>;
+  constexpr int kThreads = Cfg::kThreads, kSoftmaxWarps = Cfg::kSoftmaxWarps, kHeads = Cfg::kHeads;
+  constexpr int kSoftmaxThreads = kSoftmaxWarps * 32;
   constexpr int kQBytes = kPanels * NH * 128;
   constexpr int kPBytes = 2 * NH * 128;
   extern __shared__ uint8_t smem_raw[];
@@ -129,12 +162,11 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
   uint8_t* q_s = k_s + kPanels * kPanelBytes;            // 8 panels x NH x 128 B
   uint8_t* p_s = q_s + kQBytes;                          // 2 panels x NH x 128 B
   MlaBars* bars = reinterpret_cast<MlaBars*>(p_s + kPBytes);
-  float* smax = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 64);   // [4][NH]
-  float* m_run = smax + 4 * NH;                          // [NH]
-  float* alpha_s = m_run + NH;                           // [NH]
-  float* lsum = alpha_s + NH;                            // [4][NH]
-  float* l_run = lsum + 4 * NH;                          // [NH]
-  int* flags = reinterpret_cast<int*>(l_run + NH);       // [0] any head rescaled in this block
+  float* smax = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + kBarBytes);  // [4][NH], row sums at the end
+  float* m_run = smax + 4 * NH;                          // [NH] the maxima in use, in powers of two
+  float* minus_m = m_run + NH;                           // [NH] their negatives (0 for none yet)
+  float* limit = minus_m + NH;                           // [NH] a score above this needs a new maximum
+  float* alpha_s = limit + NH;                           // [NH]
 
   const int t = blockIdx.x, sp = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -162,199 +194,234 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
   }
 
   if (threadIdx.x == 0) {
-    mbar_init(&bars->k_full, kProducerWarps);
+    for (int p = 0; p < 5; ++p) mbar_init(&bars->k_full[p], kProducerWarps);
+    for (int j = 0; j < kPanels / 2; ++j) mbar_init(&bars->k_free[j], 1);
     mbar_init(&bars->s_full, 1);
     mbar_init(&bars->p_full, kSoftmaxWarps);
     mbar_init(&bars->pv_done, 1);
-    bars->abort_flag = 0;
+    bars->grow[0] = bars->grow[1] = 0;
     fence_barrier_init();
   }
   if (warp == 0) {
-    tmem_alloc(&bars->tmem_base, kTmemCols);
+    tmem_alloc(&bars->tmem_base, Cfg::kTmemCols);
     tmem_relinquish();
   }
-  // Q -> shared memory, K-major panels [NH x 64 dims], 128-byte swizzle; heads >= nh are zero.
-  // All global loads of a thread are issued before its stores.
-  {
-    constexpr int kChunks = NH * (kD / 8);
-    constexpr int kPer = (kChunks + kThreads - 1) / kThreads;
-    uint4 qv[kPer];
-#pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-      const int i = threadIdx.x + j * kThreads;
-      qv[j] = make_uint4(0, 0, 0, 0);
-      if (i < kChunks) {
-        const int h = i / (kD / 8), c8 = i % (kD / 8);
-        if (h < a.nh) qv[j] = __ldg(reinterpret_cast<const uint4*>(a.q + t * a.ldt + static_cast<long long>(h) * kD + c8 * 8));
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-      const int i = threadIdx.x + j * kThreads;
-      if (i < kChunks) {
-        const int h = i / (kD / 8), c8 = i % (kD / 8);
-        const int panel = c8 >> 3, c = c8 & 7;
-        *reinterpret_cast<uint4*>(q_s + panel * (NH * 128) + h * 128 + ((c ^ (h & 7)) << 4)) = qv[j];
-      }
-    }
-  }
-  if (threadIdx.x < NH) { m_run[threadIdx.x] = -INFINITY; l_run[threadIdx.x] = 0.f; }
-  fence_proxy_async();
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  if (threadIdx.x == 0) STK_TRACE(1);
-  const uint32_t tmem_base = bars->tmem_base;
-  const uint32_t tmem_s = tmem_base;                     // S^T: NH columns
-  const uint32_t tmem_o = tmem_base + NH;                // 4 x NH columns
+  // slot of row li of this token's list (-1: none), and the cache it lies in
+  auto slot_of = [&](int li) -> int {
+    if (li >= r_end) return -1;
+    return li < n_swa ? a.swa_slots[static_cast<long long>(t) * a.swa_ld + li]
+                      : a.topk_slots[static_cast<long long>(t) * a.topk_ld + (li - n_swa)];
+  };
 
-  if (warp == 0) {
-    // ------------------------------- MMA issuer -------------------------------
-    if (lane == 0) {
+  // every warp passes this once its part of the prologue is done
+  auto begin = [&]() {
+    fence_proxy_async();
+    tc_fence_before();
+    named_bar_sync(1, kThreads);
+    tc_fence_after();
+  };
+  auto load_q = [&]() {
+    // Q -> shared memory, K-major panels [NH x 64 dims], 128-byte swizzle; heads >= nh are zero.
+    constexpr int kChunks = NH * (kD / 8), kLoaders = 32 * kSoftmaxWarps, kBatch = 8;
+    for (int i0 = threadIdx.x - 128; i0 < kChunks; i0 += kLoaders * kBatch) {
+      uint4 qv[kBatch];
+#pragma unroll
+      for (int j = 0; j < kBatch; ++j) {
+        const int i = i0 + j * kLoaders, h = i / (kD / 8), c8 = i % (kD / 8);
+        qv[j] = make_uint4(0, 0, 0, 0);
+        if (i < kChunks && h < a.nh) qv[j] = __ldg(reinterpret_cast<const uint4*>(a.q + t * a.ldt + static_cast<long long>(h) * kD + c8 * 8));
+      }
+#pragma unroll
+      for (int j = 0; j < kBatch; ++j) {
+        const int i = i0 + j * kLoaders, h = i / (kD / 8), c8 = i % (kD / 8);
+        if (i < kChunks) *reinterpret_cast<uint4*>(q_s + (c8 >> 3) * (NH * 128) + h * 128 + (((c8 & 7) ^ (h & 7)) << 4)) = qv[j];
+      }
+    }
+    if (threadIdx.x - 128 < NH) m_run[threadIdx.x - 128] = -INFINITY;
+  };
+
+  if (warp < 4) {
+    reg_dec<Cfg::kIssueRegs>();
+    begin();
+    if (threadIdx.x == 0) STK_TRACE(1);
+    if (warp == 0) {
+      // ------------------------------- MMA issuer -------------------------------
+      const uint32_t tmem_s = bars->tmem_base, tmem_o = tmem_s + NH;
+      const uint32_t lead = elect_one() ? 1u : 0u, ts = __shfl_sync(0xffffffffu, tmem_s, 0), to = __shfl_sync(0xffffffffu, tmem_o, 0);
       constexpr uint32_t kIdescQK = umma_idesc(1u, 1u, 128, NH);
       constexpr uint32_t kIdescPV = umma_idesc(1u, 1u, 128, NH) | (1u << 15);     // A is MN-major
+      constexpr uint32_t kStep = kPanelBytes >> 4, kQStep = (NH * 128) >> 4;      // panels in descriptor units
+      const uint32_t k_lo = desc_lo(smem_u32(k_s)), v_lo = desc_lo(smem_u32(k_s), kPanelBytes);
+      const uint32_t q_lo = desc_lo(smem_u32(q_s)), p_lo = desc_lo(smem_u32(p_s));
       bool ok = true;
       for (int b = 0; b < n_blocks && ok; ++b) {
         const uint32_t ph = b & 1;
-        if (!mbar_wait(&bars->k_full, ph, a.status, 600)) { ok = false; break; }
-        if (b == 0) STK_TRACE(2);
-        tc_fence_after();
-#pragma unroll
-        for (int p = 0; p < kPanels; ++p) {
-          const uint64_t ad = umma_desc_sw128(smem_u32(k_s + p * kPanelBytes));
-          const uint64_t bd = umma_desc_sw128(smem_u32(q_s + p * (NH * 128)));
-#pragma unroll
-          for (int k = 0; k < 4; ++k) umma_f16(tmem_s, ad + 2 * k, bd + 2 * k, kIdescQK, (p | k) != 0);
-        }
-        umma_commit(&bars->s_full);
-        if (!mbar_wait(&bars->p_full, ph, a.status, 601)) { ok = false; break; }
-        if (b == 0) STK_TRACE(4);
-        tc_fence_after();
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-#pragma unroll
-          for (int kk = 0; kk < 8; ++kk) {
-            const uint64_t ad = umma_desc_mn_sw128(smem_u32(k_s + (2 * j) * kPanelBytes + kk * 2048), kPanelBytes);
-            const uint64_t bd = umma_desc_sw128(smem_u32(p_s + (kk >> 2) * (NH * 128))) + 2 * (kk & 3);
-            umma_f16(tmem_o + j * NH, ad, bd, kIdescPV, (b > 0 || kk > 0) ? 1u : 0u);
+#pragma unroll 1
+        for (int i = 0; i < kPanels; ++i) {
+          const int p = panel_at(i);
+          if (i != 2 && i != 4 && i != 6) {
+            ok = ok && mbar_wait(&bars->k_full[p < 6 ? p >> 1 : p - 3], ph, a.status, 600);
+            if (!ok) break;
+            tc_fence_after();
           }
+          if (b == 0 && i == 0 && lane == 0) STK_TRACE(2);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) mma_ss(ts, k_lo + p * kStep + 2 * k, q_lo + p * kQStep + 2 * k, kIdescQK, (i | k) != 0 ? 1u : 0u, lead);
         }
-        umma_commit(&bars->pv_done);
+        if (!ok) break;
+        mma_commit(&bars->s_full, lead);
+        ok = mbar_wait(&bars->p_full, ph, a.status, 601);
+        if (!ok) break;
+        tc_fence_after();
+        if (b == 0 && lane == 0) STK_TRACE(4);
+#pragma unroll 1
+        for (int i = 0; i < kPanels / 2; ++i) {
+          const int j = pair_at(i);
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)
+            mma_ss(to + j * NH, v_lo + 2 * j * kStep + kk * 128, p_lo + (kk >> 2) * kQStep + 2 * (kk & 3), kIdescPV, (b > 0 || kk > 0) ? 1u : 0u, lead);
+          mma_commit(&bars->k_free[j], lead);
+        }
       }
-      if (!ok) bars->abort_flag = 1;
+      // what was issued completes before the tensor memory goes away
+      mma_commit(&bars->pv_done, lead);
+      mbar_wait(&bars->pv_done, 0, a.status, 602);
+      __syncwarp();
     }
-  } else if (warp <= kSoftmaxWarps) {
+  } else if (warp < 4 + kSoftmaxWarps) {
     // ------------------------------- softmax / epilogue -------------------------------
+    if constexpr (Cfg::kSoftmaxRegs > Cfg::kLaunchRegs) reg_inc<Cfg::kSoftmaxRegs>();
+    load_q();
+    begin();
+    const uint32_t tmem_s = bars->tmem_base, tmem_o = tmem_s + NH;       // S^T: NH columns; O^T: 4 x NH columns
     const int q4 = warp & 3;                              // TMEM lane quarter
     const int row = q4 * 32 + lane;                       // row of the block owned by this thread
-    const int sw = warp - 1;                              // 0..3
+    const int h0 = ((warp - 4) >> 2) * kHeads;            // its first head
     const uint32_t lane_addr = static_cast<uint32_t>(q4 * 32) << 16;
     const float sl2 = a.scale * 1.4426950408889634f;
-    const int own = threadIdx.x - 32;                     // owner thread of head `own` when < NH
-    bool ok = true;
-    for (int b = 0; b < n_blocks && ok; ++b) {
+    const int own = threadIdx.x - 128;                   // owner thread of head `own` when < NH
+    uint64_t lp[kHeads / 2];                              // sums of this row's weights, two heads each
+#pragma unroll
+    for (int i = 0; i < kHeads / 2; ++i) lp[i] = 0ull;
+    // this row's place in a head's line of P: the 16-byte chunk number is turned by the head's low bits
+    uint32_t pdst[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      pdst[i] = smem_u32(p_s) + (row >> 6) * (NH * 128) + (h0 + i) * 128 + ((((row & 63) >> 3) ^ i) << 4) + (row & 7) * 2;
+    const uint64_t sl22 = pack2(sl2, sl2);
+    int slot = slot_of(r_begin + row);
+    bool ok = true;                                       // the same in every lane; barriers are passed either way
+    auto scores = [&](int c, uint32_t (&r16)[16]) {       // sixteen heads' products of this row
+      tmem_ld_32x16(tmem_s + lane_addr + h0 + c, r16);
+      tmem_ld_wait();
+    };
+    for (int b = 0; b < n_blocks; ++b) {
       const uint32_t ph = b & 1;
-      const int li = r_begin + b * kRows + row;
-      bool valid = li < r_end;
-      if (valid) {
-        const int slot = li < n_swa ? a.swa_slots[static_cast<long long>(t) * a.swa_ld + li]
-                                    : a.topk_slots[static_cast<long long>(t) * a.topk_ld + (li - n_swa)];
-        valid = slot >= 0;
-      }
-      if (!mbar_wait(&bars->s_full, ph, a.status, 610)) { ok = false; break; }
-      if (b == 0 && threadIdx.x == 32) STK_TRACE(3);
+      const bool valid = slot >= 0;
+      slot = slot_of(r_begin + (b + 1) * kRows + row);
+      ok = __all_sync(0xffffffffu, ok && mbar_wait(&bars->s_full, ph, a.status, 610));
+      if (b == 0 && threadIdx.x == 128) STK_TRACE(3);
       tc_fence_after();
-      float s[NH];
+      if (b > 0) {
+        bool grow = false;
 #pragma unroll
-      for (int c = 0; c < NH; c += 16) {
-        uint32_t r16[16];
-        tmem_ld_32x16(tmem_s + lane_addr + c, r16);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 16; ++i) s[c + i] = valid ? __uint_as_float(r16[i]) * sl2 : -INFINITY;
-      }
-      if (b == 0 && threadIdx.x == 32) STK_TRACE(8);
-      // block maximum per head over the 128 rows (destroys s; it is re-read from TMEM below)
-      bfly_reduce_store<NH, true>(s, smax + sw * NH, lane);
-      if (b == 0 && threadIdx.x == 32) STK_TRACE(9);
-      named_bar_sync(2, kSoftmaxWarps * 32);
-      if (own < NH) {
-        const float bm = fmaxf(fmaxf(smax[own], smax[NH + own]), fmaxf(smax[2 * NH + own], smax[3 * NH + own]));
-        const float mo = m_run[own];
-        const float mn = fmaxf(mo, bm);
-        const float al = (mo == -INFINITY || mn == -INFINITY) ? 1.f : exp2f(mo - mn);     // mo == mn -> 1
-        alpha_s[own] = al;
-        m_run[own] = mn;
-        l_run[own] *= al;
-      }
-      if (threadIdx.x == 32) flags[0] = 0;
-      named_bar_sync(2, kSoftmaxWarps * 32);
-      if (own < NH && b > 0 && alpha_s[own] != 1.f) flags[0] = 1;
-      if (b == 0 && threadIdx.x == 32) STK_TRACE(11);
-      // P = exp2(s - m), bf16, written as the K-major B operand [head][row]
-      const int ppanel = row >> 6, prow_in = row & 63;
-      uint8_t* pdst = p_s + ppanel * (NH * 128) + (prow_in & 7) * 2;
-#pragma unroll
-      for (int c = 0; c < NH; c += 16) {
-        uint32_t r16[16];
-        tmem_ld_32x16(tmem_s + lane_addr + c, r16);
-        float mloc[16];
-#pragma unroll
-        for (int i = 0; i < 16; i += 4) {
-          const float4 m4 = *reinterpret_cast<const float4*>(m_run + c + i);
-          mloc[i] = m4.x; mloc[i + 1] = m4.y; mloc[i + 2] = m4.z; mloc[i + 3] = m4.w;
-        }
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const int h = c + i;
-          const float p = (!valid || mloc[i] == -INFINITY) ? 0.f : ex2_approx(__uint_as_float(r16[i]) * sl2 - mloc[i]);
-          const __nv_bfloat16 pb = __float2bfloat16(p);
-          s[h] = __bfloat162float(pb);
-          *reinterpret_cast<__nv_bfloat16*>(pdst + h * 128 + (((prow_in >> 3) ^ (h & 7)) << 4)) = pb;
-        }
-      }
-      // row sums of P per head (the same rounded values the tensor core multiplies)
-      bfly_reduce_store<NH, false>(s, lsum + sw * NH, lane);
-      if (b == 0 && threadIdx.x == 32) STK_TRACE(12);
-      named_bar_sync(2, kSoftmaxWarps * 32);
-      if (b == 0 && threadIdx.x == 32) STK_TRACE(13);
-      if (own < NH) l_run[own] += lsum[own] + lsum[NH + own] + lsum[2 * NH + own] + lsum[3 * NH + own];
-      if (flags[0]) {
-        // some head's maximum moved: scale the O^T columns (the previous block's PV has completed,
-        // because this block's rows could only be loaded after it)
-#pragma unroll
-        for (int c = 0; c < NH; c += 16) {
-          float al[16];
+        for (int c = 0; c < kHeads; c += 16) {
+          uint32_t r16[16];
+          scores(c, r16);
 #pragma unroll
           for (int i = 0; i < 16; i += 4) {
-            const float4 a4 = *reinterpret_cast<const float4*>(alpha_s + c + i);
-            al[i] = a4.x; al[i + 1] = a4.y; al[i + 2] = a4.z; al[i + 3] = a4.w;
-          }
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            uint32_t r16[16];
-            tmem_ld_32x16(tmem_o + j * NH + c + lane_addr, r16);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 16; ++i) r16[i] = __float_as_uint(__uint_as_float(r16[i]) * al[i]);
-            tmem_st_32x16(tmem_o + j * NH + c + lane_addr, r16);
+            const float4 l4 = *reinterpret_cast<const float4*>(limit + h0 + c + i);
+            grow = grow || __uint_as_float(r16[i]) * sl2 > l4.x || __uint_as_float(r16[i + 1]) * sl2 > l4.y ||
+                   __uint_as_float(r16[i + 2]) * sl2 > l4.z || __uint_as_float(r16[i + 3]) * sl2 > l4.w;
           }
         }
-        tmem_st_wait();
+        if (__any_sync(0xffffffffu, grow && valid) && lane == 0) bars->grow[ph] = 1;
+        named_bar_sync(2, kSoftmaxThreads);
+      }
+      if (b == 0 || bars->grow[ph]) {
+        // new maxima for all heads
+#pragma unroll 1
+        for (int c = 0; c < kHeads; c += 16) {
+          uint32_t r16[16];
+          scores(c, r16);
+          float s[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) s[i] = valid ? __uint_as_float(r16[i]) * sl2 : -INFINITY;
+          bfly_reduce_store<16, true>(s, smax + q4 * NH + h0 + c, lane);
+        }
+        named_bar_sync(2, kSoftmaxThreads);
+        if (own < NH) {
+          const float bm = fmaxf(fmaxf(smax[own], smax[NH + own]), fmaxf(smax[2 * NH + own], smax[3 * NH + own]));
+          const float mo = m_run[own], mn = fmaxf(mo, bm);
+          alpha_s[own] = (mo == -INFINITY || mn == -INFINITY) ? 1.f : exp2f(mo - mn);
+          m_run[own] = mn;
+          minus_m[own] = mn == -INFINITY ? 0.f : -mn;
+          limit[own] = mn + kStale;
+        }
+        if (threadIdx.x == 128) bars->grow[ph] = 0;        // everybody has read it; next written two blocks on
+        named_bar_sync(2, kSoftmaxThreads);
+        if (b > 0) {
+#pragma unroll
+          for (int i = 0; i < kHeads; i += 2) lp[i / 2] = mul2(lp[i / 2], pack2(alpha_s[h0 + i], alpha_s[h0 + i + 1]));
+          // this block's scores were issued behind the previous block's value products: those are complete
+#pragma unroll 1
+          for (int c = 0; c < 4 * kHeads; c += 16) {
+            const uint32_t at = tmem_o + (c / kHeads) * NH + h0 + c % kHeads + lane_addr;
+            uint32_t r16[16];
+            tmem_ld_32x16(at, r16);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) r16[i] = __float_as_uint(__uint_as_float(r16[i]) * alpha_s[h0 + c % kHeads + i]);
+            tmem_st_32x16(at, r16);
+          }
+          tmem_st_wait();
+        }
+      }
+      // P = exp2(s - m), bf16, written as the K-major B operand [head][row]; the sums take the rounded values
+#pragma unroll
+      for (int c = 0; c < kHeads; c += 16) {
+        uint32_t r16[16];
+        scores(c, r16);
+        if (valid) {
+#pragma unroll
+          for (int i = 0; i < 16; i += 4) {
+            const ulonglong2 m4 = *reinterpret_cast<const ulonglong2*>(minus_m + h0 + c + i);
+#pragma unroll
+            for (int k = 0; k < 4; k += 2) {
+              float x, y;
+              unpack2(fma2(pack2(__uint_as_float(r16[i + k]), __uint_as_float(r16[i + k + 1])), sl22, k ? m4.y : m4.x), x, y);
+              const __nv_bfloat162 p = __floats2bfloat162_rn(ex2_approx(x), ex2_approx(y));
+              const uint32_t u = *reinterpret_cast<const uint32_t*>(&p);
+              lp[(c + i + k) / 2] = add2(lp[(c + i + k) / 2], pack2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)));
+              put16(pdst[(i + k) & 7] + (c + ((i + k) & 8)) * 128, u);
+              put16(pdst[(i + k + 1) & 7] + (c + ((i + k) & 8)) * 128, u >> 16);
+            }
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) put16(pdst[i & 7] + (c + (i & 8)) * 128, 0u);
+        }
       }
       fence_proxy_async();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars->p_full);
     }
-    // ---- epilogue: wait for the last PV, write the partial ----
-    if (ok) ok = mbar_wait(&bars->pv_done, (n_blocks - 1) & 1, a.status, 611);
-    if (threadIdx.x == 32) STK_TRACE(5);
+    // ---- epilogue: wait for the last value products, reduce the row sums ----
+    ok = __all_sync(0xffffffffu, ok && mbar_wait(&bars->pv_done, 0, a.status, 611));
+    if (threadIdx.x == 128) STK_TRACE(5);
     tc_fence_after();
-    if (ok && a.out != nullptr) {
+#pragma unroll
+    for (int c = 0; c < kHeads; c += 16) {
+      float l16[16];
+#pragma unroll
+      for (int i = 0; i < 16; i += 2) unpack2(lp[(c + i) / 2], l16[i], l16[i + 1]);
+      bfly_reduce_store<16, false>(l16, smax + q4 * NH + h0 + c, lane);
+    }
+    named_bar_sync(2, kSoftmaxThreads);
+    const float l_own = own < NH ? (smax[own] + smax[NH + own]) + (smax[2 * NH + own] + smax[3 * NH + own]) : 0.f;
+    if (a.out != nullptr) {
       // direct output: per-head factor exp(m - M) / (exp(sink - M) + l * exp(m - M)) with M = max(sink, m)
-      named_bar_sync(2, kSoftmaxWarps * 32);
       if (own < NH) {
         const float m_nat = m_run[own] * 0.6931471805599453f;
         const float sk = (a.sink != nullptr && own < a.nh) ? a.sink[own] : -INFINITY;
@@ -362,29 +429,32 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
         float f = 0.f;
         if (m_nat != -INFINITY) {
           const float w = __expf(m_nat - M);
-          const float denom = (sk != -INFINITY ? __expf(sk - M) : 0.f) + l_run[own] * w;
+          const float denom = (sk != -INFINITY ? __expf(sk - M) : 0.f) + l_own * w;
           f = denom > 0.f ? w / denom : 0.f;
         }
         alpha_s[own] = f;
       }
-      named_bar_sync(2, kSoftmaxWarps * 32);
+      named_bar_sync(2, kSoftmaxThreads);
+    }
+    if (ok && a.out != nullptr) {
       __nv_bfloat16* orow = a.out + static_cast<long long>(t) * a.ldo;
       const float pos = a.positions != nullptr ? static_cast<float>(a.positions[t]) : 0.f;
-#pragma unroll
+#pragma unroll 1
       for (int j = 0; j < 4; ++j) {
         const int d = j * 128 + row;
         const bool rot = a.positions != nullptr && j == 3 && q4 >= 2;      // d >= 448: warp-uniform
         float sn = 0.f, cs = 1.f;
         if (rot) sincosf(pos * a.inv_freq[(d - kNope) >> 1], &sn, &cs);
-#pragma unroll
-        for (int c = 0; c < NH; c += 16) {
+#pragma unroll 1
+        for (int c = 0; c < kHeads; c += 16) {
           uint32_t r16[16];
-          tmem_ld_32x16(tmem_o + j * NH + c + lane_addr, r16);
+          tmem_ld_32x16(tmem_o + j * NH + h0 + c + lane_addr, r16);
           tmem_ld_wait();
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            if (c + i < a.nh) {
-              float v = __uint_as_float(r16[i]) * alpha_s[c + i];
+            const int h = h0 + c + i;
+            if (h < a.nh) {
+              float v = __uint_as_float(r16[i]) * alpha_s[h];
               if (rot) {
                 // the pair (even d, d + 1) sits in neighbouring lanes; values are rounded to bf16 before the rotation,
                 // as the separate combine pass does
@@ -392,7 +462,7 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
                 const float p = __shfl_xor_sync(0xffffffffu, v, 1);
                 v = (d & 1) ? (-p * sn + v * cs) : (v * cs + p * sn);
               }
-              orow[static_cast<long long>(c + i) * kD + d] = __float2bfloat16(v);
+              orow[static_cast<long long>(h) * kD + d] = __float2bfloat16(v);
             }
           }
         }
@@ -401,99 +471,90 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
 #pragma unroll
-        for (int c = 0; c < NH; c += 16) {
+        for (int c = 0; c < kHeads; c += 16) {
           uint32_t r16[16];
-          tmem_ld_32x16(tmem_o + j * NH + c + lane_addr, r16);
+          tmem_ld_32x16(tmem_o + j * NH + h0 + c + lane_addr, r16);
           tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            if (c + i < a.nh) prow[(c + i) * (kD + 2) + j * 128 + row] = __uint_as_float(r16[i]);
-          }
+          for (int i = 0; i < 16; ++i)
+            if (h0 + c + i < a.nh) prow[(h0 + c + i) * (kD + 2) + j * 128 + row] = __uint_as_float(r16[i]);
         }
       }
-      named_bar_sync(2, kSoftmaxWarps * 32);
       if (own < a.nh) {
         prow[own * (kD + 2) + kD] = m_run[own] * 0.6931471805599453f;      // back to natural-log units
-        prow[own * (kD + 2) + kD + 1] = l_run[own];
+        prow[own * (kD + 2) + kD + 1] = l_own;
       }
     }
   } else {
     // ------------------------------- producers -------------------------------
-    const int pt = threadIdx.x - 32 * (1 + kSoftmaxWarps);     // 0..255
-    const int row = pt >> 1, half = pt & 1;
+    // Warp pw owns rows 8 pw .. 8 pw + 7 of every block; a lane holds 16 bytes of each 64-byte segment of one row's codes, and the
+    // row's scale bytes.
+    const int pw = warp - 4 - kSoftmaxWarps, l4 = lane & 3, row = 8 * pw + (lane >> 2);
+    uint8_t* const line = k_s + row * 128;
+    const uint32_t turn = (row & 7) << 4;
+    uint4 raw[7];
+    uint2 sc8;
+    const uint8_t* src_row;                                // row whose codes are in `raw`; nullptr: none
+    int slot_next = slot_of(r_begin + row);
+    auto next_row = [&](int b) {                           // slot_next -> row of block b; slot of block b + 1
+      const int slot = slot_next;
+      const bool swa = r_begin + b * kRows + row < n_swa;
+      src_row = nullptr;
+      sc8 = make_uint2(0, 0);
+      if (slot >= 0) {
+        const uint8_t* page = (swa ? a.swa_base : a.comp_base) + static_cast<long long>(slot >> 6) * (swa ? a.swa_stride : a.comp_stride);
+        src_row = page + (slot & 63) * kDataBytes + l4 * 16;
+        sc8 = *reinterpret_cast<const uint2*>(page + 64 * kDataBytes + (slot & 63) * 8);
+      }
+      slot_next = slot_of(r_begin + (b + 1) * kRows + row);
+    };
+    auto fetch = [&](int seg) {
+      raw[seg] = make_uint4(0, 0, 0, 0);
+      if (src_row != nullptr) raw[seg] = __ldg(reinterpret_cast<const uint4*>(src_row + seg * 64));
+    };
+    next_row(0);
+#pragma unroll
+    for (int i = 0; i < 7; ++i) fetch(panel_at(i));
+    begin();
     bool ok = true;
     for (int b = 0; b < n_blocks && ok; ++b) {
-      if (b > 0) {
-        if (!mbar_wait(&bars->pv_done, (b - 1) & 1, a.status, 620)) { ok = false; break; }
-      }
-      const int li = r_begin + b * kRows + row;
-      int slot = -1;
-      const uint8_t* cbase = a.swa_base;
-      long long cstride = a.swa_stride;
-      if (li < r_end) {
-        if (li < n_swa) slot = a.swa_slots[static_cast<long long>(t) * a.swa_ld + li];
-        else { slot = a.topk_slots[static_cast<long long>(t) * a.topk_ld + (li - n_swa)]; cbase = a.comp_base; cstride = a.comp_stride; }
-      }
-      const int sw7 = row & 7;
-      if (slot < 0) {
-        const uint4 z = make_uint4(0, 0, 0, 0);
+      const uint2 sc = sc8;
 #pragma unroll
-        for (int pp = 0; pp < 4; ++pp) {
-          uint8_t* dst = k_s + (half * 4 + pp) * kPanelBytes + row * 128;
-#pragma unroll
-          for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(dst + (c << 4)) = z;
+      for (int i = 0; i < kPanels; ++i) {
+        const int p = panel_at(i);
+        if (b > 0 && (i == 0 || i == 1 || i == 3 || i == 5)) {
+          ok = __all_sync(0xffffffffu, ok && mbar_wait(&bars->k_free[p >> 1], (b - 1) & 1, a.status, 620));
+          if (!ok) break;
         }
-      } else {
-        const uint8_t* pbase = cbase + static_cast<long long>(slot >> 6) * cstride;
-        const int rr = slot & 63;
-        const uint8_t* drow = pbase + static_cast<long long>(rr) * kDataBytes;
-        const uint8_t* srow = pbase + 64LL * kDataBytes + rr * 8;
-        const uint2 sc8 = *reinterpret_cast<const uint2*>(srow);
-        // two fp8 panels at a time: issue the eight 16-byte loads, then convert and store
-        auto fp8_panels2 = [&](int first_panel, int n_panels) {
-          uint4 w[8];
-#pragma unroll
-          for (int v = 0; v < 8; ++v)
-            if (v < n_panels * 4) w[v] = __ldg(reinterpret_cast<const uint4*>(drow + first_panel * 64) + v);
-#pragma unroll
-          for (int pp = 0; pp < 2; ++pp) {
-            if (pp < n_panels) {
-              const int panel = first_panel + pp;
-              const uint32_t sbyte = ((panel < 4 ? sc8.x : sc8.y) >> (8 * (panel & 3))) & 0xff;
-              const float sc = __uint_as_float(sbyte << 23);               // 2^(byte - 127)
-              uint8_t* dst = k_s + panel * kPanelBytes + row * 128;
-#pragma unroll
-              for (int v = 0; v < 4; ++v) {
-                const uint4 x = w[pp * 4 + v];
-                uint4 o0, o1;
-                fp8x4_to_bf16x4(x.x, sc, o0.x, o0.y);
-                fp8x4_to_bf16x4(x.y, sc, o0.z, o0.w);
-                fp8x4_to_bf16x4(x.z, sc, o1.x, o1.y);
-                fp8x4_to_bf16x4(x.w, sc, o1.z, o1.w);
-                *reinterpret_cast<uint4*>(dst + (((2 * v) ^ sw7) << 4)) = o0;
-                *reinterpret_cast<uint4*>(dst + (((2 * v + 1) ^ sw7) << 4)) = o1;
-              }
-            }
-          }
-        };
-        if (half == 0) {
-          fp8_panels2(0, 2);
-          fp8_panels2(2, 2);
+        if (i == 0) {
+          // the rotated part of this block, then where the next block's row lies
+          const uint8_t* src = src_row != nullptr ? src_row + kNope : a.swa_base;
+          copy16_async(line + 7 * kPanelBytes + ((l4 << 4) ^ turn), src, src_row != nullptr);
+          copy16_async(line + 7 * kPanelBytes + (((4 + l4) << 4) ^ turn), src_row != nullptr ? src + 64 : src, src_row != nullptr);
+          next_row(b + 1);
+        }
+        if (p < 7) {
+          const float f = __uint_as_float((((p < 4 ? sc.x : sc.y) >> (8 * (p & 3))) & 0xff) << 23);      // 2^(byte - 127)
+          const uint64_t f2 = pack2(f, f);
+          uint4 o0, o1;
+          e4m3x4_to_bf16(raw[p].x, f2, o0.x, o0.y);
+          e4m3x4_to_bf16(raw[p].y, f2, o0.z, o0.w);
+          e4m3x4_to_bf16(raw[p].z, f2, o1.x, o1.y);
+          e4m3x4_to_bf16(raw[p].w, f2, o1.z, o1.w);
+          *reinterpret_cast<uint4*>(line + p * kPanelBytes + ((l4 << 5) ^ turn)) = o0;
+          *reinterpret_cast<uint4*>(line + p * kPanelBytes + (((l4 << 5) + 16) ^ turn)) = o1;
+          fetch(p);
         } else {
-          uint4 rp[8];
-#pragma unroll
-          for (int c = 0; c < 8; ++c) rp[c] = __ldg(reinterpret_cast<const uint4*>(drow + kNope) + c);   // 64 bf16 rope dims
-          fp8_panels2(4, 2);
-          fp8_panels2(6, 1);
-          uint8_t* dst = k_s + 7 * kPanelBytes + row * 128;
-#pragma unroll
-          for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(dst + ((c ^ sw7) << 4)) = rp[c];
+          asm volatile("cp.async.wait_all;" ::: "memory");
+        }
+        if (i == 0 || i == 2 || i == 4 || i == 6 || i == 7) {
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->k_full[p < 6 ? p >> 1 : p - 3]);
         }
       }
-      fence_proxy_async();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->k_full);
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
   }
 
   tc_fence_before();
@@ -501,13 +562,13 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
   if (threadIdx.x == 0) STK_TRACE(6);
   if (warp == 0) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, kTmemCols);
+    tmem_dealloc(bars->tmem_base, Cfg::kTmemCols);
   }
 }
 
 template <int NH>
 static int launch_mla_tc(const MlaTcArgs& a, cudaStream_t st) {
-  const int smem = kPanels * kPanelBytes + kPanels * NH * 128 + 2 * NH * 128 + 64 + (4 * NH + NH + NH + 4 * NH + NH) * 4 + 64 + 1024;
+  const int smem = kPanels * kPanelBytes + kPanels * NH * 128 + 2 * NH * 128 + kBarBytes + 8 * NH * 4 + 1024;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(sparse_mla_tc_kernel<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
@@ -515,7 +576,7 @@ static int launch_mla_tc(const MlaTcArgs& a, cudaStream_t st) {
     configured = true;
   }
   dim3 grid(a.T, a.n_splits);
-  launch_pdl(sparse_mla_tc_kernel<NH>, dim3(grid), dim3(kThreads), smem, st, a);
+  launch_pdl(sparse_mla_tc_kernel<NH>, dim3(grid), dim3(MlaCfg<NH>::kThreads), smem, st, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 

@@ -413,6 +413,73 @@ def test_sparse_mla_direct_output_matches_split_path(nh):
     assert rel_err(out[sub], ref) < 1.2e-2
 
 
+@pytest.mark.parametrize("nh,T,K", [(64, 300, 512), (64, 9, 1100), (40, 300, 130), (16, 300, 300)])
+def test_sparse_mla_maxima_that_keep_growing(nh, T, K):
+    """Keys whose scores grow along the list by far more than the factor a stale maximum may be off by (the accumulators are
+    rescaled block after block), and lists that fall as steeply (they never are); ragged ends, gaps, whole blocks of gaps."""
+    torch.manual_seed(21)
+    D, R_, W = 512, 64, 128
+    n_pages = 24
+    n = n_pages * 64
+    rows = torch.randn(n, D) * (0.2 + 6.0 * torch.arange(n)[:, None] / n)
+    ccpu = C.PagedCache.allocate(n_pages, D, R_, True, "latent", "cpu")
+    ccpu.write_rows_cpu(torch.arange(n), rows)
+    cg = C.PagedCache(ccpu.buf.to(dev()), D, R_, True, "latent")
+    q = (4 * torch.randn(T, nh, D, device=dev())).to(BF16)
+    swa = torch.sort(torch.randint(0, n, (T, W), device=dev()), 1)[0].to(torch.int32)
+    top = torch.sort(torch.randint(0, n, (T, K), device=dev()), 1)[0].to(torch.int32)
+    top[::2], swa[::2] = top[::2].flip(1), swa[::2].flip(1)
+    top[torch.rand(T, K, device=dev()) < 0.1] = -1
+    swa[4], top[5, :K // 2] = -1, -1
+    swa_lens = torch.randint(0, W + 1, (T,), dtype=torch.int32, device=dev())
+    top_lens = torch.randint(0, K + 1, (T,), dtype=torch.int32, device=dev())
+    swa_lens[:4], top_lens[:4] = W, torch.tensor([K, K, 0, 1], dtype=torch.int32)
+    sink = torch.randn(nh, device=dev())
+    out = A.sparse_mla(q, cg, swa, swa_lens, cg, top, top_lens, sink, D ** -0.5)
+    sub = torch.arange(min(T, 9))
+    ref = A.sparse_mla(q[:9].cpu(), ccpu, swa[:9].cpu(), swa_lens[:9].cpu(), ccpu, top[:9].cpu(), top_lens[:9].cpu(), sink.cpu(), D ** -0.5)
+    # weights and results are rounded to bf16 (2^-9 each); scores of a few hundred carry fp32 rounding into the weights
+    for i in sub.tolist():
+        assert rel_err(out[i], ref[i]) < 1.2e-2 or float(ref[i].abs().max()) < 1e-6
+
+
+@pytest.mark.parametrize("nh", [64, 16])
+def test_sparse_mla_codes_and_scales(nh):
+    """Every e4m3 code under ordinary and extreme scale bytes (0 counts as scale zero), rotated parts as they are; NaN codes reach
+    the tokens that attend to them and no others."""
+    torch.manual_seed(22)
+    D, R_, T, W = 512, 64, 300, 128
+    n_pages = 4
+    buf = torch.zeros(n_pages, C.PagedCache.page_bytes(D, R_, True, "latent"), dtype=torch.uint8)
+    codes = torch.randint(0, 256, (n_pages, 64, 448), dtype=torch.uint8)
+    codes[(codes & 0x7f) == 0x7f] = 0x7e
+    rope = torch.randn(n_pages, 64, R_).to(BF16).view(torch.uint8)
+    scales = torch.zeros(n_pages, 64, 8, dtype=torch.uint8)
+    scales[:, :, :7] = torch.tensor([0, 1, 60, 110, 119, 120, 121, 127, 133, 134, 135, 137], dtype=torch.uint8)[
+        torch.randint(0, 12, (n_pages, 64, 7))]
+    codes[1, 7, 100] = 0xff
+    buf[:, :64 * 576] = torch.cat([codes, rope], 2).view(n_pages, -1)
+    buf[:, 64 * 576:64 * 584] = scales.view(n_pages, -1)
+    cg = C.PagedCache(buf.to(dev()), D, R_, True, "latent")
+    value = torch.cat([(codes.view(torch.float8_e4m3fn).double().view(n_pages, 64, 7, 64)
+                        * torch.where(scales[:, :, :7] == 0, 0.0, torch.exp2(scales[:, :, :7].double() - 127))[..., None]).view(n_pages * 64, 448),
+                       rope.view(BF16).double().view(n_pages * 64, R_)], 1)
+    q = (2.0 ** -19 * torch.randn(T, nh, D, device=dev())).to(BF16)
+    slots = torch.randint(0, n_pages * 64, (T, W), dtype=torch.int32, device=dev())
+    slots[slots == 71] = 70
+    slots[3, 5] = 71
+    lens = torch.full((T,), W, dtype=torch.int32, device=dev())
+    sink = torch.zeros(nh, device=dev())
+    out = A.sparse_mla(q, cg, slots, lens, None, None, None, sink, D ** -0.5)
+    assert bool(out[3].isnan().all()) and int(out.isnan().any(2).any(1).sum()) == 1
+    kv = value.to(dev())[slots.long()]
+    p = torch.softmax(torch.cat([q.double() @ kv.transpose(1, 2) * D ** -0.5, torch.zeros(T, nh, 1, device=dev(), dtype=torch.float64)], 2), 2)
+    ref = p[:, :, :-1] @ kv
+    keep = torch.arange(T, device=dev()) != 3
+    for part in (slice(0, 448), slice(448, 512)):           # weights and results are rounded to bf16
+        assert rel_err(out[keep][:, :, part], ref[keep][:, :, part]) < 8e-3
+
+
 @pytest.mark.parametrize("scoring", ["sigmoid", "sqrtsoftplus"])
 def test_router(scoring):
     T, E, k = 33, 256, 6
