@@ -775,6 +775,37 @@ def test_moe_grouped_gemm_nvfp4(T, E, k):
     assert rel_err(out, out2) < 1.5e-2
 
 
+@pytest.mark.parametrize("H,I,E,counts", [
+    (256, 128, 16, (0, 1, 15, 16, 17, 0, 31, 33)), (384, 256, 12, (127, 128, 129, 0, 300, 1)), (1024, 384, 9, (0, 0, 257, 2, 64, 65)),
+    (128, 128, 2100, (3, 0, 40, 1))])
+def test_moe_grouped_gemm_uneven_experts(H, I, E, counts):
+    """Tiles of one row to several full ones, experts without rows between and behind them, feature counts that are no multiple of
+    two weight tiles, K of a few blocks, more experts than one launch lists."""
+    torch.manual_seed(14)
+    chosen = torch.cat([torch.full((n,), (i * (E - 1)) // (len(counts) - 1), dtype=torch.int32) for i, n in enumerate(counts)])
+    T = chosen.numel()
+    ids = chosen[torch.randperm(T)][:, None].to(dev())
+    w = torch.rand(T, 1, device=dev()) + 0.5
+    scale = lambda *shape: (0.05 + torch.rand(*shape, device=dev())).to(torch.float8_e4m3fn).view(torch.uint8)
+    code = lambda *shape: torch.randint(0, 256, shape, dtype=torch.uint8, device=dev())
+    ew = M.ExpertWeights(code(E, 2 * I, H // 2), code(E, H, I // 2), scale(E, 2 * I, H // 16), scale(E, H, I // 16),
+                         0.02 + 0.02 * torch.rand(E, device=dev()), 0.02 + 0.02 * torch.rand(E, device=dev()))
+    x = torch.randn(T, H, device=dev()).to(BF16)
+    old, M.DIRECT_MAX_PAIRS = M.DIRECT_MAX_PAIRS, 0
+    try:
+        out = M.moe_experts(x, ids, w, ew, 10.0, None, E)
+    finally:
+        M.DIRECT_MAX_PAIRS = old
+    f8 = torch.float8_e4m3fn
+    ref = torch.zeros(T, H, device=dev(), dtype=torch.float64)
+    for e in ids.unique().tolist():
+        rows = (ids[:, 0] == e).nonzero()[:, 0]
+        h = x[rows].double() @ R.dequant_nvfp4(ew.w13[e], ew.s13[e].view(f8), ew.g13[e]).double().t()
+        g, u = h[:, :I].clamp(max=10.0), h[:, I:].clamp(-10.0, 10.0)
+        ref[rows] = (g * torch.sigmoid(g) * u) @ R.dequant_nvfp4(ew.w2[e], ew.s2[e].view(f8), ew.g2[e]).double().t() * w[rows].double()
+    assert rel_err(out, ref) < 5e-3                     # activations rounded to fp16 in between, expert outputs and sums to bf16
+
+
 def test_topk_candidates_and_markov_chain_match_cpu():
     """The drafter's sampling path: two-level candidate selection over the full vocabulary and the one-launch
     sequential Markov sampling against their CPU statements."""
