@@ -21,6 +21,7 @@
 #include <stdlib.h>
 
 #include "common.cuh"
+#include "pairs.cuh"
 #include "stk_c_api.h"
 #include "symm.cuh"
 
@@ -56,11 +57,6 @@ struct GemmArgs {
   // carries the current epoch.  Token tiles are visited starting with this rank's own shard.
   int gate_enabled;
   int gate_rows;
-  // Token-major mode (fp8, T >= 128): the operands swap roles -- TMEM lanes are tokens, columns are weight rows -- so
-  // the activation scale of a K block is one value per thread and the weight scale one value per tile: the per-block
-  // rescale is a single multiplier per thread instead of one per accumulator column.  T/N/tiles_* then describe the
-  // swapped problem (a.N = tokens, a.T = weight rows); out is still [tokens, ldo].
-  int token_major;
   // Whether the split-K reduction may write `out` with 16-byte (fp32) / 4-byte (bf16) vector stores: the host sets
   // it from the alignment of `out` and `ldo`; otherwise the reduction writes element by element.
   int out_vec_ok;
@@ -153,7 +149,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUt
   // Launched with programmatic serialization (plain GEMMs only): barriers, TMEM and descriptors are set up and the
   // first weight tiles of this CTA are on their way to L2 while the previous kernel finishes; activations, split-K
   // counters and epochs are touched only after the wait.
-  if (warp == 0 && lane == 0 && !a.token_major && static_cast<int>(blockIdx.x) < a.splits * a.tiles_t * a.tiles_n) {
+  if (warp == 0 && lane == 0 && static_cast<int>(blockIdx.x) < a.splits * a.tiles_t * a.tiles_n) {
     const int u = blockIdx.x;
     const int tn = u % a.tiles_n;
     const int sp = u / (a.tiles_n * a.tiles_t);
@@ -379,51 +375,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUt
         float acc[kColsPerWarp];
 #pragma unroll
         for (int j = 0; j < kColsPerWarp; ++j) acc[j] = 0.f;
-        if (a.token_major) {
-          // lane = token n, columns = weight rows t0 .. t0 + kColsPerWarp of row block tt (BT == 128)
-          for (int kb = kb0; kb < kb1 && ok; ++kb) {
-            const float s = a.w_scale[tt * a.w_scale_ld + kb] *
-                            (n_ok ? a.x_scale[static_cast<long long>(kb) * a.x_scale_ld + n] : 0.f);
-            if (!mbar_wait(&bars->tmem_full[ab], aphase, a.status, 400 + ab)) { ok = false; break; }
-            tc_fence_after();
-#pragma unroll
-            for (int c = 0; c < kChunksPerWarp; ++c) {
-              uint32_t r[32];
-              tmem_ld_chunk<CW>(tmem_base + ab * BT + col_base + c * CW + (static_cast<uint32_t>(q * 32) << 16), r);
-              tmem_ld_wait();
-#pragma unroll
-              for (int j = 0; j < CW; ++j) acc[c * CW + j] = fmaf(__uint_as_float(r[j]), s, acc[c * CW + j]);
-            }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bars->tmem_empty[ab]);
-            if (++ab == 2) { ab = 0; aphase ^= 1; }
-          }
-          if (ok && n_ok) {
-            // a thread owns kColsPerWarp consecutive outputs of its token row
-            const long long o0 = static_cast<long long>(n) * a.ldo + t0;
-            const bool vec = !a.out_fp32 && (a.ldo % 8 == 0) && ((reinterpret_cast<uintptr_t>(a.out) & 15) == 0) &&
-                             t0 + kColsPerWarp <= a.T;
-            if (vec) {
-#pragma unroll
-              for (int j = 0; j < kColsPerWarp; j += 8) {
-                uint4 ov;
-                __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&ov);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) oh[i] = __floats2bfloat162_rn(acc[j + 2 * i], acc[j + 2 * i + 1]);
-                *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.out) + o0 + j) = ov;
-              }
-            } else {
-#pragma unroll
-              for (int j = 0; j < kColsPerWarp; ++j) {
-                if (t0 + j < a.T) {
-                  if (a.out_fp32) reinterpret_cast<float*>(a.out)[o0 + j] = acc[j];
-                  else reinterpret_cast<__nv_bfloat16*>(a.out)[o0 + j] = __float2bfloat16(acc[j]);
-                }
-              }
-            }
-          }
-        } else {
         for (int kb = kb0; kb < kb1 && ok; ++kb) {
           const float sw = a.w_scale[tn * a.w_scale_ld + kb];
           const int gkb = a.group_tiles ? (tn / a.group_tiles) * a.k_blocks : 0;
@@ -454,7 +405,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUt
         if (ok) {
 #pragma unroll
           for (int j = 0; j < kColsPerWarp; ++j) store(t0 + j, acc[j]);
-        }
         }
       } else {
         if (!mbar_wait(&bars->tmem_full[ab], aphase, a.status, 400 + ab)) { ok = false; break; }
@@ -582,6 +532,16 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUt
   }
 }
 
+// ---- clusters that split K ---------------------------------------------------------
+__device__ __forceinline__ uint32_t peer_addr(uint32_t smem_addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // ---------------------------------------------------------------------------------
 // Wide tile for large bf16 problems: one CTA owns 256 tokens x 256 weight rows (token-major: TMEM lanes are tokens,
 // so an epilogue thread writes 64 contiguous bytes of its token's output row per chunk).
@@ -599,11 +559,17 @@ struct WideArgs {
   long long ldo;
   int out_fp32;
   int* status;
+  // block-diagonal weights: tn / group_tiles is the block, its X columns start at that times group_k (0: one block)
+  int group_tiles, group_k;
 };
 
 constexpr int kWideStages = 3;
 constexpr int kWideStageBytes = 2 * 128 * 128 + 256 * 128;       // two weight tiles + one token tile = 64 KB
 
+// S > 1: a cluster of S CTAs shares a tile, each with its part of K.  CTA j writes piece j of the tile (S = 2: 128 tokens; S = 4: 128
+// tokens x 128 weight rows); the others bring it their partial sums through distributed shared memory, into the operand ring that
+// is free by then.  Sums are formed in the order of the CTAs' ranks.
+template <int S>
 __global__ void __launch_bounds__(320, 1)
 gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const WideArgs a) {
   extern __shared__ uint8_t smem_raw[];
@@ -635,21 +601,26 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   pdl_trigger();
   const int units = a.tiles_n * a.tiles_t;
   constexpr uint32_t kIdesc = umma_idesc(1u, 1u, 128, 256);
+  const int rank = S > 1 ? static_cast<int>(blockIdx.x) % S : 0;
+  const int per = (a.k_blocks + S - 1) / S, k_begin = rank * per, k_end = min(a.k_blocks, k_begin + per);
+  const int u_first = blockIdx.x / S, u_step = gridDim.x / S;
 
   if (warp == 0) {
     if (lane == 0) {
       int stage = 0, issued = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+      for (int u = u_first; u < units && ok; u += u_step) {
         const int tn = u % a.tiles_n, tt = u / a.tiles_n;
-        for (int kb = 0; kb < a.k_blocks; ++kb) {
+        const int gx = a.group_tiles ? tn / a.group_tiles * a.group_k : 0;
+        for (int kb = k_begin; kb < k_end; ++kb) {
           if (!mbar_wait(&bars->empty[stage], phase ^ 1, a.status, 100 + stage)) { ok = false; break; }
           mbar_expect_tx(&bars->full[stage], kWideStageBytes);
           uint8_t* st = smem + stage * kWideStageBytes;
           // token-major: the two A operands are 128-token tiles (TMEM lanes = tokens), B is the 256-row weight tile
-          tma_load_2d(st, &tmX, &bars->full[stage], kb * 64, tt * 256);
-          tma_load_2d(st + 128 * 128, &tmX, &bars->full[stage], kb * 64, tt * 256 + 128);
+          const int kx = kb * 64 + gx;
+          tma_load_2d(st, &tmX, &bars->full[stage], kx, tt * 256);
+          tma_load_2d(st + 128 * 128, &tmX, &bars->full[stage], kx, tt * 256 + 128);
           tma_load_2d(st + 2 * 128 * 128, &tmW, &bars->full[stage], kb * 64, tn * 256);
           ++issued;
           if (++stage == kWideStages) { stage = 0; phase ^= 1; }
@@ -666,87 +637,143 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         }
       }
     }
+    __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0, aphase = 0;
-      bool ok = true;
-      for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
-        if (!mbar_wait(&bars->tmem_empty[0], aphase ^ 1, a.status, 200)) { ok = false; break; }
+    const uint32_t lead = elect_one() ? 1u : 0u, tm = __shfl_sync(0xffffffffu, tmem_base, 0), s_lo = desc_lo(smem_u32(smem));
+    int stage = 0;
+    uint32_t phase = 0, aphase = 0;
+    bool ok = true;
+    for (int u = u_first; u < units && ok; u += u_step) {
+      ok = mbar_wait(&bars->tmem_empty[0], aphase ^ 1, a.status, 200);
+      if (!ok) break;
+      tc_fence_after();
+      for (int kb = k_begin; kb < k_end; ++kb) {
+        ok = mbar_wait(&bars->full[stage], phase, a.status, 300 + stage);
+        if (!ok) break;
         tc_fence_after();
-        for (int kb = 0; kb < a.k_blocks; ++kb) {
-          if (!mbar_wait(&bars->full[stage], phase, a.status, 300 + stage)) { ok = false; break; }
-          tc_fence_after();
-          const uint8_t* st = smem + stage * kWideStageBytes;
-          const uint64_t a0 = umma_desc_sw128(smem_u32(st));
-          const uint64_t a1 = umma_desc_sw128(smem_u32(st + 128 * 128));
-          const uint64_t bd = umma_desc_sw128(smem_u32(st + 2 * 128 * 128));
+        const uint32_t st = s_lo + stage * (kWideStageBytes >> 4);
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const uint32_t acc = (kb > 0 || k > 0) ? 1u : 0u;
-            umma_f16(tmem_base, a0 + 2 * k, bd + 2 * k, kIdesc, acc);
-            umma_f16(tmem_base + 256, a1 + 2 * k, bd + 2 * k, kIdesc, acc);
-          }
-          umma_commit(&bars->empty[stage]);
-          if (++stage == kWideStages) { stage = 0; phase ^= 1; }
+        for (int k = 0; k < 4; ++k) {
+          const uint32_t acc = (kb > k_begin || k > 0) ? 1u : 0u;
+          mma_ss(tm, st + 2 * k, st + 2048 + 2 * k, kIdesc, acc, lead);
+          mma_ss(tm + 256, st + 1024 + 2 * k, st + 2048 + 2 * k, kIdesc, acc, lead);
         }
-        if (ok) umma_commit(&bars->tmem_full[0]);
-        aphase ^= 1;
+        mma_commit(&bars->empty[stage], lead);
+        if (++stage == kWideStages) { stage = 0; phase ^= 1; }
       }
+      if (ok) mma_commit(&bars->tmem_full[0], lead);
+      aphase ^= 1;
     }
+    __syncwarp();
   } else {
     // eight epilogue warps: lane quarter q = warp % 4 (the TMEM lanes a warp may read), column half h
     const int e = warp - 2;
     const int q = warp & 3, h = e >> 2;
+    const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
     uint32_t aphase = 0;
     bool ok = true;
-    for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+    for (int u = u_first; u < units && ok; u += u_step) {
       const int tn = u % a.tiles_n, tt = u / a.tiles_n;
-      if (!mbar_wait(&bars->tmem_full[0], aphase, a.status, 400)) { ok = false; break; }
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars->tmem_full[0], aphase, a.status, 400));
+      if (!ok && S == 1) break;
       tc_fence_after();
       // a thread owns one token row and, per chunk, 32 consecutive output features: 64 contiguous bytes of bf16
       const bool vec_ok = !a.out_fp32 && (a.ldo % 8 == 0) && ((reinterpret_cast<uintptr_t>(a.out) & 15) == 0);
       const bool vec32_ok = (a.ldo % 4 == 0) && ((reinterpret_cast<uintptr_t>(a.out) & 15) == 0);
-#pragma unroll
-      for (int m = 0; m < 2; ++m) {
+      auto store32 = [&](int m, int col, const uint32_t (&r)[32]) {
         const int t = tt * 256 + m * 128 + q * 32 + lane;
         const bool t_ok = t < a.T;
+        const int n0 = tn * 256 + col;
+        if (t_ok) {
+          if (vec_ok && n0 + 32 <= a.N) {
+            __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(a.out) + static_cast<long long>(t) * a.ldo + n0;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t r[32];
-          const int col = h * 128 + c * 32;
-          tmem_ld_32x32(tmem_base + m * 256 + col + (static_cast<uint32_t>(q * 32) << 16), r);
-          tmem_ld_wait();
-          const int n0 = tn * 256 + col;
-          if (t_ok) {
-            if (vec_ok && n0 + 32 <= a.N) {
-              __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(a.out) + static_cast<long long>(t) * a.ldo + n0;
+            for (int j = 0; j < 32; j += 8) {
+              uint4 ov;
+              __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&ov);
 #pragma unroll
-              for (int j = 0; j < 32; j += 8) {
-                uint4 ov;
-                __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&ov);
+              for (int i = 0; i < 4; ++i)
+                oh[i] = __floats2bfloat162_rn(__uint_as_float(r[j + 2 * i]), __uint_as_float(r[j + 2 * i + 1]));
+              *reinterpret_cast<uint4*>(o + j) = ov;
+            }
+          } else if (a.out_fp32) {
+            float* o = reinterpret_cast<float*>(a.out) + static_cast<long long>(t) * a.ldo + n0;
+            if (vec32_ok && n0 + 32 <= a.N) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-                  oh[i] = __floats2bfloat162_rn(__uint_as_float(r[j + 2 * i]), __uint_as_float(r[j + 2 * i + 1]));
-                *reinterpret_cast<uint4*>(o + j) = ov;
-              }
-            } else if (a.out_fp32) {
-              float* o = reinterpret_cast<float*>(a.out) + static_cast<long long>(t) * a.ldo + n0;
-              if (vec32_ok && n0 + 32 <= a.N) {
-#pragma unroll
-                for (int j = 0; j < 32; j += 4) *reinterpret_cast<uint4*>(o + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
-              } else {
-#pragma unroll
-                for (int j = 0; j < 32; ++j)
-                  if (n0 + j < a.N) o[j] = __uint_as_float(r[j]);
-              }
+              for (int j = 0; j < 32; j += 4) *reinterpret_cast<uint4*>(o + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
             } else {
-              __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(a.out) + static_cast<long long>(t) * a.ldo + n0;
 #pragma unroll
               for (int j = 0; j < 32; ++j)
-                if (n0 + j < a.N) o[j] = __float2bfloat16(__uint_as_float(r[j]));
+                if (n0 + j < a.N) o[j] = __uint_as_float(r[j]);
+            }
+          } else {
+            __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(a.out) + static_cast<long long>(t) * a.ldo + n0;
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (n0 + j < a.N) o[j] = __float2bfloat16(__uint_as_float(r[j]));
+          }
+        }
+      };
+      if constexpr (S == 1) {
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            uint32_t r[32];
+            tmem_ld_32x32(tmem_base + m * 256 + h * 128 + c * 32 + lane_addr, r);
+            tmem_ld_wait();
+            store32(m, h * 128 + c * 32, r);
+          }
+        }
+      } else {
+        // piece j: token tile m_of(j), columns from c_of(j); this warp's share of a piece is kShare columns of its lane quarter
+        constexpr int kCols = 512 / S, kShare = kCols / 2;
+        auto m_of = [](int j) { return S == 2 ? j : j >> 1; };
+        auto c_of = [](int j) { return S == 2 ? 0 : (j & 1) * 128; };
+        const uint32_t line = smem_u32(smem) + (q * 32 + lane) * 16;      // [slot][column / 4][token] of 16 bytes
+        cluster_sync_all();                                               // every CTA's products are done: the rings are free
+#pragma unroll 1
+        for (int d = 1; d < S; ++d) {
+          const int j = (rank + d) % S;
+          const uint32_t to = peer_addr(line + (rank < j ? rank : rank - 1) * (kCols * 512), j);
+#pragma unroll 1
+          for (int c = 0; c < kShare; c += 32) {
+            uint32_t r[32];
+            tmem_ld_32x32(tmem_base + m_of(j) * 256 + c_of(j) + h * kShare + c + lane_addr, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 32; i += 4)
+              asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};"
+                           ::"r"(to + (h * kShare + c + i) / 4 * 2048), "r"(r[i]), "r"(r[i + 1]), "r"(r[i + 2]), "r"(r[i + 3]) : "memory");
+          }
+        }
+        cluster_sync_all();                                               // all pieces have arrived
+#pragma unroll 1
+        for (int c = 0; c < kShare; c += 32) {
+          uint32_t r[32];
+          float v[32];
+          tmem_ld_32x32(tmem_base + m_of(rank) * 256 + c_of(rank) + h * kShare + c + lane_addr, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = 0.f;
+#pragma unroll
+          for (int j = 0; j < S; ++j) {
+            if (j == rank) {
+#pragma unroll
+              for (int i = 0; i < 32; ++i) v[i] += __uint_as_float(r[i]);
+            } else {
+              const uint32_t from = line + (j < rank ? j : j - 1) * (kCols * 512) + (h * kShare + c) / 4 * 2048;
+#pragma unroll
+              for (int i = 0; i < 32; i += 4) {
+                float x0, x1, x2, x3;
+                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x0), "=f"(x1), "=f"(x2), "=f"(x3) : "r"(from + i / 4 * 2048));
+                v[i] += x0; v[i + 1] += x1; v[i + 2] += x2; v[i + 3] += x3;
+              }
             }
           }
+#pragma unroll
+          for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(v[i]);
+          store32(m_of(rank), c_of(rank) + h * kShare + c, r);
         }
       }
       tc_fence_before();
@@ -754,6 +781,300 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       if (lane == 0) mbar_arrive(&bars->tmem_empty[0]);
       aphase ^= 1;
     }
+  }
+  if (S > 1 && warp < 2) {
+    // the CTAs of a cluster meet twice (one tile each)
+    cluster_sync_all();
+    cluster_sync_all();
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+// ---------------------------------------------------------------------------------
+// fp8 with at least a full tile of tokens, token-major: TMEM lanes are tokens, columns are weight rows, so the scale of a K block
+// is one multiplier per thread.  One CTA owns 128 tokens x 128 weight rows.
+//
+// What bounds it: a K block is 259 tensor-core cycles, and its 128 x 128 results have to be read back from TMEM, scaled and added
+// to the second-level accumulators (fp32, in registers).  The scales of a block are asked for four blocks ahead (loaded when their
+// block's products were done, they held every block up for a trip to memory), four accumulators are in flight, and a buffer is given
+// back as soon as it has been read.  Operands are 32 KB a block; at 4096 tokens they leave L2 at 13 TB/s, near what it gives.
+// Measured (4096 tokens, 4096 x 8192): 241 us with scales loaded on demand, 172 us now.  Sixteen epilogue warps instead of eight
+// took 238 us, 256 tokens a CTA 193 us.
+// ---------------------------------------------------------------------------------
+struct Fp8Args {
+  int T, N, k_blocks, tiles_t, tiles_n;
+  void* out;
+  long long ldo;
+  int out_fp32;
+  const float* w_scale;
+  int w_scale_ld;
+  const float* x_scale;
+  int x_scale_ld;
+  int* status;
+};
+
+constexpr int kFp8StageBytes = 2 * 128 * 128, kFp8Stages = 6;
+constexpr int kFp8Bufs = 4;                                    // accumulators in TMEM, 128 columns each
+constexpr int kFp8EpiWarps = 8, kFp8Threads = 32 * (2 + kFp8EpiWarps);
+
+struct alignas(8) Fp8Bars {
+  uint64_t full[6], empty[6], tmem_full[4], tmem_empty[4];
+  uint32_t tmem_base;
+};
+
+// D[tmem] (+)= A[smem] * B[smem], e4m3 operands, issued by a converged warp (see common.cuh)
+__device__ __forceinline__ void mma_ss_f8(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t acc, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+      "mov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %4, p;\n\t}"
+      ::"r"(d), "r"(a_lo), "r"(b_lo), "r"(kDescHi), "r"(idesc), "r"(acc), "r"(lead)
+      : "memory");
+}
+
+// S > 1: a cluster of S CTAs shares a tile, each with its part of K; CTA j writes kCols / S columns of every epilogue thread, to
+// which the others' sums come through distributed shared memory (into the operand ring, free by then), added in rank order.
+template <int S>
+__global__ void __launch_bounds__(kFp8Threads, 1)
+gemm_fp8_tokens_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const Fp8Args a) {
+  constexpr int kStages = kFp8Stages, kBufs = kFp8Bufs, kCols = 64;       // columns of an epilogue warp
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  Fp8Bars* bars = reinterpret_cast<Fp8Bars*>(smem + kStages * kFp8StageBytes);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kStages; ++i) {
+      mbar_init(&bars->full[i], 1);
+      mbar_init(&bars->empty[i], 1);
+    }
+    for (int i = 0; i < kBufs; ++i) {
+      mbar_init(&bars->tmem_full[i], 1);
+      mbar_init(&bars->tmem_empty[i], kFp8EpiWarps);
+    }
+    fence_barrier_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(&bars->tmem_base, 512);
+    tmem_relinquish();
+  }
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmX);
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = bars->tmem_base;
+  pdl_wait();
+  pdl_trigger();
+  const int units = a.tiles_t * a.tiles_n;
+  const int rank = S > 1 ? static_cast<int>(blockIdx.x) % S : 0;
+  const int per = (a.k_blocks + S - 1) / S, k_begin = min(a.k_blocks, rank * per), k_end = min(a.k_blocks, k_begin + per);
+  const int u_first = blockIdx.x / S, u_step = gridDim.x / S;
+
+  if (warp == 0) {
+    // ------------------------------ TMA producer ------------------------------
+    if (lane == 0) {
+      int stage = 0, issued = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int u = u_first; u < units && ok; u += u_step) {
+        const int tt = u % a.tiles_t, tn = u / a.tiles_t;
+        for (int kb = k_begin; kb < k_end; ++kb) {
+          if (!mbar_wait(&bars->empty[stage], phase ^ 1, a.status, 100 + stage)) { ok = false; break; }
+          mbar_expect_tx(&bars->full[stage], kFp8StageBytes);
+          uint8_t* st = smem + stage * kFp8StageBytes;
+          tma_load_2d(st, &tmX, &bars->full[stage], kb * 128, tt * 128);
+          tma_load_2d(st + 128 * 128, &tmW, &bars->full[stage], kb * 128, tn * 128);
+          ++issued;
+          if (++stage == kStages) { stage = 0; phase ^= 1; }
+        }
+      }
+      if (!ok) {
+        // drain: wait (bounded) until every load issued to the ring has landed
+        const int pending = issued < kStages ? issued : kStages;
+        int s = stage;
+        uint32_t ph = phase;
+        for (int i = 0; i < pending; ++i) {
+          if (--s < 0) { s = kStages - 1; ph ^= 1; }
+          mbar_wait(&bars->full[s], ph, nullptr, 0);
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ------------------------------ MMA issuer --------------------------------
+    const uint32_t lead = elect_one() ? 1u : 0u, tm = __shfl_sync(0xffffffffu, tmem_base, 0), s_lo = desc_lo(smem_u32(smem));
+    constexpr uint32_t kIdesc = umma_idesc(0u, 0u, 128, 128);
+    const long long total = units > u_first ? ((units - 1 - u_first) / u_step + 1LL) * (k_end - k_begin) : 0;
+    int stage = 0, ab = 0;
+    uint32_t phase = 0, aphase = 0;
+    for (long long i = 0; i < total; ++i) {
+      if (!mbar_wait(&bars->tmem_empty[ab], aphase ^ 1, a.status, 200 + ab) || !mbar_wait(&bars->full[stage], phase, a.status, 300 + stage)) break;
+      tc_fence_after();
+      const uint32_t st = s_lo + stage * (kFp8StageBytes >> 4), d = tm + ab * 128;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) mma_ss_f8(d, st + 2 * k, st + 1024 + 2 * k, kIdesc, k > 0 ? 1u : 0u, lead);
+      mma_commit(&bars->empty[stage], lead);
+      mma_commit(&bars->tmem_full[ab], lead);
+      if (++stage == kStages) { stage = 0; phase ^= 1; }
+      if (++ab == kBufs) { ab = 0; aphase ^= 1; }
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------ epilogue -----------------------------------
+    // a thread owns one token and kCols weight rows
+    const int e = warp - 2, q = warp & 3, col0 = (e >> 2) * kCols;
+    const uint32_t tile = tmem_base + col0 + (static_cast<uint32_t>(q * 32) << 16);
+    int ab = 0;
+    uint32_t aphase = 0;
+    bool ok = true;
+    for (int u = u_first; u < units && ok; u += u_step) {
+      const int tt = u % a.tiles_t, tn = u / a.tiles_t;
+      const int t = tt * 128 + q * 32 + lane;
+      const bool t_ok = t < a.T;
+      const bool live = tt * 128 + q * 32 < a.T;         // some lane of this warp has a token
+      const float* xs = a.x_scale + (t_ok ? t : 0);
+      const float* ws = a.w_scale + static_cast<long long>(tn) * a.w_scale_ld;
+      constexpr int kAhead = 4;
+      float sx[kAhead], sw[kAhead];
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) {
+        const int kb = min(k_begin + i, a.k_blocks - 1);
+        sx[i] = __ldg(xs + static_cast<long long>(kb) * a.x_scale_ld);
+        sw[i] = __ldg(ws + kb);
+      }
+      uint64_t acc[kCols / 2];
+#pragma unroll
+      for (int j = 0; j < kCols / 2; ++j) acc[j] = 0ull;
+      for (int kb0 = k_begin; kb0 < k_end && ok; kb0 += kAhead) {
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) {
+          const int kb = kb0 + i;
+          if (kb >= k_end || !ok) break;
+          const float s = sx[i] * sw[i];
+          const uint64_t s2 = pack2(s, s);
+          const int next = min(kb + kAhead, a.k_blocks - 1);
+          sx[i] = __ldg(xs + static_cast<long long>(next) * a.x_scale_ld);
+          sw[i] = __ldg(ws + next);
+          ok = __all_sync(0xffffffffu, mbar_wait(&bars->tmem_full[ab], aphase, a.status, 400 + ab));
+          if (!ok) break;
+          tc_fence_after();
+          uint32_t r[2][32];
+          if (live) {
+            tmem_ld_32x32(tile + ab * 128, r[0]);
+            tmem_ld_32x32(tile + ab * 128 + 32, r[1]);
+            tmem_ld_wait();
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->tmem_empty[ab]);
+          if (live) {
+#pragma unroll
+            for (int j = 0; j < kCols; j += 2)
+              acc[j / 2] = fma2(pack2(__uint_as_float(r[j / 32][j % 32]), __uint_as_float(r[j / 32][j % 32 + 1])), s2, acc[j / 2]);
+          }
+          if (++ab == kBufs) { ab = 0; aphase ^= 1; }
+        }
+      }
+      const bool aligned = (reinterpret_cast<uintptr_t>(a.out) & 15) == 0 && a.ldo % (a.out_fp32 ? 4 : 8) == 0;
+      auto store8 = [&](int c, const float (&v)[8]) {               // columns c .. c + 7 of this thread
+        const int n = tn * 128 + col0 + c;
+        const long long o0 = static_cast<long long>(t) * a.ldo + n;
+        if (!t_ok) return;
+        if (aligned && n + 8 <= a.N) {
+          if (a.out_fp32) {
+            float* o = reinterpret_cast<float*>(a.out) + o0;
+            *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
+            *reinterpret_cast<float4*>(o + 4) = make_float4(v[4], v[5], v[6], v[7]);
+          } else {
+            uint4 ov;
+            __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&ov);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) oh[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+            *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.out) + o0) = ov;
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            if (n + i < a.N) {
+              if (a.out_fp32) reinterpret_cast<float*>(a.out)[o0 + i] = v[i];
+              else reinterpret_cast<__nv_bfloat16*>(a.out)[o0 + i] = __float2bfloat16(v[i]);
+            }
+          }
+        }
+      };
+      auto take8 = [&](int c, float (&v)[8]) {
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) unpack2(acc[(c + i) / 2], v[i], v[i + 1]);
+      };
+      if constexpr (S == 1) {
+        if (ok) {
+#pragma unroll
+          for (int c = 0; c < kCols; c += 8) {
+            float v[8];
+            take8(c, v);
+            store8(c, v);
+          }
+        }
+      } else {
+        constexpr int kShare = kCols / S;
+        static_assert(kShare % 8 == 0, "columns of a CTA");
+        const uint32_t line = smem_u32(smem) + e * 512 + lane * 16;                     // [sender][column / 4][thread] of 16 bytes
+        cluster_sync_all();                                                             // every CTA is done with its ring
+#pragma unroll
+        for (int j = 0; j < S; ++j) {
+          if (j != rank && live) {
+            const uint32_t to = peer_addr(line + (rank < j ? rank : rank - 1) * (kShare / 4 * 4096), j);
+#pragma unroll
+            for (int c = 0; c < kShare; c += 8) {
+              float v[8];
+              take8(j * kShare + c, v);
+#pragma unroll
+              for (int i = 0; i < 8; i += 4)
+                asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};"
+                             ::"r"(to + (c + i) / 4 * 4096), "f"(v[i]), "f"(v[i + 1]), "f"(v[i + 2]), "f"(v[i + 3]) : "memory");
+            }
+          }
+        }
+        cluster_sync_all();                                                             // all sums have arrived
+#pragma unroll
+        for (int own = 0; own < S; ++own) {
+          if (own == rank && live && ok) {
+#pragma unroll
+            for (int c = 0; c < kShare; c += 8) {
+              float v[8], mine[8];
+              take8(own * kShare + c, mine);
+#pragma unroll
+              for (int i = 0; i < 8; ++i) v[i] = 0.f;
+#pragma unroll
+              for (int j = 0; j < S; ++j) {
+#pragma unroll
+                for (int i = 0; i < 8; i += 4) {
+                  float4 x = make_float4(mine[i], mine[i + 1], mine[i + 2], mine[i + 3]);
+                  if (j != own)
+                    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w)
+                                 : "r"(line + (j < own ? j : j - 1) * (kShare / 4 * 4096) + (c + i) / 4 * 4096));
+                  v[i] += x.x; v[i + 1] += x.y; v[i + 2] += x.z; v[i + 3] += x.w;
+                }
+              }
+              store8(own * kShare + c, v);
+            }
+          }
+        }
+      }
+    }
+  }
+  if (S > 1 && warp < 2) {
+    // the CTAs of a cluster meet twice (one tile each)
+    cluster_sync_all();
+    cluster_sync_all();
   }
   tc_fence_before();
   __syncthreads();
@@ -814,6 +1135,25 @@ int make_tmap_pages(CUtensorMap* tm, const void* base, long long pages, int rows
   return r == CUDA_SUCCESS ? 0 : -2;
 }
 
+// Clusters of `cluster` CTAs, with the programmatic-serialization attribute where `launch_pdl` would use it
+template <typename... KArgs, typename... Args>
+static int launch_cluster(void (*kernel)(KArgs...), int cluster, int grid, int threads, int smem, cudaStream_t st, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = cluster;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = pdl_use(st, STK_PDL_CLASS) ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...) == cudaSuccess ? 0 : -4;
+}
+
 template <int BT, bool kFp8>
 static int launch_gemm(const CUtensorMap& tw, const CUtensorMap& tx, const GemmArgs& a, int grid, cudaStream_t st) {
   using Cfg = GemmCfg<BT>;
@@ -831,6 +1171,18 @@ static int launch_gemm(const CUtensorMap& tw, const CUtensorMap& tx, const GemmA
     launch_pdl(gemm_kernel<BT, kFp8>, dim3(grid), dim3(kFp8 ? 320 : 192), smem, st, tw, tx, a);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
+}
+
+template <int S>
+static int launch_fp8_tokens(const CUtensorMap& tx, const CUtensorMap& tw, const Fp8Args& a, int sm_count, cudaStream_t st) {
+  constexpr int smem = kFp8Stages * kFp8StageBytes + static_cast<int>(sizeof(Fp8Bars)) + 1024;
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(gemm_fp8_tokens_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -3;
+    configured = true;
+  }
+  const int units = a.tiles_t * a.tiles_n;
+  return launch_cluster(gemm_fp8_tokens_kernel<S>, S, S > 1 ? units * S : units < sm_count ? units : sm_count, kFp8Threads, smem, st, tx, tw, a);
 }
 
 }  // namespace stk
@@ -860,6 +1212,36 @@ STK_API long long stk_gemm_workspace_bytes(int T, int N, int splits) {
   return splits > 1 ? static_cast<long long>(splits) * T * N * 4 : 0;
 }
 
+// CTAs that share a 256 x 256 tile of the wide kernel (as many as keep the SMs to one round, with at least four K blocks each), or 0
+// where the kernel above is better: up to 96 tokens.  Measured, us, kernel above / this one with its split:
+//   64 tokens x 4096 x 8192: 24.5 / 28.7;  128: 51.8 / 29.5;  256: 48.4 / 29.8;  777: 124 / 52;  128 x 40960 x 1536: 94 / 46;
+//   4096 tokens x 64 x 4096: 28 / 19;  777 x 4096 x 4096: 66 / 31.5 (45.3 without the split);  1500 x 4096 x 4096: 113 / 49.6.
+static int wide_split_of(int T, int N, int K, int sm_count) {
+  if (T <= 96) return 0;
+  const int units = ((T + 255) / 256) * ((N + 255) / 256), kb = (K * 2 + 127) / 128;
+  int s = 4;
+  while (s > 1 && (units * s > sm_count || kb < 4 * s)) s /= 2;
+  return s;
+}
+
+template <int S>
+static int launch_wide_s(const CUtensorMap& tx, const CUtensorMap& tw, const WideArgs& a, int grid, cudaStream_t st) {
+  constexpr int smem = kWideStages * kWideStageBytes + 256 + 1024;
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(gemm_wide_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -3;
+    configured = true;
+  }
+  return launch_cluster(gemm_wide_kernel<S>, S, grid, 320, smem, st, tw, tx, a);
+}
+
+static int launch_wide(const CUtensorMap& tx, const CUtensorMap& tw, const WideArgs& a, int split, int sm_count, cudaStream_t st) {
+  const int units = a.tiles_n * a.tiles_t;
+  if (split == 4) return launch_wide_s<4>(tx, tw, a, units * 4, st);
+  if (split == 2) return launch_wide_s<2>(tx, tw, a, units * 2, st);
+  return launch_wide_s<1>(tx, tw, a, units < sm_count ? units : sm_count, st);
+}
+
 // STK_GEMM_WIDE=0 keeps large bf16 problems on the 128 x 256 tile (A/B runs)
 static bool gemm_wide_enabled() {
   static int v = -1;
@@ -868,6 +1250,18 @@ static bool gemm_wide_enabled() {
     v = (e != nullptr && e[0] == '0') ? 0 : 1;
   }
   return v == 1;
+}
+
+// CTAs that share a tile of the fp8 token-major kernel (as many as keep the SMs to one round, with at least four K blocks each), or 0
+// where the kernel above is better: few tokens under a weight whose tiles fill the SMs.  Measured, us, kernel above / this one:
+//   64 tokens x 4096 x 8192: 18.9 / 11.5;  x 2048 x 4096: 14.2 / 7.7;  x 40960 x 1536: 32.7 / 20.2;  x 129280 x 4096: 143 / 101;
+//   12 tokens x 4096 x 8192: 13.9 / 11.8;  x 129280 x 4096: 106 / 137.
+static int fp8_tokens_split(int T, int N, int K, int sm_count) {
+  if (T <= 8) return 0;
+  const int units = ((N + 127) / 128) * ((T + 127) / 128), kb = (K + 127) / 128;
+  int s = 4;
+  while (s > 1 && (units * s > sm_count || kb < 4 * s)) s /= 2;
+  return s > 1 || T >= 48 ? s : 0;
 }
 
 static int gemm_launch(const void* W, long long ldw, const void* X, long long ldx, void* out, long long ldo, int T, int N,
@@ -881,50 +1275,43 @@ static int gemm_launch(const void* W, long long ldw, const void* X, long long ld
   if (is_fp8 && (w_scale == nullptr || x_scale == nullptr || (x_scale_ld & 3))) return -11;
   if (splits > 1 && (workspace == nullptr || counters == nullptr)) return -12;
   if (groups < 1) groups = 1;
-  // fp8 with at least a full tile of tokens: token-major orientation (see GemmArgs::token_major)
-  const bool token_major = is_fp8 && T >= 128 && groups == 1 && ar_ctx == nullptr && gate_ctx == nullptr && splits <= 1 &&
-                           (reinterpret_cast<uintptr_t>(X) & 15) == 0;
-  if (token_major) {
+  const int tokens_split = is_fp8 && groups == 1 && ar_ctx == nullptr && gate_ctx == nullptr ? fp8_tokens_split(T, N, K, sm_count) : 0;
+  if (tokens_split > 0) {
     CUtensorMap ta, tb;
     if (make_tmap_2d(&ta, X, 1, T, K, ldx, 128) != 0) return -13;        // lanes: tokens
     if (make_tmap_2d(&tb, W, 1, N, K, ldw, 128) != 0) return -14;        // columns: weight rows
-    GemmArgs a;
+    Fp8Args a;
     memset(&a, 0, sizeof(a));
-    a.T = N; a.N = T;
+    a.T = T; a.N = N;
     a.k_blocks = (K + 127) / 128;
-    a.splits = 1;
-    a.tiles_n = (T + 127) / 128;
-    a.tiles_t = (N + 127) / 128;
+    a.tiles_n = (N + 127) / 128;
     a.out = out; a.ldo = ldo; a.out_fp32 = out_fp32;
     a.w_scale = w_scale; a.w_scale_ld = w_scale_ld;
     a.x_scale = x_scale; a.x_scale_ld = x_scale_ld;
     a.status = status;
-    a.token_major = 1;
-    const int units = a.tiles_n * a.tiles_t;
-    const int grid = units < sm_count ? units : sm_count;
-    return launch_gemm<128, true>(ta, tb, a, grid, reinterpret_cast<cudaStream_t>(stream));
+    a.tiles_t = (T + 127) / 128;
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    switch (tokens_split) {
+      case 4: return launch_fp8_tokens<4>(ta, tb, a, sm_count, st);
+      case 2: return launch_fp8_tokens<2>(ta, tb, a, sm_count, st);
+      default: return launch_fp8_tokens<1>(ta, tb, a, sm_count, st);
+    }
   }
-  if (!is_fp8 && groups == 1 && ar_ctx == nullptr && gate_ctx == nullptr && splits <= 1 && bt_override == 0 && T >= 512 &&
-      N >= 512 && gemm_wide_enabled()) {
+  // block-diagonal weights take the wide tiles where blocks are whole tiles and whole 128-byte steps of K
+  const int wide_split = (groups == 1 || (N % (256 * groups) == 0 && K % 64 == 0)) ? wide_split_of(T, N, K, sm_count) : 0;
+  if (!is_fp8 && ar_ctx == nullptr && gate_ctx == nullptr && splits <= 1 && bt_override == 0 && wide_split > 0 && gemm_wide_enabled()) {
     CUtensorMap tw2, tx2;
-    if (make_tmap_2d(&tw2, W, 2, N, K, ldw, 256) != 0) return -13;       // B operand: 256 weight rows
-    if (make_tmap_2d(&tx2, X, 2, T, K, ldx, 128) != 0) return -14;       // A operands: 128 tokens each
+    if (make_tmap_2d(&tw2, W, 2, N, K, ldw, 256) != 0) return -13;                                               // B operand: 256 weight rows
+    if (make_tmap_2d(&tx2, X, 2, T, static_cast<long long>(K) * groups, ldx, 128) != 0) return -14;              // A operands: 128 tokens each
     WideArgs wa;
     wa.T = T; wa.N = N;
     wa.k_blocks = (K * 2 + 127) / 128;
     wa.tiles_n = (N + 255) / 256;
     wa.tiles_t = (T + 255) / 256;
     wa.out = out; wa.ldo = ldo; wa.out_fp32 = out_fp32; wa.status = status;
-    const int wunits = wa.tiles_n * wa.tiles_t;
-    const int wgrid = wunits < sm_count ? wunits : sm_count;
-    const int wsmem = kWideStages * kWideStageBytes + 256 + 1024;
-    static bool wide_configured = false;
-    if (!wide_configured) {
-      if (cudaFuncSetAttribute(gemm_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, wsmem) != cudaSuccess) return -3;
-      wide_configured = true;
-    }
-    launch_pdl(gemm_wide_kernel, dim3(wgrid), dim3(320), wsmem, reinterpret_cast<cudaStream_t>(stream), tw2, tx2, wa);
-    return cudaGetLastError() == cudaSuccess ? 0 : -4;
+    wa.group_tiles = groups > 1 ? N / groups / 256 : 0;
+    wa.group_k = K;
+    return launch_wide(tx2, tw2, wa, wide_split, sm_count, reinterpret_cast<cudaStream_t>(stream));
   }
   int bt = stk_gemm_pick_bt(T, is_fp8);
   if (!is_fp8 && T > 128 && groups == 1) {
@@ -970,7 +1357,6 @@ static int gemm_launch(const void* W, long long ldw, const void* X, long long ld
   }
   a.gate_enabled = 0;
   a.gate_rows = 0;
-  a.token_major = 0;
   if (gate_ctx != nullptr) {
     if (ar_ctx != nullptr || gate_rows <= 0 || a.splits != 1) return -19;
     memcpy(&a.ar, gate_ctx, sizeof(a.ar));
