@@ -775,6 +775,68 @@ def test_moe_grouped_gemm_nvfp4(T, E, k):
     assert rel_err(out, out2) < 1.5e-2
 
 
+@pytest.mark.parametrize("T", [9, 47, 48, 100, 127, 128, 129, 300, 700])
+@pytest.mark.parametrize("N,K", [(72, 192), (200, 512), (512, 2048), (2048, 4096), (20000, 1664)])
+def test_gemm_fp8_token_tiles(T, N, K):
+    """Ragged tiles of tokens and weight rows, a K that ends inside a block, K split over two and four CTAs of a cluster (with an
+    uneven last part), several tiles per CTA, fp32 results and rows of a wider matrix."""
+    torch.manual_seed(T + N)
+    lw = Fn.LinearWeight.from_master(torch.randn(N, K, device=dev()) * 0.05, "fp8", dev())
+    x = torch.randn(T, K, device=dev()).to(BF16)
+    xq, xs = R.quant_fp8_group128_act(x)
+    ref = R.dequant_fp8_group128_act(xq, xs).double() @ lw.dequant().double().t()
+    out = Fn.linear(x, lw)
+    assert rel_err(out, ref) < 3e-3                       # bf16 results; the activation's codes may differ at ties
+    wide = torch.full((T, N + 24), 7.0, dtype=F32, device=dev())
+    Fn.linear(x, lw, out=wide[:, 8:8 + N])
+    assert rel_err(wide[:, 8:8 + N], ref) < 2.5e-3
+    assert bool((wide[:, :8] == 7.0).all()) and bool((wide[:, 8 + N:] == 7.0).all())
+
+
+@pytest.mark.parametrize("T", [97, 128, 129, 255, 257, 520])
+@pytest.mark.parametrize("N,K", [(16, 4096), (272, 1088), (1000, 64), (1030, 2048), (5000, 576)])
+def test_gemm_bf16_wide_tiles_that_share_k(T, N, K):
+    """256 x 256 tiles alone and split over two and four CTAs of a cluster: ragged edges, K of one block and of uneven parts."""
+    torch.manual_seed(T + N)
+    w = (torch.randn(N, K, device=dev()) * 0.05).to(BF16)
+    x = torch.randn(T, K, device=dev()).to(BF16)
+    ref = x.double() @ w.double().t()
+    assert rel_err(Fn.linear(x, Fn.LinearWeight(w)), ref) < 2.5e-3
+    wide = torch.full((T, N + 5), 7.0, dtype=F32, device=dev())
+    Fn.linear(x, Fn.LinearWeight(w), out=wide[:, :N])
+    assert rel_err(wide[:, :N], ref) < 2e-5               # fp32 sums
+    assert bool((wide[:, N:] == 7.0).all())
+
+
+@pytest.mark.parametrize("T", [130, 600])
+@pytest.mark.parametrize("groups,n,K", [(2, 256, 128), (3, 512, 1024), (8, 128, 256)])
+def test_gemm_bf16_wide_block_diagonal(T, groups, n, K):
+    """Blocks of whole wide tiles (the last: blocks too narrow for them)."""
+    torch.manual_seed(T)
+    w = (torch.randn(groups * n, K, device=dev()) * 0.05).to(BF16)
+    x = torch.randn(T, groups * K, device=dev()).to(BF16)
+    ref = torch.cat([x[:, g * K:(g + 1) * K].double() @ w[g * n:(g + 1) * n].double().t() for g in range(groups)], 1)
+    assert rel_err(Fn.linear(x, Fn.LinearWeight(w), groups=groups), ref) < 2.5e-3
+
+
+@pytest.mark.parametrize("T,K", [(1, 128), (7, 640), (9, 512), (130, 2176)])
+def test_quant_act_codes_and_scales(T, K):
+    """Rows and groups that do not fill a thread block; a row of zeros, values at the ends of the range; equal to the plain
+    statement up to ties of the scaled value."""
+    torch.manual_seed(T)
+    x = (torch.randn(T, K, device=dev()) * torch.exp(4 * torch.randn(T, 1, device=dev()))).to(BF16)
+    x[T // 2] = 0
+    x[0, :3] = torch.tensor([3e38, -3e38, 1e-30])
+    big = torch.zeros(T, K + 64, dtype=BF16, device=dev())
+    big[:, 8:8 + K] = x
+    for src in (x, big[:, 8:8 + K], big[:, 4:4 + K]):        # the last: rows that 16-byte loads cannot take
+        qa = Fn.quant_act(src)
+        wq, ws = R.quant_fp8_group128_act(src)
+        assert torch.equal(qa.scale[:, :T].t(), ws) or rel_err(qa.scale[:, :T].t(), ws) < 1e-6
+        same = (qa.q.view(torch.uint8) == wq.view(torch.uint8)).float().mean()
+        assert float(same) > 0.999
+
+
 @pytest.mark.parametrize("H,I,E,counts", [
     (256, 128, 16, (0, 1, 15, 16, 17, 0, 31, 33)), (384, 256, 12, (127, 128, 129, 0, 300, 1)), (1024, 384, 9, (0, 0, 257, 2, 64, 65)),
     (128, 128, 2100, (3, 0, 40, 1))])
