@@ -309,6 +309,7 @@ class Engine:
         self._next_id = 0
         self.requests: Dict[int, Request] = {}
         self._graphs: Dict[tuple, object] = {}
+        self._feeds: Dict[int, int] = {}     # steps of one given token per sequence so far, by batch size
         # a captured step cannot hold the stage-to-stage sends and receives: pipeline stages run eagerly; so do steps
         # under decode context parallelism (their staging buffers are allocated as block sizes first appear)
         self.use_graphs = self.device.type == "cuda" and sc.graph_cap > 0 and pipe is None and dcp == 1
@@ -406,11 +407,16 @@ class Engine:
         t, n_req, _ = self._stage(seqs)
         self._upload(t, n_req, 0)
         max_comp_rows = max(1, max(s.start + s.n for s in seqs) // 4)
-        meta = self._build_meta(t, n_req, max_comp_rows, pure_decode=all(s.n == 1 for s in seqs))
-        X = self.model.forward_hidden(meta)
+        one_each = t == n_req
+        graph = self._feed_graph(n_req, max_comp_rows) if one_each and len(rows) == t else None
         logits = None
-        if rows:
-            logits = self.model.compute_logits(self.model.head_hidden(X, torch.tensor(rows, device=self.device))).float()
+        if graph is not None:
+            logits = graph.replay()[:t].to(torch.float32, copy=True)       # the graph's own buffer is the next step's too
+        else:
+            meta = self._build_meta(t, n_req, max_comp_rows, pure_decode=one_each)
+            X = self.model.forward_hidden(meta)
+            if rows:
+                logits = self.model.compute_logits(self.model.head_hidden(X, torch.tensor(rows, device=self.device))).float()
         self._queue_status_read()
         if self.device.type == "cuda":
             torch.cuda.current_stream().synchronize()
@@ -939,20 +945,39 @@ class Engine:
         return out
 
     # ---- CUDA graphs -----------------------------------------------------------------
-    def _decode_graph(self, n_req: int, max_comp_rows: int) -> "DecodeGraph":
+    # Steps of given tokens (one per sequence) run eagerly this often at a batch size before they are captured: a short replay
+    # never pays for a capture (a few hundred launches), a long one is no longer paced by them.
+    FEED_EAGER_STEPS = 16
+
+    def _decode_graph(self, n_req: int, max_comp_rows: int, logits: bool = False) -> "DecodeGraph":
         bucket = 1
         while bucket < n_req:
             bucket *= 2
         rows_bucket = self.model.decode_bucket(max_comp_rows)
-        key = (bucket, rows_bucket)
+        key = ("feed", bucket, rows_bucket) if logits else (bucket, rows_bucket)
         if n_req < bucket:
             # padding rows: empty query ranges => request -1, nothing is read or written for them
             self.buf.d_qstart[n_req + 1:bucket + 1].fill_(n_req)
         g = self._graphs.get(key)
         if g is None:
-            g = DecodeGraph(self, bucket, rows_bucket)
+            g = DecodeGraph(self, bucket, rows_bucket, logits)
             self._graphs[key] = g
         return g
+
+    def _feed_graph(self, n_req: int, max_comp_rows: int) -> Optional["DecodeGraph"]:
+        """The captured step that gives every sequence's logits for one given token each, once such steps are frequent."""
+        if not self.use_graphs or n_req > self.cfg.sched.graph_cap or n_req > self.cfg.sched.max_num_seqs:
+            return None
+        seen = self._feeds.get(n_req, 0)
+        if seen < self.FEED_EAGER_STEPS:
+            self._feeds[n_req] = seen + 1
+            return None
+        return self._decode_graph(n_req, max_comp_rows, logits=True)
+
+    def _run_logits(self, n: int, max_comp_rows: int) -> torch.Tensor:
+        """One token of each of n requests -> their logits [n, vocab] in the head's type."""
+        X = self.model.forward_hidden(self._build_meta(n, n, max_comp_rows, pure_decode=True))
+        return self.model.compute_logits(self.model.head_hidden(X))
 
 
 _CAPTURE_STREAMS: Dict[int, "torch.cuda.Stream"] = {}
@@ -1018,11 +1043,16 @@ class SpecGraph:
 
 
 class DecodeGraph:
-    """A captured pure-decode step for `bucket` rows (token i belongs to request i)."""
+    """A captured pure-decode step for `bucket` rows (token i belongs to request i): sampled tokens, or logits."""
 
-    def __init__(self, eng: Engine, bucket: int, rows_bucket: int):
+    def __init__(self, eng: Engine, bucket: int, rows_bucket: int, logits: bool = False):
         self.eng = eng
         self.bucket = bucket
+
+        def body():
+            if logits:
+                return eng._run_logits(bucket, rows_bucket)
+            return eng._run_model(bucket, bucket, bucket, rows_bucket, identity_rows=True)
         # warm-up outside capture (allocates scratch, configures kernels), then capture.  A recurrent state must not advance
         # here: such a model warms up on empty query ranges (every row is padding) and gets its ranges back for the replay.
         qstart = eng.buf.d_qstart[:bucket + 1]
@@ -1033,14 +1063,14 @@ class DecodeGraph:
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):
             for _ in range(2):
-                self.out = eng._run_model(bucket, bucket, bucket, rows_bucket, identity_rows=True)
+                self.out = body()
         torch.cuda.current_stream().wait_stream(side)
         torch.cuda.synchronize()
         from ..ops import _lib
         before = _lib.launch_count
         self.graph = torch.cuda.CUDAGraph()
         with _capturing(self.graph, eng.device):
-            self.out = eng._run_model(bucket, bucket, bucket, rows_bucket, identity_rows=True)
+            self.out = body()
         self.launches_per_replay = _lib.launch_count - before
         if ranges is not None:
             qstart.copy_(ranges)

@@ -189,3 +189,44 @@ def test_dspark_text_does_not_depend_on_what_the_drafter_proposes():
     replay, m1 = run(lambda: ReplayDrafter(recorded, cfg.vocab_size, acceptance=(1.0, 1.0, 1.0)))
     assert m1.spec_num_accepted_tokens > m0.spec_num_accepted_tokens + 10      # the second run really accepted drafts
     assert replay == never
+
+
+@pytest.mark.parametrize("family", ["flash", "hybrid"])
+def test_feed_steps_that_are_captured_match_eager_ones(family):
+    """Steps of one given token per sequence, captured after a while, against an engine that never captures: three sequences (a
+    padded batch), a sequence that joins later, a longer span in between; states must advance exactly once per step."""
+    from stkernel_b200.config import hybrid_stack
+    from stkernel_b200.models.hybrid import build_hybrid_weights
+    if family == "flash":
+        cfg = flash_config(num_layers=2, n_routed_experts=16, vocab_size=4096, num_hash_layers=2, dense_dtype="bf16")
+        weights = build_model_weights(cfg, RandomSource(5), "cuda:0")
+    else:
+        cfg = hybrid_stack(4, 512, heads=4, kv_heads=1, dim=128, window=160, ff=768, vocab=4096, mlstm_heads=2, mlstm_dim=64, mlstm_vdim=128)
+        weights = build_hybrid_weights(cfg, RandomSource(5), "cuda:0")
+    g = torch.Generator().manual_seed(3)
+    tokens = torch.randint(0, cfg.vocab_size, (4, 200), generator=g).tolist()
+    outs = []
+    for cap in (0, 8):
+        ec = EngineConfig(model=cfg, sched=SchedulerConfig(max_model_len=512, max_num_seqs=4, max_num_batched_tokens=512, graph_cap=cap)).validate()
+        eng = Engine(ec, weights, "cuda:0", max_context=512)
+        seqs = [eng.open_sequence() for _ in range(3)]
+        got = [eng.feed([(s, tokens[i][:70 + i], [69 + i]) for i, s in enumerate(seqs)])]
+        pos = [70, 71, 72]
+        for step in range(2 * Engine.FEED_EAGER_STEPS + 6):
+            if step == Engine.FEED_EAGER_STEPS + 4:
+                seqs.append(eng.open_sequence())
+                pos.append(0)
+                got.append(eng.feed([(seqs[3], tokens[3][:40], [39])]))
+                pos[3] = 40
+            got.append(eng.feed([(s, [tokens[i][pos[i]]], [0]) for i, s in enumerate(seqs)]))
+            pos = [p + 1 for p in pos]
+        assert (len(eng._graphs) > 0) == (cap > 0)
+        outs.append([x.clone() for x in got])
+        for s in seqs:
+            eng.close_sequence(s)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    for a, b in zip(*outs):
+        assert a.shape == b.shape and a.dtype == b.dtype == torch.float32
+        # the padded batch changes the order of sums; their bf16 roundings go through the whole model
+        assert float((a - b).norm() / a.norm()) < 2e-2
