@@ -202,6 +202,11 @@ class HostStage:
         self.event = None           # recorded after the uploads that read this set
 
 
+def step_bucket(n_req: int) -> int:
+    """Rows of the captured step that serves `n_req` requests."""
+    return 1 << max(0, n_req - 1).bit_length()
+
+
 class StepBuffers:
     """Two pinned host staging sets (the host may prepare step k+1 while the copies of step k are
     still queued) + fixed-address device tensors for the step description."""
@@ -276,8 +281,9 @@ class Engine:
                 self.kv.swa.on_pressure = pc.evict_one
                 self.kv.c4.on_pressure = pc.evict_one
         self.sched = Scheduler(cfg, self.kv, self.prefix_cache)
-        self.buf = StepBuffers(sc.max_num_batched_tokens + sc.max_num_seqs * (1 + n_spec), sc.max_num_seqs, self.device,
-                               sc.max_num_seqs * (1 + n_spec))
+        # a captured step reads its batch rounded up to a power of two: padded rows have query ranges of their own in these buffers
+        padded = step_bucket(sc.max_num_seqs)
+        self.buf = StepBuffers(sc.max_num_batched_tokens + padded * (1 + n_spec), padded, self.device, padded * (1 + n_spec))
         self.drafter = None
         if spec_on:
             pin = self.device.type == "cuda"
@@ -950,9 +956,7 @@ class Engine:
     FEED_EAGER_STEPS = 16
 
     def _decode_graph(self, n_req: int, max_comp_rows: int, logits: bool = False) -> "DecodeGraph":
-        bucket = 1
-        while bucket < n_req:
-            bucket *= 2
+        bucket = step_bucket(n_req)
         rows_bucket = self.model.decode_bucket(max_comp_rows)
         key = ("feed", bucket, rows_bucket) if logits else (bucket, rows_bucket)
         if n_req < bucket:

@@ -220,3 +220,16 @@ def test_log_probabilities_match_the_oracle_and_do_not_change_the_text():
         eng.step()
     rc = eng.requests[c]
     assert len(rc.logprobs) == 4 and all(top == [] and lp <= 0 for lp, top in rc.logprobs)
+
+
+@pytest.mark.parametrize("seqs", [1, 3, 5, 8, 33])
+def test_step_buffers_hold_the_padded_batch(seqs):
+    """A captured step of n requests reads the query ranges, rows and sampling inputs of the next power of two."""
+    from stkernel_b200.runtime.engine import step_bucket
+    cfg = tiny_config()
+    eng = make_engine(cfg, init_random_weights(cfg, seed=1), seqs=seqs)
+    bucket = step_bucket(seqs)
+    assert bucket >= seqs and bucket & (bucket - 1) == 0 and bucket < 2 * seqs
+    b = eng.buf
+    assert b.d_qstart.numel() >= bucket + 1
+    assert min(x.numel() for x in (b.d_tokens, b.d_rows, b.d_start, b.d_temp, b.d_seed, b.d_pos, b.d_topk, b.d_topp)) >= bucket
