@@ -1,6 +1,7 @@
 """Indexer scoring / top-k, per-step index metadata and sparse MLA attention."""
 from __future__ import annotations
 
+from functools import lru_cache
 from typing import Optional, Tuple
 
 import torch
@@ -228,6 +229,27 @@ USE_DECODE_MLA = True          # register-resident kernel for decode-sized steps
 MLA_DECODE_MAX_T = 8
 
 
+MLA_DIRECT_MIN_T = 37          # up to 36 tokens the combine pass spreads the final rows better (64 heads, 128 rows: 16.8 us against 19.2 at
+                               # 16 tokens, 18.7 / 19.4 at 32, 19.6 / 19.3 at 40, 29.9 / 19.9 at 148)
+
+
+@lru_cache(maxsize=4096)
+def _mla_splits(t: int, max_rows: int, sms: int) -> int:
+    """Row splits of the tensor-core kernel.  A CTA (one per SM) works through its 128-row blocks in turn and costs most of one more
+    to begin and end; every split leaves fp32 partial rows that the combine pass reads again, about 0.012 of a block's time each.
+    So: the count with the least rounds x (blocks + 0.8), partials included.  Measured against two CTAs per SM (64 heads, 2176 rows):
+    9 tokens 65 -> 29 us, 32: 52 -> 42, 64: 77 -> 60, 128: 111 -> 90.  Beyond one CTA per SM no split: 150 tokens gain a tenth by
+    one, but lose a fifth where the lists are short of their capacity (56 -> 67 us at 384 of 2176 rows)."""
+    if t > sms:
+        return 1
+    best, least = 1, None
+    for s in range(1, -(-max_rows // 128) + 1):
+        cost = -(-t * s // sms) * (-(-(-(-max_rows // s)) // 128) + 0.8) + (0.012 * t * s if s > 1 else 0.0)
+        if least is None or cost < least - 1e-9:
+            best, least = s, cost
+    return best
+
+
 def sparse_mla(q: torch.Tensor, swa_cache: PagedCache, swa_slots: torch.Tensor, swa_lens: torch.Tensor,
                comp_cache: Optional[PagedCache], topk_slots: Optional[torch.Tensor], topk_lens: Optional[torch.Tensor],
                sink: torch.Tensor, scale: float, inv_rope: Optional[Tuple[torch.Tensor, torch.Tensor]] = None,
@@ -294,10 +316,8 @@ def sparse_mla(q: torch.Tensor, swa_cache: PagedCache, swa_slots: torch.Tensor, 
     max_rows = swa_slots.shape[1] + (topk_slots.shape[1] if topk_slots is not None else 0)
     cc = comp_cache if comp_cache is not None else swa_cache
     if USE_TENSOR_CORE_MLA and swa_cache.fp8 and d == 512 and swa_cache.rope_dim == 64 and nh <= 64 and q.stride(0) % 8 == 0:
-        # tcgen05 kernel: one 64-row key block per CTA while the SMs are not full (a block is a serial chain of
-        # gather -> QK^T -> softmax -> PV, so at decode sizes more, shorter CTAs finish sooner)
-        n_splits = max(1, min((max_rows + 63) // 64, (2 * _lib.sm_count()) // max(t, 1)))
-        if n_splits == 1 and MLA_DIRECT_OUT:
+        n_splits = _mla_splits(t, max_rows, _lib.sm_count())
+        if n_splits == 1 and MLA_DIRECT_OUT and t >= MLA_DIRECT_MIN_T:
             # enough tokens to fill the GPU: the kernel writes the final rows itself (no fp32 partials, no combine pass)
             out = torch.empty(t, nh, d, dtype=BF16, device=q.device)
             _lib.call("stk_sparse_mla_tc_out", q, q.stride(0), swa_cache.buf, swa_cache.page_stride, cc.buf, cc.page_stride,

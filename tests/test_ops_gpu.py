@@ -376,6 +376,34 @@ def test_sparse_mla_matches_reference(nh, D, R_, fp8):
     assert rel_err(out2, ref2) < 1e-2
 
 
+@pytest.mark.parametrize("tokens", [9, 36, 37, 64, 148, 149])
+@pytest.mark.parametrize("K", [0, 640])
+def test_sparse_mla_splits_rows_over_idle_sms(tokens, K):
+    """Both sides of each line of the split rule, with lists that fill their capacity, end in any split, or are empty.
+    Tolerance of the tests around it: fp8 rows against the fp32 reference of the same rows."""
+    torch.manual_seed(tokens)
+    D, R_, W, nh, n_pages = 512, 64, 128, 16, 24
+    ccpu = C.PagedCache.allocate(n_pages, D, R_, True, "latent", "cpu")
+    ccpu.write_rows_cpu(torch.arange(n_pages * 64), torch.randn(n_pages * 64, D))
+    cg = C.PagedCache(ccpu.buf.to(dev()), D, R_, True, "latent")
+    q = torch.randn(tokens, nh, D).to(BF16)
+    swa_slots = torch.randint(0, n_pages * 64, (tokens, W), dtype=torch.int32)
+    swa_lens = torch.randint(0, W + 1, (tokens,), dtype=torch.int32)
+    top = torch.randint(0, n_pages * 64, (tokens, max(K, 1)), dtype=torch.int32) if K else None
+    top_lens = torch.randint(0, K + 1, (tokens,), dtype=torch.int32) if K else None
+    swa_lens[0], swa_lens[1] = W, 0
+    if K:
+        top_lens[0], top_lens[1], top_lens[2] = K, 0, 1
+    sink = torch.randn(nh)
+    out = A.sparse_mla(q.to(dev()), cg, swa_slots.to(dev()), swa_lens.to(dev()), cg if K else None, top.to(dev()) if K else None,
+                       top_lens.to(dev()) if K else None, sink.to(dev()), D ** -0.5)
+    sub = torch.tensor(sorted({0, 1, 2, tokens // 2, tokens - 1}))
+    ref = A.sparse_mla(q[sub], ccpu, swa_slots[sub], swa_lens[sub], ccpu if K else None, top[sub] if K else None,
+                       top_lens[sub] if K else None, sink, D ** -0.5)
+    assert rel_err(out[sub.to(dev())], ref) < 1.2e-2
+    assert float(out[1].float().abs().max()) == 0.0
+
+
 @pytest.mark.parametrize("nh", [64, 8])
 def test_sparse_mla_direct_output_matches_split_path(nh):
     """Steps with many tokens take the single-split kernel that writes the final rows itself (sink merge, normalisation,
