@@ -414,7 +414,8 @@ class Engine:
         self._upload(t, n_req, 0)
         max_comp_rows = max(1, max(s.start + s.n for s in seqs) // 4)
         one_each = t == n_req
-        graph = self._feed_graph(n_req, max_comp_rows) if one_each and len(rows) == t else None
+        # a captured step gives every row once, in order: other wishes (a place twice, none of a sequence) are gathered eagerly
+        graph = self._feed_graph(n_req, max_comp_rows) if one_each and rows == list(range(t)) else None
         logits = None
         if graph is not None:
             logits = graph.replay()[:t].to(torch.float32, copy=True)       # the graph's own buffer is the next step's too

@@ -233,3 +233,35 @@ def test_step_buffers_hold_the_padded_batch(seqs):
     b = eng.buf
     assert b.d_qstart.numel() >= bucket + 1
     assert min(x.numel() for x in (b.d_tokens, b.d_rows, b.d_start, b.d_temp, b.d_seed, b.d_pos, b.d_topk, b.d_topp)) >= bucket
+
+
+class PlainStep:
+    """Stands for a captured step without a GPU: `replay` runs the step's body over the padded batch."""
+
+    def __init__(self, eng, bucket, rows_bucket, logits=False):
+        self.body = lambda: eng._run_logits(bucket, rows_bucket)
+
+    def replay(self):
+        return self.body()
+
+
+@pytest.mark.parametrize("wanted", [([0, 0], []), ([], [0, 0]), ([0], [0]), ([0, 0], [0]), ([], [0])])
+def test_captured_feed_steps_give_the_wanted_rows(wanted, monkeypatch):
+    """Places that are repeated or absent: the logits are those of an engine that never captures, in the order asked for."""
+    from stkernel_b200.runtime import engine as E
+    monkeypatch.setattr(E, "DecodeGraph", PlainStep)
+    monkeypatch.setattr(Engine, "FEED_EAGER_STEPS", 0)
+    torch.manual_seed(4)
+    cfg = tiny_config()
+    w = init_random_weights(cfg, seed=2)
+    tokens = torch.randint(0, cfg.vocab_size, (2, 24)).tolist()
+    outs = []
+    for captured in (False, True):
+        ec = EngineConfig(model=cfg, sched=SchedulerConfig(max_model_len=64, max_num_seqs=2, max_num_batched_tokens=64, graph_cap=8)).validate()
+        eng = Engine(ec, build_model_weights(cfg, DictSource(w), "cpu"), "cpu", max_context=64)
+        eng.use_graphs = captured
+        a, b = eng.open_sequence(), eng.open_sequence()
+        eng.feed([(a, tokens[0][:20], []), (b, tokens[1][:17], [])])
+        outs.append(eng.feed([(a, [tokens[0][20]], wanted[0]), (b, [tokens[1][17]], wanted[1])]))
+    assert outs[0].shape[0] == len(wanted[0]) + len(wanted[1])
+    assert outs[0].shape == outs[1].shape and float((outs[0] - outs[1]).norm()) <= 1e-5 * float(outs[0].norm())

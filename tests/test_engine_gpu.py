@@ -230,3 +230,27 @@ def test_feed_steps_that_are_captured_match_eager_ones(family):
         assert a.shape == b.shape and a.dtype == b.dtype == torch.float32
         # the padded batch changes the order of sums; their bf16 roundings go through the whole model
         assert float((a - b).norm() / a.norm()) < 2e-2
+
+
+def test_feed_places_that_repeat_or_are_absent_on_both_sides_of_the_capture():
+    """The same wishes before and after steps of this batch are captured: row i of the logits is the i-th wanted place."""
+    cfg = tiny_config(dense_dtype="bf16", kv_cache_dtype="fp8_ds_mla", expert_dtype="nvfp4")
+    src = DictSource(init_random_weights(cfg, seed=2))
+    tokens = torch.randint(0, cfg.vocab_size, (2, 120), generator=torch.Generator().manual_seed(1)).tolist()
+    outs = []
+    for cap in (0, 8):
+        eng = make_engine(cfg, src, graph_cap=cap)
+        a, b = eng.open_sequence(), eng.open_sequence()
+        eng.feed([(a, tokens[0][:40], []), (b, tokens[1][:33], [])])
+        got = []
+        for i in range(Engine.FEED_EAGER_STEPS + 8):
+            wa, wb = (([0], [0]), ([0, 0], []), ([], [0, 0]), ([], [0]))[0 if i < Engine.FEED_EAGER_STEPS + 2 else i % 4]
+            got.append(eng.feed([(a, [tokens[0][40 + i]], wa), (b, [tokens[1][33 + i]], wb)]))
+            assert got[-1].shape[0] == len(wa) + len(wb)
+        assert (len(eng._graphs) > 0) == (cap > 0)
+        outs.append(got)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    for x, y in zip(*outs):
+        # bf16 roundings in another order of the sums; the other sequence's logits differ by more than the norm
+        assert x.shape == y.shape and float((x - y).norm() / x.norm()) < 2e-2
