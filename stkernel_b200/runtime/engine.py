@@ -973,6 +973,10 @@ class Engine:
         """The captured step that gives every sequence's logits for one given token each, once such steps are frequent."""
         if not self.use_graphs or n_req > self.cfg.sched.graph_cap or n_req > self.cfg.sched.max_num_seqs:
             return None
+        if self.cfg.parallel.tp_size > 1 or self.model.load_recorder is not None:
+            # whole logit rows are gathered over the ranks by a library collective, which stays outside captured steps (as it does
+            # in generation); and padded rows and a capture's warm-up would be counted among the experts' tokens
+            return None
         seen = self._feeds.get(n_req, 0)
         if seen < self.FEED_EAGER_STEPS:
             self._feeds[n_req] = seen + 1

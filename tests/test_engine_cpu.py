@@ -265,3 +265,26 @@ def test_captured_feed_steps_give_the_wanted_rows(wanted, monkeypatch):
         outs.append(eng.feed([(a, [tokens[0][20]], wanted[0]), (b, [tokens[1][17]], wanted[1])]))
     assert outs[0].shape[0] == len(wanted[0]) + len(wanted[1])
     assert outs[0].shape == outs[1].shape and float((outs[0] - outs[1]).norm()) <= 1e-5 * float(outs[0].norm())
+
+
+def test_feed_steps_of_several_ranks_or_with_recorded_loads_are_not_captured(monkeypatch):
+    """Full rows gathered over the ranks stay outside captured steps; recorded expert loads count the fed tokens alone."""
+    import dataclasses
+    from stkernel_b200.parallel.eplb import LoadRecorder
+    from stkernel_b200.runtime import engine as E
+    monkeypatch.setattr(E, "DecodeGraph", PlainStep)
+    monkeypatch.setattr(Engine, "FEED_EAGER_STEPS", 0)
+    cfg = tiny_config()
+    ec = EngineConfig(model=cfg, sched=SchedulerConfig(max_model_len=64, max_num_seqs=4, max_num_batched_tokens=64, graph_cap=8)).validate()
+    eng = Engine(ec, build_model_weights(cfg, DictSource(init_random_weights(cfg, seed=2)), "cpu"), "cpu", max_context=64)
+    eng.use_graphs = True
+    assert eng._feed_graph(3, 1) is not None
+    eng.cfg = dataclasses.replace(ec, parallel=dataclasses.replace(ec.parallel, tp_size=2))
+    assert eng._feed_graph(3, 1) is None
+    eng.cfg = ec
+    eng.model.load_recorder = rec = LoadRecorder(cfg.num_hidden_layers, cfg.n_routed_experts, torch.device("cpu"))
+    assert eng._feed_graph(3, 1) is None
+    seqs = [eng.open_sequence() for _ in range(3)]
+    for i in range(4):
+        eng.feed([(s, [7 + i], [0]) for s in seqs])
+    assert rec.counts.sum().item() == 4 * 3 * cfg.num_experts_per_tok * cfg.num_hidden_layers
