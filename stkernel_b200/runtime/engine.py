@@ -207,6 +207,13 @@ def step_bucket(n_req: int) -> int:
     return 1 << max(0, n_req - 1).bit_length()
 
 
+def feed_bucket(n_req: int) -> int:
+    """Rows of the captured step of given tokens that serves `n_req` sequences: never more than `step_bucket` (which the step's
+    buffers hold), no padding up to eight rows (where every row costs: 5 rows padded to 8 through eight layers of the flagship replayed
+    in 3.7 ms for 4.5 ms eagerly) and at most seven rows of it above."""
+    return n_req if n_req <= 8 else (n_req + 7) // 8 * 8
+
+
 class StepBuffers:
     """Two pinned host staging sets (the host may prepare step k+1 while the copies of step k are
     still queued) + fixed-address device tensors for the step description."""
@@ -315,7 +322,7 @@ class Engine:
         self._next_id = 0
         self.requests: Dict[int, Request] = {}
         self._graphs: Dict[tuple, object] = {}
-        self._feeds: Dict[int, int] = {}     # steps of one given token per sequence so far, by batch size
+        self._feeds: Dict[tuple, int] = {}   # steps of one given token per sequence that ran eagerly, by the graph that would serve them
         # a captured step cannot hold the stage-to-stage sends and receives: pipeline stages run eagerly; so do steps
         # under decode context parallelism (their staging buffers are allocated as block sizes first appear)
         self.use_graphs = self.device.type == "cuda" and sc.graph_cap > 0 and pipe is None and dcp == 1
@@ -952,22 +959,24 @@ class Engine:
         return out
 
     # ---- CUDA graphs -----------------------------------------------------------------
-    # Steps of given tokens (one per sequence) run eagerly this often at a batch size before they are captured: a short replay
-    # never pays for a capture (a few hundred launches), a long one is no longer paced by them.
+    # Steps of given tokens (one per sequence) run eagerly this often for a graph before it is captured: a short replay never pays
+    # for a capture, a long one is no longer paced by its launches.  Measured, two flagship layers: a capture costs four to six eager
+    # steps (1.7 to 2.6 ms; more where the allocator has much to give back first) and is paid back by 8 to 17 replays (0.7 to 1.6 ms).
     FEED_EAGER_STEPS = 16
+    FEED_MAX_GRAPHS = 16           # of these steps; the one that was not used for longest makes room
 
-    def _decode_graph(self, n_req: int, max_comp_rows: int, logits: bool = False) -> "DecodeGraph":
-        bucket = step_bucket(n_req)
-        rows_bucket = self.model.decode_bucket(max_comp_rows)
-        key = ("feed", bucket, rows_bucket) if logits else (bucket, rows_bucket)
+    def _decode_graph(self, n_req: int, max_comp_rows: int) -> "DecodeGraph":
+        key = (step_bucket(n_req), self.model.decode_bucket(max_comp_rows))
+        self._pad_ranges(n_req, key[0])
+        g = self._graphs.get(key)
+        if g is None:
+            g = self._graphs[key] = DecodeGraph(self, *key)
+        return g
+
+    def _pad_ranges(self, n_req: int, bucket: int) -> None:
         if n_req < bucket:
             # padding rows: empty query ranges => request -1, nothing is read or written for them
             self.buf.d_qstart[n_req + 1:bucket + 1].fill_(n_req)
-        g = self._graphs.get(key)
-        if g is None:
-            g = DecodeGraph(self, bucket, rows_bucket, logits)
-            self._graphs[key] = g
-        return g
 
     def _feed_graph(self, n_req: int, max_comp_rows: int) -> Optional["DecodeGraph"]:
         """The captured step that gives every sequence's logits for one given token each, once such steps are frequent."""
@@ -977,11 +986,23 @@ class Engine:
             # whole logit rows are gathered over the ranks by a library collective, which stays outside captured steps (as it does
             # in generation); and padded rows and a capture's warm-up would be counted among the experts' tokens
             return None
-        seen = self._feeds.get(n_req, 0)
-        if seen < self.FEED_EAGER_STEPS:
-            self._feeds[n_req] = seen + 1
-            return None
-        return self._decode_graph(n_req, max_comp_rows, logits=True)
+        key = ("feed", feed_bucket(n_req), self.model.decode_bucket(max_comp_rows))
+        g = self._graphs.pop(key, None)
+        if g is None:
+            seen = self._feeds.get(key, 0)
+            if seen < self.FEED_EAGER_STEPS:
+                self._feeds[key] = seen + 1
+                return None
+            self._feeds.pop(key, None)
+            held = [k for k in self._graphs if k[0] == "feed"]
+            if len(held) >= self.FEED_MAX_GRAPHS:
+                del self._graphs[held[0]]           # `feed` waits for its replays: none is running
+            self._pad_ranges(n_req, key[1])
+            g = DecodeGraph(self, key[1], key[2], logits=True)
+        else:
+            self._pad_ranges(n_req, key[1])
+        self._graphs[key] = g                       # in the order of their last use
+        return g
 
     def _run_logits(self, n: int, max_comp_rows: int) -> torch.Tensor:
         """One token of each of n requests -> their logits [n, vocab] in the head's type."""

@@ -288,3 +288,41 @@ def test_feed_steps_of_several_ranks_or_with_recorded_loads_are_not_captured(mon
     for i in range(4):
         eng.feed([(s, [7 + i], [0]) for s in seqs])
     assert rec.counts.sum().item() == 4 * 3 * cfg.num_experts_per_tok * cfg.num_hidden_layers
+
+
+def test_feed_graphs_are_counted_padded_and_bounded_by_the_graph_that_serves_them(monkeypatch):
+    """Each graph is captured after its own eager steps, also when a sequence grows into the next one; padding is small and within
+    the step's buffers; the graphs held are bounded and the least recently used one goes."""
+    from stkernel_b200.runtime import engine as E
+    built = []
+
+    class Step(PlainStep):
+        def __init__(self, eng, bucket, rows_bucket, logits=False):
+            super().__init__(eng, bucket, rows_bucket, logits)
+            built.append((bucket, rows_bucket))
+
+    monkeypatch.setattr(E, "DecodeGraph", Step)
+    cfg = tiny_config()
+    ec = EngineConfig(model=cfg, sched=SchedulerConfig(max_model_len=64, max_num_seqs=256, max_num_batched_tokens=256, graph_cap=256)).validate()
+    eng = Engine(ec, build_model_weights(cfg, DictSource(init_random_weights(cfg, seed=2)), "cpu"), "cpu", max_context=64)
+    eng.use_graphs = True
+    eng.model.decode_bucket = lambda rows: 64 * (rows // 64 + 1)
+    for n in range(1, 257):
+        b = E.feed_bucket(n)
+        assert n <= b <= n + 7 and b <= E.step_bucket(n) and (n > 8 or b == n)
+    steps = Engine.FEED_EAGER_STEPS
+    # 9 to 16 sequences share a graph and its count
+    assert all(eng._feed_graph(9 + i % 8, 1) is None for i in range(steps))
+    assert eng._feed_graph(12, 1) is not None and built == [(16, 64)]
+    assert eng.buf.d_qstart[13:17].tolist() == [12] * 4
+    # more rows: another graph, with eager steps of its own
+    assert all(eng._feed_graph(12, 64) is None for _ in range(steps))
+    assert eng._feed_graph(12, 64) is not None and built == [(16, 64), (16, 128)]
+    assert eng._feed_graph(16, 1) is not None and len(built) == 2
+    for n in range(1, 256, 8):
+        for _ in range(steps + 1):
+            eng._feed_graph(n, 1)
+        eng._feed_graph(12, 64)                       # kept in use
+        assert sum(k[0] == "feed" for k in eng._graphs) <= Engine.FEED_MAX_GRAPHS
+    assert ("feed", 16, 128) in eng._graphs and ("feed", 24, 64) not in eng._graphs
+    assert len(built) == len(set(built))

@@ -254,3 +254,44 @@ def test_feed_places_that_repeat_or_are_absent_on_both_sides_of_the_capture():
     for x, y in zip(*outs):
         # bf16 roundings in another order of the sums; the other sequence's logits differ by more than the norm
         assert x.shape == y.shape and float((x - y).norm() / x.norm()) < 2e-2
+
+
+@pytest.mark.parametrize("family", ["flash", "hybrid"])
+def test_captured_feeds_start_sequences_and_outgrow_their_graph(family, monkeypatch):
+    """Steps captured after two eager ones: a sequence whose first step is one token of a captured batch, in a row that another
+    sequence gave back; nine sequences in sixteen rows; contexts that outgrow the rows their graph was captured for."""
+    from stkernel_b200.config import hybrid_stack
+    from stkernel_b200.models.hybrid import build_hybrid_weights
+    monkeypatch.setattr(Engine, "FEED_EAGER_STEPS", 2)
+    if family == "flash":
+        cfg = flash_config(num_layers=2, n_routed_experts=16, vocab_size=4096, num_hash_layers=2, dense_dtype="bf16")
+        weights = build_model_weights(cfg, RandomSource(5), "cuda:0")
+    else:
+        cfg = hybrid_stack(4, 512, heads=4, kv_heads=1, dim=128, window=160, ff=768, vocab=4096, mlstm_heads=2, mlstm_dim=64, mlstm_vdim=128)
+        weights = build_hybrid_weights(cfg, RandomSource(5), "cuda:0")
+    tokens = torch.randint(0, cfg.vocab_size, (11, 80), generator=torch.Generator().manual_seed(3)).tolist()
+    outs = []
+    for cap in (0, 16):
+        ec = EngineConfig(model=cfg, sched=SchedulerConfig(max_model_len=512, max_num_seqs=10, max_num_batched_tokens=512, graph_cap=cap)).validate()
+        eng = Engine(ec, weights, "cuda:0", max_context=512)
+        eng.model.decode_bucket = lambda rows: 8 * (rows // 8 + 1)
+        live = {i: [eng.open_sequence(), 0] for i in range(8)}
+        got = []
+        for step in range(40):
+            if step == 12:
+                eng.close_sequence(live.pop(2)[0])
+                live[8] = [eng.open_sequence(), 0]
+                live[9] = [eng.open_sequence(), 0]
+            order = sorted(live)
+            got.append(eng.feed([(live[i][0], [tokens[i][live[i][1]]], [0]) for i in order]))
+            for i in order:
+                live[i][1] += 1
+        keys = [k for k in eng._graphs if k[0] == "feed"]
+        assert cap == 0 or ({k[1] for k in keys} == {8, 16} and len({k[2] for k in keys}) > 1)
+        outs.append(got)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    for step, (a, b) in enumerate(zip(*outs)):
+        assert a.shape == b.shape
+        # row by row: bf16 roundings in another order of the sums, through the whole model
+        assert float(((a - b).norm(dim=1) / a.norm(dim=1)).max()) < 4e-2, step
