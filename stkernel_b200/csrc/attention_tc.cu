@@ -9,7 +9,7 @@
 //                    O^T[dim, head] += V^T . P           (the same panels as the MN-major A operand:
 //                                                         K = V = the latent row, stored once)
 //   softmax warps    read S^T from TMEM (one row and half of the heads per thread), write P as the K-major B
-//                    operand, rescale O in TMEM only when some score outgrew its head's maximum by 2^8
+//                    operand, rescale in TMEM the columns of O whose head's maximum moved
 //
 // What bounds it: the key block (128 KB in bf16) and Q (64 KB) fill shared memory, so there is one key buffer, and a block is
 // scores -> softmax -> values in turn.  Everything else is taken off that chain:
@@ -19,11 +19,12 @@
 //     warps with twice the rows each left the conversions waiting for their own results); a load instruction takes 64 contiguous
 //     bytes of eight rows, and its two stores per lane hit every bank once.  The rotated part needs no conversion: it is copied
 //     asynchronously into the panel that is freed first and scored last;
-//   * the softmax works with a maximum that may be stale by up to 2^8 (weights keep their relative precision, only their common
-//     factor moves), so the reductions over the 128 rows that a maximum needs run for a token's first block and rarely after;
-//     the row sums of P stay in registers (one per head and row) and are reduced once per CTA.
-// Measured (4096 tokens, 64 heads, 128 + 2048 rows): 5166 us with one thread block of thirteen warps working through
-// load -> scores -> softmax -> values without overlap, 2524 us now (8400 cycles per block, 3100 of them on the tensor cores).
+//   * of O only the columns of the heads whose maximum moved are rescaled, one head at a time (a few of a block's 64; two at a time
+//     took 2753 us, four 2894, all of them 3182); the row sums of P stay in registers (one per head and row) and are reduced once
+//     per CTA.  The maxima themselves are exact: with one that may be stale by up to 2^8 the leading weights fall anywhere between
+//     two powers of two instead of just below 1, where bf16 rounds best -- 2525 us, and 2.8 % more error.
+// Measured (4096 tokens, 64 heads, 128 + 2048 rows): 5162 us with one thread block of thirteen warps working through
+// load -> scores -> softmax -> values without overlap, 2677 us now.
 //
 // Accumulators live in TMEM: S (NH columns) and four O^T tiles of [128 dims x NH heads].
 // A CTA of a split writes an un-normalised partial (o, m, l) that `sparse_mla_combine` merges with the sink.
@@ -68,11 +69,10 @@ __device__ __forceinline__ unsigned long long global_ns() {
 constexpr int kD = 512, kR = 64, kNope = 448, kDataBytes = 576, kPanels = 8, kRows = 128;
 constexpr int kPanelBytes = kRows * 128;                 // 16 KB
 constexpr int kProducerWarps = 16;
-constexpr float kStale = 8.f;                            // how far (in powers of two) a score may pass the maximum in use
 
 // Warpgroups: the first issues products (one warp of it), then the softmax warps, then the producers.  From 32 heads on two
 // softmax warps share a lane quarter of TMEM and take half of the heads each.  Registers follow the roles: what the first
-// warpgroup gives back (launch total 640 x 96) pays for the sums that the softmax warps hold.
+// warpgroup gives back (of 896 x 72 or 768 x 80 at launch) pays for the sums that the softmax warps hold.
 template <int NH>
 struct MlaCfg {
   static constexpr int kHalves = NH >= 32 ? 2 : 1;
@@ -106,10 +106,17 @@ struct alignas(8) MlaBars {
   uint64_t k_free[kPanels / 2];    // the value products of a pair of panels are done
   uint64_t s_full, p_full, pv_done;
   uint32_t tmem_base;
-  int grow[2];                     // by block parity: some score outgrew its head's maximum
+  uint32_t moved[2];               // heads whose maximum this block moved, by halves of 32
 };
 static_assert(sizeof(MlaBars) <= kBarBytes, "barrier block");
 
+// one column: 32 lanes x 32 bits
+__device__ __forceinline__ void tmem_ld_32x1(uint32_t taddr, uint32_t& r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_st_32x1(uint32_t taddr, uint32_t r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(taddr), "r"(r) : "memory");
+}
 __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
@@ -165,8 +172,7 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
   float* smax = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + kBarBytes);  // [4][NH], row sums at the end
   float* m_run = smax + 4 * NH;                          // [NH] the maxima in use, in powers of two
   float* minus_m = m_run + NH;                           // [NH] their negatives (0 for none yet)
-  float* limit = minus_m + NH;                           // [NH] a score above this needs a new maximum
-  float* alpha_s = limit + NH;                           // [NH]
+  float* alpha_s = minus_m + NH;                         // [NH]
 
   const int t = blockIdx.x, sp = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -199,7 +205,6 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
     mbar_init(&bars->s_full, 1);
     mbar_init(&bars->p_full, kSoftmaxWarps);
     mbar_init(&bars->pv_done, 1);
-    bars->grow[0] = bars->grow[1] = 0;
     fence_barrier_init();
   }
   if (warp == 0) {
@@ -322,60 +327,56 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
       ok = __all_sync(0xffffffffu, ok && mbar_wait(&bars->s_full, ph, a.status, 610));
       if (b == 0 && threadIdx.x == 128) STK_TRACE(3);
       tc_fence_after();
-      if (b > 0) {
-        bool grow = false;
+      // maxima of this block's rows per head, and the running ones
+      {
+        uint32_t raw[kHeads / 16][16];
+        float s[kHeads];
 #pragma unroll
-        for (int c = 0; c < kHeads; c += 16) {
-          uint32_t r16[16];
-          scores(c, r16);
+        for (int c = 0; c < kHeads / 16; ++c) tmem_ld_32x16(tmem_s + lane_addr + h0 + 16 * c, raw[c]);
+        tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 16; i += 4) {
-            const float4 l4 = *reinterpret_cast<const float4*>(limit + h0 + c + i);
-            grow = grow || __uint_as_float(r16[i]) * sl2 > l4.x || __uint_as_float(r16[i + 1]) * sl2 > l4.y ||
-                   __uint_as_float(r16[i + 2]) * sl2 > l4.z || __uint_as_float(r16[i + 3]) * sl2 > l4.w;
-          }
-        }
-        if (__any_sync(0xffffffffu, grow && valid) && lane == 0) bars->grow[ph] = 1;
-        named_bar_sync(2, kSoftmaxThreads);
+        for (int i = 0; i < kHeads; ++i) s[i] = valid ? __uint_as_float(raw[i / 16][i % 16]) * sl2 : -INFINITY;
+        bfly_reduce_store<kHeads, true>(s, smax + q4 * NH + h0, lane);
       }
-      if (b == 0 || bars->grow[ph]) {
-        // new maxima for all heads
-#pragma unroll 1
-        for (int c = 0; c < kHeads; c += 16) {
-          uint32_t r16[16];
-          scores(c, r16);
-          float s[16];
-#pragma unroll
-          for (int i = 0; i < 16; ++i) s[i] = valid ? __uint_as_float(r16[i]) * sl2 : -INFINITY;
-          bfly_reduce_store<16, true>(s, smax + q4 * NH + h0 + c, lane);
-        }
-        named_bar_sync(2, kSoftmaxThreads);
+      named_bar_sync(2, kSoftmaxThreads);
+      if (own < (NH < 32 ? 32 : NH)) {                     // whole warps
+        bool moved = false;
         if (own < NH) {
           const float bm = fmaxf(fmaxf(smax[own], smax[NH + own]), fmaxf(smax[2 * NH + own], smax[3 * NH + own]));
           const float mo = m_run[own], mn = fmaxf(mo, bm);
-          alpha_s[own] = (mo == -INFINITY || mn == -INFINITY) ? 1.f : exp2f(mo - mn);
+          moved = mn != mo && mo != -INFINITY;
+          alpha_s[own] = moved ? exp2f(mo - mn) : 1.f;
           m_run[own] = mn;
           minus_m[own] = mn == -INFINITY ? 0.f : -mn;
-          limit[own] = mn + kStale;
         }
-        if (threadIdx.x == 128) bars->grow[ph] = 0;        // everybody has read it; next written two blocks on
-        named_bar_sync(2, kSoftmaxThreads);
-        if (b > 0) {
+        const uint32_t some = __ballot_sync(0xffffffffu, moved);
+        if (lane == 0) bars->moved[own >> 5] = some;
+      }
+      named_bar_sync(2, kSoftmaxThreads);
+      // heads whose maximum moved: their sums, and their columns of O (this block's scores were issued behind the previous block's
+      // value products: those are complete)
+      uint32_t mask = bars->moved[h0 >> 5] >> (h0 & 31);
+      if constexpr (kHeads < 32) mask &= (1u << kHeads) - 1u;
+      if (mask != 0) {
 #pragma unroll
-          for (int i = 0; i < kHeads; i += 2) lp[i / 2] = mul2(lp[i / 2], pack2(alpha_s[h0 + i], alpha_s[h0 + i + 1]));
-          // this block's scores were issued behind the previous block's value products: those are complete
-#pragma unroll 1
-          for (int c = 0; c < 4 * kHeads; c += 16) {
-            const uint32_t at = tmem_o + (c / kHeads) * NH + h0 + c % kHeads + lane_addr;
-            uint32_t r16[16];
-            tmem_ld_32x16(at, r16);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 16; ++i) r16[i] = __float_as_uint(__uint_as_float(r16[i]) * alpha_s[h0 + c % kHeads + i]);
-            tmem_st_32x16(at, r16);
-          }
-          tmem_st_wait();
+        for (int i = 0; i < kHeads; i += 4) {
+          const ulonglong2 f4 = *reinterpret_cast<const ulonglong2*>(alpha_s + h0 + i);
+          lp[i / 2] = mul2(lp[i / 2], f4.x);
+          lp[i / 2 + 1] = mul2(lp[i / 2 + 1], f4.y);
         }
+        const uint32_t o_at = tmem_o + h0 + lane_addr;
+        while (mask != 0) {
+          const int h = __ffs(mask) - 1;
+          mask &= mask - 1;
+          uint32_t r[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) tmem_ld_32x1(o_at + j * NH + h, r[j]);
+          const float f = alpha_s[h0 + h];
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 4; ++j) tmem_st_32x1(o_at + j * NH + h, __float_as_uint(__uint_as_float(r[j]) * f));
+        }
+        tmem_st_wait();
       }
       // P = exp2(s - m), bf16, written as the K-major B operand [head][row]; the sums take the rounded values
 #pragma unroll
@@ -568,7 +569,7 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
 
 template <int NH>
 static int launch_mla_tc(const MlaTcArgs& a, cudaStream_t st) {
-  const int smem = kPanels * kPanelBytes + kPanels * NH * 128 + 2 * NH * 128 + kBarBytes + 8 * NH * 4 + 1024;
+  const int smem = kPanels * kPanelBytes + kPanels * NH * 128 + 2 * NH * 128 + kBarBytes + 7 * NH * 4 + 1024;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(sparse_mla_tc_kernel<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)

@@ -1,4 +1,6 @@
 """Each sm_100a kernel against the PyTorch fp32 statement of the same op."""
+import math
+
 import pytest
 import torch
 
@@ -374,6 +376,44 @@ def test_sparse_mla_matches_reference(nh, D, R_, fp8):
     out2 = A.sparse_mla(q, cg, swa_slots, swa_lens, None, None, None, sink, D ** -0.5)
     ref2 = A.sparse_mla(q.cpu(), ccpu, swa_slots.cpu(), swa_lens.cpu(), None, None, None, sink.cpu(), D ** -0.5)
     assert rel_err(out2, ref2) < 1e-2
+
+
+@pytest.mark.parametrize("nh", [8, 32, 64])
+def test_sparse_mla_weights_are_relative_to_the_exact_maximum(nh):
+    """Weights relative to the largest: 1 and 3/4 are bf16 numbers, so two leading rows 3 x and -4 x in the last block cancel whatever
+    came before them -- a first block of rows 4 to 9 powers of two lower, a different distance per token, which a maximum taken from
+    it would turn into weights that bf16 rounds.  Tolerance: 3/4 is met to the fp32 rounding of scores below 2^4 and of their
+    difference (a few 2^-20 of a weight), times the 4 + 3 that are subtracted; 1e-4 is ten times that and a thirtieth of a rounding."""
+    D, R_, T, W = 512, 64, 60, 128
+    levels = list(range(4, 14))
+    rows = torch.zeros((1 + len(levels)) * 64, D)
+    g = torch.Generator().manual_seed(0)
+    x = torch.randint(0, 2, (D,), generator=g).float() * 2 - 1
+    rows[0], rows[1] = 3 * x, -4 * x                          # leading rows
+    rows[0, 0], rows[1, 0] = 16, 15
+    for i, n in enumerate(levels):                            # a page of rows for each distance of the first block
+        rows[64 * (i + 1):64 * (i + 2), 0] = 16 - n
+    ccpu = C.PagedCache.allocate(1 + len(levels), D, R_, True, "latent", "cpu")
+    ccpu.write_rows_cpu(torch.arange(rows.shape[0]), rows)
+    assert torch.equal(ccpu.read_rows_cpu(torch.arange(rows.shape[0]))[0].float(), rows)
+    cg = C.PagedCache(ccpu.buf.to(dev()), D, R_, True, "latent")
+    q = torch.zeros(T, nh, D, device=dev(), dtype=BF16)
+    q[:, :, 0] = 1
+    page = torch.arange(T) % len(levels) + 1
+    slots = (page[:, None] * 64 + torch.arange(W)[None] % 64).to(torch.int32).to(dev())
+    lens = torch.full((T,), W, dtype=torch.int32, device=dev())
+    top = torch.tensor([[0, 1]], dtype=torch.int32, device=dev()).expand(T, -1).contiguous()
+    top_lens = torch.full((T,), 2, dtype=torch.int32, device=dev())
+    sink = torch.full((nh,), -1e30, device=dev())
+    scale = math.log(4 / 3)
+    out = A.sparse_mla(q, cg, slots, lens, cg, top, top_lens, sink, scale).float()
+    assert float(out[:, :, 1:].abs().max()) < 1e-4
+    # the first value does not cancel: against the weights in 64 bits
+    lead = torch.tensor([16 - n for n in levels], dtype=torch.float64)[page - 1]
+    s = torch.stack([lead, torch.full_like(lead, 16), torch.full_like(lead, 15)], 1)
+    w = torch.exp((s - 16) * scale) * torch.tensor([W, 1, 1], dtype=torch.float64)
+    ref = (w * s).sum(1) / w.sum(1)
+    assert float((out[:, :, 0].double().cpu() - ref[:, None]).abs().max()) < 2 ** -8 * 16
 
 
 @pytest.mark.parametrize("tokens", [9, 36, 37, 64, 148, 149])
