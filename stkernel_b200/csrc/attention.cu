@@ -226,9 +226,7 @@ __global__ void sparse_mla_combine_kernel(const float* __restrict__ partial, con
     o0 *= inv;
     o1 *= inv;
     if (positions != nullptr && d >= nope) {
-      // round to bf16 first: the un-fused path stores the attention output before rotating it
-      o0 = __bfloat162float(__float2bfloat16(o0));
-      o1 = __bfloat162float(__float2bfloat16(o1));
+      // rotated in 32 bits: one rounding, where a separate rotation would read a stored bf16 output and round again
       float sn, cs;
       sincosf(pos * inv_freq[(d - nope) >> 1], &sn, &cs);
       const float x = o0 * cs + o1 * sn;

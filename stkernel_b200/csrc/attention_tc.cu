@@ -457,9 +457,7 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
             if (h < a.nh) {
               float v = __uint_as_float(r16[i]) * alpha_s[h];
               if (rot) {
-                // the pair (even d, d + 1) sits in neighbouring lanes; values are rounded to bf16 before the rotation,
-                // as the separate combine pass does
-                v = __bfloat162float(__float2bfloat16(v));
+                // the pair (even d, d + 1) sits in neighbouring lanes
                 const float p = __shfl_xor_sync(0xffffffffu, v, 1);
                 v = (d & 1) ? (-p * sn + v * cs) : (v * cs + p * sn);
               }
