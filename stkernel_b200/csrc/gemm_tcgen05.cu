@@ -1196,7 +1196,7 @@ STK_API int stk_gemm_pick_bt(int T, int is_fp8) {
   return bt;
 }
 
-// Suggested split-K factor so that a skinny problem still fills the SMs.
+// Suggested split-K factor so that a skinny problem still fills the SMs (through the fp32 workspace of the 128-row tiles).
 STK_API int stk_gemm_pick_splits(int T, int N, int K, int is_fp8, int sm_count) {
   const int bt = stk_gemm_pick_bt(T, is_fp8);
   const int tiles = ((N + 127) / 128) * ((T + bt - 1) / bt);
@@ -1264,6 +1264,13 @@ static int fp8_tokens_split(int T, int N, int K, int sm_count) {
   return s > 1 || T >= 48 ? s : 0;
 }
 
+// Which token-major tiles a plain product (one block, no fused collective) without workspace splits takes: the number of CTAs that
+// share one, or 0 for the 128-row tiles.
+STK_API int stk_gemm_token_tile_ctas(int T, int N, int K, int is_fp8, int sm_count) {
+  if (is_fp8) return fp8_tokens_split(T, N, K, sm_count);
+  return gemm_wide_enabled() ? wide_split_of(T, N, K, sm_count) : 0;
+}
+
 static int gemm_launch(const void* W, long long ldw, const void* X, long long ldx, void* out, long long ldo, int T, int N,
                        int K, int is_fp8, int out_fp32, const float* w_scale, int w_scale_ld, const float* x_scale,
                        int x_scale_ld, int splits, float* workspace, int* counters, int* status, int sm_count,
@@ -1275,7 +1282,8 @@ static int gemm_launch(const void* W, long long ldw, const void* X, long long ld
   if (is_fp8 && (w_scale == nullptr || x_scale == nullptr || (x_scale_ld & 3))) return -11;
   if (splits > 1 && (workspace == nullptr || counters == nullptr)) return -12;
   if (groups < 1) groups = 1;
-  const int tokens_split = is_fp8 && groups == 1 && ar_ctx == nullptr && gate_ctx == nullptr ? fp8_tokens_split(T, N, K, sm_count) : 0;
+  // an explicit split goes through the workspace
+  const int tokens_split = is_fp8 && splits <= 1 && groups == 1 && ar_ctx == nullptr && gate_ctx == nullptr ? fp8_tokens_split(T, N, K, sm_count) : 0;
   if (tokens_split > 0) {
     CUtensorMap ta, tb;
     if (make_tmap_2d(&ta, X, 1, T, K, ldx, 128) != 0) return -13;        // lanes: tokens

@@ -888,6 +888,26 @@ def test_gemm_fp8_token_tiles(T, N, K):
     assert bool((wide[:, :8] == 7.0).all()) and bool((wide[:, 8 + N:] == 7.0).all())
 
 
+def test_gemm_fp8_workspace_serves_explicit_splits_only(monkeypatch):
+    """By default the token tiles take these sizes and no workspace is reserved; an explicit split goes through it."""
+    torch.manual_seed(3)
+    asked = []
+    scratch = Fn.scratch
+    monkeypatch.setattr(Fn, "scratch", lambda name, *a, **k: asked.append(name) or scratch(name, *a, **k))
+    for T, N, K in ((16, 2048, 4096), (40, 4096, 8192), (100, 1024, 4096)):
+        lw = Fn.LinearWeight.from_master(torch.randn(N, K, device=dev()) * 0.05, "fp8", dev())
+        x = torch.randn(T, K, device=dev()).to(BF16)
+        xq, xs = R.quant_fp8_group128_act(x)
+        ref = R.dequant_fp8_group128_act(xq, xs).double() @ lw.dequant().double().t()
+        assert rel_err(Fn.linear(x, lw), ref) < 3e-3
+        assert "gemm.splitk" not in asked
+        ws = scratch("gemm.splitk", (4 * T * N,), F32, dev())
+        ws.fill_(float("nan"))
+        assert rel_err(Fn.linear(x, lw, splits=4), ref) < 3e-3
+        assert "gemm.splitk" in asked and bool(ws.isfinite().all())
+        asked.clear()
+
+
 @pytest.mark.parametrize("T", [97, 128, 129, 255, 257, 520])
 @pytest.mark.parametrize("N,K", [(16, 4096), (272, 1088), (1000, 64), (1030, 2048), (5000, 576)])
 def test_gemm_bf16_wide_tiles_that_share_k(T, N, K):
