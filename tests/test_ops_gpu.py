@@ -445,11 +445,13 @@ def test_sparse_mla_rotates_its_output_in_32_bits(T):
 
 @pytest.mark.parametrize("tokens", [9, 36, 37, 64, 148, 149])
 @pytest.mark.parametrize("K", [0, 640])
-def test_sparse_mla_splits_rows_over_idle_sms(tokens, K):
-    """Both sides of each line of the split rule, with lists that fill their capacity, end in any split, or are empty.
+@pytest.mark.parametrize("nh", [16, 64])
+def test_sparse_mla_splits_rows_over_idle_sms(tokens, K, nh):
+    """Both sides of each line of the split rule, with lists that fill their capacity, end in any split, or are empty; one and two
+    softmax warps per quarter of the rows.
     Tolerance of the tests around it: fp8 rows against the fp32 reference of the same rows."""
     torch.manual_seed(tokens)
-    D, R_, W, nh, n_pages = 512, 64, 128, 16, 24
+    D, R_, W, n_pages = 512, 64, 128, 24
     ccpu = C.PagedCache.allocate(n_pages, D, R_, True, "latent", "cpu")
     ccpu.write_rows_cpu(torch.arange(n_pages * 64), torch.randn(n_pages * 64, D))
     cg = C.PagedCache(ccpu.buf.to(dev()), D, R_, True, "latent")
@@ -911,14 +913,16 @@ def test_gemm_fp8_workspace_serves_explicit_splits_only(monkeypatch):
 @pytest.mark.parametrize("T", [97, 128, 129, 255, 257, 520])
 @pytest.mark.parametrize("N,K", [(16, 4096), (272, 1088), (1000, 64), (1030, 2048), (5000, 576)])
 def test_gemm_bf16_wide_tiles_that_share_k(T, N, K):
-    """256 x 256 tiles alone and split over two and four CTAs of a cluster: ragged edges, K of one block and of uneven parts."""
+    """256 x 256 tiles alone and split over two and four CTAs of a cluster: ragged edges, K of one block and of uneven parts.  Without
+    workspace splits, which sizes up to 128 tokens would take by themselves."""
     torch.manual_seed(T + N)
+    assert _lib.query("stk_gemm_token_tile_ctas", T, N, K, 0, _lib.sm_count()) == (4 if K >= 1024 else 2 if K >= 512 else 1)
     w = (torch.randn(N, K, device=dev()) * 0.05).to(BF16)
     x = torch.randn(T, K, device=dev()).to(BF16)
     ref = x.double() @ w.double().t()
-    assert rel_err(Fn.linear(x, Fn.LinearWeight(w)), ref) < 2.5e-3
+    assert rel_err(Fn.linear(x, Fn.LinearWeight(w), splits=1), ref) < 2.5e-3
     wide = torch.full((T, N + 5), 7.0, dtype=F32, device=dev())
-    Fn.linear(x, Fn.LinearWeight(w), out=wide[:, :N])
+    Fn.linear(x, Fn.LinearWeight(w), out=wide[:, :N], splits=1)
     assert rel_err(wide[:, :N], ref) < 2e-5               # fp32 sums
     assert bool((wide[:, N:] == 7.0).all())
 
