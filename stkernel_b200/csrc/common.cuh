@@ -32,7 +32,7 @@ __device__ __forceinline__ void set_status(int* status, int code, int detail) {
   }
 }
 
-constexpr uint32_t kSpinBudget = 20u * 1000u * 1000u;   // try_wait polls, ~ a second at most
+constexpr uint32_t kSpinBudget = 20u * 1000u * 1000u;   // try_wait polls; one that fails returns after 4 us (7800 cycles, measured): 80 s
 
 // ---- programmatic dependent launch -------------------------------------------
 // The decode step is a chain of short kernels.  Each one is launched with the programmatic-serialization attribute:

@@ -796,8 +796,8 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 }
 
 // ---------------------------------------------------------------------------------
-// fp8 with at least a full tile of tokens, token-major: TMEM lanes are tokens, columns are weight rows, so the scale of a K block
-// is one multiplier per thread.  One CTA owns 128 tokens x 128 weight rows.
+// fp8, token-major (from nine tokens on, see fp8_tokens_split): TMEM lanes are tokens, columns are weight rows, so the scale of a K
+// block is one multiplier per thread.  One CTA owns 128 tokens x 128 weight rows.
 //
 // What bounds it: a K block is 259 tensor-core cycles, and its 128 x 128 results have to be read back from TMEM, scaled and added
 // to the second-level accumulators (fp32, in registers).  The scales of a block are asked for four blocks ahead (loaded when their
@@ -1213,7 +1213,8 @@ STK_API long long stk_gemm_workspace_bytes(int T, int N, int splits) {
 }
 
 // CTAs that share a 256 x 256 tile of the wide kernel (as many as keep the SMs to one round, with at least four K blocks each), or 0
-// where the kernel above is better: up to 96 tokens.  Measured, us, kernel above / this one with its split:
+// where the kernel above is better: up to 96 tokens.  A call that asks for workspace splits keeps the kernel above: `linear` does so up
+// to 128 tokens wherever 128-row tiles leave SMs idle.  Measured without workspace splits, us, kernel above / this one with its split:
 //   64 tokens x 4096 x 8192: 24.5 / 28.7;  128: 51.8 / 29.5;  256: 48.4 / 29.8;  777: 124 / 52;  128 x 40960 x 1536: 94 / 46;
 //   4096 tokens x 64 x 4096: 28 / 19;  777 x 4096 x 4096: 66 / 31.5 (45.3 without the split);  1500 x 4096 x 4096: 113 / 49.6.
 static int wide_split_of(int T, int N, int K, int sm_count) {
@@ -1323,8 +1324,8 @@ static int gemm_launch(const void* W, long long ldw, const void* X, long long ld
   }
   int bt = stk_gemm_pick_bt(T, is_fp8);
   if (!is_fp8 && T > 128 && groups == 1) {
-    // mid-size bf16 problems: split-K through the fp32 workspace costs more than it gains above 128 tokens
-    // (measured), so parallelism comes from narrower token tiles until about 0.7 x the SMs have a tile
+    // bf16 products that the wide tiles do not take (those fused with a collective): split-K through the fp32 workspace costs more
+    // than it gains above 128 tokens (measured), so parallelism comes from narrower token tiles until about 0.7 x the SMs have one
     const int wt = (N + 127) / 128;
     while (bt > 64 && wt * ((T + bt - 1) / bt) * 10 < sm_count * 7) bt /= 2;
   }

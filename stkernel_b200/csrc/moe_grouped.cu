@@ -20,7 +20,11 @@
 // fences and load latency of a block are paid once per 128 codes of a thread and hidden by the other three groups; with all
 // sixteen warps on the same block (32 codes each) the same conversions took 2500 cycles per block at 128 tokens and 1040 at 16.
 // Codes are fetched two own blocks ahead, past the ends of tiles.
-// Measured (256 experts, 4096 x 2048, top 6), both products: 64 tokens 1231 us before, 882 us now; 4096 tokens 3680 us before, 3684 us
+// Measured (hidden 4096, 2048 rows an expert, top 6; device time of the first + the second product, us):
+//   64 tokens, 256 experts    849 + 529 with all warps on one block, 632 + 302 now
+//   4096 tokens, 256 experts  2772 + 1512, 2399 + 1233
+//   4096 tokens, 64 experts   1901 + 1033, 1005 + 540
+//
 // This is the engine's counterpart of the reference's fused W4A16 MoE kernel and, for the
 // expert-parallel layout, of its mega-MoE grouped GEMM (overlay/nvidia_model.py:227-559).
 #include <cuda_fp4.h>
@@ -60,6 +64,10 @@ struct MoeGCfg {
   static constexpr int kStageBytes = kATiles * 128 * 128 + BT * 128;
   static constexpr int kStagesRaw = (196 * 1024) / kStageBytes;
   static constexpr int kStages = kStagesRaw > 6 ? 6 : kStagesRaw;
+  // A dequant group waits for a free stage by parity, which cannot tell "free" from "two rounds behind".  At block i it knows that
+  // block i - kMoeGroups - kStages was multiplied (its last wait); the stage is at most one round behind if that is not before
+  // block i - 2 kStages.
+  static_assert(kStages >= kMoeGroups, "stages of the ring");
   static constexpr int kAccCols = kATiles * BT;
   static constexpr int kTmemCols = (2 * kAccCols <= 32) ? 32 : (2 * kAccCols <= 64) ? 64 : (2 * kAccCols <= 128) ? 128
                                    : (2 * kAccCols <= 256) ? 256 : 512;
