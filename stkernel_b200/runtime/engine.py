@@ -960,8 +960,8 @@ class Engine:
 
     # ---- CUDA graphs -----------------------------------------------------------------
     # Steps of given tokens (one per sequence) run eagerly this often for a graph before it is captured: a short replay never pays
-    # for a capture, a long one is no longer paced by its launches.  Measured, two flagship layers: a capture costs four to six eager
-    # steps (1.7 to 2.6 ms; more where the allocator has much to give back first) and is paid back by 8 to 17 replays (0.7 to 1.6 ms).
+    # for a capture, a long one is no longer paced by its launches.  Measured, two flagship layers, 1 to 64 sequences: a step takes 1.7
+    # to 2.6 ms eagerly and 0.7 to 1.6 ms replayed; a capture costs three to five eager steps and is paid back by 5 to 13 replays.
     FEED_EAGER_STEPS = 16
     FEED_MAX_GRAPHS = 16           # of these steps; the one that was not used for longest makes room
 
@@ -1024,14 +1024,27 @@ def _capture_stream(device) -> "torch.cuda.Stream":
 
 
 @contextlib.contextmanager
-def _capturing(graph: "torch.cuda.CUDAGraph", device):
+def _capturing(graph: "torch.cuda.CUDAGraph", device, keep_cache: bool = False, pool=None):
     """Capture into `graph` without cyclic garbage collection: a collector that runs in the middle may release an earlier engine's
-    graphs and events, which is not permitted while a stream is being captured."""
+    graphs and events, which is not permitted while a stream is being captured.
+
+    keep_cache: leave the allocator's cached blocks where they are while the device has room for the capture's own memory (a
+    thirty-second of it).  Giving them back, as `torch.cuda.graph` does first, makes the steps behind the capture allocate again; the
+    caller has synchronised the device.  pool: that of another graph, to share its memory."""
     was = gc.isenabled()
     gc.disable()
     try:
-        with torch.cuda.graph(graph, stream=_capture_stream(device)):
-            yield
+        free, total = torch.cuda.mem_get_info(device) if keep_cache else (0, 1)
+        if free < total // 32:
+            with torch.cuda.graph(graph, pool=pool, stream=_capture_stream(device)):
+                yield
+        else:
+            with torch.cuda.stream(_capture_stream(device)):
+                graph.capture_begin(pool=pool)
+                try:
+                    yield
+                finally:
+                    graph.capture_end()
     finally:
         if was:
             gc.enable()
@@ -1076,7 +1089,6 @@ class DecodeGraph:
     """A captured pure-decode step for `bucket` rows (token i belongs to request i): sampled tokens, or logits."""
 
     def __init__(self, eng: Engine, bucket: int, rows_bucket: int, logits: bool = False):
-        self.eng = eng
         self.bucket = bucket
 
         def body():
@@ -1089,17 +1101,25 @@ class DecodeGraph:
         ranges = qstart.clone() if eng.model.recurrent else None
         if ranges is not None:
             qstart.zero_()
-        side = torch.cuda.Stream()
-        side.wait_stream(torch.cuda.current_stream())
-        with torch.cuda.stream(side):
-            for _ in range(2):
-                self.out = body()
-        torch.cuda.current_stream().wait_stream(side)
+        pool = None
+        if logits:
+            # in the middle of a replay: steps like it have run, so one of this size, in the blocks they left to this stream, prepares
+            # the rest.  On a stream of its own every block is allocated anew, which took from 7 to 400 ms.  Steps of given tokens
+            # share one pool: they run one after the other and their logits are copied out.
+            body()
+            pool = next((g.graph.pool() for k, g in eng._graphs.items() if k[0] == "feed"), None)
+        else:
+            side = torch.cuda.Stream()
+            side.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(side):
+                for _ in range(2):
+                    self.out = body()
+            torch.cuda.current_stream().wait_stream(side)
         torch.cuda.synchronize()
         from ..ops import _lib
         before = _lib.launch_count
         self.graph = torch.cuda.CUDAGraph()
-        with _capturing(self.graph, eng.device):
+        with _capturing(self.graph, eng.device, keep_cache=logits, pool=pool):
             self.out = body()
         self.launches_per_replay = _lib.launch_count - before
         if ranges is not None:

@@ -295,3 +295,34 @@ def test_captured_feeds_start_sequences_and_outgrow_their_graph(family, monkeypa
         assert a.shape == b.shape
         # row by row: bf16 roundings in another order of the sums, through the whole model
         assert float(((a - b).norm(dim=1) / a.norm(dim=1)).max()) < 4e-2, step
+
+
+def test_a_capture_leaves_cached_memory_alone_and_the_engine_free_to_go(monkeypatch):
+    """In the middle of a replay: the allocator keeps its cached blocks through the capture, feed graphs share one pool, and an engine
+    that holds such graphs goes with its last reference."""
+    import gc
+    import weakref
+    monkeypatch.setattr(Engine, "FEED_EAGER_STEPS", 2)
+    cfg = tiny_config(dense_dtype="bf16", kv_cache_dtype="fp8_ds_mla", expert_dtype="nvfp4")
+    eng = make_engine(cfg, DictSource(init_random_weights(cfg, seed=2)), graph_cap=8)
+    seqs = [eng.open_sequence() for _ in range(3)]
+    eng.feed([(s, [1, 2, 3], []) for s in seqs])
+    block = torch.empty(256 << 20, dtype=torch.uint8, device="cuda:0")
+    del block
+    for n in (3, 2):
+        for i in range(2):
+            eng.feed([(s, [4 + i], [0]) for s in seqs[:n]])
+        held = torch.cuda.memory_reserved()
+        eng.feed([(s, [6], [0]) for s in seqs[:n]])
+        assert len(eng._graphs) == 4 - n and torch.cuda.memory_reserved() >= held
+    assert len({g.graph.pool() for g in eng._graphs.values()}) == 1
+    torch.cuda.synchronize()
+    _lib.check_status()
+    gc.collect()
+    gc.disable()
+    try:
+        ref = weakref.ref(eng)
+        del eng
+        assert ref() is None
+    finally:
+        gc.enable()
