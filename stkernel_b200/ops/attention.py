@@ -229,8 +229,9 @@ USE_DECODE_MLA = True          # register-resident kernel for decode-sized steps
 MLA_DECODE_MAX_T = 8
 
 
-MLA_DIRECT_MIN_T = 37          # up to 36 tokens the combine pass spreads the final rows better (64 heads, 128 rows: 16.8 us against 19.2 at
-                               # 16 tokens, 18.7 / 19.4 at 32, 19.6 / 19.3 at 40, 29.9 / 19.9 at 148)
+MLA_DIRECT_MIN_T = 37          # up to 36 tokens the combine pass spreads the final rows better (128 rows, partials / direct: 64 heads
+                               # 16.6 / 19.1 us at 16 tokens, 18.7 / 19.1 at 36, 21.4 / 19.2 at 64, 29.7 / 19.6 at 148; 8 heads 10.9 /
+                               # 11.6 at 36, 11.4 / 11.6 at 64, 13.7 / 11.9 at 148)
 
 
 @lru_cache(maxsize=4096)
@@ -238,8 +239,8 @@ def _mla_splits(t: int, max_rows: int, sms: int) -> int:
     """Row splits of the tensor-core kernel.  A CTA (one per SM) works through its 128-row blocks in turn and costs most of one more
     to begin and end; every split leaves fp32 partial rows that the combine pass reads again, about 0.012 of a block's time each.
     So: the count with the least rounds x (blocks + 0.8), partials included.  Measured against two CTAs per SM (64 heads, 2176 rows):
-    9 tokens 65 -> 29 us, 32: 52 -> 42, 64: 77 -> 60, 128: 111 -> 90.  Beyond one CTA per SM no split: 150 tokens gain a tenth by
-    one, but lose a fifth where the lists are short of their capacity (56 -> 67 us at 384 of 2176 rows)."""
+    9 tokens 65 -> 30 us, 32: 54 -> 45, 64: 82 -> 65, 128: 120 -> 96 (32 tokens x 16 heads: 40 -> 34).  Beyond one CTA per SM no
+    split: 150 tokens gain a tenth by one (190 -> 167), but lose where the lists are short of their capacity (384 of 2176 rows)."""
     if t > sms:
         return 1
     best, least = 1, None
