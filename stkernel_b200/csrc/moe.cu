@@ -13,9 +13,8 @@
 // bytes of the weight rows, so each warp streams whole rows with 16-byte loads and dots them in
 // half2 against activations held in shared memory (fp32 accumulation per 16-value group).
 // Prefill-sized batches use the tcgen05 grouped GEMM instead.
-#include <cuda_fp4.h>
-
 #define STK_PDL_CLASS 1024      // bit of this file's kernels in the PDL mask (STK_PDL, stk_set_pdl_mask)
+#include "codes.cuh"
 #include "common.cuh"
 #include "router.cuh"
 
@@ -200,12 +199,10 @@ __device__ __forceinline__ float fp4_chunk_dot(const uint4& wv, uint32_t sc, con
     for (int q = 0; q < 2; ++q) {
       const uint4 xv = xs[(k * 4 + g * 2 + q) * 32 + lane];
       const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w};
-      const uint32_t w = words[g * 2 + q];
+      __half2 h[4];
+      e2m1x8_to_half(words[g * 2 + q], h);
 #pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const __half2_raw hr = __nv_cvt_fp4x2_to_halfraw2(static_cast<__nv_fp4x2_storage_t>((w >> (8 * b)) & 0xff), __NV_E2M1);
-        hs = __hfma2(*reinterpret_cast<const __half2*>(&hr), *reinterpret_cast<const __half2*>(&xw[b]), hs);
-      }
+      for (int b = 0; b < 4; ++b) hs = __hfma2(h[b], *reinterpret_cast<const __half2*>(&xw[b]), hs);
     }
     part[g] = __low2float(hs) + __high2float(hs);
   }

@@ -5,30 +5,28 @@
 // that have rows, dealt out in turn, so that every CTA has the same number of them whichever experts were chosen:
 //
 //   TMA warp         activation tile [BT tokens x 64 k] fp16, 128-byte swizzle
-//   dequant warps    e2m1 codes and e4m3 group scales -> fp16 written straight into the swizzled K-major
-//                    operand tile
-//   MMA warp         tcgen05.mma kind::f16 into TMEM (double-buffered accumulators), as many token columns as
-//                    the tile has rows (in sixteens)
-//   epilogue warps   FC1: gate and up tiles sit side by side in TMEM, so one thread holds both values
-//                    of an output and applies SwiGLU with clamp before storing fp16;
+//   weight warp      e2m1 codes of 128 weight rows x 256 k by TMA (a 128-byte line a row), their e4m3 group scales by cp.async
+//   dequant warps    codes and scales -> fp16 straight into tensor memory: a TMEM lane is a weight row, 64 k are 32 columns
+//   MMA warp         tcgen05.mma kind::f16, weights from tensor memory and activations from shared memory, as many token columns
+//                    as the tile has rows (in sixteens)
+//   epilogue warps   FC1: a warp's lanes hold sixteen gate rows and the up rows of the same features, one shuffle brings a
+//                    feature's two products together for SwiGLU with clamp, stored as fp16;
 //                    FC2: scaled bf16 store.  Rows past the expert's last token are masked.
 //
 // e2m1 x e4m3 is exact in fp16, the per-matrix fp32 scale is applied in the epilogue.
 //
-// What bounds it: a K block of 256 weight rows is 16384 codes to convert and 9.2 KB to fetch, for eight products of 40 to 65
-// tensor-core cycles.  Four groups of four dequant warps (one per scheduler) convert every fourth K block each, so the waits,
-// fences and load latency of a block are paid once per 128 codes of a thread and hidden by the other three groups; with all
-// sixteen warps on the same block (32 codes each) the same conversions took 2500 cycles per block at 128 tokens and 1040 at 16.
-// Codes are fetched two own blocks ahead, past the ends of tiles.
-// Measured (hidden 4096, 2048 rows an expert, top 6; device time of the first + the second product, us):
-//   64 tokens, 256 experts    849 + 529 with all warps on one block, 632 + 302 now
-//   4096 tokens, 256 experts  2772 + 1512, 2399 + 1233
-//   4096 tokens, 64 experts   1901 + 1033, 1005 + 540
+// What bounds it: weights are read once, 4.6 KB per 128 rows x 64 k, and their bytes in flight have to cover the trip to memory: the
+// ring holds 108 KB an SM and more (codes fetched into registers by the converting warps were 16 KB).  Converted weights do not pass
+// through shared memory, which carries the codes, the activations and the products' reads of them: 64 KB per 2 x 128 rows x 64 k at
+// 128 tokens, 512 cycles, what the products take.  Four groups of four dequant warps convert a quarter of a stage each.
+// Measured (hidden 4096, 2048 rows an expert, top 6; device time of the first + the second product, us; before: operands converted
+// into shared memory from codes in registers):
+//   64 tokens, 256 experts    632 + 302 before, 487 + 260 now
+//   4096 tokens, 256 experts  2409 + 1241, 1473 + 657
 //
 // This is the engine's counterpart of the reference's fused W4A16 MoE kernel and, for the
 // expert-parallel layout, of its mega-MoE grouped GEMM (overlay/nvidia_model.py:227-559).
-#include <cuda_fp4.h>
-
+#include "codes.cuh"
 #include "common.cuh"
 
 namespace stk {
@@ -47,6 +45,7 @@ struct MoeGArgs {
   int K;
   void* out;               // FC1: fp16 [P, I]; FC2: bf16 [P, H]
   float limit;
+  int scale_copy;          // bytes of one copy of scales: 16, 4 or (unaligned scales) 1
   int* status;
   // Expert-parallel mode: rows of expert e are pushed into the activation matrix by peers (and by this
   // GPU's own dispatch); `arrived[e]` counts the rows that have landed.  nullptr = rows are already there.
@@ -55,84 +54,98 @@ struct MoeGArgs {
 };
 
 constexpr int kMoeMaxExperts = 2048;     // of one launch (the lists of tiles lie in shared memory)
-constexpr int kMoeGroups = 4;            // dequant warps: groups x 4
+constexpr int kMoeK = 256;               // K of a weight stage: a 128-byte line of codes and 16 scales per weight row
+constexpr int kMoeSlots = 8;             // operand slots in tensor memory: 32 columns (64 K) of a weight tile each
+constexpr int kMoeThreads = 768;         // activations, products, weights, (idle), 4 epilogue warps, 4 x 4 dequant warps
 
-// kATiles: 128-row weight tiles of a unit (FC1: gate and up; FC2: two neighbours where the rows allow it)
-template <int BT, int kATiles_>
+// kTiles: weight tiles (128 TMEM lanes each) of a unit
+template <int BT, int kTiles_>
 struct MoeGCfg {
-  static constexpr int kATiles = kATiles_;
-  static constexpr int kStageBytes = kATiles * 128 * 128 + BT * 128;
-  static constexpr int kStagesRaw = (196 * 1024) / kStageBytes;
-  static constexpr int kStages = kStagesRaw > 6 ? 6 : kStagesRaw;
-  // A dequant group waits for a free stage by parity, which cannot tell "free" from "two rounds behind".  At block i it knows that
-  // block i - kMoeGroups - kStages was multiplied (its last wait); the stage is at most one round behind if that is not before
-  // block i - 2 kStages.
-  static_assert(kStages >= kMoeGroups, "stages of the ring");
-  static constexpr int kAccCols = kATiles * BT;
-  static constexpr int kTmemCols = (2 * kAccCols <= 32) ? 32 : (2 * kAccCols <= 64) ? 64 : (2 * kAccCols <= 128) ? 128
-                                   : (2 * kAccCols <= 256) ? 256 : 512;
+  static constexpr int kTiles = kTiles_;
+  static constexpr int kBoxRows = BT < 32 ? BT : 32;                    // token rows of one activation copy
+  static constexpr int kCodeBytes = 128 * 128, kScaleBytes = 128 * 16;
+  static constexpr int kWStages = BT == 128 ? 6 : 8;
+  static constexpr int kXBytes = BT * 128;
+  static constexpr int kXStages = BT == 128 ? 6 : 8;
+  static constexpr int kRingBytes = kWStages * (kCodeBytes + kScaleBytes) + kXStages * kXBytes;
+  static constexpr int kAccCols = kTiles * BT;
+  static constexpr int kAccBufs = 2 * kAccCols + kMoeSlots * 32 <= 512 ? 2 : 1;
+  static_assert(kAccBufs * kAccCols + kMoeSlots * 32 <= 512, "tensor memory");
 };
 
 struct alignas(8) MoeGBars {
-  uint64_t full[8];
-  uint64_t empty[8];
-  uint64_t tmem_full[2];
-  uint64_t tmem_empty[2];
+  uint64_t w_full[8], w_empty[8];
+  uint64_t x_full[8], x_empty[8];
+  uint64_t a_full[kMoeSlots], a_empty[kMoeSlots];
+  uint64_t tmem_full[2], tmem_empty[2];
   uint32_t tmem_base;
   int n_experts;                  // that have rows
 };
 
-// Half of a weight row's K block: 32 e2m1 codes (16 bytes) and their two e4m3 group scales.
-struct RawRow {
-  uint4 w;
-  uint32_t sc;
-};
-
-__device__ __forceinline__ void load_raw(RawRow& r, const uint8_t* w, const uint8_t* s) {
-  // codes pass by the first-level cache, which is left to the scales (a sector of them serves eight K blocks)
-  asm volatile("ld.global.nc.L1::no_allocate.L2::128B.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r.w.x), "=r"(r.w.y), "=r"(r.w.z), "=r"(r.w.w) : "l"(w));
-  r.sc = __ldg(reinterpret_cast<const uint16_t*>(s));
+__device__ __forceinline__ void moe_tmem_st_32(uint32_t taddr, const uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]),
+      "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]),
+      "r"(r[30]), "r"(r[31])
+      : "memory");
 }
+__device__ __forceinline__ void moe_tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// 32 values of one weight row -> 64 bytes of fp16, chunk i (eight values) at line + at[i].
-__device__ __forceinline__ void dequant_store(const RawRow& r, uint8_t* line, const uint32_t (&at)[4]) {
-  const uint32_t words[4] = {r.w.x, r.w.y, r.w.z, r.w.w};
-  const __half2_raw sraw = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(r.sc), __NV_E4M3);
-  const __half2 sc = *reinterpret_cast<const __half2*>(&sraw);
+// 32 e2m1 codes (16 bytes) and their two scales -> 16 words of fp16 pairs
+__device__ __forceinline__ void moe_dequant(const uint4& codes, __half2 sc, uint32_t* out) {
+  const uint32_t words[4] = {codes.x, codes.y, codes.z, codes.w};
   const __half2 sc2[2] = {__low2half2(sc), __high2half2(sc)};
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    uint4 o;
-    __half2* oh = reinterpret_cast<__half2*>(&o);
+    __half2 h[4];
+    e2m1x8_to_half(words[i], h);
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
-      const __half2_raw hr = __nv_cvt_fp4x2_to_halfraw2(static_cast<__nv_fp4x2_storage_t>((words[i] >> (8 * b)) & 0xff), __NV_E2M1);
-      oh[b] = __hmul2(*reinterpret_cast<const __half2*>(&hr), sc2[i >> 1]);
+      const __half2 v = __hmul2(h[b], sc2[i >> 1]);
+      out[4 * i + b] = *reinterpret_cast<const uint32_t*>(&v);
     }
-    *reinterpret_cast<uint4*>(line + at[i]) = o;
   }
 }
 
-template <int BT, bool kFc1, int kATiles>
-__global__ void __launch_bounds__(704, 1)
-moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const MoeGArgs a) {
-  using Cfg = MoeGCfg<BT, kATiles>;
-  constexpr int kStages = Cfg::kStages;
-  constexpr int CW = (BT >= 32 && kATiles == 1) ? 32 : 16;     // columns of an epilogue step
+// Row of a stage that TMEM lane 32 q4 + lane holds.  FC1: sixteen gate rows (rows 0..63 of the stage) and the up rows of the same
+// features (64..127) side by side in a warp, so that one shuffle brings a feature's two products together.
+template <bool kFc1>
+__device__ __forceinline__ int moe_lane_row(int q4, int lane) {
+  return kFc1 ? (lane >> 4) * 64 + q4 * 16 + (lane & 15) : q4 * 32 + lane;
+}
+
+template <int BT, bool kFc1, int kTiles>
+__global__ void __launch_bounds__(kMoeThreads, 1)
+moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const MoeGArgs a) {
+  using Cfg = MoeGCfg<BT, kTiles>;
+  constexpr int kWStages = Cfg::kWStages, kXStages = Cfg::kXStages, kAccBufs = Cfg::kAccBufs;
+  constexpr int kDepth = kMoeSlots / (4 * kTiles);              // weight stages of a tile whose operands lie in tensor memory
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* smem_a = smem;                                        // kStages x kATiles x 16 KB
-  uint8_t* smem_b = smem + kStages * kATiles * 128 * 128;        // kStages x BT*128
-  MoeGBars* bars = reinterpret_cast<MoeGBars*>(smem_b + kStages * BT * 128);
+  uint8_t* smem_w = smem;                                        // kWStages x 16 KB of codes
+  uint8_t* smem_x = smem_w + kWStages * Cfg::kCodeBytes;         // kXStages x BT x 128 B
+  uint8_t* smem_s = smem_x + kXStages * Cfg::kXBytes;            // kWStages x 2 KB of scales
+  MoeGBars* bars = reinterpret_cast<MoeGBars*>(smem_s + kWStages * Cfg::kScaleBytes);
   int* first_tile = reinterpret_cast<int*>(bars + 1);            // [experts with rows + 1] token tiles of those before
   int* expert_of = first_tile + a.e_local + 1;                   // [experts with rows]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
-      mbar_init(&bars->full[s], 1 + 4);           // TMA arrive (+tx bytes) and the four warps of a dequant group
-      mbar_init(&bars->empty[s], 1);
+    for (int s = 0; s < kWStages; ++s) {
+      mbar_init(&bars->w_full[s], 1 + 32);        // TMA arrive (+tx bytes) and the lanes that copy scales
+      mbar_init(&bars->w_empty[s], 16);           // dequant warps
+    }
+    for (int s = 0; s < kXStages; ++s) {
+      mbar_init(&bars->x_full[s], 1);
+      mbar_init(&bars->x_empty[s], 1);
+    }
+    for (int s = 0; s < kMoeSlots; ++s) {
+      mbar_init(&bars->a_full[s], 4);             // the four warps of a dequant group
+      mbar_init(&bars->a_empty[s], 1);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bars->tmem_full[i], 1);
@@ -141,11 +154,14 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const MoeGArgs a) {
     fence_barrier_init();
   }
   if (warp == 1) {
-    tmem_alloc(&bars->tmem_base, Cfg::kTmemCols);
+    tmem_alloc(&bars->tmem_base, 512);
     tmem_relinquish();
   }
   if (warp == 0) {
-    if (lane == 0) tma_prefetch_desc(&tmX);
+    if (lane == 0) {
+      tma_prefetch_desc(&tmX);
+      tma_prefetch_desc(&tmW);
+    }
     // experts that have rows, and the token tiles in front of each
     int n = 0, tiles = 0;
     for (int e0 = 0; e0 < a.e_local; e0 += 32) {
@@ -176,11 +192,13 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const MoeGArgs a) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
+  const uint32_t tmem_slots = tmem_base + kAccBufs * Cfg::kAccCols;
 
-  const int tiles_n = a.rows / (128 * kATiles);     // FC1: tiles over I; FC2: tiles over H
+  const int tiles_n = a.rows / (128 * kTiles);
   const int n_experts = bars->n_experts;
   const int units = first_tile[n_experts] * tiles_n;
-  const int k_blocks = a.K / 64;
+  const int stages_k = (a.K + kMoeK - 1) / kMoeK;               // weight stages of a tile
+  auto steps_of = [&](int sb) { return min(4, (a.K - sb * kMoeK) / 64); };      // K steps of 64 in stage sb
 
   struct Unit { int e, tn, r0, rows; };             // expert, weight tile, first row and rows of the token tile
   auto unit_at = [&](int u) {
@@ -221,11 +239,13 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const MoeGArgs a) {
           if (!here) { set_status(a.status, kTimeoutPeerFlag, 760); ok = false; break; }
           asm volatile("fence.proxy.async.global;" ::: "memory");      // peer stores (generic proxy) -> TMA reads
         }
-        for (int kb = 0; kb < k_blocks; ++kb) {
-          if (!mbar_wait(&bars->empty[stage], phase ^ 1, a.status, 700 + stage)) { ok = false; break; }
-          mbar_expect_tx(&bars->full[stage], BT * 128);
-          tma_load_2d(smem_b + stage * BT * 128, &tmX, &bars->full[stage], kb * 64, x.r0);
-          if (++stage == kStages) { stage = 0; phase ^= 1; }
+        const int boxes = (x.rows + Cfg::kBoxRows - 1) / Cfg::kBoxRows;      // only what has rows
+        for (int kb = 0; kb < a.K / 64; ++kb) {
+          if (!mbar_wait(&bars->x_empty[stage], phase ^ 1, a.status, 700 + stage)) { ok = false; break; }
+          mbar_expect_tx(&bars->x_full[stage], boxes * Cfg::kBoxRows * 128);
+          for (int i = 0; i < boxes; ++i)
+            tma_load_2d(smem_x + stage * Cfg::kXBytes + i * Cfg::kBoxRows * 128, &tmX, &bars->x_full[stage], kb * 64, x.r0 + i * Cfg::kBoxRows);
+          if (++stage == kXStages) { stage = 0; phase ^= 1; }
         }
       }
     }
@@ -233,11 +253,10 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const MoeGArgs a) {
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
     const uint32_t lead = elect_one() ? 1u : 0u, tm = __shfl_sync(0xffffffffu, tmem_base, 0);
-    const uint32_t a_lo = desc_lo(smem_u32(smem_a)), b_lo = desc_lo(smem_u32(smem_b));
-    int stage = 0;
-    uint32_t phase = 0;
-    int ab = 0;
-    uint32_t aphase = 0;
+    const uint32_t slots = tm + kAccBufs * Cfg::kAccCols, x_lo = desc_lo(smem_u32(smem_x));
+    int stage = 0, ab = 0;
+    uint32_t phase = 0, aphase = 0;
+    uint32_t step_uses[4] = {0, 0, 0, 0};           // of the slots of each step: their phases
     bool ok = true;
     for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
       const Unit x = unit_at(u);
@@ -245,30 +264,87 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const MoeGArgs a) {
       ok = mbar_wait(&bars->tmem_empty[ab], aphase ^ 1, a.status, 710 + ab);
       if (!ok) break;
       tc_fence_after();
-      for (int kb = 0; kb < k_blocks; ++kb) {
-        ok = mbar_wait(&bars->full[stage], phase, a.status, 720 + stage);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t bl = b_lo + stage * (BT * 8), al = a_lo + stage * (kATiles * 1024);
+      const uint32_t acc = tm + ab * Cfg::kAccCols;
+      for (int sb = 0; sb < stages_k && ok; ++sb) {
+        const int steps = steps_of(sb);
 #pragma unroll
-        for (int at = 0; at < kATiles; ++at)
+        for (int q = 0; q < 4; ++q) {
+          if (q < steps && ok) {
+            ok = mbar_wait(&bars->x_full[stage], phase, a.status, 720 + stage);
+            if (!ok) break;
+            const uint32_t bl = x_lo + stage * (Cfg::kXBytes >> 4);
+            const uint32_t d = step_uses[q] % kDepth, ph = (step_uses[q] / kDepth) & 1u;
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            mma_ss(tm + ab * Cfg::kAccCols + at * BT, al + at * 1024 + 2 * k, bl + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u, lead);
-        mma_commit(&bars->empty[stage], lead);
-        if (++stage == kStages) { stage = 0; phase ^= 1; }
+            for (int t = 0; t < kTiles; ++t) {
+              const int slot = (d * 4 + q) * kTiles + t;
+              ok = ok && mbar_wait(&bars->a_full[slot], ph, a.status, 750 + slot);
+              if (!ok) break;
+              tc_fence_after();
+#pragma unroll
+              for (int k = 0; k < 4; ++k)
+                mma_ts(acc + t * BT, slots + slot * 32 + k * 8, bl + 2 * k, idesc, (sb > 0 || q > 0 || k > 0) ? 1u : 0u, lead);
+              mma_commit(&bars->a_empty[slot], lead);
+            }
+            if (!ok) break;
+            mma_commit(&bars->x_empty[stage], lead);
+            ++step_uses[q];
+            if (++stage == kXStages) { stage = 0; phase ^= 1; }
+          }
+        }
       }
       if (ok) {
         mma_commit(&bars->tmem_full[ab], lead);
-        if (++ab == 2) { ab = 0; aphase ^= 1; }
+        if (++ab == kAccBufs) { ab = 0; aphase ^= 1; }
       }
     }
     __syncwarp();
-  } else if (warp < 6) {
+  } else if (warp == 2) {
+    // ------------------------------ weight producer (codes by TMA, scales by asynchronous copies) ------------------------------
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    const long long sstride = a.K / 16;
+    for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+      const Unit x = unit_at(u);
+      for (int sb = 0; sb < stages_k && ok; ++sb) {
+        for (int t = 0; t < kTiles; ++t) {
+          ok = __all_sync(0xffffffffu, mbar_wait(&bars->w_empty[stage], phase ^ 1, a.status, 740 + stage));
+          if (!ok) break;
+          const int tile = x.tn * kTiles + t;
+          const int row0 = x.e * a.rows + tile * (kFc1 ? 64 : 128), row1 = row0 + (kFc1 ? a.rows / 2 : 64);
+          if (lane == 0) {
+            mbar_expect_tx(&bars->w_full[stage], Cfg::kCodeBytes);
+            tma_load_2d(smem_w + stage * Cfg::kCodeBytes, &tmW, &bars->w_full[stage], sb * (kMoeK / 2), row0);
+            tma_load_2d(smem_w + stage * Cfg::kCodeBytes + 64 * 128, &tmW, &bars->w_full[stage], sb * (kMoeK / 2), row1);
+          }
+          const int steps = steps_of(sb);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int r = i * 32 + lane;
+            const uint8_t* src = a.s + ((r < 64 ? row0 + r : row1 + r - 64)) * sstride + sb * 16;
+            uint8_t* dst = smem_s + stage * Cfg::kScaleBytes + r * 16;
+            if (a.scale_copy == 16) {
+              asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+            } else if (a.scale_copy == 4) {
+              for (int j = 0; j < steps; ++j)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst + 4 * j)), "l"(src + 4 * j) : "memory");
+            } else {
+              for (int j = 0; j < 4 * steps; ++j) dst[j] = src[j];
+            }
+          }
+          if (a.scale_copy != 1)
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&bars->w_full[stage])) : "memory");
+          else
+            mbar_arrive(&bars->w_full[stage]);
+          if (++stage == kWStages) { stage = 0; phase ^= 1; }
+        }
+      }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  } else if (warp >= 4 && warp < 8) {
     // ------------------------------ epilogue ------------------------------
-    const int q = warp & 3;
-    const int row = q * 32 + lane;
-    const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
+    const int q4 = warp & 3;
+    const uint32_t lane_addr = static_cast<uint32_t>(q4 * 32) << 16;
     int ab = 0;
     uint32_t aphase = 0;
     bool ok = true;
@@ -278,116 +354,88 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const MoeGArgs a) {
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->tmem_full[ab], aphase, a.status, 730 + ab));
       if (!ok) break;
       tc_fence_after();
-      const int n = x.tn * (kFc1 ? 128 : 128 * kATiles) + row;      // (first) output feature of this thread
 #pragma unroll 1
-      for (int c0 = 0; c0 < x.rows; c0 += CW) {
-        uint32_t r[kATiles][32];
+      for (int c0 = 0; c0 < x.rows; c0 += 16) {
 #pragma unroll
-        for (int at = 0; at < kATiles; ++at) {
-          const uint32_t base = tmem_base + ab * Cfg::kAccCols + at * BT + c0 + lane_addr;
-          if constexpr (CW == 32) {
-            tmem_ld_32x32(base, r[at]);
-          } else {
-            uint32_t t16[16];
-            tmem_ld_32x16(base, t16);
+        for (int t = 0; t < kTiles; ++t) {
+          uint32_t r[16];
+          tmem_ld_32x16(tmem_base + ab * Cfg::kAccCols + t * BT + c0 + lane_addr, r);
+          tmem_ld_wait();
+          const int tile = x.tn * kTiles + t;
+          if constexpr (kFc1) {
+            // gate products in lanes 0..15, up products of the same features in lanes 16..31: the lower lanes finish columns
+            // 0..7, the upper ones 8..15
+            const bool upper = lane >= 16;
+            const int c = c0 + (upper ? 8 : 0);
+            __half* o = reinterpret_cast<__half*>(a.out) + static_cast<long long>(x.r0 + c) * a.n_out + tile * 64 + q4 * 16 + (lane & 15);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) r[at][i] = t16[i];
-          }
-        }
-        tmem_ld_wait();
-#pragma unroll
-        for (int j = 0; j < CW; ++j) {
-          if (c0 + j < x.rows) {
-            const long long o = static_cast<long long>(x.r0 + c0 + j) * a.n_out + n;
-            if constexpr (kFc1) {
-              float g = __uint_as_float(r[0][j]) * gs, up = __uint_as_float(r[1][j]) * gs;
+            for (int j = 0; j < 8; ++j) {
+              const uint32_t got = __shfl_xor_sync(0xffffffffu, upper ? r[j] : r[j + 8], 16);
+              float g = __uint_as_float(upper ? got : r[j]) * gs, up = __uint_as_float(upper ? r[j + 8] : got) * gs;
               if (a.limit > 0.f) {
                 g = fminf(g, a.limit);
                 up = fminf(fmaxf(up, -a.limit), a.limit);
               }
-              reinterpret_cast<__half*>(a.out)[o] = __float2half(g / (1.f + __expf(-g)) * up);
-            } else {
-#pragma unroll
-              for (int at = 0; at < kATiles; ++at)
-                reinterpret_cast<__nv_bfloat16*>(a.out)[o + at * 128] = __float2bfloat16(__uint_as_float(r[at][j]) * gs);
+              if (c + j < x.rows) o[j * a.n_out] = __float2half(g / (1.f + __expf(-g)) * up);
             }
+          } else {
+            __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(a.out) + static_cast<long long>(x.r0 + c0) * a.n_out + tile * 128 + q4 * 32 + lane;
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              if (c0 + j < x.rows) o[j * a.n_out] = __float2bfloat16(__uint_as_float(r[j]) * gs);
           }
         }
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars->tmem_empty[ab]);
-      if (++ab == 2) { ab = 0; aphase ^= 1; }
+      if (++ab == kAccBufs) { ab = 0; aphase ^= 1; }
     }
-  } else {
-    // ------------------------------ dequant producers (weights) ------------------------------
-    // Group g converts every fourth K block of the CTA's sequence of units.  A lane pair shares a weight row (32 codes each);
-    // a thread has the same half of 2 kATiles rows, 64 apart.
-    constexpr int kMine = 2 * kATiles;
-    const int group = (warp - 6) >> 2, gt = ((warp - 6) & 3) * 32 + lane;
-    const int half = gt & 1, r16 = gt >> 1;
-    uint32_t at[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) at[i] = static_cast<uint32_t>(r16 * 128 + (((half * 4 + i) ^ (r16 & 7)) << 4));
-    const long long wstride = a.K / 2, sstride = a.K / 16;
-    const long long second = (kFc1 ? a.rows / 2 : 128);             // rows between the first and the second tile
-    struct Cursor {
-      int u, kb;
-      const uint8_t* w;
-      const uint8_t* s;
-    } ld{static_cast<int>(blockIdx.x), group, nullptr, nullptr};
-    auto enter = [&]() {                                             // pointers of the cursor's unit
-      if (ld.u >= units) return;
-      const Unit x = unit_at(ld.u);
-      const long long row = static_cast<long long>(x.e) * a.rows + x.tn * (kFc1 ? 128 : 128 * kATiles) + r16;
-      ld.w = a.w + row * wstride + half * 16;
-      ld.s = a.s + row * sstride + half * 2;
-    };
-    auto settle = [&]() {                                            // the K block may lie in a later unit
-      while (ld.kb >= k_blocks && ld.u < units) {
-        ld.kb -= k_blocks;
-        ld.u += gridDim.x;
-        if (ld.kb < k_blocks) enter();
-      }
-    };
-    RawRow raw[2][kMine];
-    auto load = [&](RawRow (&r)[kMine]) {                            // the cursor's block, then on by a group's stride
-      if (ld.u < units) {
-#pragma unroll
-        for (int j = 0; j < kMine; ++j) {
-          const long long rows = (j & 1) * 64 + (j >> 1) * second;
-          load_raw(r[j], ld.w + rows * wstride + ld.kb * 32, ld.s + rows * sstride + ld.kb * 4);
-        }
-        ld.kb += kMoeGroups;
-        settle();
-      }
-    };
-    enter();
-    settle();
-    load(raw[0]);
-    load(raw[1]);
-    // blocks of this CTA's whole sequence: units, each k_blocks long
-    const long long mine = static_cast<int>(blockIdx.x) < units ? (units - 1 - static_cast<int>(blockIdx.x)) / static_cast<int>(gridDim.x) + 1 : 0;
-    const long long total = mine * k_blocks;
-    int stage = group % kStages;
-    uint32_t phase = static_cast<uint32_t>(group / kStages) & 1u;
+  } else if (warp >= 8) {
+    // ------------------------------ dequant (weights) ------------------------------
+    // Group q converts the q-th 64 values of every weight stage; a thread has one weight row.
+    const int q = (warp - 8) >> 2, q4 = warp & 3;
+    const uint32_t lane_addr = static_cast<uint32_t>(q4 * 32) << 16;
+    const int row = moe_lane_row<kFc1>(q4, lane);
+    const uint32_t code_at = row * 128 + (((2 * q) ^ (row & 7)) << 4), scale_at = row * 16 + q * 4;
+    int stage = 0;
+    uint32_t phase = 0, uses = 0;
     bool ok = true;
-    auto step = [&](RawRow (&r)[kMine]) {
-      ok = __all_sync(0xffffffffu, mbar_wait(&bars->empty[stage], phase ^ 1, a.status, 740 + stage));
-      if (!ok) return;
-#pragma unroll
-      for (int j = 0; j < kMine; ++j)
-        dequant_store(r[j], smem_a + (stage * kATiles + (j >> 1)) * 128 * 128 + (j & 1) * 64 * 128, at);
-      fence_proxy_async();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->full[stage]);
-      load(r);
-      stage += kMoeGroups;
-      while (stage >= kStages) { stage -= kStages; phase ^= 1; }
-    };
-    for (long long i = group; i < total && ok; i += 2 * kMoeGroups) {
-      step(raw[0]);
-      if (ok && i + kMoeGroups < total) step(raw[1]);
+    for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+      for (int sb = 0; sb < stages_k && ok; ++sb) {
+        const bool mine = q < steps_of(sb);
+        const uint32_t d = uses % kDepth, ph = (uses / kDepth) & 1u;
+#pragma unroll 1
+        for (int t = 0; t < kTiles; ++t) {
+          ok = __all_sync(0xffffffffu, mbar_wait(&bars->w_full[stage], phase, a.status, 770 + stage));
+          if (!ok) break;
+          uint32_t o[32];
+          if (mine) {
+            const uint8_t* codes = smem_w + stage * Cfg::kCodeBytes;
+            const uint4 c0 = *reinterpret_cast<const uint4*>(codes + code_at), c1 = *reinterpret_cast<const uint4*>(codes + (code_at ^ 16));
+            const uint32_t sc = *reinterpret_cast<const uint32_t*>(smem_s + stage * Cfg::kScaleBytes + scale_at);
+            __half2 s0, s1;
+            e4m3x4_to_half(sc, s0, s1);
+            moe_dequant(c0, s0, o);
+            moe_dequant(c1, s1, o + 16);
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->w_empty[stage]);
+          if (++stage == kWStages) { stage = 0; phase ^= 1; }
+          if (mine) {
+            const int slot = (d * 4 + q) * kTiles + t;
+            ok = __all_sync(0xffffffffu, mbar_wait(&bars->a_empty[slot], ph ^ 1, a.status, 780 + slot));
+            if (!ok) break;
+            tc_fence_after();
+            moe_tmem_st_32(tmem_slots + slot * 32 + lane_addr, o);
+            moe_tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->a_full[slot]);
+          }
+        }
+        if (mine) ++uses;
+      }
     }
   }
 
@@ -395,7 +443,7 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const MoeGArgs a) {
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, Cfg::kTmemCols);
+    tmem_dealloc(tmem_base, 512);
   }
 }
 
@@ -418,19 +466,19 @@ __global__ void moe_permute_kernel(const __nv_bfloat16* __restrict__ x, long lon
   }
 }
 
-template <int BT, bool kFc1, int kATiles>
-static int launch_moe_grouped(const CUtensorMap& tx, const MoeGArgs& a, int grid, cudaStream_t st) {
-  using Cfg = MoeGCfg<BT, kATiles>;
-  constexpr int kFixed = Cfg::kStages * Cfg::kStageBytes + static_cast<int>(sizeof(MoeGBars)) + 1024;
+template <int BT, bool kFc1, int kTiles>
+static int launch_moe_grouped(const CUtensorMap& tx, const CUtensorMap& tw, const MoeGArgs& a, int grid, cudaStream_t st) {
+  using Cfg = MoeGCfg<BT, kTiles>;
+  constexpr int kFixed = Cfg::kRingBytes + static_cast<int>(sizeof(MoeGBars)) + 1024;
   constexpr int kMost = kFixed + (2 * kMoeMaxExperts + 1) * 4;
   static_assert(kMost <= 227 * 1024, "shared memory");
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(moe_grouped_kernel<BT, kFc1, kATiles>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost) != cudaSuccess)
+    if (cudaFuncSetAttribute(moe_grouped_kernel<BT, kFc1, kTiles>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost) != cudaSuccess)
       return -3;
     configured = true;
   }
-  moe_grouped_kernel<BT, kFc1, kATiles><<<grid, 704, kFixed + (2 * a.e_local + 1) * 4, st>>>(tx, a);
+  moe_grouped_kernel<BT, kFc1, kTiles><<<grid, kMoeThreads, kFixed + (2 * a.e_local + 1) * 4, st>>>(tx, tw, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
@@ -455,7 +503,7 @@ static int moe_grouped_launch(const void* xs, long long xs_rows, const void* w, 
   if (e_local <= 0) return 0;
   if (K % 64 || n_out % 128 || (bt != 16 && bt != 32 && bt != 64 && bt != 128)) return -1;
   CUtensorMap tx;
-  if (make_tmap_2d(&tx, xs, 2, xs_rows, K, K, bt) != 0) return -2;
+  if (make_tmap_2d(&tx, xs, 2, xs_rows, K, K, bt < 32 ? bt : 32) != 0) return -2;
   MoeGArgs a;
   a.rows = fc1 ? 2 * n_out : n_out; a.n_out = n_out; a.K = K; a.out = out; a.limit = limit; a.status = status;
   a.spin_budget = spin_budget;
@@ -465,12 +513,15 @@ static int moe_grouped_launch(const void* xs, long long xs_rows, const void* w, 
     a.e_local = e_local - e0 < kMoeMaxExperts ? e_local - e0 : kMoeMaxExperts;
     a.w = (const uint8_t*)w + static_cast<long long>(e0) * a.rows * (K / 2);
     a.s = (const uint8_t*)s + static_cast<long long>(e0) * a.rows * (K / 16);
+    a.scale_copy = K % 256 == 0 && (reinterpret_cast<uintptr_t>(a.s) & 15) == 0 ? 16 : (reinterpret_cast<uintptr_t>(a.s) & 3) == 0 ? 4 : 1;
+    CUtensorMap tw;
+    if (make_tmap_2d(&tw, a.w, 1, static_cast<long long>(a.e_local) * a.rows, K / 2, K / 2, 64) != 0) return -2;
     a.gscale = gscale + e0;
     a.offsets = offsets + e0;
     a.arrived = arrived != nullptr ? arrived + e0 : nullptr;
     int rc;
-#define STK_MG(BT_) (fc1 ? launch_moe_grouped<BT_, true, 2>(tx, a, sm_count, st) \
-                         : two ? launch_moe_grouped<BT_, false, 2>(tx, a, sm_count, st) : launch_moe_grouped<BT_, false, 1>(tx, a, sm_count, st))
+#define STK_MG(BT_) (fc1 ? launch_moe_grouped<BT_, true, 2>(tx, tw, a, sm_count, st) \
+                         : two ? launch_moe_grouped<BT_, false, 2>(tx, tw, a, sm_count, st) : launch_moe_grouped<BT_, false, 1>(tx, tw, a, sm_count, st))
     switch (bt) {
       case 16: rc = STK_MG(16); break;
       case 32: rc = STK_MG(32); break;

@@ -987,6 +987,37 @@ def test_moe_grouped_gemm_uneven_experts(H, I, E, counts):
     assert rel_err(out, ref) < 5e-3                     # activations rounded to fp16 in between, expert outputs and sums to bf16
 
 
+@pytest.mark.parametrize("H,I", [(512, 256), (384, 128), (128, 128)])
+def test_moe_grouped_gemm_scales_off_alignment(H, I):
+    """Scales whose rows or base 16- and 4-byte copies cannot take, and K that ends inside a weight stage: the same bits as the
+    aligned ones give."""
+    torch.manual_seed(15)
+    E, T = 6, 90
+    ids = torch.randint(0, E, (T, 2), dtype=torch.int32, device=dev())
+    w = torch.rand(T, 2, device=dev()) + 0.5
+    scale = lambda *shape: (0.05 + torch.rand(*shape, device=dev())).to(torch.float8_e4m3fn).view(torch.uint8)
+    code = lambda *shape: torch.randint(0, 256, shape, dtype=torch.uint8, device=dev())
+    g = torch.full((E,), 0.03, device=dev())
+    w13, w2, s13, s2 = code(E, 2 * I, H // 2), code(E, H, I // 2), scale(E, 2 * I, H // 16), scale(E, H, I // 16)
+    x = torch.randn(T, H, device=dev()).to(BF16)
+
+    def moved(t, by):
+        buf = torch.zeros(t.numel() + by, dtype=torch.uint8, device=dev())
+        buf[by:] = t.reshape(-1)
+        return buf[by:].view(t.shape)
+    outs = [M.moe_experts(x, ids, w, M.ExpertWeights(w13, w2, moved(s13, by), moved(s2, by), g, g), 10.0, None, E) for by in (0, 4, 2)]
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    f8 = torch.float8_e4m3fn
+    ref = torch.zeros(T, H, device=dev(), dtype=torch.float64)
+    for e in range(E):
+        rows, place = (ids == e).nonzero(as_tuple=True)
+        h = x[rows].double() @ R.dequant_nvfp4(w13[e], s13[e].view(f8), g[e]).double().t()
+        y = h[:, :I].clamp(max=10.0)
+        y = y * torch.sigmoid(y) * h[:, I:].clamp(-10.0, 10.0)
+        ref.index_add_(0, rows, y @ R.dequant_nvfp4(w2[e], s2[e].view(f8), g[e]).double().t() * w[rows, place].double()[:, None])
+    assert rel_err(outs[0], ref) < 5e-3
+
+
 def test_topk_candidates_and_markov_chain_match_cpu():
     """The drafter's sampling path: two-level candidate selection over the full vocabulary and the one-launch
     sequential Markov sampling against their CPU statements."""
