@@ -63,11 +63,11 @@ template <int BT, int kTiles_>
 struct MoeGCfg {
   static constexpr int kTiles = kTiles_;
   static constexpr int kBoxRows = BT < 32 ? BT : 32;                    // token rows of one activation copy
-  static constexpr int kCodeBytes = 128 * 128, kScaleBytes = 128 * 16;
-  static constexpr int kWStages = BT == 128 ? 6 : 8;
+  static constexpr int kCodeBytes = 128 * 128, kScaleBytes = 128 * 16;  // of a weight tile in a stage
+  static constexpr int kSteps = kMoeSlots / kTiles;                     // K steps of 64 whose operands are ready or being written
+  static constexpr int kWStages = kTiles == 2 ? (BT >= 64 ? 4 : 5) : (BT == 128 ? 4 : 8);
   static constexpr int kXBytes = BT * 128;
-  static constexpr int kXStages = BT == 128 ? 6 : 8;
-  static constexpr int kRingBytes = kWStages * (kCodeBytes + kScaleBytes) + kXStages * kXBytes;
+  static constexpr int kRingBytes = kWStages * kTiles * (kCodeBytes + kScaleBytes) + kSteps * kXBytes;
   static constexpr int kAccCols = kTiles * BT;
   static constexpr int kAccBufs = 2 * kAccCols + kMoeSlots * 32 <= 512 ? 2 : 1;
   static_assert(kAccBufs * kAccCols + kMoeSlots * 32 <= 512, "tensor memory");
@@ -75,8 +75,7 @@ struct MoeGCfg {
 
 struct alignas(8) MoeGBars {
   uint64_t w_full[8], w_empty[8];
-  uint64_t x_full[8], x_empty[8];
-  uint64_t a_full[kMoeSlots], a_empty[kMoeSlots];
+  uint64_t s_full[kMoeSlots], s_empty[kMoeSlots];     // a step's weights (tensor memory) and activations (shared memory)
   uint64_t tmem_full[2], tmem_empty[2];
   uint32_t tmem_base;
   int n_experts;                  // that have rows
@@ -111,6 +110,11 @@ __device__ __forceinline__ void moe_dequant(const uint4& codes, __half2 sc, uint
   }
 }
 
+template <int N>
+__device__ __forceinline__ void moe_regs_less() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void moe_regs_more() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+
 // Row of a stage that TMEM lane 32 q4 + lane holds.  FC1: sixteen gate rows (rows 0..63 of the stage) and the up rows of the same
 // features (64..127) side by side in a warp, so that one shuffle brings a feature's two products together.
 template <bool kFc1>
@@ -122,14 +126,14 @@ template <int BT, bool kFc1, int kTiles>
 __global__ void __launch_bounds__(kMoeThreads, 1)
 moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const MoeGArgs a) {
   using Cfg = MoeGCfg<BT, kTiles>;
-  constexpr int kWStages = Cfg::kWStages, kXStages = Cfg::kXStages, kAccBufs = Cfg::kAccBufs;
-  constexpr int kDepth = kMoeSlots / (4 * kTiles);              // weight stages of a tile whose operands lie in tensor memory
+  constexpr int kWStages = Cfg::kWStages, kSteps = Cfg::kSteps, kAccBufs = Cfg::kAccBufs;
+  constexpr int kWCodes = kTiles * Cfg::kCodeBytes, kWScales = kTiles * Cfg::kScaleBytes;      // of a weight stage
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* smem_w = smem;                                        // kWStages x 16 KB of codes
-  uint8_t* smem_x = smem_w + kWStages * Cfg::kCodeBytes;         // kXStages x BT x 128 B
-  uint8_t* smem_s = smem_x + kXStages * Cfg::kXBytes;            // kWStages x 2 KB of scales
-  MoeGBars* bars = reinterpret_cast<MoeGBars*>(smem_s + kWStages * Cfg::kScaleBytes);
+  uint8_t* smem_w = smem;                                        // kWStages x kTiles x 16 KB of codes
+  uint8_t* smem_x = smem_w + kWStages * kWCodes;                 // kSteps x BT x 128 B
+  uint8_t* smem_s = smem_x + kSteps * Cfg::kXBytes;              // kWStages x kTiles x 2 KB of scales
+  MoeGBars* bars = reinterpret_cast<MoeGBars*>(smem_s + kWStages * kWScales);
   int* first_tile = reinterpret_cast<int*>(bars + 1);            // [experts with rows + 1] token tiles of those before
   int* expert_of = first_tile + a.e_local + 1;                   // [experts with rows]
 
@@ -139,13 +143,9 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       mbar_init(&bars->w_full[s], 1 + 32);        // TMA arrive (+tx bytes) and the lanes that copy scales
       mbar_init(&bars->w_empty[s], 16);           // dequant warps
     }
-    for (int s = 0; s < kXStages; ++s) {
-      mbar_init(&bars->x_full[s], 1);
-      mbar_init(&bars->x_empty[s], 1);
-    }
-    for (int s = 0; s < kMoeSlots; ++s) {
-      mbar_init(&bars->a_full[s], 4);             // the four warps of a dequant group
-      mbar_init(&bars->a_empty[s], 1);
+    for (int s = 0; s < kSteps; ++s) {
+      mbar_init(&bars->s_full[s], 1 + 4);         // TMA arrive (+tx bytes) and the four warps of a dequant group
+      mbar_init(&bars->s_empty[s], 1);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bars->tmem_full[i], 1);
@@ -198,7 +198,14 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   const int n_experts = bars->n_experts;
   const int units = first_tile[n_experts] * tiles_n;
   const int stages_k = (a.K + kMoeK - 1) / kMoeK;               // weight stages of a tile
-  auto steps_of = [&](int sb) { return min(4, (a.K - sb * kMoeK) / 64); };      // K steps of 64 in stage sb
+  const int steps_k = a.K / 64;                                 // K steps of a unit
+  // K step kb of this CTA's i-th unit is the use'th of its place in a stage (kb % 4): the buffers it takes and their phase
+  struct Step { int buf; uint32_t phase; };
+  auto step_at = [&](int i, int kb) {
+    const int q = kb & 3, use = i * ((steps_k + 3 - q) >> 2) + (kb >> 2);
+    if constexpr (kSteps == 4) return Step{q, static_cast<uint32_t>(use) & 1u};
+    else return Step{(use & 1) * 4 + q, static_cast<uint32_t>(use >> 1) & 1u};
+  };
 
   struct Unit { int e, tn, r0, rows; };             // expert, weight tile, first row and rows of the token tile
   auto unit_at = [&](int u) {
@@ -218,13 +225,15 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     return x;
   };
 
+  // Registers follow the roles: of 768 x 80 at launch, 128 x 56 + 128 x 64 + 512 x 88
+  if (warp < 4) {
+    moe_regs_less<56>();
   if (warp == 0) {
     // ------------------------------ TMA producer (activations) ------------------------------
     if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
       bool ok = true;
-      for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+      int i = 0;
+      for (int u = blockIdx.x; u < units && ok; u += gridDim.x, ++i) {
         const Unit x = unit_at(u);
         if (a.arrived != nullptr) {
           // rows of this expert come over NVLink: start as soon as they are all here (bounded wait)
@@ -240,12 +249,12 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
           asm volatile("fence.proxy.async.global;" ::: "memory");      // peer stores (generic proxy) -> TMA reads
         }
         const int boxes = (x.rows + Cfg::kBoxRows - 1) / Cfg::kBoxRows;      // only what has rows
-        for (int kb = 0; kb < a.K / 64; ++kb) {
-          if (!mbar_wait(&bars->x_empty[stage], phase ^ 1, a.status, 700 + stage)) { ok = false; break; }
-          mbar_expect_tx(&bars->x_full[stage], boxes * Cfg::kBoxRows * 128);
-          for (int i = 0; i < boxes; ++i)
-            tma_load_2d(smem_x + stage * Cfg::kXBytes + i * Cfg::kBoxRows * 128, &tmX, &bars->x_full[stage], kb * 64, x.r0 + i * Cfg::kBoxRows);
-          if (++stage == kXStages) { stage = 0; phase ^= 1; }
+        for (int kb = 0; kb < steps_k; ++kb) {
+          const Step st = step_at(i, kb);
+          if (!mbar_wait(&bars->s_empty[st.buf], st.phase ^ 1, a.status, 700 + st.buf)) { ok = false; break; }
+          mbar_expect_tx(&bars->s_full[st.buf], boxes * Cfg::kBoxRows * 128);
+          for (int j = 0; j < boxes; ++j)
+            tma_load_2d(smem_x + st.buf * Cfg::kXBytes + j * Cfg::kBoxRows * 128, &tmX, &bars->s_full[st.buf], kb * 64, x.r0 + j * Cfg::kBoxRows);
         }
       }
     }
@@ -254,43 +263,27 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     // ------------------------------ MMA issuer ------------------------------
     const uint32_t lead = elect_one() ? 1u : 0u, tm = __shfl_sync(0xffffffffu, tmem_base, 0);
     const uint32_t slots = tm + kAccBufs * Cfg::kAccCols, x_lo = desc_lo(smem_u32(smem_x));
-    int stage = 0, ab = 0;
-    uint32_t phase = 0, aphase = 0;
-    uint32_t step_uses[4] = {0, 0, 0, 0};           // of the slots of each step: their phases
+    int ab = 0, i = 0;
+    uint32_t aphase = 0;
     bool ok = true;
-    for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+    for (int u = blockIdx.x; u < units && ok; u += gridDim.x, ++i) {
       const Unit x = unit_at(u);
       const uint32_t idesc = umma_idesc(0u, 0u, 128, 0) | static_cast<uint32_t>(((x.rows + 15) >> 4) << 1) << 17;   // fp16 x fp16 -> fp32
       ok = mbar_wait(&bars->tmem_empty[ab], aphase ^ 1, a.status, 710 + ab);
       if (!ok) break;
       tc_fence_after();
       const uint32_t acc = tm + ab * Cfg::kAccCols;
-      for (int sb = 0; sb < stages_k && ok; ++sb) {
-        const int steps = steps_of(sb);
+      for (int kb = 0; kb < steps_k; ++kb) {
+        const Step st = step_at(i, kb);
+        ok = mbar_wait(&bars->s_full[st.buf], st.phase, a.status, 720 + st.buf);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t bl = x_lo + st.buf * (Cfg::kXBytes >> 4), al = slots + st.buf * (kTiles * 32);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          if (q < steps && ok) {
-            ok = mbar_wait(&bars->x_full[stage], phase, a.status, 720 + stage);
-            if (!ok) break;
-            const uint32_t bl = x_lo + stage * (Cfg::kXBytes >> 4);
-            const uint32_t d = step_uses[q] % kDepth, ph = (step_uses[q] / kDepth) & 1u;
+        for (int t = 0; t < kTiles; ++t)
 #pragma unroll
-            for (int t = 0; t < kTiles; ++t) {
-              const int slot = (d * 4 + q) * kTiles + t;
-              ok = ok && mbar_wait(&bars->a_full[slot], ph, a.status, 750 + slot);
-              if (!ok) break;
-              tc_fence_after();
-#pragma unroll
-              for (int k = 0; k < 4; ++k)
-                mma_ts(acc + t * BT, slots + slot * 32 + k * 8, bl + 2 * k, idesc, (sb > 0 || q > 0 || k > 0) ? 1u : 0u, lead);
-              mma_commit(&bars->a_empty[slot], lead);
-            }
-            if (!ok) break;
-            mma_commit(&bars->x_empty[stage], lead);
-            ++step_uses[q];
-            if (++stage == kXStages) { stage = 0; phase ^= 1; }
-          }
-        }
+          for (int k = 0; k < 4; ++k) mma_ts(acc + t * BT, al + t * 32 + k * 8, bl + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u, lead);
+        mma_commit(&bars->s_empty[st.buf], lead);
       }
       if (ok) {
         mma_commit(&bars->tmem_full[ab], lead);
@@ -306,23 +299,25 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     const long long sstride = a.K / 16;
     for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
       const Unit x = unit_at(u);
-      for (int sb = 0; sb < stages_k && ok; ++sb) {
+      for (int sb = 0; sb < stages_k; ++sb) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&bars->w_empty[stage], phase ^ 1, a.status, 740 + stage));
+        if (!ok) break;
+        const int steps = min(4, steps_k - 4 * sb);
+        if (lane == 0) mbar_expect_tx(&bars->w_full[stage], kWCodes);
+#pragma unroll
         for (int t = 0; t < kTiles; ++t) {
-          ok = __all_sync(0xffffffffu, mbar_wait(&bars->w_empty[stage], phase ^ 1, a.status, 740 + stage));
-          if (!ok) break;
           const int tile = x.tn * kTiles + t;
           const int row0 = x.e * a.rows + tile * (kFc1 ? 64 : 128), row1 = row0 + (kFc1 ? a.rows / 2 : 64);
           if (lane == 0) {
-            mbar_expect_tx(&bars->w_full[stage], Cfg::kCodeBytes);
-            tma_load_2d(smem_w + stage * Cfg::kCodeBytes, &tmW, &bars->w_full[stage], sb * (kMoeK / 2), row0);
-            tma_load_2d(smem_w + stage * Cfg::kCodeBytes + 64 * 128, &tmW, &bars->w_full[stage], sb * (kMoeK / 2), row1);
+            uint8_t* to = smem_w + stage * kWCodes + t * Cfg::kCodeBytes;
+            tma_load_2d(to, &tmW, &bars->w_full[stage], sb * (kMoeK / 2), row0);
+            tma_load_2d(to + 64 * 128, &tmW, &bars->w_full[stage], sb * (kMoeK / 2), row1);
           }
-          const int steps = steps_of(sb);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int r = i * 32 + lane;
             const uint8_t* src = a.s + ((r < 64 ? row0 + r : row1 + r - 64)) * sstride + sb * 16;
-            uint8_t* dst = smem_s + stage * Cfg::kScaleBytes + r * 16;
+            uint8_t* dst = smem_s + stage * kWScales + t * Cfg::kScaleBytes + r * 16;
             if (a.scale_copy == 16) {
               asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
             } else if (a.scale_copy == 4) {
@@ -332,16 +327,18 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
               for (int j = 0; j < 4 * steps; ++j) dst[j] = src[j];
             }
           }
-          if (a.scale_copy != 1)
-            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&bars->w_full[stage])) : "memory");
-          else
-            mbar_arrive(&bars->w_full[stage]);
-          if (++stage == kWStages) { stage = 0; phase ^= 1; }
         }
+        if (a.scale_copy != 1)
+          asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&bars->w_full[stage])) : "memory");
+        else
+          mbar_arrive(&bars->w_full[stage]);
+        if (++stage == kWStages) { stage = 0; phase ^= 1; }
       }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
-  } else if (warp >= 4 && warp < 8) {
+  }
+  } else if (warp < 8) {
+    moe_regs_less<64>();
     // ------------------------------ epilogue ------------------------------
     const int q4 = warp & 3;
     const uint32_t lane_addr = static_cast<uint32_t>(q4 * 32) << 16;
@@ -376,7 +373,7 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
                 g = fminf(g, a.limit);
                 up = fminf(fmaxf(up, -a.limit), a.limit);
               }
-              if (c + j < x.rows) o[j * a.n_out] = __float2half(g / (1.f + __expf(-g)) * up);
+              if (c + j < x.rows) o[j * a.n_out] = __float2half(__fdividef(g, 1.f + __expf(-g)) * up);
             }
           } else {
             __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(a.out) + static_cast<long long>(x.r0 + c0) * a.n_out + tile * 128 + q4 * 32 + lane;
@@ -391,50 +388,58 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       if (lane == 0) mbar_arrive(&bars->tmem_empty[ab]);
       if (++ab == kAccBufs) { ab = 0; aphase ^= 1; }
     }
-  } else if (warp >= 8) {
+  } else {
+    moe_regs_more<88>();
     // ------------------------------ dequant (weights) ------------------------------
     // Group q converts the q-th 64 values of every weight stage; a thread has one weight row.
     const int q = (warp - 8) >> 2, q4 = warp & 3;
     const uint32_t lane_addr = static_cast<uint32_t>(q4 * 32) << 16;
     const int row = moe_lane_row<kFc1>(q4, lane);
     const uint32_t code_at = row * 128 + (((2 * q) ^ (row & 7)) << 4), scale_at = row * 16 + q * 4;
-    int stage = 0;
-    uint32_t phase = 0, uses = 0;
+    int stage = 0, i = 0;
+    uint32_t phase = 0;
     bool ok = true;
-    for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
-      for (int sb = 0; sb < stages_k && ok; ++sb) {
-        const bool mine = q < steps_of(sb);
-        const uint32_t d = uses % kDepth, ph = (uses / kDepth) & 1u;
-#pragma unroll 1
-        for (int t = 0; t < kTiles; ++t) {
-          ok = __all_sync(0xffffffffu, mbar_wait(&bars->w_full[stage], phase, a.status, 770 + stage));
-          if (!ok) break;
-          uint32_t o[32];
-          if (mine) {
-            const uint8_t* codes = smem_w + stage * Cfg::kCodeBytes;
-            const uint4 c0 = *reinterpret_cast<const uint4*>(codes + code_at), c1 = *reinterpret_cast<const uint4*>(codes + (code_at ^ 16));
-            const uint32_t sc = *reinterpret_cast<const uint32_t*>(smem_s + stage * Cfg::kScaleBytes + scale_at);
-            __half2 s0, s1;
-            e4m3x4_to_half(sc, s0, s1);
-            moe_dequant(c0, s0, o);
-            moe_dequant(c1, s1, o + 16);
-          }
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bars->w_empty[stage]);
-          if (++stage == kWStages) { stage = 0; phase ^= 1; }
-          if (mine) {
-            const int slot = (d * 4 + q) * kTiles + t;
-            ok = __all_sync(0xffffffffu, mbar_wait(&bars->a_empty[slot], ph ^ 1, a.status, 780 + slot));
-            if (!ok) break;
-            tc_fence_after();
-            moe_tmem_st_32(tmem_slots + slot * 32 + lane_addr, o);
-            moe_tmem_st_wait();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bars->a_full[slot]);
+    for (int u = blockIdx.x; u < units && ok; u += gridDim.x, ++i) {
+      for (int sb = 0; sb < stages_k; ++sb) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&bars->w_full[stage], phase, a.status, 770 + stage));
+        if (!ok) break;
+        const bool mine = 4 * sb + q < steps_k;
+        uint4 c0[kTiles], c1[kTiles];
+        uint32_t sc[kTiles];
+        if (mine) {
+#pragma unroll
+          for (int t = 0; t < kTiles; ++t) {
+            const uint8_t* codes = smem_w + stage * kWCodes + t * Cfg::kCodeBytes;
+            c0[t] = *reinterpret_cast<const uint4*>(codes + code_at);
+            c1[t] = *reinterpret_cast<const uint4*>(codes + (code_at ^ 16));
+            sc[t] = *reinterpret_cast<const uint32_t*>(smem_s + stage * kWScales + t * Cfg::kScaleBytes + scale_at);
           }
         }
-        if (mine) ++uses;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->w_empty[stage]);
+        if (++stage == kWStages) { stage = 0; phase ^= 1; }
+        if (mine) {
+          const Step st = step_at(i, 4 * sb + q);
+#pragma unroll
+          for (int t = 0; t < kTiles; ++t) {
+            uint32_t o[32];
+            __half2 s0, s1;
+            e4m3x4_to_half(sc[t], s0, s1);
+            moe_dequant(c0[t], s0, o);
+            moe_dequant(c1[t], s1, o + 16);
+            if (t == 0) {
+              ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_empty[st.buf], st.phase ^ 1, a.status, 780 + st.buf));
+              if (!ok) break;
+              tc_fence_after();
+            }
+            moe_tmem_st_32(tmem_slots + (st.buf * kTiles + t) * 32 + lane_addr, o);
+          }
+          if (!ok) break;
+          moe_tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->s_full[st.buf]);
+        }
       }
     }
   }
