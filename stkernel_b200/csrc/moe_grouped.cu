@@ -15,14 +15,17 @@
 //
 // e2m1 x e4m3 is exact in fp16, the per-matrix fp32 scale is applied in the epilogue.
 //
-// What bounds it: weights are read once, 4.6 KB per 128 rows x 64 k, and their bytes in flight have to cover the trip to memory: the
-// ring holds 108 KB an SM and more (codes fetched into registers by the converting warps were 16 KB).  Converted weights do not pass
-// through shared memory, which carries the codes, the activations and the products' reads of them: 64 KB per 2 x 128 rows x 64 k at
-// 128 tokens, 512 cycles, what the products take.  Four groups of four dequant warps convert a quarter of a stage each.
+// What bounds it.  Few rows: memory; the bytes in flight have to cover the trip (the ring holds 108 KB an SM and more; codes fetched
+// into registers by the converting warps were 16 KB), and the issuing warp may not be in the way: a wait for a barrier that has long
+// completed takes it 70 to 95 cycles, so a K step's barriers are looked at while the step before is issued, and its products are issued by
+// one lane (N / 2 + 10 cycles each with weights in tensor memory; 82 to 90 under a lane predicate).  Many rows: a step of 2 x 128
+// weight rows x 64 k and 128 tokens is 512 tensor-core cycles, 24 KB from L2 (550 cycles when every SM asks) and 300 cycles of
+// conversion, which overlap as far as four steps in tensor memory allow.  Converted weights do not pass through shared memory.
 // Measured (hidden 4096, 2048 rows an expert, top 6; device time of the first + the second product, us; before: operands converted
 // into shared memory from codes in registers):
-//   64 tokens, 256 experts    632 + 302 before, 487 + 260 now
-//   4096 tokens, 256 experts  2409 + 1241, 1473 + 657
+//   64 tokens, 256 experts    632 + 302 before, 350 + 193 now (5.3 TB/s)
+//   4096 tokens, 256 experts  2409 + 1241, 1105 + 590
+//   4096 tokens, 32 experts   756 + 398 now (1090 TFLOP/s); one weight tile x 256 tokens a unit: 1542 us for the whole, 1310 as it is
 //
 // This is the engine's counterpart of the reference's fused W4A16 MoE kernel and, for the
 // expert-parallel layout, of its mega-MoE grouped GEMM (overlay/nvidia_model.py:227-559).
@@ -65,9 +68,9 @@ struct MoeGCfg {
   static constexpr int kBoxRows = BT < 32 ? BT : 32;                    // token rows of one activation copy
   static constexpr int kCodeBytes = 128 * 128, kScaleBytes = 128 * 16;  // of a weight tile in a stage
   static constexpr int kSteps = kMoeSlots / kTiles;                     // K steps of 64 whose operands are ready or being written
-  static constexpr int kWStages = kTiles == 2 ? (BT >= 64 ? 4 : 5) : (BT == 128 ? 4 : 8);
-  static constexpr int kXBytes = BT * 128;
-  static constexpr int kRingBytes = kWStages * kTiles * (kCodeBytes + kScaleBytes) + kSteps * kXBytes;
+  static constexpr int kXBytes = BT * 128, kXStages = BT == 128 ? 6 : 8;
+  static constexpr int kWStages = kTiles == 2 ? (BT == 128 ? 3 : BT == 16 ? 5 : 4) : (BT == 128 ? 6 : 8);
+  static constexpr int kRingBytes = kWStages * kTiles * (kCodeBytes + kScaleBytes) + kXStages * kXBytes;
   static constexpr int kAccCols = kTiles * BT;
   static constexpr int kAccBufs = 2 * kAccCols + kMoeSlots * 32 <= 512 ? 2 : 1;
   static_assert(kAccBufs * kAccCols + kMoeSlots * 32 <= 512, "tensor memory");
@@ -75,7 +78,8 @@ struct MoeGCfg {
 
 struct alignas(8) MoeGBars {
   uint64_t w_full[8], w_empty[8];
-  uint64_t s_full[kMoeSlots], s_empty[kMoeSlots];     // a step's weights (tensor memory) and activations (shared memory)
+  uint64_t x_full[8], x_empty[8];
+  uint64_t s_full[kMoeSlots], s_empty[kMoeSlots];     // a step's converted weights
   uint64_t tmem_full[2], tmem_empty[2];
   uint32_t tmem_base;
   int n_experts;                  // that have rows
@@ -110,10 +114,27 @@ __device__ __forceinline__ void moe_dequant(const uint4& codes, __half2 sc, uint
   }
 }
 
-template <int N>
-__device__ __forceinline__ void moe_regs_less() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int N>
-__device__ __forceinline__ void moe_regs_more() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+// D[tmem] (+)= A[tmem] * B[smem], in code that one lane runs.  With the operands in tensor memory a product takes N / 2 + 10 cycles this
+// way; issued by a converged warp under a lane predicate (mma_ts) it takes 82 to 90 however few columns it has.
+__device__ __forceinline__ void moe_mma(uint32_t d, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\tmov.b64 b, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n\t}"
+      ::"r"(d), "r"(a_tmem), "r"(b_lo), "r"(kDescHi), "r"(idesc), "r"(acc)
+      : "memory");
+}
+
+// Whether the phase has completed, without waiting for it
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+  return ok != 0;
+}
 
 // Row of a stage that TMEM lane 32 q4 + lane holds.  FC1: sixteen gate rows (rows 0..63 of the stage) and the up rows of the same
 // features (64..127) side by side in a warp, so that one shuffle brings a feature's two products together.
@@ -126,13 +147,13 @@ template <int BT, bool kFc1, int kTiles>
 __global__ void __launch_bounds__(kMoeThreads, 1)
 moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const MoeGArgs a) {
   using Cfg = MoeGCfg<BT, kTiles>;
-  constexpr int kWStages = Cfg::kWStages, kSteps = Cfg::kSteps, kAccBufs = Cfg::kAccBufs;
+  constexpr int kWStages = Cfg::kWStages, kXStages = Cfg::kXStages, kSteps = Cfg::kSteps, kAccBufs = Cfg::kAccBufs;
   constexpr int kWCodes = kTiles * Cfg::kCodeBytes, kWScales = kTiles * Cfg::kScaleBytes;      // of a weight stage
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* smem_w = smem;                                        // kWStages x kTiles x 16 KB of codes
-  uint8_t* smem_x = smem_w + kWStages * kWCodes;                 // kSteps x BT x 128 B
-  uint8_t* smem_s = smem_x + kSteps * Cfg::kXBytes;              // kWStages x kTiles x 2 KB of scales
+  uint8_t* smem_x = smem_w + kWStages * kWCodes;                 // kXStages x BT x 128 B
+  uint8_t* smem_s = smem_x + kXStages * Cfg::kXBytes;            // kWStages x kTiles x 2 KB of scales
   MoeGBars* bars = reinterpret_cast<MoeGBars*>(smem_s + kWStages * kWScales);
   int* first_tile = reinterpret_cast<int*>(bars + 1);            // [experts with rows + 1] token tiles of those before
   int* expert_of = first_tile + a.e_local + 1;                   // [experts with rows]
@@ -143,8 +164,12 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       mbar_init(&bars->w_full[s], 1 + 32);        // TMA arrive (+tx bytes) and the lanes that copy scales
       mbar_init(&bars->w_empty[s], 16);           // dequant warps
     }
+    for (int s = 0; s < kXStages; ++s) {
+      mbar_init(&bars->x_full[s], 1);
+      mbar_init(&bars->x_empty[s], 1);
+    }
     for (int s = 0; s < kSteps; ++s) {
-      mbar_init(&bars->s_full[s], 1 + 4);         // TMA arrive (+tx bytes) and the four warps of a dequant group
+      mbar_init(&bars->s_full[s], 4 * kTiles);    // the four warps of each tile's dequant group
       mbar_init(&bars->s_empty[s], 1);
     }
     for (int i = 0; i < 2; ++i) {
@@ -199,12 +224,17 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   const int units = first_tile[n_experts] * tiles_n;
   const int stages_k = (a.K + kMoeK - 1) / kMoeK;               // weight stages of a tile
   const int steps_k = a.K / 64;                                 // K steps of a unit
-  // K step kb of this CTA's i-th unit is the use'th of its place in a stage (kb % 4): the buffers it takes and their phase
+  // Buffers of K step kb of this CTA's i-th unit, and their phase.  Four of them: those of the step's place in a weight stage (a dequant
+  // group then sees every use of its buffers, which a wait by parity needs, also where a unit's last stage is not whole).  Eight: in turn.
   struct Step { int buf; uint32_t phase; };
   auto step_at = [&](int i, int kb) {
-    const int q = kb & 3, use = i * ((steps_k + 3 - q) >> 2) + (kb >> 2);
-    if constexpr (kSteps == 4) return Step{q, static_cast<uint32_t>(use) & 1u};
-    else return Step{(use & 1) * 4 + q, static_cast<uint32_t>(use >> 1) & 1u};
+    if constexpr (kSteps == 4) {
+      const int q = kb & 3, use = i * ((steps_k + 3 - q) >> 2) + (kb >> 2);
+      return Step{q, static_cast<uint32_t>(use) & 1u};
+    } else {
+      const int n = i * steps_k + kb;
+      return Step{n & (kSteps - 1), static_cast<uint32_t>(n / kSteps) & 1u};
+    }
   };
 
   struct Unit { int e, tn, r0, rows; };             // expert, weight tile, first row and rows of the token tile
@@ -225,15 +255,13 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     return x;
   };
 
-  // Registers follow the roles: of 768 x 80 at launch, 128 x 56 + 128 x 64 + 512 x 88
-  if (warp < 4) {
-    moe_regs_less<56>();
   if (warp == 0) {
     // ------------------------------ TMA producer (activations) ------------------------------
     if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0;
       bool ok = true;
-      int i = 0;
-      for (int u = blockIdx.x; u < units && ok; u += gridDim.x, ++i) {
+      for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
         const Unit x = unit_at(u);
         if (a.arrived != nullptr) {
           // rows of this expert come over NVLink: start as soon as they are all here (bounded wait)
@@ -250,11 +278,11 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         }
         const int boxes = (x.rows + Cfg::kBoxRows - 1) / Cfg::kBoxRows;      // only what has rows
         for (int kb = 0; kb < steps_k; ++kb) {
-          const Step st = step_at(i, kb);
-          if (!mbar_wait(&bars->s_empty[st.buf], st.phase ^ 1, a.status, 700 + st.buf)) { ok = false; break; }
-          mbar_expect_tx(&bars->s_full[st.buf], boxes * Cfg::kBoxRows * 128);
+          if (!mbar_wait(&bars->x_empty[stage], phase ^ 1, a.status, 700 + stage)) { ok = false; break; }
+          mbar_expect_tx(&bars->x_full[stage], boxes * Cfg::kBoxRows * 128);
           for (int j = 0; j < boxes; ++j)
-            tma_load_2d(smem_x + st.buf * Cfg::kXBytes + j * Cfg::kBoxRows * 128, &tmX, &bars->s_full[st.buf], kb * 64, x.r0 + j * Cfg::kBoxRows);
+            tma_load_2d(smem_x + stage * Cfg::kXBytes + j * Cfg::kBoxRows * 128, &tmX, &bars->x_full[stage], kb * 64, x.r0 + j * Cfg::kBoxRows);
+          if (++stage == kXStages) { stage = 0; phase ^= 1; }
         }
       }
     }
@@ -263,30 +291,50 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     // ------------------------------ MMA issuer ------------------------------
     const uint32_t lead = elect_one() ? 1u : 0u, tm = __shfl_sync(0xffffffffu, tmem_base, 0);
     const uint32_t slots = tm + kAccBufs * Cfg::kAccCols, x_lo = desc_lo(smem_u32(smem_x));
-    int ab = 0, i = 0;
-    uint32_t aphase = 0;
+    int ab = 0, n = 0, stage = 0;
+    uint32_t aphase = 0, xphase = 0, phases = 0;               // kSteps == 4: phase of each buffer; else buffers are taken in turn, n counts steps
     bool ok = true;
-    for (int u = blockIdx.x; u < units && ok; u += gridDim.x, ++i) {
+    for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
       const Unit x = unit_at(u);
       const uint32_t idesc = umma_idesc(0u, 0u, 128, 0) | static_cast<uint32_t>(((x.rows + 15) >> 4) << 1) << 17;   // fp16 x fp16 -> fp32
-      ok = mbar_wait(&bars->tmem_empty[ab], aphase ^ 1, a.status, 710 + ab);
+      ok = mbar_wait(&bars->tmem_empty[ab], aphase ^ 1, a.status, 705 + ab);
       if (!ok) break;
       tc_fence_after();
       const uint32_t acc = tm + ab * Cfg::kAccCols;
-      for (int kb = 0; kb < steps_k; ++kb) {
-        const Step st = step_at(i, kb);
-        ok = mbar_wait(&bars->s_full[st.buf], st.phase, a.status, 720 + st.buf);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t bl = x_lo + st.buf * (Cfg::kXBytes >> 4), al = slots + st.buf * (kTiles * 32);
+      bool ready = false;                          // the next step's barriers were seen complete while this step's products were issued
+      for (int kb0 = 0; kb0 < steps_k && ok; kb0 += 4) {
 #pragma unroll
-        for (int t = 0; t < kTiles; ++t)
+        for (int q = 0; q < 4; ++q) {
+          if (kb0 + q >= steps_k) break;
+          const int buf = kSteps == 4 ? q : n & (kSteps - 1);
+          const uint32_t phase = kSteps == 4 ? (phases >> q) & 1u : static_cast<uint32_t>(n / kSteps) & 1u;
+          if (!__all_sync(0xffffffffu, ready)) {
+            ok = mbar_wait(&bars->x_full[stage], xphase, a.status, 710 + stage) && mbar_wait(&bars->s_full[buf], phase, a.status, 720 + buf);
+            if (!ok) break;
+          }
+          const uint32_t bl = x_lo + stage * (Cfg::kXBytes >> 4), al = slots + buf * (kTiles * 32);
+          uint64_t* const x_done = &bars->x_empty[stage];
+          if (++stage == kXStages) { stage = 0; xphase ^= 1; }
+          ++n;
+          phases ^= 1u << q;
+          const int after = kSteps == 4 ? (q + 1) & 3 : n & (kSteps - 1);
+          ready = mbar_test(&bars->s_full[after], kSteps == 4 ? (phases >> after) & 1u : static_cast<uint32_t>(n / kSteps) & 1u);
+          ready = mbar_test(&bars->x_full[stage], xphase) && ready && kb0 + q + 1 < steps_k;
+          tc_fence_after();
+          if (lead) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) mma_ts(acc + t * BT, al + t * 32 + k * 8, bl + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u, lead);
-        mma_commit(&bars->s_empty[st.buf], lead);
+            for (int t = 0; t < kTiles; ++t)
+#pragma unroll
+              for (int k = 0; k < 4; ++k) moe_mma(acc + t * BT, al + t * 32 + k * 8, bl + 2 * k, idesc, (q > 0 || k > 0) ? 1u : (kb0 > 0 ? 1u : 0u));
+            umma_commit(&bars->s_empty[buf]);
+            umma_commit(x_done);
+          }
+          __syncwarp();
+        }
       }
       if (ok) {
-        mma_commit(&bars->tmem_full[ab], lead);
+        if (lead) umma_commit(&bars->tmem_full[ab]);
+        __syncwarp();
         if (++ab == kAccBufs) { ab = 0; aphase ^= 1; }
       }
     }
@@ -336,9 +384,7 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
-  }
-  } else if (warp < 8) {
-    moe_regs_less<64>();
+  } else if (warp >= 4 && warp < 8) {
     // ------------------------------ epilogue ------------------------------
     const int q4 = warp & 3;
     const uint32_t lane_addr = static_cast<uint32_t>(q4 * 32) << 16;
@@ -365,6 +411,7 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
             const bool upper = lane >= 16;
             const int c = c0 + (upper ? 8 : 0);
             __half* o = reinterpret_cast<__half*>(a.out) + static_cast<long long>(x.r0 + c) * a.n_out + tile * 64 + q4 * 16 + (lane & 15);
+            __half v[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
               const uint32_t got = __shfl_xor_sync(0xffffffffu, upper ? r[j] : r[j + 8], 16);
@@ -373,13 +420,29 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
                 g = fminf(g, a.limit);
                 up = fminf(fmaxf(up, -a.limit), a.limit);
               }
-              if (c + j < x.rows) o[j * a.n_out] = __float2half(__fdividef(g, 1.f + __expf(-g)) * up);
+              v[j] = __float2half(__fdividef(g, 1.f + __expf(-g)) * up);
+            }
+            if (c0 + 16 <= x.rows) {
+#pragma unroll
+              for (int j = 0; j < 8; ++j) o[j * a.n_out] = v[j];
+            } else {
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                if (c + j < x.rows) o[j * a.n_out] = v[j];
             }
           } else {
             __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(a.out) + static_cast<long long>(x.r0 + c0) * a.n_out + tile * 128 + q4 * 32 + lane;
+            __nv_bfloat16 v[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
-              if (c0 + j < x.rows) o[j * a.n_out] = __float2bfloat16(__uint_as_float(r[j]) * gs);
+            for (int j = 0; j < 16; ++j) v[j] = __float2bfloat16(__uint_as_float(r[j]) * gs);
+            if (c0 + 16 <= x.rows) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) o[j * a.n_out] = v[j];
+            } else {
+#pragma unroll
+              for (int j = 0; j < 16; ++j)
+                if (c0 + j < x.rows) o[j * a.n_out] = v[j];
+            }
           }
         }
       }
@@ -388,58 +451,53 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       if (lane == 0) mbar_arrive(&bars->tmem_empty[ab]);
       if (++ab == kAccBufs) { ab = 0; aphase ^= 1; }
     }
-  } else {
-    moe_regs_more<88>();
+  } else if (warp >= 8) {
     // ------------------------------ dequant (weights) ------------------------------
-    // Group q converts the q-th 64 values of every weight stage; a thread has one weight row.
-    const int q = (warp - 8) >> 2, q4 = warp & 3;
-    const uint32_t lane_addr = static_cast<uint32_t>(q4 * 32) << 16;
+    // A tile has 4 / kTiles groups of four warps, which take its K steps in turn; a thread has one weight row.  Operands are converted
+    // before their place in tensor memory is waited for.
+    constexpr int kTurns = 4 / kTiles;
+    const int group = (warp - 8) >> 2, t = group % kTiles, turn = group / kTiles, q4 = warp & 3;
+    const uint32_t to = tmem_slots + t * 32 + (static_cast<uint32_t>(q4 * 32) << 16);
     const int row = moe_lane_row<kFc1>(q4, lane);
-    const uint32_t code_at = row * 128 + (((2 * q) ^ (row & 7)) << 4), scale_at = row * 16 + q * 4;
+    const uint32_t code_at = t * Cfg::kCodeBytes + row * 128, scale_at = t * Cfg::kScaleBytes + row * 16, swap = (row & 7) << 4;
     int stage = 0, i = 0;
     uint32_t phase = 0;
     bool ok = true;
     for (int u = blockIdx.x; u < units && ok; u += gridDim.x, ++i) {
-      for (int sb = 0; sb < stages_k; ++sb) {
+      for (int sb = 0; sb < stages_k && ok; ++sb) {
         ok = __all_sync(0xffffffffu, mbar_wait(&bars->w_full[stage], phase, a.status, 770 + stage));
         if (!ok) break;
-        const bool mine = 4 * sb + q < steps_k;
-        uint4 c0[kTiles], c1[kTiles];
-        uint32_t sc[kTiles];
-        if (mine) {
 #pragma unroll
-          for (int t = 0; t < kTiles; ++t) {
-            const uint8_t* codes = smem_w + stage * kWCodes + t * Cfg::kCodeBytes;
-            c0[t] = *reinterpret_cast<const uint4*>(codes + code_at);
-            c1[t] = *reinterpret_cast<const uint4*>(codes + (code_at ^ 16));
-            sc[t] = *reinterpret_cast<const uint32_t*>(smem_s + stage * kWScales + t * Cfg::kScaleBytes + scale_at);
-          }
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bars->w_empty[stage]);
-        if (++stage == kWStages) { stage = 0; phase ^= 1; }
-        if (mine) {
-          const Step st = step_at(i, 4 * sb + q);
-#pragma unroll
-          for (int t = 0; t < kTiles; ++t) {
-            uint32_t o[32];
+        for (int j = 0; j < kTiles; ++j) {
+          const int q = j * kTurns + turn;
+          const bool mine = 4 * sb + q < steps_k;
+          uint32_t o[32];
+          if (mine) {
+            const uint8_t* codes = smem_w + stage * kWCodes + code_at;
+            const uint4 c0 = *reinterpret_cast<const uint4*>(codes + ((2 * q) << 4 ^ swap)), c1 = *reinterpret_cast<const uint4*>(codes + ((2 * q + 1) << 4 ^ swap));
+            const uint32_t sc = *reinterpret_cast<const uint32_t*>(smem_s + stage * kWScales + scale_at + q * 4);
             __half2 s0, s1;
-            e4m3x4_to_half(sc[t], s0, s1);
-            moe_dequant(c0[t], s0, o);
-            moe_dequant(c1[t], s1, o + 16);
-            if (t == 0) {
-              ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_empty[st.buf], st.phase ^ 1, a.status, 780 + st.buf));
-              if (!ok) break;
-              tc_fence_after();
-            }
-            moe_tmem_st_32(tmem_slots + (st.buf * kTiles + t) * 32 + lane_addr, o);
+            e4m3x4_to_half(sc, s0, s1);
+            moe_dequant(c0, s0, o);
+            moe_dequant(c1, s1, o + 16);
           }
-          if (!ok) break;
-          moe_tmem_st_wait();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bars->s_full[st.buf]);
+          if (j == kTiles - 1) {                                 // the last of this warp's parts of the stage
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->w_empty[stage]);
+          }
+          if (mine) {
+            const Step st = step_at(i, 4 * sb + q);
+            ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_empty[st.buf], st.phase ^ 1, a.status, 780 + st.buf));
+            if (!ok) break;
+            tc_fence_after();
+            moe_tmem_st_32(to + st.buf * (kTiles * 32), o);
+            moe_tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->s_full[st.buf]);
+          }
         }
+        if (++stage == kWStages) { stage = 0; phase ^= 1; }
       }
     }
   }

@@ -127,7 +127,10 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, ew: E
         if USE_GROUPED_GEMM and h % 64 == 0 and inter % 128 == 0 and h % 128 == 0:
             # tensor-core path: permute the activations into expert order, then two grouped GEMMs
             avg = max(1, n_pairs // max(1, total_experts or ew.num_local))
-            bt = 16 if avg <= 8 else 32 if avg <= 24 else 64 if avg <= 48 else 128
+            # Rows of an expert vary, and a second tile converts its weights again, so tiles are a few times the average.  256 experts,
+            # us with tiles of 16 / 32 / 64 / 128 rows: 5 rows on average 809 / 778; 9: 1081 / 945 / 885; 19: 1605 / 1165 / 1012 / 1063;
+            # 35: 2527 / 1605 / 1221 / 1194; 96: - / 3487 / 2259 / 1862.
+            bt = 16 if avg <= 3 else 32 if avg <= 6 else 64 if avg <= 24 else 128
             xs = scratch("moe.xs", (n_pairs + 128, h), torch.float16, dev, zero=True)
             act_p = scratch("moe.act_p", (n_pairs + 128, inter), torch.float16, dev, zero=True)
             _lib.call("stk_moe_permute", x, x.stride(0), sorted_p, offsets, ew.num_local, k, xs, n_pairs, h, st)

@@ -987,12 +987,12 @@ def test_moe_grouped_gemm_uneven_experts(H, I, E, counts):
     assert rel_err(out, ref) < 5e-3                     # activations rounded to fp16 in between, expert outputs and sums to bf16
 
 
-@pytest.mark.parametrize("H,I", [(512, 256), (384, 128), (128, 128)])
-def test_moe_grouped_gemm_scales_off_alignment(H, I):
+@pytest.mark.parametrize("H,I,E", [(512, 256, 6), (384, 128, 36), (128, 128, 6)])
+def test_moe_grouped_gemm_scales_off_alignment(H, I, E):
     """Scales whose rows or base 16- and 4-byte copies cannot take, and K that ends inside a weight stage: the same bits as the
     aligned ones give."""
     torch.manual_seed(15)
-    E, T = 6, 90
+    T = 90
     ids = torch.randint(0, E, (T, 2), dtype=torch.int32, device=dev())
     w = torch.rand(T, 2, device=dev()) + 0.5
     scale = lambda *shape: (0.05 + torch.rand(*shape, device=dev())).to(torch.float8_e4m3fn).view(torch.uint8)
