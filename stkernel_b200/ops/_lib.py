@@ -97,13 +97,26 @@ class KernelError(RuntimeError):
 
 
 launch_count = 0
+_entries: Dict[str, tuple] = {}        # name -> (function, positions of its pointer parameters)
+
+
+def _entry(name: str) -> tuple:
+    fn = getattr(lib(), name)
+    types = fn.argtypes
+    # a function that the sources do not declare may take a tensor anywhere
+    return _entries.setdefault(name, (fn, tuple(i for i, t in enumerate(types) if t is ctypes.c_void_p) if types is not None else None))
 
 
 def call(name: str, *args: Any) -> int:
     """Launch `name`; tensors become pointers.  Raises on a rejected launch."""
     global launch_count
-    fn = getattr(lib(), name)
-    conv = [a.data_ptr() if isinstance(a, torch.Tensor) else a for a in args]
+    fn, pointers = _entries.get(name) or _entry(name)
+    conv = list(args)
+    # only pointer parameters can be tensors; looking at every argument took 3.5 of the 6.2 us of a call of 23, this 1.7
+    for i in range(len(conv)) if pointers is None else pointers:
+        a = conv[i]
+        if a is not None and a.__class__ is not int and isinstance(a, torch.Tensor):
+            conv[i] = a.data_ptr()
     rc = fn(*conv)
     if rc != 0:
         raise KernelError(f"{name} returned {rc}")
@@ -112,7 +125,7 @@ def call(name: str, *args: Any) -> int:
 
 
 def query(name: str, *args: int) -> int:
-    return getattr(lib(), name)(*args)
+    return (_entries.get(name) or _entry(name))[0](*args)
 
 
 _sm_count: Dict[int, int] = {}
