@@ -3,7 +3,7 @@
 // One CTA per (query token, row split).  The row list (SWA window rows, then top-k compressed rows)
 // is walked in blocks of 128 rows:
 //
-//   producer warps   gather the 584-byte rows by slot id, dequantise fp8 x UE8M0 -> bf16 and write them
+//   producer warps   gather the 584-byte rows by slot id, dequantise fp8 x UE8M0 -> fp16 and write them
 //                    into shared memory as 8 panels of [128 rows x 64 dims], 128-byte swizzled
 //   MMA warp         S^T[row, head] = K_block . Q^T      (K panels as the K-major A operand)
 //                    O^T[dim, head] += V^T . P           (the same panels as the MN-major A operand:
@@ -11,20 +11,24 @@
 //   softmax warps    read S^T from TMEM (one row and half of the heads per thread), write P as the K-major B
 //                    operand, rescale in TMEM the columns of O whose head's maximum moved
 //
-// What bounds it: the key block (128 KB in bf16) and Q (64 KB) fill shared memory, so there is one key buffer, and a block is
+// Operands are fp16: codes times a power of two are exact, weights keep three bits more than bf16 leaves them.  A row that passes
+// fp16's range is divided by a power of two, which its scores get back, and its weights carry it to the values (`lift`).
+//
+// What bounds it: the key block (128 KB in fp16) and Q (64 KB) fill shared memory, so there is one key buffer, and a block is
 // scores -> softmax -> values in turn.  Everything else is taken off that chain:
 //   * panels change hands one by one: scores start on the first panel that has landed, and a pair of panels goes back to the
 //     producers as soon as its 128 output dims are accumulated, so the next block is written under the value products;
 //   * sixteen producer warps hold the codes of the whole next block in registers, so no gather latency is on the chain (eight
 //     warps with twice the rows each left the conversions waiting for their own results); a load instruction takes 64 contiguous
-//     bytes of eight rows, and its two stores per lane hit every bank once.  The rotated part needs no conversion: it is copied
-//     asynchronously into the panel that is freed first and scored last;
+//     bytes of eight rows, and its two stores per lane hit every bank once;
 //   * of O only the columns of the heads whose maximum moved are rescaled, one head at a time (a few of a block's 64; two at a time
-//     took 2753 us, four 2894, all of them 3182); the row sums of P stay in registers (one per head and row) and are reduced once
-//     per CTA.  The maxima themselves are exact: with one that may be stale by up to 2^8 the leading weights fall anywhere between
-//     two powers of two instead of just below 1, where bf16 rounds best -- 2525 us, and 2.8 % more error.
+//     took 2753 us, four 2894, all of them 3182), and that only in blocks where a weight would pass 2^kSlack: the others cost one
+//     look at the scores and a vote.  The row sums of P stay in registers (one per head and row) and are reduced once per CTA.
+// The value products read 6 KB of shared memory each and the next block's panels are written under them: 2500 cycles alone, 5600
+// with the writes.  A first block and the end of a token (queries, first gather, output) are 16000 cycles, a block 8800.
 // Measured (4096 tokens, 64 heads, 128 + 2048 rows): 5162 us with one thread block of thirteen warps working through
-// load -> scores -> softmax -> values without overlap, 2677 us now.
+// load -> scores -> softmax -> values without overlap, 2677 with bf16 operands, exact maxima in every block and two-byte stores of the
+// output, 2475 now; 128 rows alone: 576 -> 415.
 //
 // Accumulators live in TMEM: S (NH columns) and four O^T tiles of [128 dims x NH heads].
 // A CTA of a split writes an un-normalised partial (o, m, l) that `sparse_mla_combine` merges with the sink.
@@ -33,6 +37,7 @@
 // Replaces the reference's FlashInfer sparse-MLA decode/prefill kernels
 // (overlay/flashinfer_sparse.py:323-541).
 #define STK_PDL_CLASS 128      // bit of this file's kernels in the PDL mask (STK_PDL, stk_set_pdl_mask)
+#include "codes.cuh"
 #include "common.cuh"
 #include "pairs.cuh"
 #include "warp_reduce.cuh"
@@ -87,14 +92,11 @@ struct MlaCfg {
 };
 
 constexpr int kBarBytes = 192;
+constexpr float kSlack = 1.5f;        // powers of two by which weights may pass the maxima in use before these are taken anew
 // Order in which panels are written and scored, and in which pairs of them are summed and freed: the rotated part (panel 7)
 // is freed first and needed last.
 __device__ __forceinline__ constexpr int panel_at(int i) { return i == 0 ? 6 : i == 7 ? 7 : i - 1; }
 __device__ __forceinline__ constexpr int pair_at(int i) { return i == 0 ? 3 : i - 1; }
-
-__device__ __forceinline__ void copy16_async(void* smem_dst, const void* src, bool valid) {     // zeros where there is no row
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(smem_dst)), "l"(src), "r"(valid ? 16 : 0) : "memory");
-}
 
 template <int N>
 __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
@@ -106,7 +108,8 @@ struct alignas(8) MlaBars {
   uint64_t k_free[kPanels / 2];    // the value products of a pair of panels are done
   uint64_t s_full, p_full, pv_done;
   uint32_t tmem_base;
-  uint32_t moved[2];               // heads whose maximum this block moved, by halves of 32
+  uint32_t moved[2];               // heads whose maximum the last block that took maxima moved, by halves of 32
+  uint32_t unset[2];               // heads that have none yet
 };
 static_assert(sizeof(MlaBars) <= kBarBytes, "barrier block");
 
@@ -137,21 +140,31 @@ __device__ __forceinline__ void put16(uint32_t smem_addr, uint32_t v) {
   asm volatile("st.shared.b16 [%0], %1;" ::"r"(smem_addr), "h"(static_cast<unsigned short>(v)) : "memory");
 }
 
+// barrier `id` of n threads; whether any of them came with `pred`
+__device__ __forceinline__ bool bar_any(int id, int n, bool pred) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %3, 0;\n\t"
+      "barrier.cta.red.or.pred q, %1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r) : "r"(id), "r"(n), "r"(pred ? 1u : 0u) : "memory");
+  return r != 0;
+}
 __device__ __forceinline__ void named_bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 
-// Four e4m3 codes (one word) times a power of two -> four bf16.  (Moving the codes' bits into place and one product per pair
-// measured half this rate: shifts and logic share one pipe, which these conversions mostly leave alone.)
-__device__ __forceinline__ void e4m3x4_to_bf16(uint32_t w, uint64_t scale2, uint32_t& lo, uint32_t& hi) {
+// Eight bf16 values (16 bytes) times a power of two -> fp16
+__device__ __forceinline__ uint4 bf16x8_to_half(const uint4& v, float f) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  uint4 o;
+  __half2* oh = reinterpret_cast<__half2*>(&o);
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(i ? w >> 16 : w & 0xffff), __NV_E4M3);
-    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
-    float x, y;
-    unpack2(mul2(pack2(f.x, f.y), scale2), x, y);
-    const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
-    (i ? hi : lo) = *reinterpret_cast<const uint32_t*>(&v);
-  }
+  for (int i = 0; i < 4; ++i) oh[i] = __floats2half2_rn(__uint_as_float(w[i] << 16) * f, __uint_as_float(w[i] & 0xffff0000u) * f);
+  return o;
 }
+
+__device__ __forceinline__ uint32_t half2_bits(__half2 v) { return *reinterpret_cast<const uint32_t*>(&v); }
+
+// Larger of the magnitudes of two words of bf16 pairs, by halves (their bits order as the magnitudes do)
+__device__ __forceinline__ uint32_t bf16x2_absmax(uint32_t a, uint32_t b) { return __vmaxu2(a & 0x7fff7fffu, b & 0x7fff7fffu); }
 
 template <int NH>
 __global__ void __launch_bounds__(MlaCfg<NH>::kThreads, 1)
@@ -173,6 +186,7 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
   float* m_run = smax + 4 * NH;                          // [NH] the maxima in use, in powers of two
   float* minus_m = m_run + NH;                           // [NH] their negatives (0 for none yet)
   float* alpha_s = minus_m + NH;                         // [NH]
+  int* lift_s = reinterpret_cast<int*>(alpha_s + NH);    // [kRows] what the block's rows were divided by, in powers of two
 
   const int t = blockIdx.x, sp = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -202,6 +216,7 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
   if (threadIdx.x == 0) {
     for (int p = 0; p < 5; ++p) mbar_init(&bars->k_full[p], kProducerWarps);
     for (int j = 0; j < kPanels / 2; ++j) mbar_init(&bars->k_free[j], 1);
+    bars->unset[0] = bars->unset[1] = 0;
     mbar_init(&bars->s_full, 1);
     mbar_init(&bars->p_full, kSoftmaxWarps);
     mbar_init(&bars->pv_done, 1);
@@ -227,7 +242,7 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
   };
   auto load_q = [&]() {
     // Q -> shared memory, K-major panels [NH x 64 dims], 128-byte swizzle; heads >= nh are zero.
-    constexpr int kChunks = NH * (kD / 8), kLoaders = 32 * kSoftmaxWarps, kBatch = 8;
+    constexpr int kChunks = NH * (kD / 8), kLoaders = 32 * kSoftmaxWarps, kBatch = 16;
     for (int i0 = threadIdx.x - 128; i0 < kChunks; i0 += kLoaders * kBatch) {
       uint4 qv[kBatch];
 #pragma unroll
@@ -239,7 +254,7 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
 #pragma unroll
       for (int j = 0; j < kBatch; ++j) {
         const int i = i0 + j * kLoaders, h = i / (kD / 8), c8 = i % (kD / 8);
-        if (i < kChunks) *reinterpret_cast<uint4*>(q_s + (c8 >> 3) * (NH * 128) + h * 128 + (((c8 & 7) ^ (h & 7)) << 4)) = qv[j];
+        if (i < kChunks) *reinterpret_cast<uint4*>(q_s + (c8 >> 3) * (NH * 128) + h * 128 + (((c8 & 7) ^ (h & 7)) << 4)) = bf16x8_to_half(qv[j], 1.f);
       }
     }
     if (threadIdx.x - 128 < NH) m_run[threadIdx.x - 128] = -INFINITY;
@@ -253,8 +268,8 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
       // ------------------------------- MMA issuer -------------------------------
       const uint32_t tmem_s = bars->tmem_base, tmem_o = tmem_s + NH;
       const uint32_t lead = elect_one() ? 1u : 0u, ts = __shfl_sync(0xffffffffu, tmem_s, 0), to = __shfl_sync(0xffffffffu, tmem_o, 0);
-      constexpr uint32_t kIdescQK = umma_idesc(1u, 1u, 128, NH);
-      constexpr uint32_t kIdescPV = umma_idesc(1u, 1u, 128, NH) | (1u << 15);     // A is MN-major
+      constexpr uint32_t kIdescQK = umma_idesc(0u, 0u, 128, NH);
+      constexpr uint32_t kIdescPV = umma_idesc(0u, 0u, 128, NH) | (1u << 15);     // A is MN-major
       constexpr uint32_t kStep = kPanelBytes >> 4, kQStep = (NH * 128) >> 4;      // panels in descriptor units
       const uint32_t k_lo = desc_lo(smem_u32(k_s)), v_lo = desc_lo(smem_u32(k_s), kPanelBytes);
       const uint32_t q_lo = desc_lo(smem_u32(q_s)), p_lo = desc_lo(smem_u32(p_s));
@@ -313,7 +328,6 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
 #pragma unroll
     for (int i = 0; i < 8; ++i)
       pdst[i] = smem_u32(p_s) + (row >> 6) * (NH * 128) + (h0 + i) * 128 + ((((row & 63) >> 3) ^ i) << 4) + (row & 7) * 2;
-    const uint64_t sl22 = pack2(sl2, sl2);
     int slot = slot_of(r_begin + row);
     bool ok = true;                                       // the same in every lane; barriers are passed either way
     auto scores = [&](int c, uint32_t (&r16)[16]) {       // sixteen heads' products of this row
@@ -324,10 +338,35 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
       const uint32_t ph = b & 1;
       const bool valid = slot >= 0;
       slot = slot_of(r_begin + (b + 1) * kRows + row);
-      ok = __all_sync(0xffffffffu, ok && mbar_wait(&bars->s_full, ph, a.status, 610));
+      // (the row's power of two was left before the first panel was handed over: a barrier that has long completed)
+      ok = __all_sync(0xffffffffu, ok && mbar_wait(&bars->s_full, ph, a.status, 610) && mbar_wait(&bars->k_full[3], ph, a.status, 612));
       if (b == 0 && threadIdx.x == 128) STK_TRACE(3);
       tc_fence_after();
-      // maxima of this block's rows per head, and the running ones
+      const int lift = lift_s[row];
+      const float liftf = static_cast<float>(lift), sl = sl2 * __int_as_float((127 + lift) << 23), back = __int_as_float((127 - lift) << 23);
+      const uint64_t sl22 = pack2(sl, sl), lift2 = pack2(liftf, liftf), back2 = pack2(back, back);
+      // Whether a weight would pass 2^kSlack with the maxima in use
+      bool over = b == 0 || (bars->unset[0] | bars->unset[1]) != 0;
+      if (!over) {
+        float top = -INFINITY;
+#pragma unroll
+        for (int c = 0; c < kHeads; c += 16) {
+          uint32_t r16[16];
+          scores(c, r16);
+#pragma unroll
+          for (int i = 0; i < 16; i += 4) {
+            const ulonglong2 m4 = *reinterpret_cast<const ulonglong2*>(minus_m + h0 + c + i);
+            float x, y;
+            unpack2(fma2(pack2(__uint_as_float(r16[i]), __uint_as_float(r16[i + 1])), sl22, m4.x), x, y);
+            top = fmaxf(top, fmaxf(x, y));
+            unpack2(fma2(pack2(__uint_as_float(r16[i + 2]), __uint_as_float(r16[i + 3])), sl22, m4.y), x, y);
+            top = fmaxf(top, fmaxf(x, y));
+          }
+        }
+        over = valid && !(top + liftf <= kSlack);
+      }
+      if (bar_any(2, kSoftmaxThreads, over)) {
+      // exact maxima of this block's rows per head, and the running ones
       {
         uint32_t raw[kHeads / 16][16];
         float s[kHeads];
@@ -335,22 +374,26 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
         for (int c = 0; c < kHeads / 16; ++c) tmem_ld_32x16(tmem_s + lane_addr + h0 + 16 * c, raw[c]);
         tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < kHeads; ++i) s[i] = valid ? __uint_as_float(raw[i / 16][i % 16]) * sl2 : -INFINITY;
+        for (int i = 0; i < kHeads; ++i) s[i] = valid ? fmaf(__uint_as_float(raw[i / 16][i % 16]), sl, liftf) : -INFINITY;
         bfly_reduce_store<kHeads, true>(s, smax + q4 * NH + h0, lane);
       }
       named_bar_sync(2, kSoftmaxThreads);
       if (own < (NH < 32 ? 32 : NH)) {                     // whole warps
-        bool moved = false;
+        bool moved = false, unset = false;
         if (own < NH) {
           const float bm = fmaxf(fmaxf(smax[own], smax[NH + own]), fmaxf(smax[2 * NH + own], smax[3 * NH + own]));
           const float mo = m_run[own], mn = fmaxf(mo, bm);
           moved = mn != mo && mo != -INFINITY;
           alpha_s[own] = moved ? exp2f(mo - mn) : 1.f;
           m_run[own] = mn;
-          minus_m[own] = mn == -INFINITY ? 0.f : -mn;
+          unset = mn == -INFINITY;
+          minus_m[own] = unset ? 0.f : -mn;
         }
-        const uint32_t some = __ballot_sync(0xffffffffu, moved);
-        if (lane == 0) bars->moved[own >> 5] = some;
+        const uint32_t some = __ballot_sync(0xffffffffu, moved), none = __ballot_sync(0xffffffffu, unset);
+        if (lane == 0) {
+          bars->moved[own >> 5] = some;
+          bars->unset[own >> 5] = none;
+        }
       }
       named_bar_sync(2, kSoftmaxThreads);
       // heads whose maximum moved: their sums, and their columns of O (this block's scores were issued behind the previous block's
@@ -378,7 +421,8 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
         }
         tmem_st_wait();
       }
-      // P = exp2(s - m), bf16, written as the K-major B operand [head][row]; the sums take the rounded values
+      }
+      // P = exp2(s - m), fp16, written as the K-major B operand [head][row]; the sums take the rounded values
 #pragma unroll
       for (int c = 0; c < kHeads; c += 16) {
         uint32_t r16[16];
@@ -390,10 +434,11 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
 #pragma unroll
             for (int k = 0; k < 4; k += 2) {
               float x, y;
-              unpack2(fma2(pack2(__uint_as_float(r16[i + k]), __uint_as_float(r16[i + k + 1])), sl22, k ? m4.y : m4.x), x, y);
-              const __nv_bfloat162 p = __floats2bfloat162_rn(ex2_approx(x), ex2_approx(y));
+              unpack2(fma2(pack2(__uint_as_float(r16[i + k]), __uint_as_float(r16[i + k + 1])), sl22, add2(k ? m4.y : m4.x, lift2)), x, y);
+              const __half2 p = __floats2half2_rn(ex2_approx(x), ex2_approx(y));
               const uint32_t u = *reinterpret_cast<const uint32_t*>(&p);
-              lp[(c + i + k) / 2] = add2(lp[(c + i + k) / 2], pack2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)));
+              const float2 pf = __half22float2(p);
+              lp[(c + i + k) / 2] = fma2(pack2(pf.x, pf.y), back2, lp[(c + i + k) / 2]);
               put16(pdst[(i + k) & 7] + (c + ((i + k) & 8)) * 128, u);
               put16(pdst[(i + k + 1) & 7] + (c + ((i + k) & 8)) * 128, u >> 16);
             }
@@ -438,7 +483,11 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
       named_bar_sync(2, kSoftmaxThreads);
     }
     if (ok && a.out != nullptr) {
+      // The sums lie by dims in TMEM: they are turned in shared memory (the panels are no longer needed) and leave in one copy.  Stored
+      // two bytes a lane straight to memory, with a branch per value, they took 16000 cycles a token.
       __nv_bfloat16* orow = a.out + static_cast<long long>(t) * a.ldo;
+      const bool turned = ((reinterpret_cast<uintptr_t>(a.out) | static_cast<uintptr_t>(a.ldo * 2)) & 15) == 0;
+      const uint32_t stage = smem_u32(k_s);
       const float pos = a.positions != nullptr ? static_cast<float>(a.positions[t]) : 0.f;
 #pragma unroll 1
       for (int j = 0; j < 4; ++j) {
@@ -451,19 +500,39 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
           uint32_t r16[16];
           tmem_ld_32x16(tmem_o + j * NH + h0 + c + lane_addr, r16);
           tmem_ld_wait();
+          float v[16];
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const int h = h0 + c + i;
-            if (h < a.nh) {
-              float v = __uint_as_float(r16[i]) * alpha_s[h];
-              if (rot) {
-                // the pair (even d, d + 1) sits in neighbouring lanes
-                const float p = __shfl_xor_sync(0xffffffffu, v, 1);
-                v = (d & 1) ? (-p * sn + v * cs) : (v * cs + p * sn);
-              }
-              orow[static_cast<long long>(h) * kD + d] = __float2bfloat16(v);
+          for (int i = 0; i < 16; i += 4) {
+            const float4 f4 = *reinterpret_cast<const float4*>(alpha_s + h0 + c + i);
+            v[i] = __uint_as_float(r16[i]) * f4.x;
+            v[i + 1] = __uint_as_float(r16[i + 1]) * f4.y;
+            v[i + 2] = __uint_as_float(r16[i + 2]) * f4.z;
+            v[i + 3] = __uint_as_float(r16[i + 3]) * f4.w;
+          }
+          if (rot) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              // the pair (even d, d + 1) sits in neighbouring lanes
+              const float p = __shfl_xor_sync(0xffffffffu, v[i], 1);
+              v[i] = (d & 1) ? (-p * sn + v[i] * cs) : (v[i] * cs + p * sn);
             }
           }
+          if (turned) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) put16(stage + (h0 + c + i) * (kD * 2) + d * 2, __bfloat16_as_ushort(__float2bfloat16(v[i])));
+          } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              if (h0 + c + i < a.nh) orow[static_cast<long long>(h0 + c + i) * kD + d] = __float2bfloat16(v[i]);
+          }
+        }
+      }
+      if (turned) {
+        fence_proxy_async();
+        named_bar_sync(2, kSoftmaxThreads);
+        if (own == 0) {
+          asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(orow), "r"(stage), "r"(a.nh * kD * 2) : "memory");
+          asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group 0;" ::: "memory");
         }
       }
     } else if (ok) {
@@ -491,7 +560,7 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
     const int pw = warp - 4 - kSoftmaxWarps, l4 = lane & 3, row = 8 * pw + (lane >> 2);
     uint8_t* const line = k_s + row * 128;
     const uint32_t turn = (row & 7) << 4;
-    uint4 raw[7];
+    uint4 raw[7], rot[2];                                  // codes, and the rotated part (bf16)
     uint2 sc8;
     const uint8_t* src_row;                                // row whose codes are in `raw`; nullptr: none
     int slot_next = slot_of(r_begin + row);
@@ -511,13 +580,31 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
       raw[seg] = make_uint4(0, 0, 0, 0);
       if (src_row != nullptr) raw[seg] = __ldg(reinterpret_cast<const uint4*>(src_row + seg * 64));
     };
+    auto fetch_rot = [&]() {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        rot[i] = make_uint4(0, 0, 0, 0);
+        if (src_row != nullptr) rot[i] = __ldg(reinterpret_cast<const uint4*>(src_row + kNope + i * 64));
+      }
+    };
     next_row(0);
 #pragma unroll
     for (int i = 0; i < 7; ++i) fetch(panel_at(i));
+    fetch_rot();
     begin();
     bool ok = true;
     for (int b = 0; b < n_blocks && ok; ++b) {
       const uint2 sc = sc8;
+      // Power of two that brings the row into fp16's range: 0 unless a scale is above 2^7 (a code's magnitude is at most 448) or a
+      // rotated value above 2^16
+      const uint32_t top = __vmaxu2(__vmaxu2(sc.x & 0x00ff00ffu, (sc.x >> 8) & 0x00ff00ffu), __vmaxu2(sc.y & 0x00ff00ffu, (sc.y >> 8) & 0x000000ffu));
+      uint32_t big = __vmaxu2(__vmaxu2(bf16x2_absmax(rot[0].x, rot[0].y), bf16x2_absmax(rot[0].z, rot[0].w)),
+                              __vmaxu2(bf16x2_absmax(rot[1].x, rot[1].y), bf16x2_absmax(rot[1].z, rot[1].w)));
+      big = __vmaxu2(big, __shfl_xor_sync(0xffffffffu, big, 1));
+      big = __vmaxu2(big, __shfl_xor_sync(0xffffffffu, big, 2));
+      const int lift = max(0, max(max(static_cast<int>(top & 0xffff), static_cast<int>(top >> 16)) - 134,
+                                  (max(static_cast<int>(big & 0xffff), static_cast<int>(big >> 16)) >> 7) - 142));
+      const float back = __int_as_float((127 - lift) << 23);
 #pragma unroll
       for (int i = 0; i < kPanels; ++i) {
         const int p = panel_at(i);
@@ -525,35 +612,45 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
           ok = __all_sync(0xffffffffu, ok && mbar_wait(&bars->k_free[p >> 1], (b - 1) & 1, a.status, 620));
           if (!ok) break;
         }
-        if (i == 0) {
-          // the rotated part of this block, then where the next block's row lies
-          const uint8_t* src = src_row != nullptr ? src_row + kNope : a.swa_base;
-          copy16_async(line + 7 * kPanelBytes + ((l4 << 4) ^ turn), src, src_row != nullptr);
-          copy16_async(line + 7 * kPanelBytes + (((4 + l4) << 4) ^ turn), src_row != nullptr ? src + 64 : src, src_row != nullptr);
-          next_row(b + 1);
-        }
+        if (i == 0 && l4 == 0) lift_s[row] = lift;
+        uint4 o0, o1;
+        uint32_t at0, at1;
         if (p < 7) {
-          const float f = __uint_as_float((((p < 4 ? sc.x : sc.y) >> (8 * (p & 3))) & 0xff) << 23);      // 2^(byte - 127)
-          const uint64_t f2 = pack2(f, f);
-          uint4 o0, o1;
-          e4m3x4_to_bf16(raw[p].x, f2, o0.x, o0.y);
-          e4m3x4_to_bf16(raw[p].y, f2, o0.z, o0.w);
-          e4m3x4_to_bf16(raw[p].z, f2, o1.x, o1.y);
-          e4m3x4_to_bf16(raw[p].w, f2, o1.z, o1.w);
-          *reinterpret_cast<uint4*>(line + p * kPanelBytes + ((l4 << 5) ^ turn)) = o0;
-          *reinterpret_cast<uint4*>(line + p * kPanelBytes + (((l4 << 5) + 16) ^ turn)) = o1;
-          fetch(p);
+          const uint32_t w = p < 4 ? sc.x : sc.y;
+          const float f = __uint_as_float(((p & 3) == 3 ? w >> 1 : w << (23 - 8 * (p & 3))) & 0x7f800000u) * back;      // 2^(byte - 127 - lift)
+          const __half2 f2 = __float2half2_rn(f);
+          const uint32_t codes[4] = {raw[p].x, raw[p].y, raw[p].z, raw[p].w};
+          __half2 h[8];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            e4m3x4_to_half(codes[j], h[2 * j], h[2 * j + 1]);
+            h[2 * j] = __hmul2(h[2 * j], f2);
+            h[2 * j + 1] = __hmul2(h[2 * j + 1], f2);
+          }
+          o0 = make_uint4(half2_bits(h[0]), half2_bits(h[1]), half2_bits(h[2]), half2_bits(h[3]));
+          o1 = make_uint4(half2_bits(h[4]), half2_bits(h[5]), half2_bits(h[6]), half2_bits(h[7]));
+          at0 = (l4 << 5) ^ turn;
+          at1 = ((l4 << 5) + 16) ^ turn;
         } else {
-          asm volatile("cp.async.wait_all;" ::: "memory");
+          o0 = bf16x8_to_half(rot[0], back);
+          o1 = bf16x8_to_half(rot[1], back);
+          at0 = (l4 << 4) ^ turn;
+          at1 = ((4 + l4) << 4) ^ turn;
         }
+        *reinterpret_cast<uint4*>(line + p * kPanelBytes + at0) = o0;
+        *reinterpret_cast<uint4*>(line + p * kPanelBytes + at1) = o1;
         if (i == 0 || i == 2 || i == 4 || i == 6 || i == 7) {
           fence_proxy_async();
           __syncwarp();
           if (lane == 0) mbar_arrive(&bars->k_full[p < 6 ? p >> 1 : p - 3]);
         }
       }
+      // the next block's codes: asked for once all of this one is handed over, they arrive under its softmax
+      next_row(b + 1);
+#pragma unroll
+      for (int i = 0; i < 7; ++i) fetch(panel_at(i));
+      fetch_rot();
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
   }
 
   tc_fence_before();
@@ -567,7 +664,7 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
 
 template <int NH>
 static int launch_mla_tc(const MlaTcArgs& a, cudaStream_t st) {
-  const int smem = kPanels * kPanelBytes + kPanels * NH * 128 + 2 * NH * 128 + kBarBytes + 7 * NH * 4 + 1024;
+  const int smem = kPanels * kPanelBytes + kPanels * NH * 128 + 2 * NH * 128 + kBarBytes + 7 * NH * 4 + kRows * 4 + 1024;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(sparse_mla_tc_kernel<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)

@@ -378,6 +378,42 @@ def test_sparse_mla_matches_reference(nh, D, R_, fp8):
     assert rel_err(out2, ref2) < 1e-2
 
 
+@pytest.mark.parametrize("nh", [8, 64])
+@pytest.mark.parametrize("off", [0, 4])
+def test_sparse_mla_rows_beyond_fp16(nh, off):
+    """Rows whose scales or rotated part pass fp16's range beside ordinary ones, maxima that first rise a little and then a lot, a
+    list that ends inside a block, and an output that 16-byte copies cannot take (off).  Output rounded to bf16: 2^-9, 1.7e-3 in the
+    2-norm; 3e-3 leaves as much again for fp16 weights."""
+    D, R_, T, W, n = 512, 64, 150, 300, 512
+    g = torch.Generator().manual_seed(3)
+    rows = torch.randn(n, D, generator=g)
+    size = torch.ones(n)
+    size[1::4] = 3e4                                          # within the range, its products are not
+    size[2::4] = 1e6                                          # scales up to 2^12, rotated values above 65504
+    rows *= size[:, None]
+    rows[3::8, D - R_:] *= 1e5                                # only the rotated part
+    ccpu = C.PagedCache.allocate(n // 64, D, R_, True, "latent", "cpu")
+    ccpu.write_rows_cpu(torch.arange(n), rows)
+    kv = ccpu.read_rows_cpu(torch.arange(n))[0].double().to(dev())
+    cg = C.PagedCache(ccpu.buf.to(dev()), D, R_, True, "latent")
+    q = torch.randn(T, nh, D, generator=g).to(dev()).to(BF16)
+    order = torch.argsort(size, stable=True).to(torch.int32)                # small rows first
+    slots = order[torch.arange(W) * 512 // W].repeat(T, 1).to(dev())
+    lens = torch.full((T,), W, dtype=torch.int32, device=dev())
+    sink = torch.randn(nh, device=dev())
+    scale = 2e-7
+    buf = torch.zeros(T * nh * D + 8, dtype=BF16, device=dev())
+    out = buf[off:off + T * nh * D].view(T, nh, D)
+    _lib.call("stk_sparse_mla_tc_out", q, q.stride(0), cg.buf, cg.page_stride, cg.buf, cg.page_stride, slots, slots.stride(0), lens, None, 0,
+              None, T, nh, D, R_, W, scale, out, out.stride(0), sink, None, None, _lib.status_buffer(), _lib.stream())
+    k = kv[slots[0].long()]
+    s = q.double() @ k.t() * scale
+    p = torch.softmax(torch.cat([s, sink.double()[None, :, None].expand(T, -1, 1)], 2), 2)[:, :, :-1]
+    assert rel_err(out, p @ k) < 3e-3
+    assert float(buf[:off].abs().sum()) == 0 and float(buf[off + T * nh * D:].abs().sum()) == 0
+    _lib.check_status()
+
+
 @pytest.mark.parametrize("nh", [8, 32, 64])
 def test_sparse_mla_weights_are_relative_to_the_exact_maximum(nh):
     """Weights relative to the largest: 1 and 3/4 are bf16 numbers, so two leading rows 3 x and -4 x in the last block cancel whatever
