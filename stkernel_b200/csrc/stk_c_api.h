@@ -121,6 +121,7 @@ int stk_token_maps(const int* query_start, const int* req_rows, const int* start
 int stk_mhc_pick_splits(int T, int HC);
 int stk_mhc_dots(const void* x, const float* fn, float* partial, int T, int H, int hc, int n_mix, int n_splits, void* stream);
 int stk_mhc_finalize(const void* x, const float* partial, int n_splits, int partial_ld, int sumsq_in_partial, const float* base, const float* scale, const void* norm_w, float* post, float* comb, void* y, int T, int H, int hc, float rms_eps, float hc_eps, int sinkhorn_iters, float post_mult, int mode, void* q_out, float* q_scale, int q_scale_ld, void* stream);
+int stk_mhc_finalize_rows(const void* x, const float* prod, int prod_ld, int lo_at, const float* base, const float* scale, const void* norm_w, float* post, float* comb, void* y, int T, int H, int hc, float rms_eps, float hc_eps, int sinkhorn_iters, float post_mult, void* stream);
 int stk_mhc_post(const void* x, const void* res, const float* post, const float* comb, void* out, int T, int H, int hc, void* stream);
 int stk_mhc_cluster(const void* x, const float* fn, const float* base, const float* scale, const void* norm_w, float* post, float* comb, void* y, int T, int H, int hc, int n_mix, float rms_eps, float hc_eps, int sinkhorn_iters, float post_mult, int mode, void* stream);
 int stk_mhc_post_pre(const void* fa, const void* res_old, const float* post_old, const float* comb_old, void* x_out, const float* fn, const float* base, const float* scale, const void* norm_w, float* post, float* comb, void* y, int T, int H, int hc, int n_mix, float rms_eps, float hc_eps, int sinkhorn_iters, float post_mult, int mode, void* stream);

@@ -505,6 +505,14 @@ def mhc_pre(residual: torch.Tensor, fn: torch.Tensor, base: torch.Tensor, scale:
             cnt = scratch("gemm.counters", (4096,), torch.int32, dev, zero=True)
         _lib.call("stk_gemm_tile", wcat, wcat.stride(0), x2d, x2d.stride(0), prod, 128, t, 128, hc * h, 1, 32, splits, ws, cnt,
                   _lib.status_buffer(), _lib.sm_count(), _lib.stream())
+        if hc == 4 and h % 8 == 0 and h <= 8192 and not quant and residual.data_ptr() % 16 == 0 and (norm_w is None or norm_w.data_ptr() % 16 == 0):
+            # whole rows in 16-byte parts: the squares are summed where the streams are read anyway
+            y = torch.empty(t, h, dtype=BF16, device=dev)
+            post = torch.empty(t, hc, dtype=F32, device=dev)
+            comb = torch.empty(t, hc * hc, dtype=F32, device=dev)
+            _lib.call("stk_mhc_finalize_rows", residual, prod, 128, 32, base, scale, norm_w, post, comb, y, t, h, hc, rms_eps, hc_eps,
+                      iters, 2.0, _lib.stream())
+            return y, post, comb
         partial = scratch("mhc.partial", (t * (n_mix + 1),), F32, dev).view(t, n_mix + 1)
         torch.add(prod[:, :n_mix], prod[:, 32:32 + n_mix], out=partial[:, :n_mix])
         _lib.call("stk_row_sumsq", x2d, x2d.stride(0), partial[:, n_mix:], n_mix + 1, t, hc * h, _lib.stream())

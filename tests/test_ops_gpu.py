@@ -136,6 +136,57 @@ def test_mhc_pre_post_head(T, H):
     assert rel_err(hh, R.hc_head(res, hfn, hb, hs, 1e-6, 1e-6)) < 5e-3
 
 
+@pytest.mark.parametrize("H", [272, 2064, 6144])
+@pytest.mark.parametrize("norm", [True, False])
+def test_mhc_pre_in_whole_rows(H, norm):
+    """Widths that end inside a thread block's pass, and of one, two and four passes; without a norm behind the sum."""
+    torch.manual_seed(2)
+    T, hc = 259, 4
+    res = torch.randn(T, hc, H, device=dev()).to(BF16)
+    fn = torch.randn(24, hc * H, device=dev()) * 0.02
+    base, scale = torch.randn(24, device=dev()) * 0.1, torch.tensor([1.0, 0.7, 1.3], device=dev())
+    nw = (1 + 0.1 * torch.randn(H, device=dev())).to(BF16) if norm else None
+    y, post, comb = Fn.mhc_pre(res, fn, base, scale, nw, 1e-6, 1e-6, 20)
+    yr, pr, cr = R.mhc_pre(res, fn, base, scale, nw, 1e-6, 1e-6, 20, round_bf16=True)
+    assert rel_err(y, yr) < 5e-3                          # two roundings to bf16
+    assert torch.allclose(post, pr, atol=1e-4, rtol=1e-4) and torch.allclose(comb.view(T, hc, hc), cr, atol=1e-4, rtol=1e-3)
+    x = torch.randn(T, H, device=dev()).to(BF16)
+    assert rel_err(Fn.mhc_post(x, res, post, comb), R.mhc_post(x, res, pr, cr)) < 5e-3
+
+
+@pytest.mark.parametrize("n,e_local,start", [(2049, 300, 0), (5000, 37, 3), (24576, 256, 0)])
+def test_moe_align_many_pairs(n, e_local, start):
+    """Chunks and experts that fill neither a batch of counts nor a warp; pairs of other ranks' experts."""
+    g = torch.Generator().manual_seed(n)
+    ids = torch.randint(0, e_local + 5, (n,), generator=g, dtype=torch.int32)
+    sorted_p, sorted_e, pair_row = (torch.full((n,), -7, dtype=torch.int32, device=dev()) for _ in range(3))
+    offsets = torch.empty(e_local + 1, dtype=torch.int32, device=dev())
+    counts = torch.empty((n + 255) // 256 * e_local, dtype=torch.int32, device=dev())
+    _lib.call("stk_moe_align", ids.to(dev()), n, start, e_local, sorted_p, pair_row, offsets, sorted_e, counts, _lib.stream())
+    local = ids - start
+    mine = (local >= 0) & (local < e_local)
+    order = torch.argsort(torch.where(mine, local, e_local), stable=True)[:int(mine.sum())]
+    assert torch.equal(sorted_p.cpu()[:order.numel()], order.to(torch.int32))
+    assert torch.equal(sorted_e.cpu()[:order.numel()], local[order])
+    assert torch.equal(offsets.cpu()[1:], torch.bincount(local[mine].long(), minlength=e_local).cumsum(0).to(torch.int32))
+    want = torch.full((n,), -1, dtype=torch.int32)
+    want[order] = torch.arange(order.numel(), dtype=torch.int32)
+    assert torch.equal(pair_row.cpu(), want)
+
+
+@pytest.mark.parametrize("topk", [1, 8, 9, 16])
+def test_moe_combine_places(topk):
+    torch.manual_seed(topk)
+    T, H = 70, 1096
+    y, w = torch.randn(T * topk, H, device=dev()).to(BF16), torch.rand(T, topk, device=dev())
+    rows = torch.randperm(T * topk).to(torch.int32).to(dev())
+    rows[::5] = -1
+    shared, out = torch.randn(T, H, device=dev()).to(BF16), torch.empty(T, H, dtype=BF16, device=dev())
+    _lib.call("stk_moe_combine", y, w, rows, shared, out, T, H, topk, None, _lib.stream())
+    picked = torch.where(rows[:, None] >= 0, y.double()[rows.clamp(min=0).long()], 0.0).view(T, topk, H)
+    assert rel_err(out, (picked * w.double()[:, :, None]).sum(1) + shared.double()) < 2.5e-3      # rounded to bf16 once
+
+
 @pytest.mark.parametrize("T,H", [(1, 4096), (5, 4096), (16, 1024), (40, 512)])
 def test_mhc_post_pre_fused(T, H):
     """Post-mix of one sub-block fused into the next pre-mix (one cluster launch for T <= 16) against the two
