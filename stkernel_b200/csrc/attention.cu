@@ -192,49 +192,80 @@ sparse_mla_split_kernel(MlaArgs a) {
   }
 }
 
-// grid (T, nh); merges splits, adds the sink to the denominator, optionally applies the inverse
-// RoPE on the last R dims (the rotation the output projection expects), writes bf16.
-__global__ void sparse_mla_combine_kernel(const float* __restrict__ partial, const float* __restrict__ sink,
-                                          __nv_bfloat16* __restrict__ out, long long ldo, int nh, int D, int n_splits,
-                                          const int64_t* __restrict__ positions, const float* __restrict__ inv_freq,
-                                          int R) {
+// A warp per (token, head): merges splits, adds the sink to the denominator, optionally applies the inverse RoPE on the last R dims
+// (the rotation the output projection expects), writes bf16.  The splits' maxima and sums are read by a lane each and their weights
+// handed round; a lane's parts of a split's row are all asked for at once, two splits at a time.  Measured (64 tokens x 64 heads, 2
+// splits of 512 dims, 17 MB): 10.6 us with a thread block per head that read the maxima again for every pair of dims, 5 now.
+constexpr int kCombineWarps = 4;
+__global__ void __launch_bounds__(32 * kCombineWarps)
+sparse_mla_combine_kernel(const float* __restrict__ partial, const float* __restrict__ sink, __nv_bfloat16* __restrict__ out,
+                          long long ldo, int T, int nh, int D, int n_splits, const int64_t* __restrict__ positions,
+                          const float* __restrict__ inv_freq, int R) {
   pdl_wait();
   pdl_trigger();
-  const int t = blockIdx.x, h = blockIdx.y;
+  const int w = blockIdx.x * kCombineWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (w >= T * nh) return;
+  const int t = w / nh, h = w - t * nh;
   const float* base = partial + (static_cast<long long>(t) * n_splits * nh + h) * (D + 2);
   const long long sstride = static_cast<long long>(nh) * (D + 2);
-  float M = sink ? sink[h] : -INFINITY;
-  for (int s = 0; s < n_splits; ++s) M = fmaxf(M, base[s * sstride + D]);
-  float denom = sink ? __expf(sink[h] - M) : 0.f;
-  for (int s = 0; s < n_splits; ++s) {
+  const float sk = sink ? sink[h] : -INFINITY;
+  float M = sk;
+  for (int s = lane; s < n_splits; s += 32) M = fmaxf(M, base[s * sstride + D]);
+  M = warp_max(M);
+  float denom = 0.f;
+  for (int s = lane; s < n_splits; s += 32) {
     const float ms = base[s * sstride + D];
     if (ms != -INFINITY) denom += base[s * sstride + D + 1] * __expf(ms - M);
   }
+  denom = warp_sum(denom) + (sink ? __expf(sk - M) : 0.f);
   const float inv = denom > 0.f ? 1.f / denom : 0.f;
   const int nope = D - R;
   const float pos = positions ? static_cast<float>(positions[t]) : 0.f;
-  for (int d = threadIdx.x * 2; d < D; d += blockDim.x * 2) {
-    float o0 = 0.f, o1 = 0.f;
-    for (int s = 0; s < n_splits; ++s) {
-      const float ms = base[s * sstride + D];
-      if (ms != -INFINITY) {
-        const float w = __expf(ms - M);
-        o0 = fmaf(base[s * sstride + d], w, o0);
-        o1 = fmaf(base[s * sstride + d + 1], w, o1);
+  constexpr int kPairs = 8;                              // pairs of dims of a lane in a pass of 512
+  for (int d0 = 0; d0 < D; d0 += 64 * kPairs) {
+    float2 o[kPairs];
+#pragma unroll
+    for (int i = 0; i < kPairs; ++i) o[i] = make_float2(0.f, 0.f);
+    for (int s0 = 0; s0 < n_splits; s0 += 2) {
+      float2 v[2][kPairs];
+      float ws[2];
+#pragma unroll
+      for (int z = 0; z < 2; ++z) {
+        const float* row = base + (s0 + z) * sstride;
+        const bool there = s0 + z < n_splits;
+        const float ms = there ? row[D] : -INFINITY;
+        ws[z] = ms != -INFINITY ? __expf(ms - M) : 0.f;
+#pragma unroll
+        for (int i = 0; i < kPairs; ++i) {
+          const int d = d0 + 64 * i + 2 * lane;
+          v[z][i] = make_float2(0.f, 0.f);
+          if (ms != -INFINITY && d < D) v[z][i] = *reinterpret_cast<const float2*>(row + d);
+        }
       }
+#pragma unroll
+      for (int z = 0; z < 2; ++z)
+#pragma unroll
+        for (int i = 0; i < kPairs; ++i) {
+          o[i].x = fmaf(v[z][i].x, ws[z], o[i].x);
+          o[i].y = fmaf(v[z][i].y, ws[z], o[i].y);
+        }
     }
-    o0 *= inv;
-    o1 *= inv;
-    if (positions != nullptr && d >= nope) {
-      // rotated in 32 bits: one rounding, where a separate rotation would read a stored bf16 output and round again
-      float sn, cs;
-      sincosf(pos * inv_freq[(d - nope) >> 1], &sn, &cs);
-      const float x = o0 * cs + o1 * sn;
-      const float y = -o0 * sn + o1 * cs;
-      o0 = x;
-      o1 = y;
+#pragma unroll
+    for (int i = 0; i < kPairs; ++i) {
+      const int d = d0 + 64 * i + 2 * lane;
+      if (d >= D) continue;
+      float o0 = o[i].x * inv, o1 = o[i].y * inv;
+      if (positions != nullptr && d >= nope) {
+        // rotated in 32 bits: one rounding, where a separate rotation would read a stored bf16 output and round again
+        float sn, cs;
+        sincosf(pos * inv_freq[(d - nope) >> 1], &sn, &cs);
+        const float x = o0 * cs + o1 * sn;
+        const float y = -o0 * sn + o1 * cs;
+        o0 = x;
+        o1 = y;
+      }
+      *reinterpret_cast<__nv_bfloat162*>(out + t * ldo + static_cast<long long>(h) * D + d) = __floats2bfloat162_rn(o0, o1);
     }
-    *reinterpret_cast<__nv_bfloat162*>(out + t * ldo + static_cast<long long>(h) * D + d) = __floats2bfloat162_rn(o0, o1);
   }
 }
 
@@ -295,8 +326,8 @@ STK_API int stk_sparse_mla(const void* q, long long ldt, const void* swa_cache, 
     default: return -2;
   }
 #undef STK_MLA
-  dim3 g2(T, nh);
-  launch_pdl(sparse_mla_combine_kernel, dim3(g2), dim3(128), 0, st, workspace, sink, (__nv_bfloat16*)out, ldo, nh, D, n_splits, nullptr, nullptr, 0);
+  launch_pdl(sparse_mla_combine_kernel, dim3((T * nh + kCombineWarps - 1) / kCombineWarps), dim3(32 * kCombineWarps), 0, st, workspace, sink,
+             (__nv_bfloat16*)out, ldo, T, nh, D, n_splits, nullptr, nullptr, 0);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
@@ -305,8 +336,7 @@ STK_API int stk_sparse_mla_combine(const float* workspace, const float* sink, vo
                                    void* stream) {
   if (T <= 0) return 0;
   if (D % 2) return -1;
-  dim3 g2(T, nh);
-  launch_pdl(sparse_mla_combine_kernel, dim3(g2), dim3(128), 0, (cudaStream_t)stream, workspace, sink, (__nv_bfloat16*)out, ldo, nh, D, n_splits,
-                                                                  positions, inv_freq, R);
+  launch_pdl(sparse_mla_combine_kernel, dim3((T * nh + kCombineWarps - 1) / kCombineWarps), dim3(32 * kCombineWarps), 0, (cudaStream_t)stream,
+             workspace, sink, (__nv_bfloat16*)out, ldo, T, nh, D, n_splits, positions, inv_freq, R);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }

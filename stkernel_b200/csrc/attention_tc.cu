@@ -543,9 +543,15 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
           uint32_t r16[16];
           tmem_ld_32x16(tmem_o + j * NH + h0 + c + lane_addr, r16);
           tmem_ld_wait();
+          float* o = prow + (h0 + c) * (kD + 2) + j * 128 + row;
+          if (h0 + c + 16 <= a.nh) {                       // without a branch per value
 #pragma unroll
-          for (int i = 0; i < 16; ++i)
-            if (h0 + c + i < a.nh) prow[(h0 + c + i) * (kD + 2) + j * 128 + row] = __uint_as_float(r16[i]);
+            for (int i = 0; i < 16; ++i) o[i * (kD + 2)] = __uint_as_float(r16[i]);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              if (h0 + c + i < a.nh) o[i * (kD + 2)] = __uint_as_float(r16[i]);
+          }
         }
       }
       if (own < a.nh) {
