@@ -195,7 +195,7 @@ sparse_mla_split_kernel(MlaArgs a) {
 // A warp per (token, head): merges splits, adds the sink to the denominator, optionally applies the inverse RoPE on the last R dims
 // (the rotation the output projection expects), writes bf16.  The splits' maxima and sums are read by a lane each and their weights
 // handed round; a lane's parts of a split's row are all asked for at once, two splits at a time.  Measured (64 tokens x 64 heads, 2
-// splits of 512 dims, 17 MB): 10.6 us with a thread block per head that read the maxima again for every pair of dims, 5 now.
+// splits of 512 dims, 17 MB): 10.6 us with a thread block per head that read the maxima again for every pair of dims, 7.5 now.
 constexpr int kCombineWarps = 4;
 __global__ void __launch_bounds__(32 * kCombineWarps)
 sparse_mla_combine_kernel(const float* __restrict__ partial, const float* __restrict__ sink, __nv_bfloat16* __restrict__ out,

@@ -1085,6 +1085,238 @@ gemm_fp8_tokens_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
 }
 
 // ---------------------------------------------------------------------------------
+// fp8, a pair of CTAs on 256 tokens x 256 weight rows: each holds 128 tokens and half of the weight rows of a K block, one product of
+// the pair reads both halves (cta_group::2), and each CTA's accumulators are its own tokens x all 256 weight rows.
+//
+// What bounds it: the single CTAs above fetch 32 KB of operands per 128 x 128 x 128 products, 2.1 GB for 4096 x 4096 x 8192, near the
+// 12 TB/s that L2 gives; a pair fetches the same 32 KB per CTA for twice the products (512 tensor-core cycles).  Each epilogue warp
+// adds 128 columns to its fp32 sums in that time, 360 cycles and as much again for hand-overs; packed multiply-adds took 760.  Large
+// products meet the power limit first.
+// ---------------------------------------------------------------------------------
+constexpr int kPairStages = 6, kPairStageBytes = 2 * 128 * 128;
+constexpr int kPairThreads = 384;      // four warps that issue, eight that add up; registers follow (of 384 x 168: 128 x 40 + 256 x 232)
+
+struct alignas(8) PairBars {
+  uint64_t full[6], empty[6], tmem_full[2], tmem_empty[2];
+  uint32_t tmem_base;
+};
+
+// Copy into this CTA's shared memory whose bytes count on a barrier of the pair's first CTA
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t smem_dst, const void* tmap, uint32_t bar, int x, int y) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void mma_pair_f8(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t acc, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+      "mov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], a, b, %4, p;\n\t}"
+      ::"r"(d), "r"(a_lo), "r"(b_lo), "r"(kDescHi), "r"(idesc), "r"(acc), "r"(lead)
+      : "memory");
+}
+// The barrier at this offset in both CTAs of the pair counts one arrival when the products issued so far are done.
+__device__ __forceinline__ void mma_commit_pair(uint64_t* bar, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t.reg .b16 both;\n\tsetp.ne.b32 q, %1, 0;\n\tmov.b16 both, 3;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], both;\n\t}"
+      ::"r"(smem_u32(bar)), "r"(lead) : "memory");
+}
+// (What these arrivals order is reads of tensor memory, which the fence in front of them covers; with cluster-wide release they waited
+// for the scales in flight, 1300 cycles a K block.)
+__device__ __forceinline__ void mbar_arrive_at(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// Whether the phase has completed, without waiting for it
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+  return ok != 0;
+}
+
+__global__ void __launch_bounds__(kPairThreads, 1)
+gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const Fp8Args a) {
+  constexpr int kCols = 128;                             // weight rows of an epilogue warp
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  PairBars* bars = reinterpret_cast<PairBars*>(smem + kPairStages * kPairStageBytes);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = blockIdx.x & 1u;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kPairStages; ++i) {
+      mbar_init(&bars->full[i], 1);
+      mbar_init(&bars->empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&bars->tmem_full[i], 1);
+      mbar_init(&bars->tmem_empty[i], 16);             // epilogue warps of both CTAs
+    }
+    fence_barrier_init();
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem_base)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmX);
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();                                    // the other CTA's barriers are ready
+  tc_fence_after();
+  const uint32_t tmem_base = bars->tmem_base;
+  pdl_wait();
+  pdl_trigger();
+  const int units = a.tiles_t * a.tiles_n;
+  const int u_first = blockIdx.x >> 1, u_step = gridDim.x >> 1;
+
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    if (warp == 0) {
+      // ------------------------------ TMA producer: this CTA's tokens and half of the weight rows ------------------------------
+      if (lane == 0) {
+        int stage = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int u = u_first; u < units && ok; u += u_step) {
+          const int tt = u % a.tiles_t, tn = u / a.tiles_t;
+          for (int kb = 0; kb < a.k_blocks; ++kb) {
+            if (!mbar_wait(&bars->empty[stage], phase ^ 1, a.status, 100 + stage)) { ok = false; break; }
+            if (rank == 0) mbar_expect_tx(&bars->full[stage], 2 * kPairStageBytes);
+            const uint32_t st = smem_u32(smem + stage * kPairStageBytes), full = peer_addr(smem_u32(&bars->full[stage]), 0);
+            tma_load_2d_pair(st, &tmX, full, kb * 128, tt * 256 + rank * 128);
+            tma_load_2d_pair(st + 128 * 128, &tmW, full, kb * 128, tn * 256 + rank * 128);
+            if (++stage == kPairStages) { stage = 0; phase ^= 1; }
+          }
+        }
+      }
+    } else if (warp == 1 && rank == 0) {
+      // ------------------------------ MMA issuer (first CTA) --------------------------------
+      const uint32_t lead = elect_one() ? 1u : 0u, tm = __shfl_sync(0xffffffffu, tmem_base, 0), s_lo = desc_lo(smem_u32(smem));
+      constexpr uint32_t kIdesc = umma_idesc(0u, 0u, 256, 256);
+      const long long total = units > u_first ? ((units - 1 - u_first) / u_step + 1LL) * a.k_blocks : 0;
+      int stage = 0, ab = 0;
+      uint32_t phase = 0, aphase = 0;
+      for (long long i = 0; i < total; ++i) {
+        if (!mbar_wait(&bars->full[stage], phase, a.status, 300 + stage) || !mbar_wait(&bars->tmem_empty[ab], aphase ^ 1, a.status, 200 + ab)) break;
+        tc_fence_after();
+        const uint32_t st = s_lo + stage * (kPairStageBytes >> 4), d = tm + ab * 256;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) mma_pair_f8(d, st + 2 * k, st + 1024 + 2 * k, kIdesc, k > 0 ? 1u : 0u, lead);
+        mma_commit_pair(&bars->tmem_full[ab], lead);
+        mma_commit_pair(&bars->empty[stage], lead);
+        if (++stage == kPairStages) { stage = 0; phase ^= 1; }
+        if (++ab == 2) { ab = 0; aphase ^= 1; }
+      }
+    }
+    __syncwarp();
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
+    // ------------------------------ epilogue: a thread owns one token and kCols weight rows -----------------------------------
+    const int q = warp & 3, col0 = ((warp - 4) >> 2) * kCols;
+    const uint32_t tile = tmem_base + col0 + (static_cast<uint32_t>(q * 32) << 16);
+    const uint32_t empty0 = peer_addr(smem_u32(&bars->tmem_empty[0]), 0);
+    int ab = 0;
+    uint32_t aphase = 0;
+    bool ok = true, ready = false;
+    for (int u = u_first; u < units && ok; u += u_step) {
+      const int tt = u % a.tiles_t, tn = u / a.tiles_t;
+      const int t0 = tt * 256 + static_cast<int>(rank) * 128 + q * 32, t = t0 + lane, n0 = tn * 256 + col0;
+      const bool t_ok = t < a.T;
+      const bool live = t0 < a.T && n0 < a.N;             // some lane of this warp has a token, some column a weight row
+      const float* xs = a.x_scale + (t_ok ? t : 0);
+      const float* ws = a.w_scale + (live ? static_cast<long long>(n0 / 128) * a.w_scale_ld : 0LL);
+      constexpr int kAhead = 4;
+      float sx[kAhead], sw[kAhead];
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) {
+        const int kb = min(i, a.k_blocks - 1);
+        sx[i] = __ldg(xs + static_cast<long long>(kb) * a.x_scale_ld);
+        sw[i] = __ldg(ws + kb);
+      }
+      float acc[kCols];
+#pragma unroll
+      for (int j = 0; j < kCols; ++j) acc[j] = 0.f;
+      for (int kb0 = 0; kb0 < a.k_blocks && ok; kb0 += kAhead) {
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) {
+          const int kb = kb0 + i;
+          if (kb >= a.k_blocks || !ok) break;
+          const float s = sx[i] * sw[i];
+          const int next = min(kb + kAhead, a.k_blocks - 1);
+          sx[i] = __ldg(xs + static_cast<long long>(next) * a.x_scale_ld);
+          sw[i] = __ldg(ws + next);
+          if (!__all_sync(0xffffffffu, ready)) {
+            ok = __all_sync(0xffffffffu, mbar_wait(&bars->tmem_full[ab], aphase, a.status, 400 + ab));
+            if (!ok) break;
+          }
+          tc_fence_after();
+          if (live) {
+#pragma unroll
+            for (int c = 0; c < kCols; c += 64) {
+              uint32_t r[2][32];
+              tmem_ld_32x32(tile + ab * 256 + c, r[0]);
+              tmem_ld_32x32(tile + ab * 256 + c + 32, r[1]);
+              tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < 64; ++j) acc[c + j] = fmaf(__uint_as_float(r[j / 32][j % 32]), s, acc[c + j]);
+            }
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_at(empty0 + ab * 8);
+          if (++ab == 2) { ab = 0; aphase ^= 1; }
+          ready = mbar_test(&bars->tmem_full[ab], aphase);
+        }
+      }
+      if (ok && t_ok) {
+        const bool aligned = (reinterpret_cast<uintptr_t>(a.out) & 15) == 0 && a.ldo % (a.out_fp32 ? 4 : 8) == 0;
+        if (aligned && n0 + kCols <= a.N) {
+#pragma unroll
+          for (int c = 0; c < kCols; c += 8) {
+            const float* v = acc + c;
+            const long long o0 = static_cast<long long>(t) * a.ldo + n0 + c;
+            if (a.out_fp32) {
+              float* o = reinterpret_cast<float*>(a.out) + o0;
+              *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
+              *reinterpret_cast<float4*>(o + 4) = make_float4(v[4], v[5], v[6], v[7]);
+            } else {
+              uint4 ov;
+              __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&ov);
+#pragma unroll
+              for (int i = 0; i < 4; ++i) oh[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+              *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.out) + o0) = ov;
+            }
+          }
+        } else {
+#pragma unroll
+          for (int c = 0; c < kCols; ++c) {
+            if (n0 + c < a.N) {
+              const long long o = static_cast<long long>(t) * a.ldo + n0 + c;
+              if (a.out_fp32) reinterpret_cast<float*>(a.out)[o] = acc[c];
+              else reinterpret_cast<__nv_bfloat16*>(a.out)[o] = __float2bfloat16(acc[c]);
+            }
+          }
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();                                    // nobody reads this CTA's operands or arrives at its barriers any more
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+  }
+}
+
+// ---------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -1185,6 +1417,17 @@ static int launch_fp8_tokens(const CUtensorMap& tx, const CUtensorMap& tw, const
   return launch_cluster(gemm_fp8_tokens_kernel<S>, S, S > 1 ? units * S : units < sm_count ? units : sm_count, kFp8Threads, smem, st, tx, tw, a);
 }
 
+static int launch_fp8_pair(const CUtensorMap& tx, const CUtensorMap& tw, const Fp8Args& a, int sm_count, cudaStream_t st) {
+  constexpr int smem = kPairStages * kPairStageBytes + static_cast<int>(sizeof(PairBars)) + 1024;
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(gemm_fp8_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -3;
+    configured = true;
+  }
+  const int units = a.tiles_t * a.tiles_n, pairs = sm_count / 2;
+  return launch_cluster(gemm_fp8_pair_kernel, 2, 2 * (units < pairs ? units : pairs), kPairThreads, smem, st, tx, tw, a);
+}
+
 }  // namespace stk
 
 using namespace stk;
@@ -1265,6 +1508,19 @@ static int fp8_tokens_split(int T, int N, int K, int sm_count) {
   return s > 1 || T >= 48 ? s : 0;
 }
 
+// Whether pairs of CTAs take a product that the single CTAs above would take without splitting K.  A round of pairs does the work of two
+// rounds of single CTAs in 1.62 to 1.92 times the time of one, so they are taken where they need no more than half the rounds.
+// Measured, us, single / pair (rounds): 512 tokens x 16384 x 4096: 59 / 50 (4 / 2);  3000 x 4096 x 4096: 84 / 70 (6 / 3);
+//   4096 x 1024 x 8192: 55 / 46 (2 / 1);  4096 x 40960 x 1536: 456 / 424 (70 / 35);  1500 x 4096 x 8192: 79 / 86 (3 / 2);
+//   4096 x 4096 x 8192: 176 / 192 (7 / 4): at K = 8192 both run into the power limit (1.3 to 1.5 GHz).
+static bool fp8_pair_serves(int T, int N, int sm_count) {
+  const int pairs = sm_count / 2;
+  if (pairs < 1) return false;
+  const long long single = (static_cast<long long>((T + 127) / 128) * ((N + 127) / 128) + sm_count - 1) / sm_count;
+  const long long paired = (static_cast<long long>((T + 255) / 256) * ((N + 255) / 256) + pairs - 1) / pairs;
+  return 2 * paired <= single;
+}
+
 // Which token-major tiles a plain product (one block, no fused collective) without workspace splits takes: the number of CTAs that
 // share one, or 0 for the 128-row tiles.
 STK_API int stk_gemm_token_tile_ctas(int T, int N, int K, int is_fp8, int sm_count) {
@@ -1300,6 +1556,11 @@ static int gemm_launch(const void* W, long long ldw, const void* X, long long ld
     a.status = status;
     a.tiles_t = (T + 127) / 128;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    if (tokens_split == 1 && fp8_pair_serves(T, N, sm_count)) {
+      a.tiles_t = (T + 255) / 256;
+      a.tiles_n = (N + 255) / 256;
+      return launch_fp8_pair(ta, tb, a, sm_count, st);
+    }
     switch (tokens_split) {
       case 4: return launch_fp8_tokens<4>(ta, tb, a, sm_count, st);
       case 2: return launch_fp8_tokens<2>(ta, tb, a, sm_count, st);

@@ -977,6 +977,23 @@ def test_gemm_fp8_token_tiles(T, N, K):
     assert bool((wide[:, :8] == 7.0).all()) and bool((wide[:, 8 + N:] == 7.0).all())
 
 
+@pytest.mark.parametrize("T,N,K", [(520, 6136, 272), (600, 6144, 1664), (2100, 2040, 1040), (700, 24600, 128)])
+def test_gemm_fp8_pairs_of_ctas(T, N, K):
+    """Products that pairs of CTAs take: ragged tiles of tokens and weight rows (a second CTA without tokens or weight rows of its
+    own), a K that ends inside a block, one block only, several tiles per pair; rows of a wider matrix, in fp32."""
+    torch.manual_seed(T + N)
+    lw = Fn.LinearWeight.from_master(torch.randn(N, K, device=dev()) * 0.05, "fp8", dev())
+    x = torch.randn(T, K, device=dev()).to(BF16)
+    xq, xs = R.quant_fp8_group128_act(x)
+    ref = R.dequant_fp8_group128_act(xq, xs).double() @ lw.dequant().double().t()
+    assert rel_err(Fn.linear(x, lw), ref) < 3e-3          # bf16 results; the activation's codes may differ at ties
+    wide = torch.full((T, N + 21), 7.0, dtype=F32, device=dev())
+    Fn.linear(x, lw, out=wide[:, 8:8 + N])
+    assert rel_err(wide[:, 8:8 + N], ref) < 2.5e-3
+    assert bool((wide[:, :8] == 7.0).all()) and bool((wide[:, 8 + N:] == 7.0).all())
+    _lib.check_status()
+
+
 def test_gemm_fp8_workspace_serves_explicit_splits_only(monkeypatch):
     """By default the token tiles take these sizes and no workspace is reserved; an explicit split goes through it."""
     torch.manual_seed(3)
