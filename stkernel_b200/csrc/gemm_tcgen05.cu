@@ -566,12 +566,12 @@ struct WideArgs {
 constexpr int kWideStages = 3;
 constexpr int kWideStageBytes = 2 * 128 * 128 + 256 * 128;       // two weight tiles + one token tile = 64 KB
 
-// S > 1: a cluster of S CTAs shares a tile, each with its part of K.  CTA j writes piece j of the tile (S = 2: 128 tokens; S = 4: 128
-// tokens x 128 weight rows); the others bring it their partial sums through distributed shared memory, into the operand ring that
-// is free by then.  Sums are formed in the order of the CTAs' ranks.
-template <int S>
+// A cluster of four CTAs shares a tile, each with its part of K.  CTA j writes piece j of the tile (128 tokens x 128 weight rows); the
+// others bring it their partial sums through distributed shared memory, into the operand ring that is free by then.  Sums are formed in
+// the order of the CTAs' ranks.  (Tiles that one or two CTAs can have to themselves are left to the pairs below.)
 __global__ void __launch_bounds__(320, 1)
 gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const WideArgs a) {
+  constexpr int S = 4;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   GemmBarriers* bars = reinterpret_cast<GemmBarriers*>(smem + kWideStages * kWideStageBytes);
@@ -601,7 +601,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   pdl_trigger();
   const int units = a.tiles_n * a.tiles_t;
   constexpr uint32_t kIdesc = umma_idesc(1u, 1u, 128, 256);
-  const int rank = S > 1 ? static_cast<int>(blockIdx.x) % S : 0;
+  const int rank = static_cast<int>(blockIdx.x) % S;
   const int per = (a.k_blocks + S - 1) / S, k_begin = rank * per, k_end = min(a.k_blocks, k_begin + per);
   const int u_first = blockIdx.x / S, u_step = gridDim.x / S;
 
@@ -675,7 +675,6 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     for (int u = u_first; u < units && ok; u += u_step) {
       const int tn = u % a.tiles_n, tt = u / a.tiles_n;
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->tmem_full[0], aphase, a.status, 400));
-      if (!ok && S == 1) break;
       tc_fence_after();
       // a thread owns one token row and, per chunk, 32 consecutive output features: 64 contiguous bytes of bf16
       const bool vec_ok = !a.out_fp32 && (a.ldo % 8 == 0) && ((reinterpret_cast<uintptr_t>(a.out) & 15) == 0);
@@ -714,22 +713,11 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
           }
         }
       };
-      if constexpr (S == 1) {
-#pragma unroll
-        for (int m = 0; m < 2; ++m) {
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            uint32_t r[32];
-            tmem_ld_32x32(tmem_base + m * 256 + h * 128 + c * 32 + lane_addr, r);
-            tmem_ld_wait();
-            store32(m, h * 128 + c * 32, r);
-          }
-        }
-      } else {
+      {
         // piece j: token tile m_of(j), columns from c_of(j); this warp's share of a piece is kShare columns of its lane quarter
         constexpr int kCols = 512 / S, kShare = kCols / 2;
-        auto m_of = [](int j) { return S == 2 ? j : j >> 1; };
-        auto c_of = [](int j) { return S == 2 ? 0 : (j & 1) * 128; };
+        auto m_of = [](int j) { return j >> 1; };
+        auto c_of = [](int j) { return (j & 1) * 128; };
         const uint32_t line = smem_u32(smem) + (q * 32 + lane) * 16;      // [slot][column / 4][token] of 16 bytes
         cluster_sync_all();                                               // every CTA's products are done: the rings are free
 #pragma unroll 1
@@ -782,7 +770,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       aphase ^= 1;
     }
   }
-  if (S > 1 && warp < 2) {
+  if (warp < 2) {
     // the CTAs of a cluster meet twice (one tile each)
     cluster_sync_all();
     cluster_sync_all();
@@ -1317,6 +1305,172 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
 }
 
 // ---------------------------------------------------------------------------------
+// bf16, a pair of CTAs on 256 tokens x 256 weight rows (operands as in the fp8 pair): a CTA's accumulators are its 128 tokens x 256
+// weight rows, half of its tensor memory, so the epilogue of a tile runs under the products of the next, and a tile that would leave
+// SMs idle is shared by two CTAs without partial sums to exchange.
+//
+// What bounds it: 32 KB of operands per CTA and 512 tensor-core cycles, as for the wide tile above; large products meet the power limit.
+// Measured, us, wide tile (with its split) / pair: 777 x 4096 x 4096: 31.5 / 27.1;  1904 x 11264 x 2048: 82 / 64;
+//   4096 x 8192 x 2048: 121 / 90;  4096 x 32768 x 1536: 372 / 318;  4096 x 4096 x 2048: 82 / 72;  4096 x 4096 x 8192: 236 / 229.
+// ---------------------------------------------------------------------------------
+__device__ __forceinline__ void mma_pair_f16(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t acc, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+      "mov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %4, p;\n\t}"
+      ::"r"(d), "r"(a_lo), "r"(b_lo), "r"(kDescHi), "r"(idesc), "r"(acc), "r"(lead)
+      : "memory");
+}
+
+__global__ void __launch_bounds__(320, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const WideArgs a) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  PairBars* bars = reinterpret_cast<PairBars*>(smem + kPairStages * kPairStageBytes);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = blockIdx.x & 1u;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kPairStages; ++i) {
+      mbar_init(&bars->full[i], 1);
+      mbar_init(&bars->empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&bars->tmem_full[i], 1);
+      mbar_init(&bars->tmem_empty[i], 16);             // epilogue warps of both CTAs
+    }
+    fence_barrier_init();
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem_base)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmX);
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();                                    // the other CTA's barriers are ready
+  tc_fence_after();
+  const uint32_t tmem_base = bars->tmem_base;
+  pdl_wait();
+  pdl_trigger();
+  const int units = a.tiles_t * a.tiles_n;
+  const int u_first = blockIdx.x >> 1, u_step = gridDim.x >> 1;
+
+  if (warp == 0) {
+    // ------------------------------ TMA producer: this CTA's tokens and half of the weight rows ------------------------------
+    if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int u = u_first; u < units && ok; u += u_step) {
+        const int tn = u % a.tiles_n, tt = u / a.tiles_n;
+        const int gx = a.group_tiles ? tn / a.group_tiles * a.group_k : 0;
+        for (int kb = 0; kb < a.k_blocks; ++kb) {
+          if (!mbar_wait(&bars->empty[stage], phase ^ 1, a.status, 100 + stage)) { ok = false; break; }
+          if (rank == 0) mbar_expect_tx(&bars->full[stage], 2 * kPairStageBytes);
+          const uint32_t st = smem_u32(smem + stage * kPairStageBytes), full = peer_addr(smem_u32(&bars->full[stage]), 0);
+          tma_load_2d_pair(st, &tmX, full, kb * 64 + gx, tt * 256 + rank * 128);
+          tma_load_2d_pair(st + 128 * 128, &tmW, full, kb * 64, tn * 256 + rank * 128);
+          if (++stage == kPairStages) { stage = 0; phase ^= 1; }
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ------------------------------ MMA issuer (first CTA) --------------------------------
+    if (rank == 0) {
+      const uint32_t lead = elect_one() ? 1u : 0u, tm = __shfl_sync(0xffffffffu, tmem_base, 0), s_lo = desc_lo(smem_u32(smem));
+      constexpr uint32_t kIdesc = umma_idesc(1u, 1u, 256, 256);
+      int stage = 0, ab = 0;
+      uint32_t phase = 0, aphase = 0;
+      bool ok = true;
+      for (int u = u_first; u < units && ok; u += u_step) {
+        ok = mbar_wait(&bars->tmem_empty[ab], aphase ^ 1, a.status, 200 + ab);
+        if (!ok) break;
+        for (int kb = 0; kb < a.k_blocks; ++kb) {
+          ok = mbar_wait(&bars->full[stage], phase, a.status, 300 + stage);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t st = s_lo + stage * (kPairStageBytes >> 4), d = tm + ab * 256;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) mma_pair_f16(d, st + 2 * k, st + 1024 + 2 * k, kIdesc, (kb > 0 || k > 0) ? 1u : 0u, lead);
+          mma_commit_pair(&bars->empty[stage], lead);
+          if (++stage == kPairStages) { stage = 0; phase ^= 1; }
+        }
+        if (ok) mma_commit_pair(&bars->tmem_full[ab], lead);
+        if (++ab == 2) { ab = 0; aphase ^= 1; }
+      }
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------ epilogue: a thread owns one token and half of the weight rows -----------------------------
+    const int q = warp & 3, h = (warp - 2) >> 2;
+    const uint32_t tile = tmem_base + h * 128 + (static_cast<uint32_t>(q * 32) << 16);
+    const uint32_t empty0 = peer_addr(smem_u32(&bars->tmem_empty[0]), 0);
+    const bool vec_ok = (a.ldo % (a.out_fp32 ? 4 : 8) == 0) && ((reinterpret_cast<uintptr_t>(a.out) & 15) == 0);
+    int ab = 0;
+    uint32_t aphase = 0;
+    for (int u = u_first; u < units; u += u_step) {
+      const int tn = u % a.tiles_n, tt = u / a.tiles_n;
+      const int t = tt * 256 + static_cast<int>(rank) * 128 + q * 32 + lane, n0 = tn * 256 + h * 128;
+      if (!__all_sync(0xffffffffu, mbar_wait(&bars->tmem_full[ab], aphase, a.status, 400 + ab))) break;
+      tc_fence_after();
+#pragma unroll 1
+      for (int c = 0; c < 128; c += 32) {
+        uint32_t r[32];
+        tmem_ld_32x32(tile + ab * 256 + c, r);
+        tmem_ld_wait();
+        if (c == 96) {                                     // all of this warp's columns have been read
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_at(empty0 + ab * 8);
+        }
+        const int n = n0 + c;
+        if (t < a.T) {
+          const long long o0 = static_cast<long long>(t) * a.ldo + n;
+          if (vec_ok && n + 32 <= a.N) {
+            if (a.out_fp32) {
+              float* o = reinterpret_cast<float*>(a.out) + o0;
+#pragma unroll
+              for (int j = 0; j < 32; j += 4) *reinterpret_cast<uint4*>(o + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
+            } else {
+              __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(a.out) + o0;
+#pragma unroll
+              for (int j = 0; j < 32; j += 8) {
+                uint4 ov;
+                __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&ov);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) oh[i] = __floats2bfloat162_rn(__uint_as_float(r[j + 2 * i]), __uint_as_float(r[j + 2 * i + 1]));
+                *reinterpret_cast<uint4*>(o + j) = ov;
+              }
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              if (n + j < a.N) {
+                if (a.out_fp32) reinterpret_cast<float*>(a.out)[o0 + j] = __uint_as_float(r[j]);
+                else reinterpret_cast<__nv_bfloat16*>(a.out)[o0 + j] = __float2bfloat16(__uint_as_float(r[j]));
+              }
+            }
+          }
+        }
+      }
+      if (++ab == 2) { ab = 0; aphase ^= 1; }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();                                    // nobody reads this CTA's operands or arrives at its barriers any more
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+  }
+}
+
+// ---------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -1455,11 +1609,12 @@ STK_API long long stk_gemm_workspace_bytes(int T, int N, int splits) {
   return splits > 1 ? static_cast<long long>(splits) * T * N * 4 : 0;
 }
 
-// CTAs that share a 256 x 256 tile of the wide kernel (as many as keep the SMs to one round, with at least four K blocks each), or 0
-// where the kernel above is better: up to 96 tokens.  A call that asks for workspace splits keeps the kernel above: `linear` does so up
-// to 128 tokens wherever 128-row tiles leave SMs idle.  Measured without workspace splits, us, kernel above / this one with its split:
+// CTAs that share a 256 x 256 tile of a token-major kernel: four with a part of K each where that keeps the SMs to one round (with at
+// least four K blocks each), else a pair (1 and 2 here); or 0 where the kernel above is better: up to 96 tokens.  A call that asks for
+// workspace splits keeps the kernel above: `linear` does so up to 128 tokens wherever 128-row tiles leave SMs idle.  Measured without
+// workspace splits, us, kernel above / these:
 //   64 tokens x 4096 x 8192: 24.5 / 28.7;  128: 51.8 / 29.5;  256: 48.4 / 29.8;  777: 124 / 52;  128 x 40960 x 1536: 94 / 46;
-//   4096 tokens x 64 x 4096: 28 / 19;  777 x 4096 x 4096: 66 / 31.5 (45.3 without the split);  1500 x 4096 x 4096: 113 / 49.6.
+//   4096 tokens x 64 x 4096: 28 / 19;  777 x 4096 x 4096: 66 / 27;  1500 x 4096 x 4096: 113 / 47.
 static int wide_split_of(int T, int N, int K, int sm_count) {
   if (T <= 96) return 0;
   const int units = ((T + 255) / 256) * ((N + 255) / 256), kb = (K * 2 + 127) / 128;
@@ -1468,22 +1623,25 @@ static int wide_split_of(int T, int N, int K, int sm_count) {
   return s;
 }
 
-template <int S>
-static int launch_wide_s(const CUtensorMap& tx, const CUtensorMap& tw, const WideArgs& a, int grid, cudaStream_t st) {
+static int launch_wide(const CUtensorMap& tx, const CUtensorMap& tw, const WideArgs& a, cudaStream_t st) {
   constexpr int smem = kWideStages * kWideStageBytes + 256 + 1024;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(gemm_wide_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -3;
+    if (cudaFuncSetAttribute(gemm_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -3;
     configured = true;
   }
-  return launch_cluster(gemm_wide_kernel<S>, S, grid, 320, smem, st, tw, tx, a);
+  return launch_cluster(gemm_wide_kernel, 4, a.tiles_n * a.tiles_t * 4, 320, smem, st, tw, tx, a);
 }
 
-static int launch_wide(const CUtensorMap& tx, const CUtensorMap& tw, const WideArgs& a, int split, int sm_count, cudaStream_t st) {
-  const int units = a.tiles_n * a.tiles_t;
-  if (split == 4) return launch_wide_s<4>(tx, tw, a, units * 4, st);
-  if (split == 2) return launch_wide_s<2>(tx, tw, a, units * 2, st);
-  return launch_wide_s<1>(tx, tw, a, units < sm_count ? units : sm_count, st);
+static int launch_pair(const CUtensorMap& tx, const CUtensorMap& tw, const WideArgs& a, int sm_count, cudaStream_t st) {
+  constexpr int smem = kPairStages * kPairStageBytes + static_cast<int>(sizeof(PairBars)) + 1024;
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -3;
+    configured = true;
+  }
+  const int units = a.tiles_n * a.tiles_t, pairs = sm_count >= 2 ? sm_count / 2 : 1;
+  return launch_cluster(gemm_pair_kernel, 2, 2 * (units < pairs ? units : pairs), 320, smem, st, tx, tw, a);
 }
 
 // STK_GEMM_WIDE=0 keeps large bf16 problems on the 128 x 256 tile (A/B runs)
@@ -1571,7 +1729,7 @@ static int gemm_launch(const void* W, long long ldw, const void* X, long long ld
   const int wide_split = (groups == 1 || (N % (256 * groups) == 0 && K % 64 == 0)) ? wide_split_of(T, N, K, sm_count) : 0;
   if (!is_fp8 && ar_ctx == nullptr && gate_ctx == nullptr && splits <= 1 && bt_override == 0 && wide_split > 0 && gemm_wide_enabled()) {
     CUtensorMap tw2, tx2;
-    if (make_tmap_2d(&tw2, W, 2, N, K, ldw, 256) != 0) return -13;                                               // B operand: 256 weight rows
+    if (make_tmap_2d(&tw2, W, 2, N, K, ldw, wide_split == 4 ? 256 : 128) != 0) return -13;                       // B operand: 256 weight rows, or a CTA's half
     if (make_tmap_2d(&tx2, X, 2, T, static_cast<long long>(K) * groups, ldx, 128) != 0) return -14;              // A operands: 128 tokens each
     WideArgs wa;
     wa.T = T; wa.N = N;
@@ -1581,7 +1739,8 @@ static int gemm_launch(const void* W, long long ldw, const void* X, long long ld
     wa.out = out; wa.ldo = ldo; wa.out_fp32 = out_fp32; wa.status = status;
     wa.group_tiles = groups > 1 ? N / groups / 256 : 0;
     wa.group_k = K;
-    return launch_wide(tx2, tw2, wa, wide_split, sm_count, reinterpret_cast<cudaStream_t>(stream));
+    if (wide_split == 4) return launch_wide(tx2, tw2, wa, reinterpret_cast<cudaStream_t>(stream));
+    return launch_pair(tx2, tw2, wa, sm_count, reinterpret_cast<cudaStream_t>(stream));
   }
   int bt = stk_gemm_pick_bt(T, is_fp8);
   if (!is_fp8 && T > 128 && groups == 1) {
