@@ -1610,13 +1610,12 @@ STK_API long long stk_gemm_workspace_bytes(int T, int N, int splits) {
 }
 
 // CTAs that share a 256 x 256 tile of a token-major kernel: four with a part of K each where that keeps the SMs to one round (with at
-// least four K blocks each), else a pair (1 and 2 here); or 0 where the kernel above is better: up to 96 tokens.  A call that asks for
-// workspace splits keeps the kernel above: `linear` does so up to 128 tokens wherever 128-row tiles leave SMs idle.  Measured without
-// workspace splits, us, kernel above / these:
-//   64 tokens x 4096 x 8192: 24.5 / 28.7;  128: 51.8 / 29.5;  256: 48.4 / 29.8;  777: 124 / 52;  128 x 40960 x 1536: 94 / 46;
-//   4096 tokens x 64 x 4096: 28 / 19;  777 x 4096 x 4096: 66 / 27;  1500 x 4096 x 4096: 113 / 47.
+// least four K blocks each), else a pair (1 and 2 here); or 0 where the kernel above is better: up to 64 tokens.  A call that asks for
+// workspace splits keeps the kernel above.  Measured, us, kernel above with the split that it would ask for / these:
+//   64 tokens x 4096 x 8192: 26 / 31;  x 4096 x 2048: 18 / 16;  80 tokens x 4096 x 8192: 47 / 31;  x 2048 x 4096: 33 / 20;
+//   x 32768 x 1536: 66 / 24;  128 x 2048 x 4096: 38 / 20;  777 x 4096 x 4096: 66 / 27;  1500 x 4096 x 4096: 113 / 47.
 static int wide_split_of(int T, int N, int K, int sm_count) {
-  if (T <= 96) return 0;
+  if (T <= 64) return 0;
   const int units = ((T + 255) / 256) * ((N + 255) / 256), kb = (K * 2 + 127) / 128;
   int s = 4;
   while (s > 1 && (units * s > sm_count || kb < 4 * s)) s /= 2;

@@ -243,9 +243,9 @@ def linear(x, lw: LinearWeight, out: Optional[torch.Tensor] = None, out_dtype=BF
     is_fp8 = 1 if lw.is_fp8 else 0
     sms = _lib.sm_count()
     if splits is None:
-        # fp8 on token-major tiles splits K over clusters, without a workspace
-        plain = is_fp8 and groups == 1 and ar_ctx is None
-        splits = 1 if plain and _lib.query("stk_gemm_token_tile_ctas", t, n, k, 1, sms) else _lib.query("stk_gemm_pick_splits", t, n, k, is_fp8, sms)
+        # token-major tiles split K over clusters, without a workspace
+        plain = groups == 1 and ar_ctx is None
+        splits = 1 if plain and _lib.query("stk_gemm_token_tile_ctas", t, n, k, is_fp8, sms) else _lib.query("stk_gemm_pick_splits", t, n, k, is_fp8, sms)
     ws = cnt = None
     if splits > 1:
         ws = scratch("gemm.splitk", (splits * t * n,), F32, dev)

@@ -1031,6 +1031,22 @@ def test_gemm_bf16_wide_tiles_that_share_k(T, N, K):
     assert bool((wide[:, N:] == 7.0).all())
 
 
+@pytest.mark.parametrize("T,N,K", [(64, 1030, 2048), (65, 1030, 2048), (96, 5000, 576), (600, 7500, 192), (1100, 6200, 1088), (2900, 3333, 64)])
+def test_gemm_bf16_pairs_of_ctas(T, N, K):
+    """Up to and from where `linear` leaves its workspace splits; pairs of CTAs with one tile and with several, a second CTA without
+    tokens or weight rows, one K block; rows of a wider matrix in fp32."""
+    torch.manual_seed(T + N)
+    w = (torch.randn(N, K, device=dev()) * 0.05).to(BF16)
+    x = torch.randn(T, K, device=dev()).to(BF16)
+    ref = x.double() @ w.double().t()
+    assert rel_err(Fn.linear(x, Fn.LinearWeight(w)), ref) < 2.5e-3
+    wide = torch.full((T, N + 5), 7.0, dtype=F32, device=dev())
+    Fn.linear(x, Fn.LinearWeight(w), out=wide[:, :N])
+    assert rel_err(wide[:, :N], ref) < 2e-5               # fp32 sums
+    assert bool((wide[:, N:] == 7.0).all())
+    _lib.check_status()
+
+
 @pytest.mark.parametrize("T", [130, 600])
 @pytest.mark.parametrize("groups,n,K", [(2, 256, 128), (3, 512, 1024), (8, 128, 256)])
 def test_gemm_bf16_wide_block_diagonal(T, groups, n, K):
