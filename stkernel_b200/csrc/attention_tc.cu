@@ -1,6 +1,6 @@
 // Sparse multi-head latent attention on the 5th-generation tensor cores (fp8_ds_mla rows, D = 512).
 //
-// One CTA per (query token, row split).  The row list (SWA window rows, then top-k compressed rows)
+// One CTA per SM, which walks through (query token, row split) items.  The row list (SWA window rows, then top-k compressed rows)
 // is walked in blocks of 128 rows:
 //
 //   producer warps   gather the 584-byte rows by slot id, dequantise fp8 x UE8M0 -> fp16 and write them
@@ -25,10 +25,12 @@
 //     took 2753 us, four 2894, all of them 3182), and that only in blocks where a weight would pass 2^kSlack: the others cost one
 //     look at the scores and a vote.  The row sums of P stay in registers (one per head and row) and are reduced once per CTA.
 // The value products read 6 KB of shared memory each and the next block's panels are written under them: 2500 cycles alone, 5600
-// with the writes.  A first block and the end of a token (queries, first gather, output) are 16000 cycles, a block 8800.
+// with the writes.  The beginning and the end of a token (queries, first gather, output) were 26000 cycles with a thread block per
+// token, a block is 8200: thread blocks stay and walk through tokens, the next one's queries and first codes are fetched under this
+// one's last softmax, value products and output.
 // Measured (4096 tokens, 64 heads, 128 + 2048 rows): 5162 us with one thread block of thirteen warps working through
 // load -> scores -> softmax -> values without overlap, 2677 with bf16 operands, exact maxima in every block and two-byte stores of the
-// output, 2475 now; 128 rows alone: 576 -> 415.
+// output, 2387 now; 128 rows alone: 576 -> 281.
 //
 // Accumulators live in TMEM: S (NH columns) and four O^T tiles of [128 dims x NH heads].
 // A CTA of a split writes an un-normalised partial (o, m, l) that `sparse_mla_combine` merges with the sink.
@@ -41,6 +43,8 @@
 #include "common.cuh"
 #include "pairs.cuh"
 #include "warp_reduce.cuh"
+
+#include <type_traits>
 
 namespace stk {
 
@@ -69,7 +73,7 @@ __device__ __forceinline__ unsigned long long global_ns() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
-#define STK_TRACE(slot) do { if (a.trace && blockIdx.x == 0 && blockIdx.y == 0) a.trace[slot] = global_ns(); } while (0)
+#define STK_TRACE(slot) do { if (a.trace && blockIdx.x == 0) a.trace[slot] = global_ns(); } while (0)
 
 constexpr int kD = 512, kR = 64, kNope = 448, kDataBytes = 576, kPanels = 8, kRows = 128;
 constexpr int kPanelBytes = kRows * 128;                 // 16 KB
@@ -106,7 +110,7 @@ __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.al
 struct alignas(8) MlaBars {
   uint64_t k_full[5];              // panels 0 + 1, 2 + 3, 4 + 5, 6, 7 of the block are in shared memory
   uint64_t k_free[kPanels / 2];    // the value products of a pair of panels are done
-  uint64_t s_full, p_full, pv_done;
+  uint64_t s_full, p_full, pv_done, q_full;
   uint32_t tmem_base;
   uint32_t moved[2];               // heads whose maximum the last block that took maxima moved, by halves of 32
   uint32_t unset[2];               // heads that have none yet
@@ -186,32 +190,36 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
   float* m_run = smax + 4 * NH;                          // [NH] the maxima in use, in powers of two
   float* minus_m = m_run + NH;                           // [NH] their negatives (0 for none yet)
   float* alpha_s = minus_m + NH;                         // [NH]
-  int* lift_s = reinterpret_cast<int*>(alpha_s + NH);    // [kRows] what the block's rows were divided by, in powers of two
+  int* lift_s = reinterpret_cast<int*>(alpha_s + NH);    // [kRows] what the block's rows were divided by, in powers of two; -1: no row
 
-  const int t = blockIdx.x, sp = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n_swa = a.swa_lens[t];
-  const int n_top = a.topk_slots ? a.topk_lens[t] : 0;
-  const int L = n_swa + n_top;
-  const int r_begin = sp * a.rows_per_split;
-  const int r_end = min(L, r_begin + a.rows_per_split);
-  const int n_blocks = r_end > r_begin ? (r_end - r_begin + kRows - 1) / kRows : 0;
-  float* prow = a.partial + (static_cast<long long>(t) * a.n_splits + sp) * a.nh * (kD + 2);
-
   if (threadIdx.x == 0) STK_TRACE(0);
-  if (n_blocks == 0 && a.out != nullptr) {
-    // no keys at all: only the sink takes probability mass, the output is zero
-    __nv_bfloat16* orow = a.out + static_cast<long long>(t) * a.ldo;
-    for (int i = threadIdx.x; i < a.nh * kD; i += blockDim.x) orow[i] = __float2bfloat16(0.f);
-    return;
-  }
-  if (n_blocks == 0) {
-    for (int i = threadIdx.x; i < a.nh * (kD + 2); i += blockDim.x) {
-      const int d = i % (kD + 2);
-      prow[i] = d == kD ? -INFINITY : 0.f;
+  // Items of this CTA: a token and its part of the row list.  Every role walks through those that have rows.
+  const int items = a.T * a.n_splits;
+  struct Item { int i, t, sp, n_swa, r_begin, r_end, n_blocks; };
+  auto item_at = [&](int i) {
+    Item w;
+    w.i = i;
+    w.sp = i / a.T;
+    w.t = i - w.sp * a.T;
+    w.n_swa = a.swa_lens[w.t];
+    const int L = w.n_swa + (a.topk_slots ? a.topk_lens[w.t] : 0);
+    w.r_begin = w.sp * a.rows_per_split;
+    w.r_end = min(L, w.r_begin + a.rows_per_split);
+    w.n_blocks = w.r_end > w.r_begin ? (w.r_end - w.r_begin + kRows - 1) / kRows : 0;
+    return w;
+  };
+  auto item_from = [&](int i) {                          // the first that has rows from i on; i >= items: none left
+    Item w;
+    w.i = i;
+    w.n_blocks = 0;
+    for (; i < items; i += gridDim.x) {
+      w = item_at(i);
+      if (w.n_blocks > 0) return w;
     }
-    return;
-  }
+    w.i = i;
+    return w;
+  };
 
   if (threadIdx.x == 0) {
     for (int p = 0; p < 5; ++p) mbar_init(&bars->k_full[p], kProducerWarps);
@@ -220,19 +228,13 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
     mbar_init(&bars->s_full, 1);
     mbar_init(&bars->p_full, kSoftmaxWarps);
     mbar_init(&bars->pv_done, 1);
+    mbar_init(&bars->q_full, kProducerWarps);
     fence_barrier_init();
   }
   if (warp == 0) {
     tmem_alloc(&bars->tmem_base, Cfg::kTmemCols);
     tmem_relinquish();
   }
-  // slot of row li of this token's list (-1: none), and the cache it lies in
-  auto slot_of = [&](int li) -> int {
-    if (li >= r_end) return -1;
-    return li < n_swa ? a.swa_slots[static_cast<long long>(t) * a.swa_ld + li]
-                      : a.topk_slots[static_cast<long long>(t) * a.topk_ld + (li - n_swa)];
-  };
-
   // every warp passes this once its part of the prologue is done
   auto begin = [&]() {
     fence_proxy_async();
@@ -240,26 +242,23 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
     named_bar_sync(1, kThreads);
     tc_fence_after();
   };
-  auto load_q = [&]() {
-    // Q -> shared memory, K-major panels [NH x 64 dims], 128-byte swizzle; heads >= nh are zero.
-    constexpr int kChunks = NH * (kD / 8), kLoaders = 32 * kSoftmaxWarps, kBatch = 16;
-    for (int i0 = threadIdx.x - 128; i0 < kChunks; i0 += kLoaders * kBatch) {
-      uint4 qv[kBatch];
+  // Q of a token -> shared memory, K-major panels [NH x 64 dims], 128-byte swizzled; heads >= nh are zero.  `who` of kLoaders threads.
+  auto load_q = [&](int t, int who, auto loaders) {
+    constexpr int kLoaders = decltype(loaders)::value, kChunks = NH * (kD / 8), kBatch = kChunks / kLoaders;
+    static_assert(kChunks % kLoaders == 0, "chunks of Q");
+    uint4 qv[kBatch];
 #pragma unroll
-      for (int j = 0; j < kBatch; ++j) {
-        const int i = i0 + j * kLoaders, h = i / (kD / 8), c8 = i % (kD / 8);
-        qv[j] = make_uint4(0, 0, 0, 0);
-        if (i < kChunks && h < a.nh) qv[j] = __ldg(reinterpret_cast<const uint4*>(a.q + t * a.ldt + static_cast<long long>(h) * kD + c8 * 8));
-      }
-#pragma unroll
-      for (int j = 0; j < kBatch; ++j) {
-        const int i = i0 + j * kLoaders, h = i / (kD / 8), c8 = i % (kD / 8);
-        if (i < kChunks) *reinterpret_cast<uint4*>(q_s + (c8 >> 3) * (NH * 128) + h * 128 + (((c8 & 7) ^ (h & 7)) << 4)) = bf16x8_to_half(qv[j], 1.f);
-      }
+    for (int j = 0; j < kBatch; ++j) {
+      const int i = who + j * kLoaders, h = i / (kD / 8), c8 = i % (kD / 8);
+      qv[j] = make_uint4(0, 0, 0, 0);
+      if (h < a.nh) qv[j] = __ldg(reinterpret_cast<const uint4*>(a.q + t * a.ldt + static_cast<long long>(h) * kD + c8 * 8));
     }
-    if (threadIdx.x - 128 < NH) m_run[threadIdx.x - 128] = -INFINITY;
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) {
+      const int i = who + j * kLoaders, h = i / (kD / 8), c8 = i % (kD / 8);
+      *reinterpret_cast<uint4*>(q_s + (c8 >> 3) * (NH * 128) + h * 128 + (((c8 & 7) ^ (h & 7)) << 4)) = bf16x8_to_half(qv[j], 1.f);
+    }
   };
-
   if (warp < 4) {
     reg_dec<Cfg::kIssueRegs>();
     begin();
@@ -274,8 +273,13 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
       const uint32_t k_lo = desc_lo(smem_u32(k_s)), v_lo = desc_lo(smem_u32(k_s), kPanelBytes);
       const uint32_t q_lo = desc_lo(smem_u32(q_s)), p_lo = desc_lo(smem_u32(p_s));
       bool ok = true;
-      for (int b = 0; b < n_blocks && ok; ++b) {
-        const uint32_t ph = b & 1;
+      uint32_t g = 0, k = 0;                                   // blocks and items before this one: phases of their barriers
+      for (int at = blockIdx.x; at < items && ok; at += gridDim.x) {
+      const int n_blocks = item_at(at).n_blocks;
+      if (n_blocks == 0) continue;
+      if (k > 0) ok = mbar_wait(&bars->q_full, (k - 1) & 1, a.status, 603);
+      for (int b = 0; b < n_blocks && ok; ++b, ++g) {
+        const uint32_t ph = g & 1;
 #pragma unroll 1
         for (int i = 0; i < kPanels; ++i) {
           const int p = panel_at(i);
@@ -303,15 +307,23 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
           mma_commit(&bars->k_free[j], lead);
         }
       }
-      // what was issued completes before the tensor memory goes away
       mma_commit(&bars->pv_done, lead);
-      mbar_wait(&bars->pv_done, 0, a.status, 602);
+      ++k;
+      }
+      // what was issued completes before the tensor memory goes away
+      if (k > 0) mbar_wait(&bars->pv_done, (k - 1) & 1, a.status, 602);
       __syncwarp();
     }
   } else if (warp < 4 + kSoftmaxWarps) {
     // ------------------------------- softmax / epilogue -------------------------------
     if constexpr (Cfg::kSoftmaxRegs > Cfg::kLaunchRegs) reg_inc<Cfg::kSoftmaxRegs>();
-    load_q();
+    int at = blockIdx.x, n_blocks = 0;                    // this item, and its blocks
+    {
+      const Item e = item_from(at);
+      at = e.i;
+      n_blocks = e.n_blocks;
+    }
+    if (at < items) load_q(at % a.T, threadIdx.x - 128, std::integral_constant<int, kSoftmaxThreads>{});
     begin();
     const uint32_t tmem_s = bars->tmem_base, tmem_o = tmem_s + NH;       // S^T: NH columns; O^T: 4 x NH columns
     const int q4 = warp & 3;                              // TMEM lane quarter
@@ -321,28 +333,41 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
     const float sl2 = a.scale * 1.4426950408889634f;
     const int own = threadIdx.x - 128;                   // owner thread of head `own` when < NH
     uint64_t lp[kHeads / 2];                              // sums of this row's weights, two heads each
-#pragma unroll
-    for (int i = 0; i < kHeads / 2; ++i) lp[i] = 0ull;
     // this row's place in a head's line of P: the 16-byte chunk number is turned by the head's low bits
     uint32_t pdst[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
       pdst[i] = smem_u32(p_s) + (row >> 6) * (NH * 128) + (h0 + i) * 128 + ((((row & 63) >> 3) ^ i) << 4) + (row & 7) * 2;
-    int slot = slot_of(r_begin + row);
+    // items without rows: only the sink takes probability mass, the output is zero
+    for (int i = blockIdx.x; i < items; i += gridDim.x) {
+      const Item e = item_at(i);
+      if (e.n_blocks > 0) continue;
+      if (a.out != nullptr) {
+        __nv_bfloat16* orow = a.out + static_cast<long long>(e.t) * a.ldo;
+        for (int j = own; j < a.nh * kD; j += kSoftmaxThreads) orow[j] = __float2bfloat16(0.f);
+      } else {
+        float* prow = a.partial + (static_cast<long long>(e.t) * a.n_splits + e.sp) * a.nh * (kD + 2);
+        for (int j = own; j < a.nh * (kD + 2); j += kSoftmaxThreads) prow[j] = j % (kD + 2) == kD ? -INFINITY : 0.f;
+      }
+    }
     bool ok = true;                                       // the same in every lane; barriers are passed either way
     auto scores = [&](int c, uint32_t (&r16)[16]) {       // sixteen heads' products of this row
       tmem_ld_32x16(tmem_s + lane_addr + h0 + c, r16);
       tmem_ld_wait();
     };
-    for (int b = 0; b < n_blocks; ++b) {
-      const uint32_t ph = b & 1;
-      const bool valid = slot >= 0;
-      slot = slot_of(r_begin + (b + 1) * kRows + row);
+    uint32_t g = 0, k = 0;
+    for (; at < items; ++k) {
+#pragma unroll
+    for (int i = 0; i < kHeads / 2; ++i) lp[i] = 0ull;
+    if (own < NH) m_run[own] = -INFINITY;
+    for (int b = 0; b < n_blocks; ++b, ++g) {
+      const uint32_t ph = g & 1;
       // (the row's power of two was left before the first panel was handed over: a barrier that has long completed)
       ok = __all_sync(0xffffffffu, ok && mbar_wait(&bars->s_full, ph, a.status, 610) && mbar_wait(&bars->k_full[3], ph, a.status, 612));
       if (b == 0 && threadIdx.x == 128) STK_TRACE(3);
       tc_fence_after();
-      const int lift = lift_s[row];
+      const int mark = lift_s[row], lift = max(mark, 0);
+      const bool valid = mark >= 0;
       const float liftf = static_cast<float>(lift), sl = sl2 * __int_as_float((127 + lift) << 23), back = __int_as_float((127 - lift) << 23);
       const uint64_t sl22 = pack2(sl, sl), lift2 = pack2(liftf, liftf), back2 = pack2(back, back);
       // Whether a weight would pass 2^kSlack with the maxima in use
@@ -454,7 +479,14 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
       if (lane == 0) mbar_arrive(&bars->p_full);
     }
     // ---- epilogue: wait for the last value products, reduce the row sums ----
-    ok = __all_sync(0xffffffffu, ok && mbar_wait(&bars->pv_done, 0, a.status, 611));
+    const int sp = at / a.T, t = at - sp * a.T;
+    float* prow = a.partial + (static_cast<long long>(t) * a.n_splits + sp) * a.nh * (kD + 2);
+    {
+      const Item e = item_from(at + gridDim.x);
+      at = e.i;
+      n_blocks = e.n_blocks;
+    }
+    ok = __all_sync(0xffffffffu, ok && mbar_wait(&bars->pv_done, k & 1, a.status, 611));
     if (threadIdx.x == 128) STK_TRACE(5);
     tc_fence_after();
 #pragma unroll
@@ -483,11 +515,9 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
       named_bar_sync(2, kSoftmaxThreads);
     }
     if (ok && a.out != nullptr) {
-      // The sums lie by dims in TMEM: they are turned in shared memory (the panels are no longer needed) and leave in one copy.  Stored
-      // two bytes a lane straight to memory, with a branch per value, they took 16000 cycles a token.
+      // 64 bytes of a row a store: without a branch per value these are as fast as a turn through shared memory (with one per value
+      // they took 16000 cycles a token)
       __nv_bfloat16* orow = a.out + static_cast<long long>(t) * a.ldo;
-      const bool turned = ((reinterpret_cast<uintptr_t>(a.out) | static_cast<uintptr_t>(a.ldo * 2)) & 15) == 0;
-      const uint32_t stage = smem_u32(k_s);
       const float pos = a.positions != nullptr ? static_cast<float>(a.positions[t]) : 0.f;
 #pragma unroll 1
       for (int j = 0; j < 4; ++j) {
@@ -517,22 +547,15 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
               v[i] = (d & 1) ? (-p * sn + v[i] * cs) : (v[i] * cs + p * sn);
             }
           }
-          if (turned) {
+          __nv_bfloat16* o = orow + (h0 + c) * kD + d;
+          if (h0 + c + 16 <= a.nh) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) put16(stage + (h0 + c + i) * (kD * 2) + d * 2, __bfloat16_as_ushort(__float2bfloat16(v[i])));
+            for (int i = 0; i < 16; ++i) o[i * kD] = __float2bfloat16(v[i]);
           } else {
 #pragma unroll
             for (int i = 0; i < 16; ++i)
-              if (h0 + c + i < a.nh) orow[static_cast<long long>(h0 + c + i) * kD + d] = __float2bfloat16(v[i]);
+              if (h0 + c + i < a.nh) o[i * kD] = __float2bfloat16(v[i]);
           }
-        }
-      }
-      if (turned) {
-        fence_proxy_async();
-        named_bar_sync(2, kSoftmaxThreads);
-        if (own == 0) {
-          asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(orow), "r"(stage), "r"(a.nh * kD * 2) : "memory");
-          asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group 0;" ::: "memory");
         }
       }
     } else if (ok) {
@@ -559,6 +582,9 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
         prow[own * (kD + 2) + kD + 1] = l_own;
       }
     }
+    // O has been read: the next item's value products wait for its weights, which come behind this fence
+    tc_fence_before();
+    }
   } else {
     // ------------------------------- producers -------------------------------
     // Warp pw owns rows 8 pw .. 8 pw + 7 of every block; a lane holds 16 bytes of each 64-byte segment of one row's codes, and the
@@ -569,18 +595,38 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
     uint4 raw[7], rot[2];                                  // codes, and the rotated part (bf16)
     uint2 sc8;
     const uint8_t* src_row;                                // row whose codes are in `raw`; nullptr: none
-    int slot_next = slot_of(r_begin + row);
-    auto next_row = [&](int b) {                           // slot_next -> row of block b; slot of block b + 1
-      const int slot = slot_next;
-      const bool swa = r_begin + b * kRows + row < n_swa;
+    // The item, its blocks, and the list's next row of this lane (registers are short here: no more is kept)
+    int at, t = 0, n_swa = 0, r_end = 0, n_blocks = 0, li = 0, slot_next = -1;
+    constexpr int kWindow = 1 << 30;                       // marks a slot of the first cache (a slot is far below)
+    auto look_up = [&]() {                                 // li -> slot_next, and on to the same row of the next block
+      slot_next = -1;
+      if (li < n_swa && li < r_end) slot_next = a.swa_slots[static_cast<long long>(t) * a.swa_ld + li] | kWindow;
+      else if (li < r_end) slot_next = a.topk_slots[static_cast<long long>(t) * a.topk_ld + (li - n_swa)];
+      li += kRows;
+    };
+    auto enter = [&](int from) {
+      const Item w = item_from(from);
+      at = w.i;
+      if (at >= items) return;
+      t = w.t;
+      n_swa = w.n_swa;
+      r_end = w.r_end;
+      n_blocks = w.n_blocks;
+      li = w.r_begin + row;
+      look_up();
+    };
+    enter(blockIdx.x);
+    auto next_row = [&]() {                                // slot_next -> row to be fetched; slot of the block after
+      const int slot = slot_next & ~kWindow;
+      const bool swa = (slot_next & kWindow) != 0;
       src_row = nullptr;
       sc8 = make_uint2(0, 0);
-      if (slot >= 0) {
+      if (slot_next >= 0) {
         const uint8_t* page = (swa ? a.swa_base : a.comp_base) + static_cast<long long>(slot >> 6) * (swa ? a.swa_stride : a.comp_stride);
         src_row = page + (slot & 63) * kDataBytes + l4 * 16;
         sc8 = *reinterpret_cast<const uint2*>(page + 64 * kDataBytes + (slot & 63) * 8);
       }
-      slot_next = slot_of(r_begin + (b + 1) * kRows + row);
+      look_up();
     };
     auto fetch = [&](int seg) {
       raw[seg] = make_uint4(0, 0, 0, 0);
@@ -593,13 +639,17 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
         if (src_row != nullptr) rot[i] = __ldg(reinterpret_cast<const uint4*>(src_row + kNope + i * 64));
       }
     };
-    next_row(0);
+    auto fetch_row = [&]() {
+      next_row();
 #pragma unroll
-    for (int i = 0; i < 7; ++i) fetch(panel_at(i));
-    fetch_rot();
+      for (int i = 0; i < 7; ++i) fetch(panel_at(i));
+      fetch_rot();
+    };
+    if (at < items) fetch_row();
     begin();
     bool ok = true;
-    for (int b = 0; b < n_blocks && ok; ++b) {
+    uint32_t g = 0;
+    while (at < items) {
       const uint2 sc = sc8;
       // Power of two that brings the row into fp16's range: 0 unless a scale is above 2^7 (a code's magnitude is at most 448) or a
       // rotated value above 2^16
@@ -614,11 +664,11 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
 #pragma unroll
       for (int i = 0; i < kPanels; ++i) {
         const int p = panel_at(i);
-        if (b > 0 && (i == 0 || i == 1 || i == 3 || i == 5)) {
-          ok = __all_sync(0xffffffffu, ok && mbar_wait(&bars->k_free[p >> 1], (b - 1) & 1, a.status, 620));
+        if (g > 0 && (i == 0 || i == 1 || i == 3 || i == 5)) {
+          ok = __all_sync(0xffffffffu, ok && mbar_wait(&bars->k_free[p >> 1], (g - 1) & 1, a.status, 620));
           if (!ok) break;
         }
-        if (i == 0 && l4 == 0) lift_s[row] = lift;
+        if (i == 0 && l4 == 0) lift_s[row] = src_row != nullptr ? lift : -1;
         uint4 o0, o1;
         uint32_t at0, at1;
         if (p < 7) {
@@ -651,11 +701,21 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
           if (lane == 0) mbar_arrive(&bars->k_full[p < 6 ? p >> 1 : p - 3]);
         }
       }
+      if (!ok) break;
+      ++g;
+      if (--n_blocks == 0) {
+        // the next item's queries as soon as this one's last scores have been formed, under its softmax, value products and output
+        enter(at + gridDim.x);
+        if (at >= items) break;
+        ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full, (g - 1) & 1, a.status, 621));
+        if (!ok) break;
+        load_q(t, threadIdx.x - (4 + kSoftmaxWarps) * 32, std::integral_constant<int, 32 * kProducerWarps>{});
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->q_full);
+      }
       // the next block's codes: asked for once all of this one is handed over, they arrive under its softmax
-      next_row(b + 1);
-#pragma unroll
-      for (int i = 0; i < 7; ++i) fetch(panel_at(i));
-      fetch_rot();
+      fetch_row();
     }
   }
 
@@ -677,8 +737,11 @@ static int launch_mla_tc(const MlaTcArgs& a, cudaStream_t st) {
       return -3;
     configured = true;
   }
-  dim3 grid(a.T, a.n_splits);
-  launch_pdl(sparse_mla_tc_kernel<NH>, dim3(grid), dim3(MlaCfg<NH>::kThreads), smem, st, a);
+  int device = 0, sms = 1;
+  if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return -5;
+  const long long items = static_cast<long long>(a.T) * a.n_splits;
+  if (items > 0x7fffffffLL - sms) return -6;
+  launch_pdl(sparse_mla_tc_kernel<NH>, dim3(static_cast<unsigned>(items < sms ? items : sms)), dim3(MlaCfg<NH>::kThreads), smem, st, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 

@@ -429,6 +429,40 @@ def test_sparse_mla_matches_reference(nh, D, R_, fp8):
     assert rel_err(out2, ref2) < 1e-2
 
 
+@pytest.mark.parametrize("nh,T", [(8, 700), (32, 331), (64, 460)])
+def test_sparse_mla_several_tokens_per_thread_block(nh, T):
+    """More tokens than SMs, with lists of no rows, of one, of whole blocks and of parts of them next to one another, tokens without
+    any at the beginning and the end of a thread block's share, slots of -1 inside; the second half of the lists from another cache."""
+    D, R_, W, K, n = 512, 64, 128, 300, 1024
+    g = torch.Generator().manual_seed(T)
+    caches = []
+    for _ in range(2):
+        ccpu = C.PagedCache.allocate(n // 64, D, R_, True, "latent", "cpu")
+        ccpu.write_rows_cpu(torch.arange(n), torch.randn(n, D, generator=g))
+        caches.append((ccpu.read_rows_cpu(torch.arange(n))[0].double().to(dev()), C.PagedCache(ccpu.buf.to(dev()), D, R_, True, "latent")))
+    q = torch.randn(T, nh, D, generator=g).to(dev()).to(BF16)
+    slots = torch.randint(0, n, (T, W), generator=g, dtype=torch.int32).to(dev())
+    tops = torch.randint(0, n, (T, K), generator=g, dtype=torch.int32).to(dev())
+    tops[:, 7::31] = -1
+    lens = torch.tensor([0, 1, 127, 128, 64, 0, 128])[torch.arange(T) % 7].to(torch.int32).to(dev())
+    tlens = torch.tensor([0, 300, 129, 0, 128])[torch.arange(T) % 5].to(torch.int32).to(dev())
+    lens[:150] = torch.where(torch.arange(150, device=dev()) % 3 == 0, 0, lens[:150])
+    tlens[:150] = torch.where(torch.arange(150, device=dev()) % 3 == 0, 0, tlens[:150])
+    lens[-20:], tlens[-20:] = 0, 0
+    sink = torch.randn(nh, device=dev())
+    out = A.sparse_mla(q, caches[0][1], slots, lens, caches[1][1], tops, tlens, sink, D ** -0.5)
+    kv = torch.cat([caches[0][0][slots.long()], caches[1][0][tops.clamp(min=0).long()]], 1)
+    at = torch.arange(W + K, device=dev())[None]
+    there = torch.where(at < W, at < lens[:, None], at - W < tlens[:, None]) & torch.cat([slots >= 0, tops >= 0], 1)
+    s = (q.double() @ kv.transpose(1, 2) * D ** -0.5).masked_fill(~there[:, None], -math.inf)
+    p = torch.softmax(torch.cat([s, sink.double()[None, :, None].expand(T, -1, 1)], 2), 2)[:, :, :-1]
+    ref = p @ kv
+    assert rel_err(out, ref) < 3e-3                       # output rounded to bf16, weights to fp16
+    none = (lens + tlens) == 0
+    assert bool((out[none] == 0).all()) and rel_err(out[-21:], ref[-21:]) < 4e-3
+    _lib.check_status()
+
+
 @pytest.mark.parametrize("nh", [8, 64])
 @pytest.mark.parametrize("off", [0, 4])
 def test_sparse_mla_rows_beyond_fp16(nh, off):
