@@ -1081,6 +1081,25 @@ def test_gemm_bf16_pairs_of_ctas(T, N, K):
     _lib.check_status()
 
 
+@pytest.mark.parametrize("T", [9, 16, 17, 33, 64])
+@pytest.mark.parametrize("N,K,groups", [(1024, 4096, 1), (1000, 2080, 1), (4096, 2048, 1), (9000, 576, 1), (1024, 1024, 8), (512, 2112, 2)])
+def test_gemm_bf16_small_clusters(T, N, K, groups):
+    """Two, four and eight CTAs per 128-row tile, parts of K that are uneven or empty, a last tile that is not whole, block-diagonal
+    weights; every width of the token tile, results in rows of a wider matrix."""
+    torch.manual_seed(T + N)
+    assert _lib.query("stk_gemm_token_tile_ctas", T, N, K, 0, _lib.sm_count()) in (2, 4, 8)
+    w = (torch.randn(N, K, device=dev()) * 0.05).to(BF16)
+    x = torch.randn(T, K * groups, device=dev()).to(BF16)
+    m = N // groups
+    ref = torch.cat([x[:, g * K:(g + 1) * K].double() @ w[g * m:(g + 1) * m].double().t() for g in range(groups)], 1)
+    assert rel_err(Fn.linear(x, Fn.LinearWeight(w), groups=groups), ref) < 2.5e-3
+    wide = torch.full((T, N + 5), 7.0, dtype=F32, device=dev())
+    Fn.linear(x, Fn.LinearWeight(w), out=wide[:, :N], groups=groups)
+    assert rel_err(wide[:, :N], ref) < 2e-5               # fp32 sums
+    assert bool((wide[:, N:] == 7.0).all())
+    _lib.check_status()
+
+
 @pytest.mark.parametrize("T", [130, 600])
 @pytest.mark.parametrize("groups,n,K", [(2, 256, 128), (3, 512, 1024), (8, 128, 256)])
 def test_gemm_bf16_wide_block_diagonal(T, groups, n, K):
@@ -1139,6 +1158,34 @@ def test_moe_grouped_gemm_uneven_experts(H, I, E, counts):
         g, u = h[:, :I].clamp(max=10.0), h[:, I:].clamp(-10.0, 10.0)
         ref[rows] = (g * torch.sigmoid(g) * u) @ R.dequant_nvfp4(ew.w2[e], ew.s2[e].view(f8), ew.g2[e]).double().t() * w[rows].double()
     assert rel_err(out, ref) < 5e-3                     # activations rounded to fp16 in between, expert outputs and sums to bf16
+
+
+@pytest.mark.parametrize("H,I,T,k,start,local", [(4096, 2048, 1, 6, 0, 32), (1024, 640, 8, 6, 8, 8), (160, 1056, 3, 2, 0, 16), (7168, 2112, 2, 4, 4, 5), (512, 1024, 5, 3, 16, 4)])
+def test_moe_direct_pairs(H, I, T, k, start, local):
+    """A handful of pairs without a sort: widths that end inside a warp's pass and of one to eight passes, outputs that the thread
+    blocks do not divide, few, some or no pairs with local experts (the rest adds nothing)."""
+    torch.manual_seed(H + T)
+    E, f8 = 16, torch.float8_e4m3fn
+    scale = lambda *shape: (0.05 + torch.rand(*shape, device=dev())).to(f8).view(torch.uint8)
+    code = lambda *shape: torch.randint(0, 256, shape, dtype=torch.uint8, device=dev())
+    ew = M.ExpertWeights(code(local, 2 * I, H // 2), code(local, H, I // 2), scale(local, 2 * I, H // 16), scale(local, H, I // 16),
+                         0.02 + 0.02 * torch.rand(local, device=dev()), 0.02 + 0.02 * torch.rand(local, device=dev()), expert_start=start)
+    x = torch.randn(T, H, device=dev()).to(BF16)
+    ids = torch.stack([torch.randperm(E)[:k] for _ in range(T)]).to(torch.int32).to(dev())
+    w = torch.rand(T, k, device=dev()) + 0.5
+    shared = torch.randn(T, H, device=dev()).to(BF16)
+    out = M.moe_experts(x, ids, w, ew, 10.0, shared, E)
+    ref = shared.double()
+    for t in range(T):
+        for j in range(k):
+            e = int(ids[t, j]) - start
+            if not 0 <= e < local:
+                continue
+            h = x[t].double() @ R.dequant_nvfp4(ew.w13[e], ew.s13[e].view(f8), ew.g13[e]).double().t()
+            g, u = h[:I].clamp(max=10.0), h[I:].clamp(-10.0, 10.0)
+            ref[t] += (g * torch.sigmoid(g) * u) @ R.dequant_nvfp4(ew.w2[e], ew.s2[e].view(f8), ew.g2[e]).double().t() * w[t, j].double()
+    assert rel_err(out, ref) < 6e-3                       # fp16 sums of sixteen products, activations in fp16, outputs in bf16
+    _lib.check_status()
 
 
 @pytest.mark.parametrize("H,I,E", [(512, 256, 6), (384, 128, 36), (128, 128, 6)])
