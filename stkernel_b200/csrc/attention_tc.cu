@@ -366,8 +366,8 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
       ok = __all_sync(0xffffffffu, ok && mbar_wait(&bars->s_full, ph, a.status, 610) && mbar_wait(&bars->k_full[3], ph, a.status, 612));
       if (b == 0 && threadIdx.x == 128) STK_TRACE(3);
       tc_fence_after();
-      const int mark = lift_s[row], lift = max(mark, 0);
-      const bool valid = mark >= 0;
+      const int row_slot = lift_s[row], lift = max(row_slot, 0);   // -1: no slot in this row
+      const bool valid = row_slot >= 0;
       const float liftf = static_cast<float>(lift), sl = sl2 * __int_as_float((127 + lift) << 23), back = __int_as_float((127 - lift) << 23);
       const uint64_t sl22 = pack2(sl, sl), lift2 = pack2(liftf, liftf), back2 = pack2(back, back);
       // Whether a weight would pass 2^kSlack with the maxima in use
@@ -596,12 +596,12 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
     uint2 sc8;
     const uint8_t* src_row;                                // row whose codes are in `raw`; nullptr: none
     // The item, its blocks, and the list's next row of this lane (registers are short here: no more is kept)
-    int at, t = 0, n_swa = 0, r_end = 0, n_blocks = 0, li = 0, slot_next = -1;
+    int at, t = 0, n_swa = 0, r_end = 0, n_blocks = 0, li = 0, next_slot = -1;
     constexpr int kWindow = 1 << 30;                       // marks a slot of the first cache (a slot is far below)
-    auto look_up = [&]() {                                 // li -> slot_next, and on to the same row of the next block
-      slot_next = -1;
-      if (li < n_swa && li < r_end) slot_next = a.swa_slots[static_cast<long long>(t) * a.swa_ld + li] | kWindow;
-      else if (li < r_end) slot_next = a.topk_slots[static_cast<long long>(t) * a.topk_ld + (li - n_swa)];
+    auto look_up = [&]() {                                 // li -> next_slot, and on to the same row of the next block
+      next_slot = -1;
+      if (li < n_swa && li < r_end) next_slot = a.swa_slots[static_cast<long long>(t) * a.swa_ld + li] | kWindow;
+      else if (li < r_end) next_slot = a.topk_slots[static_cast<long long>(t) * a.topk_ld + (li - n_swa)];
       li += kRows;
     };
     auto enter = [&](int from) {
@@ -616,12 +616,12 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
       look_up();
     };
     enter(blockIdx.x);
-    auto next_row = [&]() {                                // slot_next -> row to be fetched; slot of the block after
-      const int slot = slot_next & ~kWindow;
-      const bool swa = (slot_next & kWindow) != 0;
+    auto next_row = [&]() {                                // next_slot -> row to be fetched; slot of the block after
+      const int slot = next_slot & ~kWindow;
+      const bool swa = (next_slot & kWindow) != 0;
       src_row = nullptr;
       sc8 = make_uint2(0, 0);
-      if (slot_next >= 0) {
+      if (next_slot >= 0) {
         const uint8_t* page = (swa ? a.swa_base : a.comp_base) + static_cast<long long>(slot >> 6) * (swa ? a.swa_stride : a.comp_stride);
         src_row = page + (slot & 63) * kDataBytes + l4 * 16;
         sc8 = *reinterpret_cast<const uint2*>(page + 64 * kDataBytes + (slot & 63) * 8);
