@@ -1471,6 +1471,174 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
 }
 
 // ---------------------------------------------------------------------------------
+// bf16, up to 128 tokens under weights of few 128-row tiles: a cluster of S CTAs shares a tile, each with its part of K.  TMEM lanes are
+// weight rows, columns tokens; CTA j finishes the j-th part of the tokens, to which the others bring their sums through distributed
+// shared memory, added in the order of the ranks.
+//
+// What bounds it: at 17 MB of weights (2.6 us of memory) the fixed costs, of which the meeting in an fp32 workspace -- sums out, a
+// counter, the last CTA reading them all back -- was the largest.  Measured, us, workspace splits / cluster:
+//   9 tokens x 1024 x 4096: 9.5 / 4.8;  32 x 4096 x 2048: 12.1 / 6.1;  x 4096 x 8192: 20.5 / 14.1;
+//   64 x 1024 x 4096: 22.4 / 6.6;  x 2048 x 4096: 19.8 / 8.8;  x 8192 x 2048: 20.6 / 10.2.
+// 256 x 256 tiles / cluster: 128 x 1024 x 4096: 19.7 / 8.8;  x 2048 x 4096: 20.4 / 11.2;  x 4096 x 2048: 16.2 / 10.0;
+//   x 4096 x 8192: 31.7 / 18.4.
+// ---------------------------------------------------------------------------------
+struct SmallArgs {
+  int T, N, k_blocks;
+  void* out;
+  long long ldo;
+  int out_fp32;
+  int* status;
+  int group_tiles, group_k;            // block-diagonal weights: tile / group_tiles is the block (0: one block)
+};
+
+template <int BT, int S>
+struct SmallCfg {
+  static constexpr int kStageBytes = 128 * 128 + BT * 128;
+  static constexpr int kStages = BT == 128 ? 5 : BT == 64 ? 6 : 8;
+  static constexpr int kShare = BT / S;                                 // token columns that a CTA finishes
+  static constexpr int kMeetBytes = (S - 1) * kShare * 128 * 4;         // [sender][column][weight row]
+  static constexpr int kSmem = kStages * kStageBytes + kMeetBytes + 256 + 1024;
+  static_assert(kSmem <= 227 * 1024, "shared memory");
+};
+
+template <int BT, int S>
+__global__ void __launch_bounds__(192, 1)
+gemm_small_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const SmallArgs a) {
+  using Cfg = SmallCfg<BT, S>;
+  constexpr int kStages = Cfg::kStages, kShare = Cfg::kShare;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem_x = smem + kStages * 128 * 128;
+  uint8_t* meet = smem_x + kStages * BT * 128;
+  GemmBarriers* bars = reinterpret_cast<GemmBarriers*>(meet + Cfg::kMeetBytes);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = static_cast<int>(blockIdx.x) % S, tile = static_cast<int>(blockIdx.x) / S;
+  const int per = (a.k_blocks + S - 1) / S, k_begin = min(a.k_blocks, rank * per), k_end = min(a.k_blocks, k_begin + per);
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kStages; ++i) {
+      mbar_init(&bars->full[i], 1);
+      mbar_init(&bars->empty[i], 1);
+    }
+    mbar_init(&bars->tmem_full[0], 1);
+    fence_barrier_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(&bars->tmem_base, BT < 32 ? 32 : BT);
+    tmem_relinquish();
+  }
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmX);
+    // weights are immutable: this CTA's first tiles are on their way to L2 while the kernel before finishes
+    for (int kb = k_begin; kb < min(k_end, k_begin + kStages); ++kb) tma_prefetch_2d(&tmW, kb * 64, tile * 128);
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = bars->tmem_base;
+  pdl_wait();
+  pdl_trigger();
+  if (warp == 0) {
+    if (lane == 0) {
+      const int gx = a.group_tiles ? tile / a.group_tiles * a.group_k : 0;
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int kb = k_begin; kb < k_end; ++kb) {
+        if (!mbar_wait(&bars->empty[stage], phase ^ 1, a.status, 100 + stage)) break;
+        mbar_expect_tx(&bars->full[stage], Cfg::kStageBytes);
+        tma_load_2d(smem + stage * 128 * 128, &tmW, &bars->full[stage], kb * 64, tile * 128);
+        tma_load_2d(smem_x + stage * BT * 128, &tmX, &bars->full[stage], gx + kb * 64, 0);
+        if (++stage == kStages) { stage = 0; phase ^= 1; }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    const uint32_t lead = elect_one() ? 1u : 0u, tm = __shfl_sync(0xffffffffu, tmem_base, 0);
+    const uint32_t w_lo = desc_lo(smem_u32(smem)), x_lo = desc_lo(smem_u32(smem_x));
+    constexpr uint32_t kIdesc = umma_idesc(1u, 1u, 128, BT);
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int kb = k_begin; kb < k_end; ++kb) {
+      if (!mbar_wait(&bars->full[stage], phase, a.status, 300 + stage)) break;
+      tc_fence_after();
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        mma_ss(tm, w_lo + stage * 1024 + 2 * k, x_lo + stage * (BT * 8) + 2 * k, kIdesc, (kb > k_begin || k > 0) ? 1u : 0u, lead);
+      mma_commit(&bars->empty[stage], lead);
+      if (++stage == kStages) { stage = 0; phase ^= 1; }
+    }
+    mma_commit(&bars->tmem_full[0], lead);
+    __syncwarp();
+  }
+  cluster_sync_all();                                      // every CTA runs: its meeting place may be written
+  bool ok = true;
+  const int q = warp & 3, row = q * 32 + lane;
+  uint32_t r[BT];
+  if (warp >= 2) {
+    ok = __all_sync(0xffffffffu, mbar_wait(&bars->tmem_full[0], 0, a.status, 400));
+    tc_fence_after();
+#pragma unroll
+    for (int c = 0; c < BT; c += 16) {
+      uint32_t t16[16];
+      tmem_ld_32x16(tmem_base + c + (static_cast<uint32_t>(q * 32) << 16), t16);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) r[c + i] = t16[i];
+    }
+    tmem_ld_wait();
+    if (k_begin < k_end) {
+#pragma unroll
+      for (int j = 0; j < S; ++j) {
+        if (j != rank) {
+          const uint32_t to = peer_addr(smem_u32(meet) + ((rank < j ? rank : rank - 1) * kShare * 128 + row) * 4, j);
+#pragma unroll
+          for (int c = 0; c < kShare; ++c) asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(to + c * 512), "r"(r[j * kShare + c]) : "memory");
+        }
+      }
+    }
+  }
+  cluster_sync_all();                                      // all sums have arrived
+  if (warp >= 2 && ok) {
+    const int n = tile * 128 + row;
+    float v[kShare];
+#pragma unroll
+    for (int c = 0; c < kShare; ++c) v[c] = 0.f;
+#pragma unroll
+    for (int j = 0; j < S; ++j) {
+      if (j * per >= a.k_blocks) continue;                 // a part of K without blocks
+      if (j == rank) {
+#pragma unroll
+        for (int o = 0; o < S; ++o)
+          if (o == rank) {
+#pragma unroll
+            for (int c = 0; c < kShare; ++c) v[c] += __uint_as_float(r[o * kShare + c]);
+          }
+      } else {
+        const float* from = reinterpret_cast<const float*>(meet) + (j < rank ? j : j - 1) * kShare * 128 + row;
+#pragma unroll
+        for (int c = 0; c < kShare; ++c) v[c] += from[c * 128];
+      }
+    }
+    if (n < a.N) {
+#pragma unroll
+      for (int c = 0; c < kShare; ++c) {
+        const int t = rank * kShare + c;
+        if (t < a.T) {
+          const long long o = static_cast<long long>(t) * a.ldo + n;
+          if (a.out_fp32) reinterpret_cast<float*>(a.out)[o] = v[c];
+          else reinterpret_cast<__nv_bfloat16*>(a.out)[o] = __float2bfloat16(v[c]);
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, BT < 32 ? 32 : BT);
+  }
+}
+
+// ---------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -1610,10 +1778,10 @@ STK_API long long stk_gemm_workspace_bytes(int T, int N, int splits) {
 }
 
 // CTAs that share a 256 x 256 tile of a token-major kernel: four with a part of K each where that keeps the SMs to one round (with at
-// least four K blocks each), else a pair (1 and 2 here); or 0 where the kernel above is better: up to 64 tokens.  A call that asks for
-// workspace splits keeps the kernel above.  Measured, us, kernel above with the split that it would ask for / these:
-//   64 tokens x 4096 x 8192: 26 / 31;  x 4096 x 2048: 18 / 16;  80 tokens x 4096 x 8192: 47 / 31;  x 2048 x 4096: 33 / 20;
-//   x 32768 x 1536: 66 / 24;  128 x 2048 x 4096: 38 / 20;  777 x 4096 x 4096: 66 / 27;  1500 x 4096 x 4096: 113 / 47.
+// least four K blocks each), else a pair (1 and 2 here); or 0 up to 64 tokens, where a tile would be mostly padding.  Up to 128 tokens
+// clusters on 128-row tiles come first where those leave SMs idle (small_split_of).  A call that asks for workspace splits keeps the
+// kernel above.  Measured, us, kernel above with the split that it would ask for / these:
+//   80 tokens x 32768 x 1536: 66 / 24;  777 x 4096 x 4096: 66 / 27;  1500 x 4096 x 4096: 113 / 47.
 static int wide_split_of(int T, int N, int K, int sm_count) {
   if (T <= 64) return 0;
   const int units = ((T + 255) / 256) * ((N + 255) / 256), kb = (K * 2 + 127) / 128;
@@ -1630,6 +1798,22 @@ static int launch_wide(const CUtensorMap& tx, const CUtensorMap& tw, const WideA
     configured = true;
   }
   return launch_cluster(gemm_wide_kernel, 4, a.tiles_n * a.tiles_t * 4, 320, smem, st, tw, tx, a);
+}
+
+template <int BT, int S>
+static int launch_small_s(const CUtensorMap& tw, const CUtensorMap& tx, const SmallArgs& a, int tiles, cudaStream_t st) {
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(gemm_small_kernel<BT, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, SmallCfg<BT, S>::kSmem) != cudaSuccess) return -3;
+    configured = true;
+  }
+  return launch_cluster(gemm_small_kernel<BT, S>, S, tiles * S, 192, SmallCfg<BT, S>::kSmem, st, tw, tx, a);
+}
+template <int BT>
+static int launch_small(const CUtensorMap& tw, const CUtensorMap& tx, const SmallArgs& a, int split, int tiles, cudaStream_t st) {
+  if (split == 8) return launch_small_s<BT, 8>(tw, tx, a, tiles, st);
+  if (split == 4) return launch_small_s<BT, 4>(tw, tx, a, tiles, st);
+  return launch_small_s<BT, 2>(tw, tx, a, tiles, st);
 }
 
 static int launch_pair(const CUtensorMap& tx, const CUtensorMap& tw, const WideArgs& a, int sm_count, cudaStream_t st) {
@@ -1678,11 +1862,25 @@ static bool fp8_pair_serves(int T, int N, int sm_count) {
   return 2 * paired <= single;
 }
 
-// Which token-major tiles a plain product (one block, no fused collective) without workspace splits takes: the number of CTAs that
-// share one, or 0 for the 128-row tiles.
+// CTAs that share a 128-row tile of up to 128 tokens (as many as keep the SMs to one round, with at least four K blocks each), or 1: no
+// split, the persistent kernel above.  Clusters of eight only where they ask for half of the SMs: sixteen of them do not run at once
+// (2048 x 4096, 9 tokens: 9.6 us against 4.8 for eight of them on 1024 x 4096).
+static int small_split_of(int T, int N, int K, int sm_count) {
+  if (T > 128) return 1;
+  const int tiles = (N + 127) / 128, kb = (K * 2 + 127) / 128;
+  int s = tiles * 16 <= sm_count ? 8 : 4;
+  while (s > 1 && (tiles * s > sm_count || kb < 4 * s)) s /= 2;
+  return s;
+}
+
+// Which tiles a plain product (no fused collective) without workspace splits takes: the number of CTAs that share one through a
+// cluster or as a pair, or 0 for 128-row tiles of one CTA each.  (For 65 to 128 bf16 tokens the answer is that for the 256 x 256 tiles:
+// it is never 0, and small_split_of may still put the product on 128-row tiles.)
 STK_API int stk_gemm_token_tile_ctas(int T, int N, int K, int is_fp8, int sm_count) {
   if (is_fp8) return fp8_tokens_split(T, N, K, sm_count);
-  return gemm_wide_enabled() ? wide_split_of(T, N, K, sm_count) : 0;
+  if (!gemm_wide_enabled()) return 0;
+  const int small = T <= 64 ? small_split_of(T, N, K, sm_count) : 1;
+  return small > 1 ? small : wide_split_of(T, N, K, sm_count);
 }
 
 static int gemm_launch(const void* W, long long ldw, const void* X, long long ldx, void* out, long long ldo, int T, int N,
@@ -1723,6 +1921,24 @@ static int gemm_launch(const void* W, long long ldw, const void* X, long long ld
       case 2: return launch_fp8_tokens<2>(ta, tb, a, sm_count, st);
       default: return launch_fp8_tokens<1>(ta, tb, a, sm_count, st);
     }
+  }
+  const int small_split = groups == 1 || (N % (128 * groups) == 0 && K % 64 == 0) ? small_split_of(T, N, K, sm_count) : 1;
+  if (!is_fp8 && ar_ctx == nullptr && gate_ctx == nullptr && splits <= 1 && bt_override == 0 && small_split > 1 && gemm_wide_enabled()) {
+    const int tiles = (N + 127) / 128, columns = T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : 128;
+    CUtensorMap tw3, tx3;
+    if (make_tmap_2d(&tw3, W, 2, N, K, ldw, 128) != 0) return -13;
+    if (make_tmap_2d(&tx3, X, 2, T, static_cast<long long>(K) * groups, ldx, columns) != 0) return -14;
+    SmallArgs sa;
+    sa.T = T; sa.N = N;
+    sa.k_blocks = (K * 2 + 127) / 128;
+    sa.out = out; sa.ldo = ldo; sa.out_fp32 = out_fp32; sa.status = status;
+    sa.group_tiles = groups > 1 ? N / groups / 128 : 0;
+    sa.group_k = K;
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    if (columns == 16) return launch_small<16>(tw3, tx3, sa, small_split, tiles, st);
+    if (columns == 32) return launch_small<32>(tw3, tx3, sa, small_split, tiles, st);
+    if (columns == 64) return launch_small<64>(tw3, tx3, sa, small_split, tiles, st);
+    return launch_small<128>(tw3, tx3, sa, small_split, tiles, st);
   }
   // block-diagonal weights take the wide tiles where blocks are whole tiles and whole 128-byte steps of K
   const int wide_split = (groups == 1 || (N % (256 * groups) == 0 && K % 64 == 0)) ? wide_split_of(T, N, K, sm_count) : 0;

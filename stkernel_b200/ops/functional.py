@@ -243,8 +243,8 @@ def linear(x, lw: LinearWeight, out: Optional[torch.Tensor] = None, out_dtype=BF
     is_fp8 = 1 if lw.is_fp8 else 0
     sms = _lib.sm_count()
     if splits is None:
-        # token-major tiles split K over clusters, without a workspace
-        plain = groups == 1 and ar_ctx is None
+        # clusters split K without a workspace, also of block-diagonal weights of whole tiles and 128-byte steps of K
+        plain = ar_ctx is None and (groups == 1 or (not is_fp8 and t <= 128 and n % (128 * groups) == 0 and k % 64 == 0))
         splits = 1 if plain and _lib.query("stk_gemm_token_tile_ctas", t, n, k, is_fp8, sms) else _lib.query("stk_gemm_pick_splits", t, n, k, is_fp8, sms)
     ws = cnt = None
     if splits > 1:

@@ -1081,7 +1081,7 @@ def test_gemm_bf16_pairs_of_ctas(T, N, K):
     _lib.check_status()
 
 
-@pytest.mark.parametrize("T", [9, 16, 17, 33, 64])
+@pytest.mark.parametrize("T", [9, 16, 17, 33, 64, 65, 128])
 @pytest.mark.parametrize("N,K,groups", [(1024, 4096, 1), (1000, 2080, 1), (4096, 2048, 1), (9000, 576, 1), (1024, 1024, 8), (512, 2112, 2)])
 def test_gemm_bf16_small_clusters(T, N, K, groups):
     """Two, four and eight CTAs per 128-row tile, parts of K that are uneven or empty, a last tile that is not whole, block-diagonal
