@@ -340,7 +340,7 @@ skinny_linear_kernel(const uint8_t* __restrict__ W, long long ldw_bytes, const f
 using namespace stk;
 
 // T <= 8.  K must be a multiple of 16 (fp8) / 8 (bf16); rows 16-byte aligned.
-// STK_SKINNY_MMA=0 keeps five to eight tokens on the CUDA-core kernel (A/B runs)
+// STK_SKINNY_MMA=0 keeps every batch on the CUDA-core kernel (A/B runs)
 static bool stk_skinny_mma_enabled() {
   static int v = -1;
   if (v < 0) {
@@ -359,8 +359,13 @@ static int skinny_launch(const void* W, long long ldw, int is_fp8, const float* 
   if (K % 16 || K > 16384) return -1;
   const long long ldw_bytes = ldw * (is_fp8 ? 1 : 2);
   if (ldw_bytes % 16 || (reinterpret_cast<uintptr_t>(W) & 15)) return -2;
-  // five to eight tokens: the eight-token warp-level tensor-core stream (skinny_mma.cuh)
-  if (T > 4 && !ex.route && stk_skinny_mma_enabled())
+  // The eight-token warp-level tensor-core stream (skinny_mma.cuh): five to eight tokens, and fewer under bf16 weights of a form that it
+  // takes.  (fp8 weights of up to four tokens stay here: their activations are not quantised.)
+  const bool few = T <= 4 && !is_fp8 && ex.k_split <= 1 && N % 16 == 0 && K % 128 == 0 && K <= 8192 && ldx % 8 == 0 &&
+                   (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(ex.norm_w) & 15) == 0 &&
+                   ((ex.norm_w == nullptr && !ex.use_ll) || (groups <= 1 && !swiglu)) && (groups <= 1 || (N / groups) % 16 == 0) &&
+                   (!ex.use_ll || static_cast<long long>(T) * N / 2 <= ex.ll.words);
+  if ((T > 4 || few) && !ex.route && stk_skinny_mma_enabled())
     return skinny_mma_launch(W, ldw_bytes, is_fp8, w_scale, w_scale_ld, x, ldx, out, ldo, T, N, K, out_fp32, groups, swiglu,
                              limit, ex, (cudaStream_t)stream);
   const int iters16 = ((K / 16) + 31) / 32;

@@ -1,4 +1,4 @@
-// Weight-streaming projection for 5..8 tokens (speculative verification rows, small decode batches).
+// Weight-streaming projection for 5..8 tokens (speculative verification rows, small decode batches), and for 1..4 under bf16 weights.
 //
 // At these sizes the op is still a stream over the weight matrix (a few MB, once), but the CUDA-core dot products of
 // the 1..4-token kernel pay tokens x the shared-memory reads and multiplies, and a tcgen05 tile pays its fixed costs
@@ -16,6 +16,10 @@
 // fp8: activations are quantised per (token, 128 values) exactly like the tensor-core GEMM path (scale = amax / 448)
 // by the CTA itself in its prologue (optionally after the fused RMSNorm), each 64-byte block is accumulated on its
 // own and folded into the fp32 result with w_scale x x_scale (two-level accumulation).
+//
+// One to four tokens, bf16: the dot products of the CUDA-core kernel cost about as much as the stream for one token and twice as much for
+// four.  Measured, us with a cold L2, CUDA cores / here: 129280 x 4096, 1 token 279 / 168 (6.3 TB/s), 4 tokens 463 / 174;
+// 4096 x 8192, 38.9 / 22.6 and 59.6 / 24.6;  32768 x 1536, 41.1 / 30.8 and 59.5 / 32.8;  1024 x 4096, 11.1 / 10.3 and 16.4 / 10.2.
 //
 // Shares `SkinnyExtra` (norm prologue, folded all-reduce push) and the SwiGLU / grouped modes with skinny.cu, which
 // includes this file.
@@ -46,9 +50,13 @@ __device__ __forceinline__ void mma_bf16_16x8x16(float (&d)[4], uint32_t a0, uin
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// Shared-memory layout (dynamic): activation rows [8][row_bytes + 64] (the pad spreads the eight rows over the banks),
+// Shared-memory layout (dynamic): activation rows [slots][row_bytes + 64] (the pad spreads the rows over the banks; the batch's rows and,
+// below eight, one of zeros that the remaining token slots of the mma share: with one token a CTA takes a quarter of the space, and more
+// of them reside on an SM),
 // then fp8 only: x scales [8][K / 128] floats, then the cross-warp reduction buffer [8 warps][16][8] floats, then the
 // staging area of the prologue (fp8: the raw bf16 rows [T][2K]; with the fused norm: its weights [2K bytes]).
+__host__ __device__ constexpr int smma_slots(int T) { return T < kSmTokens ? T + 1 : kSmTokens; }
+
 template <bool kFp8, bool kSwiglu>
 __global__ void __launch_bounds__(kSmWarps * 32, 2)
 skinny_mma_kernel(const uint8_t* __restrict__ W, long long ldw_bytes, const float* __restrict__ w_scale, int w_scale_ld,
@@ -59,8 +67,6 @@ skinny_mma_kernel(const uint8_t* __restrict__ W, long long ldw_bytes, const floa
   const int xstride = row_bytes + 64;
   const int kgroups = K >> 7;
   uint8_t* xs = sm_raw;
-  float* xsc = reinterpret_cast<float*>(sm_raw + kSmTokens * xstride);
-  float* red = xsc + (kFp8 ? kSmTokens * kgroups : 0);
   __shared__ float s_nr[kSmTokens];
   __shared__ float s_ss[kSmWarps][kSmTokens];
 
@@ -72,6 +78,8 @@ skinny_mma_kernel(const uint8_t* __restrict__ W, long long ldw_bytes, const floa
   // more than eight tokens (narrow weights only, see the launcher): blockIdx.y picks a group of eight
   const int t_base = blockIdx.y * kSmTokens;
   const int T = min(kSmTokens, T_all - t_base);
+  float* xsc = reinterpret_cast<float*>(sm_raw + smma_slots(T_all) * xstride);
+  float* red = xsc + (kFp8 ? kSmTokens * kgroups : 0);
   const __nv_bfloat16* xg = x + static_cast<long long>(grp) * K + static_cast<long long>(t_base) * ldx;
 
   uint4 a_lo[kSmBatch], a_hi[kSmBatch];
@@ -117,13 +125,10 @@ skinny_mma_kernel(const uint8_t* __restrict__ W, long long ldw_bytes, const floa
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(nw_s + kc * 16)), "l"(ex.norm_w + kc * 8)
                    : "memory");
   asm volatile("cp.async.commit_group;" ::: "memory");
-  // token slots beyond the batch: zeros (their results are never stored)
-  {
-    const int row16 = row_bytes >> 4;
-    for (int idx = threadIdx.x; idx < (kSmTokens - T) * row16; idx += blockDim.x) {
-      const int t = T + idx / row16, k16 = idx % row16;
-      *reinterpret_cast<uint4*>(xs + t * xstride + k16 * 16) = make_uint4(0, 0, 0, 0);
-    }
+  // token slots beyond the batch: one row of zeros (their results are never stored)
+  if (T < kSmTokens) {
+    for (int idx = threadIdx.x; idx < (row_bytes >> 4); idx += blockDim.x)
+      *reinterpret_cast<uint4*>(xs + T * xstride + idx * 16) = make_uint4(0, 0, 0, 0);
     if constexpr (kFp8)
       for (int idx = threadIdx.x; idx < (kSmTokens - T) * kgroups; idx += blockDim.x) xsc[T * kgroups + idx] = 0.f;
   }
@@ -211,6 +216,7 @@ skinny_mma_kernel(const uint8_t* __restrict__ W, long long ldw_bytes, const floa
   __syncthreads();
 
   // ---- the stream over this CTA's rows ----
+  const uint8_t* const x_row = xs + min(g, T) * xstride + c * 16;
   float res[kSwiglu ? 2 : 1] = {};
   const int r_out = threadIdx.x >> 3, t_out = threadIdx.x & 7;       // reduction mapping of threads 0..127
 #pragma unroll
@@ -223,7 +229,7 @@ skinny_mma_kernel(const uint8_t* __restrict__ W, long long ldw_bytes, const floa
       for (int i = 0; i < kSmBatch; ++i) {
         const int b = b0 + i * kSmWarps;
         if (b < nblk) {
-          const uint4 bx = *reinterpret_cast<const uint4*>(xs + g * xstride + b * 64 + c * 16);
+          const uint4 bx = *reinterpret_cast<const uint4*>(x_row + b * 64);
           if constexpr (kFp8) {
             float tmp[4] = {0.f, 0.f, 0.f, 0.f};
             mma_e4m3_16x8x32(tmp, a_lo[i].x, a_hi[i].x, a_lo[i].y, a_hi[i].y, bx.x, bx.y);
@@ -289,7 +295,7 @@ skinny_mma_kernel(const uint8_t* __restrict__ W, long long ldw_bytes, const floa
   }
 }
 
-// Host side: called by skinny_launch for 5..8 tokens.  Returns -20.. for shapes outside this kernel.
+// Host side: called by skinny_launch.  Returns -20.. for shapes outside this kernel.
 static int skinny_mma_launch(const void* W, long long ldw_bytes, int is_fp8, const float* w_scale, int w_scale_ld,
                              const void* x, long long ldx, void* out, long long ldo, int T, int N, int K, int out_fp32,
                              int groups, int swiglu, float limit, const SkinnyExtra& ex, cudaStream_t st) {
@@ -314,7 +320,7 @@ static int skinny_mma_launch(const void* W, long long ldw_bytes, int is_fp8, con
   }
   const int row_bytes = is_fp8 ? K : 2 * K;
   // activation rows + x scales + reduction buffer + staging (raw bf16 rows for the fp8 path, norm weights)
-  const size_t smem = static_cast<size_t>(kSmTokens) * (row_bytes + 64) + (is_fp8 ? kSmTokens * (K / 128) * 4 : 0) +
+  const size_t smem = static_cast<size_t>(smma_slots(T)) * (row_bytes + 64) + (is_fp8 ? kSmTokens * (K / 128) * 4 : 0) +
                       kSmWarps * kSmRows * kSmTokens * 4 + (is_fp8 ? static_cast<size_t>(T < kSmTokens ? T : kSmTokens) * 2 * K : 0) +
                       (ex.norm_w != nullptr ? 2 * K : 0);
   if (smem > 200 * 1024) return -24;

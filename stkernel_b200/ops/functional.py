@@ -108,7 +108,7 @@ def ll_reduce(p: LLPending) -> torch.Tensor:
     return out
 
 
-# largest batch served by the weight-streaming kernels: CUDA-core dot products up to four tokens, the eight-token
+# largest batch served by the weight-streaming kernels: CUDA-core dot products up to four tokens under fp8 weights, the eight-token
 # warp-level tensor-core stream above (speculative verification rows, small decode batches)
 SKINNY_MAX_T = min(8, int(_os.environ.get("STK_SKINNY_MAX_T", "8")))
 MHC_CLUSTER_MAX_T = int(_os.environ.get("STK_MHC_CLUSTER_MAX_T", "64"))

@@ -863,6 +863,28 @@ def test_skinny_linear(dtype, T, N, K):
     assert rel_err(out16, ref) < 1e-2
 
 
+@pytest.mark.parametrize("T", [1, 2, 3, 4])
+@pytest.mark.parametrize("N,K,groups", [(16, 128, 1), (48, 8192, 1), (4112, 384, 1), (64, 256, 4), (40, 256, 1), (48, 144, 1)])
+def test_skinny_bf16_few_tokens(T, N, K, groups):
+    """One to four tokens under bf16 weights: the smallest and largest K, rows and K of the other kernel (40 rows, K 144), groups, strided
+    rows and values beyond fp16.  A sum in fp32 of K products with partial sums in any order is off by at most K x 2^-24 of the sum of
+    magnitudes, a value of bf16 by 2^-8 of itself."""
+    torch.manual_seed(T + N)
+    x = (torch.randn(T, K * groups + 8, device=dev()) * 1e5).to(BF16)[:, :K * groups]
+    w = (torch.randn(N, K, device=dev()) * 0.05).to(BF16)
+    xd, wd = x.double().view(T, groups, K), w.double().view(groups, N // groups, K)
+    ref = torch.einsum("tgk,gnk->tgn", xd, wd).reshape(T, N)
+    slack = torch.einsum("tgk,gnk->tgn", xd.abs(), wd.abs()).reshape(T, N) * K * 2.0 ** -24
+    if groups > 1 or (N % 16 == 0 and K % 128 == 0):
+        lw = Fn.LinearWeight(w)
+        assert bool(((Fn.linear(x, lw, out_dtype=F32, groups=groups).double() - ref).abs() <= slack).all())
+        assert bool(((Fn.linear(x, lw, groups=groups).double() - ref).abs() <= slack + ref.abs() * 2.0 ** -8).all())
+    else:                                          # fp16 activations: no larger than 65504
+        small = (x * 1e-5).to(BF16)
+        ref = small.double() @ w.double().t()
+        assert rel_err(Fn.linear(small, Fn.LinearWeight(w), out_dtype=F32), ref.float()) < 2e-3
+
+
 def test_skinny_linear_grouped():
     G, Ng, K, T = 8, 1024, 4096, 2
     x = torch.randn(T, G * K, device=dev()).to(BF16)
