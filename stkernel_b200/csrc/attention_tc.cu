@@ -11,8 +11,10 @@
 //   softmax warps    read S^T from TMEM (one row and half of the heads per thread), write P as the K-major B
 //                    operand, rescale in TMEM the columns of O whose head's maximum moved
 //
-// Operands are fp16: codes times a power of two are exact, weights keep three bits more than bf16 leaves them.  A row that passes
-// fp16's range is divided by a power of two, which its scores get back, and its weights carry it to the values (`lift`).
+// Operands are fp16: weights keep three bits more than bf16 leaves them, and values from 2^-14 to 2^16 all of theirs.  A row, or a
+// head's queries, whose largest magnitude lies outside 2^-8 .. 2^16 is divided by a power of two that brings it back (`range_shift`):
+// its scores get it back, and a row's weights carry it to the values (`lift`).  What is below 2^-14 beside something large in the same
+// row or head is held to 2^-25, a group of codes with a scale below 2^-24 to 2^-16: at most 2^-17 of the largest.
 //
 // What bounds it: the key block (128 KB in fp16) and Q (64 KB) fill shared memory, so there is one key buffer, and a block is
 // scores -> softmax -> values in turn.  Everything else is taken off that chain:
@@ -29,8 +31,8 @@
 // token, a block is 8200: thread blocks stay and walk through tokens, the next one's queries and first codes are fetched under this
 // one's last softmax, value products and output.
 // Measured (4096 tokens, 64 heads, 128 + 2048 rows): 5162 us with one thread block of thirteen warps working through
-// load -> scores -> softmax -> values without overlap, 2677 with bf16 operands, exact maxima in every block and two-byte stores of the
-// output, 2387 now; 128 rows alone: 576 -> 281.
+// load -> scores -> softmax -> values without overlap, 2677 with bf16 operands, exact maxima in every block and a branch per stored
+// value, 2403 now, 16 of them for looking at ranges; 128 rows alone: 576 -> 281.
 //
 // Accumulators live in TMEM: S (NH columns) and four O^T tiles of [128 dims x NH heads].
 // A CTA of a split writes an un-normalised partial (o, m, l) that `sparse_mla_combine` merges with the sink.
@@ -96,6 +98,7 @@ struct MlaCfg {
 };
 
 constexpr int kBarBytes = 192;
+constexpr int kNoRow = 1 << 20;       // `lift` of a place in the list without a row
 constexpr float kSlack = 1.5f;        // powers of two by which weights may pass the maxima in use before these are taken anew
 // Order in which panels are written and scored, and in which pairs of them are summed and freed: the rotated part (panel 7)
 // is freed first and needed last.
@@ -165,7 +168,26 @@ __device__ __forceinline__ uint4 bf16x8_to_half(const uint4& v, float f) {
   return o;
 }
 
+constexpr int kMostExponent = 142, kLeastExponent = 119;      // 2^15, 2^-8
+// Power of two that a row or a head is divided by, from the biased exponent of its largest magnitude: none from 2^-8 to below 2^16,
+// else what brings that to 2^15 or 2^1 (a row lifted no higher than ordinary ones leaves fp16's range to their weights).  `low`: it
+// holds a scale that fp16 does not, which asks for 2^1 as well.  Below 2^-98 it stays where 2^100 puts it: sums of weights times that
+// have to be finite in fp32.
+__device__ __forceinline__ int range_shift(int e, bool low) {
+  return e > kMostExponent ? e - kMostExponent : e >= (low ? 128 : kLeastExponent) || e == 0 ? 0 : max(e - 128, -100);
+}
+__device__ __forceinline__ float power_of_two(int e) { return __int_as_float((127 + e) << 23); }
+
 __device__ __forceinline__ uint32_t half2_bits(__half2 v) { return *reinterpret_cast<const uint32_t*>(&v); }
+
+// Eight bf16 values times a power of two (exact, but for what falls below bf16's own range)
+__device__ __forceinline__ uint4 bf16x8_times(uint4 v, float f) {
+  const __nv_bfloat162 f2 = __float2bfloat162_rn(f);
+  __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) h[i] = __hmul2(h[i], f2);
+  return v;
+}
 
 // Larger of the magnitudes of two words of bf16 pairs, by halves (their bits order as the magnitudes do)
 __device__ __forceinline__ uint32_t bf16x2_absmax(uint32_t a, uint32_t b) { return __vmaxu2(a & 0x7fff7fffu, b & 0x7fff7fffu); }
@@ -190,7 +212,8 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
   float* m_run = smax + 4 * NH;                          // [NH] the maxima in use, in powers of two
   float* minus_m = m_run + NH;                           // [NH] their negatives (0 for none yet)
   float* alpha_s = minus_m + NH;                         // [NH]
-  int* lift_s = reinterpret_cast<int*>(alpha_s + NH);    // [kRows] what the block's rows were divided by, in powers of two; -1: no row
+  int* lift_s = reinterpret_cast<int*>(alpha_s + NH);    // [kRows] what the block's rows were divided by, in powers of two; kNoRow: no row
+  float* q_mul = reinterpret_cast<float*>(lift_s + kRows);      // [2][NH] what the heads' queries were divided by, items in turn
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) STK_TRACE(0);
@@ -242,21 +265,50 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
     named_bar_sync(1, kThreads);
     tc_fence_after();
   };
-  // Q of a token -> shared memory, K-major panels [NH x 64 dims], 128-byte swizzled; heads >= nh are zero.  `who` of kLoaders threads.
-  auto load_q = [&](int t, int who, auto loaders) {
-    constexpr int kLoaders = decltype(loaders)::value, kChunks = NH * (kD / 8), kBatch = kChunks / kLoaders;
-    static_assert(kChunks % kLoaders == 0, "chunks of Q");
-    uint4 qv[kBatch];
+  // Q of a token -> shared memory, K-major panels [NH x 64 dims], 128-byte swizzled; heads >= nh are zero.  `who` of kLoaders threads,
+  // a warp to a head; `turn`: which of the two lists of powers of two the token's heads get.
+  auto load_q = [&](int t, int who, uint32_t turn, auto loaders) {
+    constexpr int kLoaders = decltype(loaders)::value, kWarps = kLoaders / 32, kMine = NH / kWarps;
+    static_assert(NH % kWarps == 0, "heads of a warp");
+    const int w = who >> 5, lane = who & 31;
+    uint4 qv[kMine][2];
 #pragma unroll
-    for (int j = 0; j < kBatch; ++j) {
-      const int i = who + j * kLoaders, h = i / (kD / 8), c8 = i % (kD / 8);
-      qv[j] = make_uint4(0, 0, 0, 0);
-      if (h < a.nh) qv[j] = __ldg(reinterpret_cast<const uint4*>(a.q + t * a.ldt + static_cast<long long>(h) * kD + c8 * 8));
+    for (int j = 0; j < kMine; ++j) {
+      const int h = w + j * kWarps;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        qv[j][i] = make_uint4(0, 0, 0, 0);
+        if (h < a.nh) qv[j][i] = __ldg(reinterpret_cast<const uint4*>(a.q + t * a.ldt + static_cast<long long>(h) * kD + (i * 32 + lane) * 8));
+      }
     }
+    // Largest magnitudes of the lane's parts.  Whether heads need a power of two is voted on; which one is asked only then (with the
+    // reductions and products for all, 4096 tokens took 29 us more).
+    uint32_t big[kMine], all = 0;
+    bool shifted = false;
 #pragma unroll
-    for (int j = 0; j < kBatch; ++j) {
-      const int i = who + j * kLoaders, h = i / (kD / 8), c8 = i % (kD / 8);
-      *reinterpret_cast<uint4*>(q_s + (c8 >> 3) * (NH * 128) + h * 128 + (((c8 & 7) ^ (h & 7)) << 4)) = bf16x8_to_half(qv[j], 1.f);
+    for (int j = 0; j < kMine; ++j) {
+      big[j] = __vmaxu2(__vmaxu2(bf16x2_absmax(qv[j][0].x, qv[j][0].y), bf16x2_absmax(qv[j][0].z, qv[j][0].w)),
+                        __vmaxu2(bf16x2_absmax(qv[j][1].x, qv[j][1].y), bf16x2_absmax(qv[j][1].z, qv[j][1].w)));
+      all = __vmaxu2(all, big[j]);
+      shifted |= !__any_sync(0xffffffffu, w + j * kWarps >= a.nh || max(big[j] & 0xffffu, big[j] >> 16) >= kLeastExponent << 7);
+    }
+    shifted |= __any_sync(0xffffffffu, max(all & 0xffffu, all >> 16) > (kMostExponent << 7 | 127));
+#pragma unroll
+    for (int j = 0; j < kMine; ++j) {
+      const int h = w + j * kWarps;
+      int shift = 0;
+      if (shifted) {
+        const uint32_t most = __reduce_max_sync(0xffffffffu, max(big[j] & 0xffffu, big[j] >> 16));
+        shift = range_shift(static_cast<int>(most >> 7), false);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) qv[j][i] = bf16x8_times(qv[j][i], power_of_two(-shift));
+      }
+      if (lane == 0) q_mul[turn * NH + h] = power_of_two(shift);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int c8 = i * 32 + lane;
+        *reinterpret_cast<uint4*>(q_s + (c8 >> 3) * (NH * 128) + h * 128 + (((c8 & 7) ^ (h & 7)) << 4)) = bf16x8_to_half(qv[j][i], 1.f);
+      }
     }
   };
   if (warp < 4) {
@@ -323,7 +375,7 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
       at = e.i;
       n_blocks = e.n_blocks;
     }
-    if (at < items) load_q(at % a.T, threadIdx.x - 128, std::integral_constant<int, kSoftmaxThreads>{});
+    if (at < items) load_q(at % a.T, threadIdx.x - 128, 0, std::integral_constant<int, kSoftmaxThreads>{});
     begin();
     const uint32_t tmem_s = bars->tmem_base, tmem_o = tmem_s + NH;       // S^T: NH columns; O^T: 4 x NH columns
     const int q4 = warp & 3;                              // TMEM lane quarter
@@ -360,19 +412,22 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
 #pragma unroll
     for (int i = 0; i < kHeads / 2; ++i) lp[i] = 0ull;
     if (own < NH) m_run[own] = -INFINITY;
+    bool lifted = false;                                  // a row of this item so far has a power of two (the same in every warp)
+    bool q_lifted = false;                                // a head of this warp has
+    const float* const qm = q_mul + (k & 1) * NH + h0;
     for (int b = 0; b < n_blocks; ++b, ++g) {
       const uint32_t ph = g & 1;
       // (the row's power of two was left before the first panel was handed over: a barrier that has long completed)
       ok = __all_sync(0xffffffffu, ok && mbar_wait(&bars->s_full, ph, a.status, 610) && mbar_wait(&bars->k_full[3], ph, a.status, 612));
       if (b == 0 && threadIdx.x == 128) STK_TRACE(3);
       tc_fence_after();
-      const int row_slot = lift_s[row], lift = max(row_slot, 0);   // -1: no slot in this row
-      const bool valid = row_slot >= 0;
-      const float liftf = static_cast<float>(lift), sl = sl2 * __int_as_float((127 + lift) << 23), back = __int_as_float((127 - lift) << 23);
-      const uint64_t sl22 = pack2(sl, sl), lift2 = pack2(liftf, liftf), back2 = pack2(back, back);
-      // Whether a weight would pass 2^kSlack with the maxima in use
-      bool over = b == 0 || (bars->unset[0] | bars->unset[1]) != 0;
+      const int row_lift = lift_s[row];
+      const bool valid = row_lift != kNoRow, has_lift = valid && row_lift != 0;
+      if (b == 0) q_lifted = __any_sync(0xffffffffu, qm[lane & (kHeads - 1)] != 1.f);
+      // Whether a weight would pass 2^kSlack with the maxima in use (not asked where powers of two are about)
+      bool over = b == 0 || (bars->unset[0] | bars->unset[1]) != 0 || lifted || q_lifted;
       if (!over) {
+        const uint64_t sl22 = pack2(sl2, sl2);
         float top = -INFINITY;
 #pragma unroll
         for (int c = 0; c < kHeads; c += 16) {
@@ -388,7 +443,7 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
             top = fmaxf(top, fmaxf(x, y));
           }
         }
-        over = valid && !(top + liftf <= kSlack);
+        over = (valid && !(top <= kSlack)) || has_lift;
       }
       if (bar_any(2, kSoftmaxThreads, over)) {
       // exact maxima of this block's rows per head, and the running ones
@@ -399,10 +454,25 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
         for (int c = 0; c < kHeads / 16; ++c) tmem_ld_32x16(tmem_s + lane_addr + h0 + 16 * c, raw[c]);
         tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < kHeads; ++i) s[i] = valid ? fmaf(__uint_as_float(raw[i / 16][i % 16]), sl, liftf) : -INFINITY;
+        for (int i = 0; i < kHeads; ++i) s[i] = valid ? __uint_as_float(raw[i / 16][i % 16]) * sl2 : -INFINITY;
+        if (q_lifted) {
+#pragma unroll
+          for (int i = 0; i < kHeads; i += 4) {
+            const float4 q4m = *reinterpret_cast<const float4*>(qm + i);
+            s[i] *= q4m.x;
+            s[i + 1] *= q4m.y;
+            s[i + 2] *= q4m.z;
+            s[i + 3] *= q4m.w;
+          }
+        }
+        if (has_lift) {
+          const float f = power_of_two(row_lift), l = static_cast<float>(row_lift);
+#pragma unroll
+          for (int i = 0; i < kHeads; ++i) s[i] = fmaf(s[i], f, l);
+        }
         bfly_reduce_store<kHeads, true>(s, smax + q4 * NH + h0, lane);
       }
-      named_bar_sync(2, kSoftmaxThreads);
+      lifted = bar_any(2, kSoftmaxThreads, has_lift) || lifted;
       if (own < (NH < 32 ? 32 : NH)) {                     // whole warps
         bool moved = false, unset = false;
         if (own < NH) {
@@ -447,32 +517,51 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
         tmem_st_wait();
       }
       }
-      // P = exp2(s - m), fp16, written as the K-major B operand [head][row]; the sums take the rounded values
+      // P = exp2(s - m), fp16, written as the K-major B operand [head][row].  The sums take the rounded values, unless powers of two are
+      // about: these move a maximum away from the largest weight, which may then be below what fp16 holds.
+      auto weights = [&](auto plain) {
+        constexpr bool kPlain = decltype(plain)::value;
+        const int lift = kPlain || !valid ? 0 : row_lift;
+        const float sl = sl2 * power_of_two(lift), liftf = static_cast<float>(lift), back = power_of_two(-lift);
+        const uint64_t sl22 = pack2(sl, sl), lift2 = pack2(liftf, liftf), back2 = pack2(back, back);
 #pragma unroll
-      for (int c = 0; c < kHeads; c += 16) {
-        uint32_t r16[16];
-        scores(c, r16);
-        if (valid) {
+        for (int c = 0; c < kHeads; c += 16) {
+          uint32_t r16[16];
+          scores(c, r16);
+          if (valid) {
 #pragma unroll
-          for (int i = 0; i < 16; i += 4) {
-            const ulonglong2 m4 = *reinterpret_cast<const ulonglong2*>(minus_m + h0 + c + i);
+            for (int i = 0; i < 16; i += 4) {
+              const ulonglong2 m4 = *reinterpret_cast<const ulonglong2*>(minus_m + h0 + c + i);
+              ulonglong2 q4m = make_ulonglong2(0ull, 0ull);
+              if constexpr (!kPlain) q4m = *reinterpret_cast<const ulonglong2*>(qm + c + i);
 #pragma unroll
-            for (int k = 0; k < 4; k += 2) {
-              float x, y;
-              unpack2(fma2(pack2(__uint_as_float(r16[i + k]), __uint_as_float(r16[i + k + 1])), sl22, add2(k ? m4.y : m4.x, lift2)), x, y);
-              const __half2 p = __floats2half2_rn(ex2_approx(x), ex2_approx(y));
-              const uint32_t u = *reinterpret_cast<const uint32_t*>(&p);
-              const float2 pf = __half22float2(p);
-              lp[(c + i + k) / 2] = fma2(pack2(pf.x, pf.y), back2, lp[(c + i + k) / 2]);
-              put16(pdst[(i + k) & 7] + (c + ((i + k) & 8)) * 128, u);
-              put16(pdst[(i + k + 1) & 7] + (c + ((i + k) & 8)) * 128, u >> 16);
+              for (int j = 0; j < 4; j += 2) {
+                const uint64_t r2 = pack2(__uint_as_float(r16[i + j]), __uint_as_float(r16[i + j + 1])), m2 = j ? m4.y : m4.x;
+                float x, y;
+                if constexpr (kPlain) unpack2(fma2(r2, sl22, m2), x, y);
+                else unpack2(fma2(r2, mul2(sl22, j ? q4m.y : q4m.x), add2(m2, lift2)), x, y);
+                const float ex = ex2_approx(x), ey = ex2_approx(y);
+                const __half2 p = __floats2half2_rn(ex, ey);
+                const uint32_t u = half2_bits(p);
+                uint64_t& sum = lp[(c + i + j) / 2];
+                if constexpr (kPlain) {
+                  const float2 pf = __half22float2(p);
+                  sum = add2(sum, pack2(pf.x, pf.y));
+                } else {
+                  sum = fma2(pack2(ex, ey), back2, sum);
+                }
+                put16(pdst[(i + j) & 7] + (c + ((i + j) & 8)) * 128, u);
+                put16(pdst[(i + j + 1) & 7] + (c + ((i + j) & 8)) * 128, u >> 16);
+              }
             }
-          }
-        } else {
+          } else {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) put16(pdst[i & 7] + (c + (i & 8)) * 128, 0u);
+            for (int i = 0; i < 16; ++i) put16(pdst[i & 7] + (c + (i & 8)) * 128, 0u);
+          }
         }
-      }
+      };
+      if (lifted || q_lifted) weights(std::false_type{});
+      else weights(std::true_type{});
       fence_proxy_async();
       tc_fence_before();
       __syncwarp();
@@ -597,6 +686,7 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
     const uint8_t* src_row;                                // row whose codes are in `raw`; nullptr: none
     // The item, its blocks, and the list's next row of this lane (registers are short here: no more is kept)
     int at, t = 0, n_swa = 0, r_end = 0, n_blocks = 0, li = 0, next_slot = -1;
+    uint32_t turn_q = 0;                                   // list of the powers of two of this item's queries
     constexpr int kWindow = 1 << 30;                       // marks a slot of the first cache (a slot is far below)
     auto look_up = [&]() {                                 // li -> next_slot, and on to the same row of the next block
       next_slot = -1;
@@ -651,16 +741,16 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
     uint32_t g = 0;
     while (at < items) {
       const uint2 sc = sc8;
-      // Power of two that brings the row into fp16's range: 0 unless a scale is above 2^7 (a code's magnitude is at most 448) or a
-      // rotated value above 2^16
-      const uint32_t top = __vmaxu2(__vmaxu2(sc.x & 0x00ff00ffu, (sc.x >> 8) & 0x00ff00ffu), __vmaxu2(sc.y & 0x00ff00ffu, (sc.y >> 8) & 0x000000ffu));
+      // The row's largest magnitude: a code's is below 2^9.  Scales (by halves: bytes 0 2, 1 3, 4 6, 5 -)
+      const uint32_t s0 = sc.x & 0x00ff00ffu, s1 = (sc.x >> 8) & 0x00ff00ffu, s2 = sc.y & 0x00ff00ffu, s3 = (sc.y >> 8) & 0x000000ffu;
+      const uint32_t top = __vmaxu2(__vmaxu2(s0, s1), __vmaxu2(s2, s3)), low = __vminu2(__vminu2(s0, s1), __vminu2(s2, s3 | 0x00ff0000u));
       uint32_t big = __vmaxu2(__vmaxu2(bf16x2_absmax(rot[0].x, rot[0].y), bf16x2_absmax(rot[0].z, rot[0].w)),
                               __vmaxu2(bf16x2_absmax(rot[1].x, rot[1].y), bf16x2_absmax(rot[1].z, rot[1].w)));
       big = __vmaxu2(big, __shfl_xor_sync(0xffffffffu, big, 1));
       big = __vmaxu2(big, __shfl_xor_sync(0xffffffffu, big, 2));
-      const int lift = max(0, max(max(static_cast<int>(top & 0xffff), static_cast<int>(top >> 16)) - 134,
-                                  (max(static_cast<int>(big & 0xffff), static_cast<int>(big >> 16)) >> 7) - 142));
-      const float back = __int_as_float((127 - lift) << 23);
+      const int lift = range_shift(max(max(static_cast<int>(top & 0xffff), static_cast<int>(top >> 16)) + 8, static_cast<int>(max(big & 0xffff, big >> 16) >> 7)),
+                                   min(low & 0xffff, low >> 16) < 103);
+      const float back = power_of_two(-lift);
 #pragma unroll
       for (int i = 0; i < kPanels; ++i) {
         const int p = panel_at(i);
@@ -668,7 +758,7 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
           ok = __all_sync(0xffffffffu, ok && mbar_wait(&bars->k_free[p >> 1], (g - 1) & 1, a.status, 620));
           if (!ok) break;
         }
-        if (i == 0 && l4 == 0) lift_s[row] = src_row != nullptr ? lift : -1;
+        if (i == 0 && l4 == 0) lift_s[row] = src_row != nullptr ? lift : kNoRow;
         uint4 o0, o1;
         uint32_t at0, at1;
         if (p < 7) {
@@ -709,7 +799,8 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
         if (at >= items) break;
         ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full, (g - 1) & 1, a.status, 621));
         if (!ok) break;
-        load_q(t, threadIdx.x - (4 + kSoftmaxWarps) * 32, std::integral_constant<int, 32 * kProducerWarps>{});
+        turn_q ^= 1;
+        load_q(t, threadIdx.x - (4 + kSoftmaxWarps) * 32, turn_q, std::integral_constant<int, 32 * kProducerWarps>{});
         fence_proxy_async();
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->q_full);
@@ -730,7 +821,7 @@ sparse_mla_tc_kernel(const MlaTcArgs a) {
 
 template <int NH>
 static int launch_mla_tc(const MlaTcArgs& a, cudaStream_t st) {
-  const int smem = kPanels * kPanelBytes + kPanels * NH * 128 + 2 * NH * 128 + kBarBytes + 7 * NH * 4 + kRows * 4 + 1024;
+  const int smem = kPanels * kPanelBytes + kPanels * NH * 128 + 2 * NH * 128 + kBarBytes + 9 * NH * 4 + kRows * 4 + 1024;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(sparse_mla_tc_kernel<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
@@ -787,7 +878,7 @@ STK_API int stk_sparse_mla_tc(const void* q, long long ldt, const void* swa_cach
                     nullptr, status, trace, stream);
 }
 
-// One CTA per token over its whole row list, final output written by the kernel (sink merged, normalised, inverse
+// An item is a token's whole row list, final output written by the kernel (sink merged, normalised, inverse
 // RoPE on the rope dims when positions != null): for steps with enough tokens to fill the GPU without row splits.
 STK_API int stk_sparse_mla_tc_out(const void* q, long long ldt, const void* swa_cache, long long swa_stride,
                                   const void* comp_cache, long long comp_stride, const int* swa_slots, int swa_ld,

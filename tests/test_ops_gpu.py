@@ -499,6 +499,58 @@ def test_sparse_mla_rows_beyond_fp16(nh, off):
     _lib.check_status()
 
 
+@pytest.mark.parametrize("T", [12, 150])
+@pytest.mark.parametrize("nh", [8, 32, 64])
+@pytest.mark.parametrize("kind", ["small", "mixed", "far", "groups", "scales", "large queries", "small queries"])
+def test_sparse_mla_magnitudes_that_fp16_does_not_hold(kind, nh, T):
+    """Against 64 bits, per head: rows around 1e-6, alone and beside ordinary ones; a few rows of 1e12 beside ordinary ones that carry
+    most of the weight; rows whose groups are 2^20 apart (every group of the output by itself); scales of 2^-67 as another writer may
+    leave them; queries above 65504 and far below 2^-14 beside ordinary heads.  Partial rows and final ones.
+    Output rounded to bf16, at most 2^-9 of a value (1.2e-3 in the 2-norm), weights to fp16 (2^-11); 3e-3 leaves half as much again."""
+    D, R_, W, n = 512, 64, 300, 512
+    g = torch.Generator().manual_seed(11)
+    rows = torch.randn(n, D, generator=g)
+    q = torch.randn(T, nh, D, generator=g)
+    scale = D ** -0.5
+    if kind == "small":
+        rows, scale = rows * 1e-6, scale * 1e6
+    elif kind == "mixed":
+        rows[1::2] *= 1e-6
+    elif kind == "far":
+        rows[::30] *= 1e12
+        scale *= 1e-12
+    elif kind == "groups":
+        rows *= (10.0 ** torch.tensor([3, 0, -3, 1, -2, 2, -1, -3])).repeat_interleave(64)
+        scale *= 1e-3
+    elif kind == "large queries":
+        q[:, ::4] *= 2.0 ** 20
+        scale *= 2.0 ** -20
+    elif kind == "small queries":
+        q *= 2.0 ** -30
+        q[:, 0] = 0
+        scale *= 2.0 ** 30
+    ccpu = C.PagedCache.allocate(n // 64, D, R_, True, "latent", "cpu")
+    ccpu.write_rows_cpu(torch.arange(n), rows)
+    if kind == "scales":
+        data = ccpu.buf[:, :64 * 576].view(-1, 64, 576)[:, :, D - R_:].contiguous().view(BF16)
+        ccpu.buf[:, :64 * 576].view(-1, 64, 576)[:, :, D - R_:] = (data.float() * 2.0 ** -60).to(BF16).view(torch.uint8)
+        ccpu.buf[:, 64 * 576:64 * 584].view(-1, 64, 8)[:, :, :7] -= 60
+        scale *= 2.0 ** 60
+    kv = ccpu.read_rows_cpu(torch.arange(n))[0].double().to(dev())
+    cg = C.PagedCache(ccpu.buf.to(dev()), D, R_, True, "latent")
+    q = q.to(dev()).to(BF16)
+    slots = torch.arange(W, dtype=torch.int32, device=dev()).repeat(T, 1)
+    lens = torch.full((T,), W, dtype=torch.int32, device=dev())
+    sink = torch.randn(nh, generator=g).to(dev())
+    out = A.sparse_mla(q, cg, slots, lens, None, None, None, sink, scale).double()
+    s = q.double() @ kv[:W].t() * scale
+    ref = torch.softmax(torch.cat([s, sink.double()[None, :, None].expand(T, -1, 1)], 2), 2)[:, :, :-1] @ kv[:W]
+    cut = (T, nh, 8, 64) if kind == "groups" else (T, nh, 1, D)
+    err = (out - ref).view(cut).pow(2).sum((0, 3)) / ref.view(cut).pow(2).sum((0, 3))
+    assert float(err.sqrt().max()) < 3e-3
+    _lib.check_status()
+
+
 @pytest.mark.parametrize("nh", [8, 32, 64])
 def test_sparse_mla_weights_are_relative_to_the_exact_maximum(nh):
     """Weights relative to the largest: 1 and 3/4 are bf16 numbers, so two leading rows 3 x and -4 x in the last block cancel whatever
