@@ -552,6 +552,36 @@ def test_sparse_mla_magnitudes_that_fp16_does_not_hold(kind, nh, T):
 
 
 @pytest.mark.parametrize("nh", [8, 32, 64])
+def test_sparse_mla_weights_relative_to_stale_maxima(nh):
+    """A first block of rows 0 to 3 x log2(4 / 3) powers of two below two leading rows 3 x and -4 x of the last block, with weights 1
+    and 3/4 of the largest: the maximum in use may stay (up to 2^1.5), so both weights are rounded to fp16.  Tolerance per element:
+    2^-11 of each weight times what cancels, 3 + 4 * 3/4, over the sum of all weights; 1 % and 1e-5 for exponentials and output."""
+    D, R_, T, W = 512, 64, 60, 128
+    levels = [0, 1, 2, 3]
+    rows = torch.zeros((1 + len(levels)) * 64, D)
+    g = torch.Generator().manual_seed(0)
+    x = torch.randint(0, 2, (D,), generator=g).float() * 2 - 1
+    rows[0], rows[1] = 3 * x, -4 * x
+    rows[0, 0], rows[1, 0] = 16, 15
+    for i, n in enumerate(levels):
+        rows[64 * (i + 1):64 * (i + 2), 0] = 16 - n
+    ccpu = C.PagedCache.allocate(1 + len(levels), D, R_, True, "latent", "cpu")
+    ccpu.write_rows_cpu(torch.arange(rows.shape[0]), rows)
+    cg = C.PagedCache(ccpu.buf.to(dev()), D, R_, True, "latent")
+    q = torch.zeros(T, nh, D, device=dev(), dtype=BF16)
+    q[:, :, 0] = 1
+    page = torch.arange(T) % len(levels) + 1
+    slots = (page[:, None] * 64 + torch.arange(W)[None] % 64).to(torch.int32).to(dev())
+    lens = torch.full((T,), W, dtype=torch.int32, device=dev())
+    top = torch.tensor([[0, 1]], dtype=torch.int32, device=dev()).expand(T, -1).contiguous()
+    top_lens = torch.full((T,), 2, dtype=torch.int32, device=dev())
+    sink = torch.full((nh,), -1e30, device=dev())
+    out = A.sparse_mla(q, cg, slots, lens, cg, top, top_lens, sink, math.log(4 / 3)).double().cpu()
+    total = 1.75 + W * 0.75 ** torch.tensor(levels, dtype=torch.float64)[page - 1]
+    assert bool((out[:, :, 1:].abs().amax((1, 2)) <= 6 * 2.0 ** -11 * 1.01 / total + 1e-5).all())
+
+
+@pytest.mark.parametrize("nh", [8, 32, 64])
 def test_sparse_mla_weights_are_relative_to_the_exact_maximum(nh):
     """Weights relative to the largest: 1 and 3/4 are bf16 numbers, so two leading rows 3 x and -4 x in the last block cancel whatever
     came before them -- a first block of rows 4 to 9 powers of two lower, a different distance per token, which a maximum taken from
