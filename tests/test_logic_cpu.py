@@ -334,3 +334,26 @@ def test_model_config_rejects_wrongly_typed_fields_as_configuration_errors():
             [cfg.layer_kind(i) for i in range(cfg.num_hidden_layers)]
         except ConfigError:
             pass
+
+
+# ---- library calls and scratch views ------------------------------------------------------------
+def test_library_call_takes_tensors_wherever_it_took_them(monkeypatch):
+    import ctypes
+    from stkernel_b200.ops import _lib
+    got = []
+
+    def first(p, n, f):
+        got.append((p, n, f))
+        return 0
+
+    fn = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p, ctypes.c_longlong, ctypes.c_float)(first)
+    lib = type("Lib", (), {"stk_first": fn})
+    monkeypatch.setattr(_lib, "lib", lambda: lib)
+    monkeypatch.setattr(_lib, "_entries", {})
+    t = torch.zeros(4)
+    _lib.call("stk_first", t, 3, 0.5)
+    _lib.call("stk_first", None, t, 1)                 # an address as an integer
+    _lib.call("stk_first", t[1:], True, 2.0)
+    assert got == [(t.data_ptr(), 3, 0.5), (None, t.data_ptr(), 1.0), (t.data_ptr() + 4, 1, 2.0)]
+    with pytest.raises(TypeError):                     # too few arguments: what ctypes says, not an index out of range
+        _lib.call("stk_first")
