@@ -67,6 +67,7 @@ def lib() -> ctypes.CDLL:
             raise RuntimeError(
                 f"{_LIB_PATH} is missing: run `python -m stkernel_b200.csrc.build` (the CUDA ops have no fallback "
                 "on a GPU machine)")
+        _entries.clear()                          # of a library that was loaded before
         _lib = ctypes.CDLL(str(_LIB_PATH), mode=os.RTLD_GLOBAL if hasattr(os, "RTLD_GLOBAL") else ctypes.DEFAULT_MODE)
         for name, (ret, types) in _parse_signatures().items():
             fn = getattr(_lib, name, None)

@@ -357,3 +357,13 @@ def test_library_call_takes_tensors_wherever_it_took_them(monkeypatch):
     assert got == [(t.data_ptr(), 3, 0.5), (None, t.data_ptr(), 1.0), (t.data_ptr() + 4, 1, 2.0)]
     with pytest.raises(TypeError):                     # too few arguments: what ctypes says, not an index out of range
         _lib.call("stk_first")
+
+
+def test_library_entries_do_not_outlive_their_library(monkeypatch):
+    from stkernel_b200.ops import _lib
+    if not _lib.available():
+        pytest.skip("the library is not built")
+    monkeypatch.setattr(_lib, "_entries", {"stk_gemm_pick_bt": (lambda *a: -1, ())})
+    monkeypatch.setattr(_lib, "_lib", None)
+    _lib.lib()
+    assert _lib.query("stk_gemm_pick_bt", 16, 0) > 0
