@@ -367,3 +367,31 @@ def test_library_entries_do_not_outlive_their_library(monkeypatch):
     monkeypatch.setattr(_lib, "_lib", None)
     _lib.lib()
     assert _lib.query("stk_gemm_pick_bt", 16, 0) > 0
+
+
+def test_scratch_views_follow_mode_graph_growth_and_branch(monkeypatch):
+    """A view that was handed out before is handed out again only where a new one would be the same."""
+    import contextlib
+    from stkernel_b200.ops import scratch as S
+    for name, empty in (("_pool", {}), ("_views", {}), ("_outgrown", [])):
+        monkeypatch.setattr(S, name, empty)
+    monkeypatch.setattr(torch.cuda, "stream", lambda s: contextlib.nullcontext())
+    get = lambda *shape, dtype=torch.float32: S.scratch("t.views", shape, dtype, "cpu")
+    with torch.inference_mode():
+        a = get(2, 3)
+    b = get(2, 3)
+    b.zero_()                                          # not an inference tensor, which refuses this
+    assert a.data_ptr() == b.data_ptr() and get(2, 3) is b
+    b.copy_(torch.ones(2, 3, requires_grad=True))      # b is part of a graph now
+    assert not get(2, 3).requires_grad
+    for shape in ((3, 2), (2, 3), (6,), (2, 3)):       # two shapes in turn
+        assert get(*shape).shape == torch.Size(shape) and get(*shape).data_ptr() == b.data_ptr()
+    assert get(2, 3, dtype=torch.int32).dtype == torch.int32
+    with S.side_branch(None):
+        side = get(2, 3)
+        assert side.data_ptr() != b.data_ptr() and get(2, 3) is side
+    assert get(2, 3).data_ptr() == b.data_ptr()
+    get(4096)                                          # the buffer grows: its old place is not handed out any more
+    assert get(2, 3).data_ptr() == S._pool[("t.views", "cpu")].data_ptr() != b.data_ptr()
+    S.reset()
+    assert not S._views and get(2, 3).shape == (2, 3)
