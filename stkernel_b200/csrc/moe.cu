@@ -598,10 +598,17 @@ expert_fc2_direct_kernel(const __half* __restrict__ act, ExpertW w2, int e_local
   }
 }
 
-static int direct_blocks(int per_sm) {
-  int device = 0, sms = 1;
+// Thread blocks of these kernels for pairs of this width on a GPU (or a part of one) of so many SMs, or 0 where they do not serve: a
+// pair without a block of its own would be left out.
+static int direct_blocks(int pairs, int width, int sms) {
+  const int iters = (width / 32 + 31) / 32, blocks = sms * (iters <= 4 ? 2 : 1);
+  return pairs <= kDirectPairs && iters <= 8 && blocks >= pairs ? blocks : 0;
+}
+
+static int device_sms() {
+  int device = 0, sms = 0;
   if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
-  return sms * per_sm;
+  return sms;
 }
 
 }  // namespace stk
@@ -639,6 +646,9 @@ STK_API int stk_moe_align(const int* ids, int n_pairs, int e_start, int e_local,
 }
 
 // max_rows bounds the grid (rows beyond offsets[e_local] exit at once).
+// Thread blocks that take a handful of unsorted pairs of this width, or 0: a thread block per part of a pair's rows, as for sorted ones.
+STK_API int stk_moe_direct_blocks(int n_pairs, int width, int sm_count) { return direct_blocks(n_pairs, width, sm_count); }
+
 STK_API int stk_moe_expert_fc1(const void* x, long long ldx, const void* w13, const void* s13, const float* g13,
                                const int* sorted, const int* sorted_expert, const int* offsets, int e_local, int topk,
                                void* act, int max_rows, int H, int I, float limit, const int* direct_ids, int e_start,
@@ -650,9 +660,7 @@ STK_API int stk_moe_expert_fc1(const void* x, long long ldx, const void* w13, co
   const size_t smem = ((H + 1023) / 1024) * 2048;
   cudaStream_t st = (cudaStream_t)stream;
   const int iters = (H / 32 + 31) / 32;
-  if (direct_ids != nullptr && max_rows <= kDirectPairs && iters <= 8) {
-    const int grid1 = direct_blocks(iters <= 4 ? 2 : 1);
-    if (grid1 <= 0) return -5;
+  if (const int grid1 = direct_ids != nullptr ? direct_blocks(max_rows, H, device_sms()) : 0; grid1 > 0) {
 #define STK_FC1D(I_) launch_pdl(expert_fc1_direct_kernel<I_>, dim3(grid1), dim3(256), smem, st, (const __nv_bfloat16*)x, ldx, w, e_local, topk, (__half*)act, max_rows, H, I, limit, direct_ids, e_start)
     if (iters <= 1) STK_FC1D(1); else if (iters <= 2) STK_FC1D(2); else if (iters <= 4) STK_FC1D(4); else STK_FC1D(8);
 #undef STK_FC1D
@@ -684,9 +692,7 @@ STK_API int stk_moe_expert_fc2(const void* act, const void* w2, const void* s2, 
   }
   dim3 grid((H + 31) / 32, max_rows);
   const int iters = (I / 32 + 31) / 32;
-  if (direct_ids != nullptr && max_rows <= kDirectPairs && iters <= 8) {
-    const int grid1 = direct_blocks(iters <= 4 ? 2 : 1);
-    if (grid1 <= 0) return -5;
+  if (const int grid1 = direct_ids != nullptr ? direct_blocks(max_rows, I, device_sms()) : 0; grid1 > 0) {
 #define STK_FC2D(I_) launch_pdl(expert_fc2_direct_kernel<I_>, dim3(grid1), dim3(256), smem, st, (const __half*)act, w, e_local, (__nv_bfloat16*)y, max_rows, H, I, direct_ids, e_start)
     if (iters <= 1) STK_FC2D(1); else if (iters <= 2) STK_FC2D(2); else if (iters <= 4) STK_FC2D(4); else STK_FC2D(8);
 #undef STK_FC2D

@@ -147,6 +147,7 @@ int stk_mlstm_finish(const float* num, const float* den, const float* mt, float*
 // ---- moe.cu ----
 int stk_router(const float* logits, long long ldl, const float* bias, const int* tid2eid, const int64_t* token_ids, int vocab, int* ids, float* weights, int T, int E, int topk, int always, int groups, int keep, int scoring, int renorm, float scaling, int* status, void* stream);
 int stk_moe_align(const int* ids, int n_pairs, int e_start, int e_local, int* sorted, int* pair_row, int* offsets, int* sorted_expert, int* counts, void* stream);
+int stk_moe_direct_blocks(int n_pairs, int width, int sm_count);
 int stk_moe_expert_fc1(const void* x, long long ldx, const void* w13, const void* s13, const float* g13, const int* sorted, const int* sorted_expert, const int* offsets, int e_local, int topk, void* act, int max_rows, int H, int I, float limit, const int* direct_ids, int e_start, void* stream);
 int stk_moe_expert_fc2(const void* act, const void* w2, const void* s2, const float* g2, const int* sorted_expert, const int* offsets, int e_local, void* y, int max_rows, int H, int I, const int* direct_ids, int e_start, void* stream);
 

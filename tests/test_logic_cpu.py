@@ -395,3 +395,16 @@ def test_scratch_views_follow_mode_graph_growth_and_branch(monkeypatch):
     assert get(2, 3).data_ptr() == S._pool[("t.views", "cpu")].data_ptr() != b.data_ptr()
     S.reset()
     assert not S._views and get(2, 3).shape == (2, 3)
+
+
+@pytest.mark.parametrize("sms", [1, 16, 31, 32, 63, 64, 148])
+def test_every_pair_has_a_thread_block_of_its_own(sms):
+    """The expert kernels for a handful of unsorted pairs deal thread blocks out to pairs: fewer of them than pairs would leave some out."""
+    from stkernel_b200.ops import _lib
+    if not _lib.available():
+        pytest.skip("the library is not built")
+    for width in (32, 4096, 4128, 8192, 8224, 16384):
+        for pairs in (1, 6, 16, 17, 32, 33, 48, 64, 65):
+            blocks = _lib.query("stk_moe_direct_blocks", pairs, width, sms)
+            per_sm = 2 if width <= 4096 else 1
+            assert blocks == (sms * per_sm if pairs <= 64 and width <= 8192 and sms * per_sm >= pairs else 0)

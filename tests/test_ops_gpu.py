@@ -1323,6 +1323,21 @@ def test_moe_grouped_gemm_scales_off_alignment(H, I, E):
     assert rel_err(outs[0], ref) < 5e-3
 
 
+@pytest.mark.parametrize("H,I", [(8704, 128), (128, 8704)])
+def test_moe_experts_of_a_handful_of_pairs_beyond_8192(H, I):
+    """Widths that the thread blocks that stay do not take: a thread block per part of a pair's rows, without a sort."""
+    torch.manual_seed(15)
+    E, T, k = 3, 5, 2
+    assert _lib.query("stk_moe_direct_blocks", T * k, max(H, I), _lib.sm_count()) == 0
+    ew = M.ExpertWeights.from_master(torch.randn(E, 2 * I, H, device=dev()) * 0.02, torch.randn(E, H, I, device=dev()) * 0.02, "nvfp4", dev())
+    x = torch.randn(T, H, device=dev()).to(BF16)
+    ids, w = M.router(torch.randn(T, E, device=dev()), None, k, "sigmoid", True, 1.0)
+    d13, d2 = ew.dequant()
+    assert rel_err(M.moe_experts(x, ids, w, ew, 10.0), R.moe_experts(x, ids, w, d13, d2, 10.0)) < 1.5e-2
+    hi = M.ExpertWeights(ew.w13[1:], ew.w2[1:], ew.s13[1:], ew.s2[1:], ew.g13[1:], ew.g2[1:], 1)         # the first belongs to another rank
+    assert rel_err(M.moe_experts(x, ids, w, hi, 10.0), R.moe_experts(x, ids, w, d13[1:], d2[1:], 10.0, 1)) < 1.5e-2
+
+
 def test_topk_candidates_and_markov_chain_match_cpu():
     """The drafter's sampling path: two-level candidate selection over the full vocabulary and the one-launch
     sequential Markov sampling against their CPU statements."""
