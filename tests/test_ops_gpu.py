@@ -1323,6 +1323,37 @@ def test_moe_grouped_gemm_scales_off_alignment(H, I, E):
     assert rel_err(outs[0], ref) < 5e-3
 
 
+@pytest.mark.parametrize("bt", [16, 128])
+def test_moe_swiglu_against_64_bits(bt):
+    """Rows of one value, so that gate and up products are exact whichever kernel forms them: SwiGLU of the grouped product and of a
+    handful of pairs against 64 bits, down to gates whose exponential is infinite.  Tolerance: one rounding to fp16 (2^-11 of the
+    value, 2^-25 where it is subnormal); in fp32 the exponential's 2 + 1.17 |g| units -- felt while the gate is above -17, below it the
+    result is at most 2^-19 times the up value -- and a few of the quotient and the products: 30 x 2^-23."""
+    H, I, T = 64, 1024, 960
+    g = torch.Generator().manual_seed(5)
+    w = torch.randint(0, 256, (1, 2 * I, H // 2), generator=g, dtype=torch.uint8).to(dev())
+    s = (0.25 + 2 * torch.rand(1, 2 * I, H // 16, generator=g)).to(torch.float8_e4m3fn).view(torch.uint8).to(dev())
+    gs = torch.ones(1, device=dev())
+    x = torch.zeros(T, H)
+    x[torch.arange(T), torch.arange(T) % H] = torch.randn(T, generator=g) * 4.0 ** (torch.arange(T) % 3).float()
+    x = x.to(BF16).to(dev())
+    ids = torch.zeros(T, 1, dtype=torch.int32, device=dev())
+    few, grouped = (torch.empty(T + 128, I, dtype=torch.float16, device=dev()) for _ in range(2))
+    for i in range(0, T, 48):
+        _lib.call("stk_moe_expert_fc1", x[i:], x.stride(0), w, s, gs, None, None, None, 1, 1, few[i:], 48, H, I, 10.0, ids, 0, _lib.stream())
+    rows = torch.zeros(T + 128, H, dtype=torch.float16, device=dev())
+    rows[:T] = x.to(torch.float16)
+    offsets = torch.tensor([0, T], dtype=torch.int32, device=dev())
+    _lib.call("stk_moe_grouped", rows, T + 128, w, s, gs, offsets, 1, I, H, grouped, 1, 10.0, bt, _lib.status_buffer(), _lib.sm_count(),
+              _lib.stream())
+    h = x.double() @ R.dequant_nvfp4(w[0], s[0].view(torch.float8_e4m3fn), gs[0]).double().t()
+    gate, up = h[:, :I].clamp(max=10.0), h[:, I:].clamp(-10.0, 10.0)
+    assert float(gate.min()) < -100
+    ref = gate * torch.sigmoid(gate) * up
+    for out in (few[:T], grouped[:T]):
+        assert float(((out.double() - ref).abs() - (2.0 ** -11 + 30 * 2.0 ** -23) * ref.abs()).max()) <= 2.0 ** -24
+
+
 @pytest.mark.parametrize("H,I", [(8704, 128), (128, 8704)])
 def test_moe_experts_of_a_handful_of_pairs_beyond_8192(H, I):
     """Widths that the thread blocks that stay do not take: a thread block per part of a pair's rows, without a sort."""
