@@ -226,6 +226,8 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   const int steps_k = a.K / 64;                                 // K steps of a unit
   // Buffers of K step kb of this CTA's i-th unit, and their phase.  Four of them: those of the step's place in a weight stage (a dequant
   // group then sees every use of its buffers, which a wait by parity needs, also where a unit's last stage is not whole).  Eight: in turn.
+  // There a group does not see every use, but its own steps are at most seven apart (seven steps a unit: 3, 10), so its last wait, for the
+  // products of a step at most fifteen back, tells it that those of sixteen back are done, and parity can only mean those of eight back.
   struct Step { int buf; uint32_t phase; };
   auto step_at = [&](int i, int kb) {
     if constexpr (kSteps == 4) {

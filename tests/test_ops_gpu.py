@@ -1354,6 +1354,30 @@ def test_moe_swiglu_against_64_bits(bt):
         assert float(((out.double() - ref).abs() - (2.0 ** -11 + 30 * 2.0 ** -23) * ref.abs()).max()) <= 2.0 ** -24
 
 
+@pytest.mark.parametrize("I", [384, 640, 448])
+@pytest.mark.parametrize("rows", [5, 40, 130])
+def test_moe_grouped_gemm_steps_of_one_weight_tile(I, rows):
+    """Single weight tiles (features no multiple of 256) with six, ten and seven K steps of 64, more tiles than thread blocks: operand
+    places are taken in turn across tiles whose last stage is not whole."""
+    H, E = 384, 64
+    g = torch.Generator().manual_seed(I + rows)
+    P = E * rows
+    w = torch.randint(0, 256, (E, H, I // 2), generator=g, dtype=torch.uint8).to(dev())
+    s = (0.05 + torch.rand(E, H, I // 16, generator=g)).to(torch.float8_e4m3fn).view(torch.uint8).to(dev())
+    gs = torch.full((E,), 0.03, device=dev())
+    x = torch.zeros(P + 128, I, dtype=torch.float16)
+    x[:P] = torch.randn(P, I, generator=g)
+    x = x.to(dev())
+    offsets = (torch.arange(E + 1, dtype=torch.int32) * rows).to(dev())
+    out = torch.empty(P, H, dtype=BF16, device=dev())
+    _lib.call("stk_moe_grouped", x, P + 128, w, s, gs, offsets, E, H, I, out, 0, 0.0, 16 if rows < 16 else 64 if rows < 100 else 128,
+              _lib.status_buffer(), _lib.sm_count(), _lib.stream())
+    deq = torch.stack([R.dequant_nvfp4(w[e], s[e].view(torch.float8_e4m3fn), gs[e]) for e in range(E)]).double()
+    ref = torch.bmm(x[:P].double().view(E, rows, I), deq.transpose(1, 2)).view(P, H)
+    assert rel_err(out, ref) < 2.5e-3                     # rounded to bf16 once: 1.7e-3
+    _lib.check_status()
+
+
 @pytest.mark.parametrize("H,I", [(8704, 128), (128, 8704)])
 def test_moe_experts_of_a_handful_of_pairs_beyond_8192(H, I):
     """Widths that the thread blocks that stay do not take: a thread block per part of a pair's rows, without a sort."""
