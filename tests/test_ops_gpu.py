@@ -1378,6 +1378,29 @@ def test_moe_grouped_gemm_steps_of_one_weight_tile(I, rows):
     _lib.check_status()
 
 
+@pytest.mark.parametrize("bt", [16, 64, 128])
+def test_moe_grouped_gemm_of_rows_that_have_arrived(bt):
+    """The expert-parallel first product with every row in place and every count at (or past) its expert's: the same bits as without."""
+    H, I, E = 320, 256, 9
+    g = torch.Generator().manual_seed(bt)
+    counts = torch.tensor([3, 0, 70, 1, 0, 129, 16, 17, 0], dtype=torch.int32)
+    offsets = torch.cat([torch.zeros(1, dtype=torch.int32), counts.cumsum(0).to(torch.int32)]).to(dev())
+    P = int(counts.sum())
+    w = torch.randint(0, 256, (E, 2 * I, H // 2), generator=g, dtype=torch.uint8).to(dev())
+    s = (0.05 + torch.rand(E, 2 * I, H // 16, generator=g)).to(torch.float8_e4m3fn).view(torch.uint8).to(dev())
+    gs = torch.full((E,), 0.03, device=dev())
+    x = torch.zeros(P + 128, H, dtype=torch.float16)
+    x[:P] = torch.randn(P, H, generator=g)
+    x = x.to(dev())
+    plain, ep = (torch.full((P + 128, I), 7.0, dtype=torch.float16, device=dev()) for _ in range(2))
+    arrived = (counts + torch.tensor([0, 5, 0, 0, 0, 0, 1, 0, 0], dtype=torch.int32)).to(dev())
+    _lib.call("stk_moe_grouped", x, P + 128, w, s, gs, offsets, E, I, H, plain, 1, 10.0, bt, _lib.status_buffer(), _lib.sm_count(), _lib.stream())
+    _lib.call("stk_moe_grouped_ep", x, P + 128, w, s, gs, offsets, E, I, H, ep, 1, 10.0, bt, _lib.status_buffer(), _lib.sm_count(), arrived,
+              1000, _lib.stream())
+    assert torch.equal(plain.view(torch.int16), ep.view(torch.int16)) and bool((plain[P:] == 7.0).all())
+    _lib.check_status()
+
+
 @pytest.mark.parametrize("H,I", [(8704, 128), (128, 8704)])
 def test_moe_experts_of_a_handful_of_pairs_beyond_8192(H, I):
     """Widths that the thread blocks that stay do not take: a thread block per part of a pair's rows, without a sort."""
