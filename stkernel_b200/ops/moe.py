@@ -89,6 +89,16 @@ def router(logits: torch.Tensor, bias: Optional[torch.Tensor], top_k: int, scori
     return ids, w
 
 
+def tile_rows(avg_rows: float) -> int:
+    """Token rows of a tile of the grouped product, for so many rows per expert on average.
+
+    Rows of an expert vary, and a second tile converts its weights again, so tiles are a few times the average.  256 experts, us with
+    tiles of 16 / 32 / 64 / 128 rows: 5 rows on average 809 / 778; 9: 1081 / 945 / 885; 19: 1605 / 1165 / 1012 / 1063; 35: 2527 / 1605 /
+    1221 / 1194; 96: - / 3487 / 2259 / 1862."""
+    avg = int(avg_rows)
+    return 16 if avg <= 3 else 32 if avg <= 6 else 64 if avg <= 24 else 128
+
+
 def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, ew: ExpertWeights, limit: float,
                 shared: Optional[torch.Tensor] = None, total_experts: int = 0, shared_ready=None, ll=None):
     """x [T, H] bf16 -> sum_k w_k * expert_k(x) (+ shared) as bf16 [T, H]; experts that are not local add nothing.
@@ -126,11 +136,7 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, ew: E
                   counts, st)
         if USE_GROUPED_GEMM and h % 64 == 0 and inter % 128 == 0 and h % 128 == 0:
             # tensor-core path: permute the activations into expert order, then two grouped GEMMs
-            avg = max(1, n_pairs // max(1, total_experts or ew.num_local))
-            # Rows of an expert vary, and a second tile converts its weights again, so tiles are a few times the average.  256 experts,
-            # us with tiles of 16 / 32 / 64 / 128 rows: 5 rows on average 809 / 778; 9: 1081 / 945 / 885; 19: 1605 / 1165 / 1012 / 1063;
-            # 35: 2527 / 1605 / 1221 / 1194; 96: - / 3487 / 2259 / 1862.
-            bt = 16 if avg <= 3 else 32 if avg <= 6 else 64 if avg <= 24 else 128
+            bt = tile_rows(n_pairs / max(1, total_experts or ew.num_local))
             xs = scratch("moe.xs", (n_pairs + 128, h), torch.float16, dev, zero=True)
             act_p = scratch("moe.act_p", (n_pairs + 128, inter), torch.float16, dev, zero=True)
             _lib.call("stk_moe_permute", x, x.stride(0), sorted_p, offsets, ew.num_local, k, xs, n_pairs, h, st)

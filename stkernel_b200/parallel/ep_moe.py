@@ -16,7 +16,7 @@ import torch
 import torch.distributed as dist
 
 from ..ops import _lib
-from ..ops.moe import ExpertWeights
+from ..ops.moe import ExpertWeights, tile_rows
 from .symm import SymmetricHeap
 
 BF16 = torch.bfloat16
@@ -24,7 +24,7 @@ I32 = torch.int32
 
 
 def pick_bt(avg_rows: float) -> int:
-    return 16 if avg_rows <= 8 else 32 if avg_rows <= 24 else 64 if avg_rows <= 48 else 128
+    return tile_rows(avg_rows)                    # the kernel of one GPU, the rule of one GPU
 
 
 class EpMoE:

@@ -408,3 +408,11 @@ def test_every_pair_has_a_thread_block_of_its_own(sms):
             blocks = _lib.query("stk_moe_direct_blocks", pairs, width, sms)
             per_sm = 2 if width <= 4096 else 1
             assert blocks == (sms * per_sm if pairs <= 64 and width <= 8192 and sms * per_sm >= pairs else 0)
+
+
+def test_expert_tiles_have_one_rule():
+    """The expert-parallel layer launches the grouped kernel of one GPU, with tiles by the same rule (tiles measured for it)."""
+    from stkernel_b200.ops.moe import tile_rows
+    from stkernel_b200.parallel.ep_moe import pick_bt
+    for avg, rows in ((0.2, 16), (3.9, 16), (4, 32), (6.5, 32), (7, 64), (24.9, 64), (25, 128), (900, 128)):
+        assert pick_bt(avg) == tile_rows(avg) == rows
