@@ -1873,9 +1873,30 @@ static int small_split_of(int T, int N, int K, int sm_count) {
   return s;
 }
 
-// Which tiles a plain product (no fused collective) without workspace splits takes: the number of CTAs that share one through a
-// cluster or as a pair, or 0 for 128-row tiles of one CTA each.  (For 65 to 128 bf16 tokens the answer is that for the 256 x 256 tiles:
-// it is never 0, and small_split_of may still put the product on 128-row tiles.)
+// The kernel of a plain product (no fused collective, no workspace splits) and the CTAs that share a tile of it
+enum GemmKind { kGemmTiles, kGemmFp8Tokens, kGemmFp8Pair, kGemmSmall, kGemmWide, kGemmPair };
+struct GemmPlan { int kind, ctas; };
+static GemmPlan gemm_plan(int T, int N, int K, int groups, int is_fp8, int sm_count) {
+  if (is_fp8) {
+    const int s = groups == 1 ? fp8_tokens_split(T, N, K, sm_count) : 0;
+    if (s == 1 && fp8_pair_serves(T, N, sm_count)) return {kGemmFp8Pair, 2};
+    return s > 0 ? GemmPlan{kGemmFp8Tokens, s} : GemmPlan{kGemmTiles, 1};
+  }
+  if (!gemm_wide_enabled()) return {kGemmTiles, 1};
+  // block-diagonal weights take clusters and wide tiles where blocks are whole tiles and whole 128-byte steps of K
+  const int small = groups == 1 || (N % (128 * groups) == 0 && K % 64 == 0) ? small_split_of(T, N, K, sm_count) : 1;
+  if (small > 1) return {kGemmSmall, small};
+  const int wide = groups == 1 || (N % (256 * groups) == 0 && K % 64 == 0) ? wide_split_of(T, N, K, sm_count) : 0;
+  return wide == 4 ? GemmPlan{kGemmWide, 4} : wide > 0 ? GemmPlan{kGemmPair, 2} : GemmPlan{kGemmTiles, 1};
+}
+// 16 x kind + CTAs
+STK_API int stk_gemm_plan(int T, int N, int K, int groups, int is_fp8, int sm_count) {
+  const GemmPlan p = gemm_plan(T, N, K, groups < 1 ? 1 : groups, is_fp8, sm_count);
+  return 16 * p.kind + p.ctas;
+}
+
+// Whether a plain product does without workspace splits (not 0: it leaves the 128-row tiles of one CTA each).  Which kernel takes it is
+// gemm_plan's answer; this one does not look at small clusters from 65 tokens on, where the wide tiles serve as well.
 STK_API int stk_gemm_token_tile_ctas(int T, int N, int K, int is_fp8, int sm_count) {
   if (is_fp8) return fp8_tokens_split(T, N, K, sm_count);
   if (!gemm_wide_enabled()) return 0;
@@ -1895,8 +1916,9 @@ static int gemm_launch(const void* W, long long ldw, const void* X, long long ld
   if (splits > 1 && (workspace == nullptr || counters == nullptr)) return -12;
   if (groups < 1) groups = 1;
   // an explicit split goes through the workspace
-  const int tokens_split = is_fp8 && splits <= 1 && groups == 1 && ar_ctx == nullptr && gate_ctx == nullptr ? fp8_tokens_split(T, N, K, sm_count) : 0;
-  if (tokens_split > 0) {
+  const bool plain = splits <= 1 && ar_ctx == nullptr && gate_ctx == nullptr && (is_fp8 || bt_override == 0);
+  const GemmPlan plan = plain ? gemm_plan(T, N, K, groups, is_fp8, sm_count) : GemmPlan{kGemmTiles, 1};
+  if (plan.kind == kGemmFp8Tokens || plan.kind == kGemmFp8Pair) {
     CUtensorMap ta, tb;
     if (make_tmap_2d(&ta, X, 1, T, K, ldx, 128) != 0) return -13;        // lanes: tokens
     if (make_tmap_2d(&tb, W, 1, N, K, ldw, 128) != 0) return -14;        // columns: weight rows
@@ -1911,19 +1933,18 @@ static int gemm_launch(const void* W, long long ldw, const void* X, long long ld
     a.status = status;
     a.tiles_t = (T + 127) / 128;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    if (tokens_split == 1 && fp8_pair_serves(T, N, sm_count)) {
+    if (plan.kind == kGemmFp8Pair) {
       a.tiles_t = (T + 255) / 256;
       a.tiles_n = (N + 255) / 256;
       return launch_fp8_pair(ta, tb, a, sm_count, st);
     }
-    switch (tokens_split) {
+    switch (plan.ctas) {
       case 4: return launch_fp8_tokens<4>(ta, tb, a, sm_count, st);
       case 2: return launch_fp8_tokens<2>(ta, tb, a, sm_count, st);
       default: return launch_fp8_tokens<1>(ta, tb, a, sm_count, st);
     }
   }
-  const int small_split = groups == 1 || (N % (128 * groups) == 0 && K % 64 == 0) ? small_split_of(T, N, K, sm_count) : 1;
-  if (!is_fp8 && ar_ctx == nullptr && gate_ctx == nullptr && splits <= 1 && bt_override == 0 && small_split > 1 && gemm_wide_enabled()) {
+  if (plan.kind == kGemmSmall) {
     const int tiles = (N + 127) / 128, columns = T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : 128;
     CUtensorMap tw3, tx3;
     if (make_tmap_2d(&tw3, W, 2, N, K, ldw, 128) != 0) return -13;
@@ -1935,16 +1956,14 @@ static int gemm_launch(const void* W, long long ldw, const void* X, long long ld
     sa.group_tiles = groups > 1 ? N / groups / 128 : 0;
     sa.group_k = K;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    if (columns == 16) return launch_small<16>(tw3, tx3, sa, small_split, tiles, st);
-    if (columns == 32) return launch_small<32>(tw3, tx3, sa, small_split, tiles, st);
-    if (columns == 64) return launch_small<64>(tw3, tx3, sa, small_split, tiles, st);
-    return launch_small<128>(tw3, tx3, sa, small_split, tiles, st);
+    if (columns == 16) return launch_small<16>(tw3, tx3, sa, plan.ctas, tiles, st);
+    if (columns == 32) return launch_small<32>(tw3, tx3, sa, plan.ctas, tiles, st);
+    if (columns == 64) return launch_small<64>(tw3, tx3, sa, plan.ctas, tiles, st);
+    return launch_small<128>(tw3, tx3, sa, plan.ctas, tiles, st);
   }
-  // block-diagonal weights take the wide tiles where blocks are whole tiles and whole 128-byte steps of K
-  const int wide_split = (groups == 1 || (N % (256 * groups) == 0 && K % 64 == 0)) ? wide_split_of(T, N, K, sm_count) : 0;
-  if (!is_fp8 && ar_ctx == nullptr && gate_ctx == nullptr && splits <= 1 && bt_override == 0 && wide_split > 0 && gemm_wide_enabled()) {
+  if (plan.kind == kGemmWide || plan.kind == kGemmPair) {
     CUtensorMap tw2, tx2;
-    if (make_tmap_2d(&tw2, W, 2, N, K, ldw, wide_split == 4 ? 256 : 128) != 0) return -13;                       // B operand: 256 weight rows, or a CTA's half
+    if (make_tmap_2d(&tw2, W, 2, N, K, ldw, plan.kind == kGemmWide ? 256 : 128) != 0) return -13;                       // B operand: 256 weight rows, or a CTA's half
     if (make_tmap_2d(&tx2, X, 2, T, static_cast<long long>(K) * groups, ldx, 128) != 0) return -14;              // A operands: 128 tokens each
     WideArgs wa;
     wa.T = T; wa.N = N;
@@ -1954,7 +1973,7 @@ static int gemm_launch(const void* W, long long ldw, const void* X, long long ld
     wa.out = out; wa.ldo = ldo; wa.out_fp32 = out_fp32; wa.status = status;
     wa.group_tiles = groups > 1 ? N / groups / 256 : 0;
     wa.group_k = K;
-    if (wide_split == 4) return launch_wide(tx2, tw2, wa, reinterpret_cast<cudaStream_t>(stream));
+    if (plan.kind == kGemmWide) return launch_wide(tx2, tw2, wa, reinterpret_cast<cudaStream_t>(stream));
     return launch_pair(tx2, tw2, wa, sm_count, reinterpret_cast<cudaStream_t>(stream));
   }
   int bt = stk_gemm_pick_bt(T, is_fp8);

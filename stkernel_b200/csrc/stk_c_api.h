@@ -47,6 +47,7 @@ int stk_gate_route_cluster(const void* W, long long ldw, const void* x, long lon
 int stk_gemm_pick_bt(int T, int is_fp8);
 int stk_gemm_pick_splits(int T, int N, int K, int is_fp8, int sm_count);
 long long stk_gemm_workspace_bytes(int T, int N, int splits);
+int stk_gemm_plan(int T, int N, int K, int groups, int is_fp8, int sm_count);
 int stk_gemm_token_tile_ctas(int T, int N, int K, int is_fp8, int sm_count);
 int stk_gemm(const void* W, long long ldw, const void* X, long long ldx, void* out, long long ldo, int T, int N, int K, int is_fp8, int out_fp32, const float* w_scale, int w_scale_ld, const float* x_scale, int x_scale_ld, int splits, float* workspace, int* counters, int* status, int sm_count, int groups, const void* ar_ctx, void* stream);
 int stk_gemm_tile(const void* W, long long ldw, const void* X, long long ldx, void* out, long long ldo, int T, int N, int K, int out_fp32, int bt, int splits, float* workspace, int* counters, int* status, int sm_count, void* stream);

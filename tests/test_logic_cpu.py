@@ -416,3 +416,24 @@ def test_expert_tiles_have_one_rule():
     from stkernel_b200.parallel.ep_moe import pick_bt
     for avg, rows in ((0.2, 16), (3.9, 16), (4, 32), (6.5, 32), (7, 64), (24.9, 64), (25, 128), (900, 128)):
         assert pick_bt(avg) == tile_rows(avg) == rows
+
+
+TILES, FP8_TOKENS, FP8_PAIR, SMALL, WIDE, PAIR = range(6)
+
+
+@pytest.mark.parametrize("T,N,K,groups,fp8,kind,ctas", [
+    (16, 1024, 4096, 1, 0, SMALL, 8), (64, 4096, 2048, 1, 0, SMALL, 4), (64, 4096, 448, 1, 0, TILES, 1), (64, 16384, 4096, 1, 0, TILES, 1),
+    (65, 1030, 2048, 1, 0, SMALL, 8), (97, 16, 4096, 1, 0, SMALL, 8), (128, 9472, 512, 1, 0, SMALL, 2), (128, 9473, 4096, 1, 0, PAIR, 2),
+    (97, 16, 448, 1, 0, PAIR, 2), (129, 16, 4096, 1, 0, WIDE, 4), (300, 4096, 4096, 1, 0, WIDE, 4), (777, 4096, 4096, 1, 0, PAIR, 2),
+    (4096, 8192, 2048, 1, 0, PAIR, 2), (100, 8192, 4096, 8, 0, SMALL, 2), (100, 16384, 4096, 8, 0, PAIR, 2), (100, 8320, 4096, 8, 0, TILES, 1),
+    (300, 8192, 4096, 8, 0, PAIR, 2), (300, 9216, 4096, 8, 0, TILES, 1),
+    (48, 4096, 8192, 1, 1, FP8_TOKENS, 4), (512, 16384, 4096, 1, 1, FP8_PAIR, 2), (4096, 4096, 8192, 1, 1, FP8_TOKENS, 1), (64, 4096, 1024, 4, 1, TILES, 1)])
+def test_which_kernel_takes_a_product(T, N, K, groups, fp8, kind, ctas):
+    """What the launcher itself asks: the kernel, and how many thread blocks share a tile (148 SMs)."""
+    from stkernel_b200.ops import _lib
+    if not _lib.available():
+        pytest.skip("the library is not built")
+    plan = _lib.query("stk_gemm_plan", T, N, K, groups, fp8, 148)
+    assert (plan // 16, plan % 16) == (kind, ctas)
+    if groups == 1:                                    # `linear` asks for workspace splits only where the 128-row tiles take the product
+        assert (_lib.query("stk_gemm_token_tile_ctas", T, N, K, fp8, 148) == 0) == (kind == TILES)
