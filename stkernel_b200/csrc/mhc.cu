@@ -353,7 +353,7 @@ mhc_finalize_rows_kernel(const __nv_bfloat16* __restrict__ x, const float* __res
       if (act) rs += other;
     }
     c = act ? e / rs + hc_eps : 0.f;
-    for (int it = 0; it < 2 * sinkhorn_iters - 1; ++it) {
+    for (int it = 0; it < max(2 * sinkhorn_iters - 1, 1); ++it) {
       // even steps normalise columns, odd steps rows
       const bool col = (it & 1) == 0;
       float s = c;
@@ -700,7 +700,7 @@ mhc_cluster_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
         row_src[o] = j * hc + ((k + o) % hc);
         col_src[o] = ((j + o) % hc) * hc + k;
       }
-      for (int it = 0; it < 2 * sinkhorn_iters - 1; ++it) {
+      for (int it = 0; it < max(2 * sinkhorn_iters - 1, 1); ++it) {
         // even steps normalise columns, odd steps rows
         const bool col = (it & 1) == 0;
         float s = c;

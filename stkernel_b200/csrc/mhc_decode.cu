@@ -292,7 +292,7 @@ mhc_decode_kernel(const MhcDecodeArgs a) {
 #pragma unroll
     for (int o = 1; o < 4; ++o) rs += __shfl_sync(0xffffffffu, e, row_src[o]);
     c = act ? e / rs + a.hc_eps : 0.f;
-    for (int it = 0; it < 2 * a.sinkhorn_iters - 1; ++it) {
+    for (int it = 0; it < max(2 * a.sinkhorn_iters - 1, 1); ++it) {
       const bool col = (it & 1) == 0;                 // even steps normalise columns, odd steps rows
       const float a1 = __shfl_sync(0xffffffffu, c, col ? col_src[1] : row_src[1]);
       const float a2 = __shfl_sync(0xffffffffu, c, col ? col_src[2] : row_src[2]);

@@ -154,6 +154,21 @@ def test_mhc_pre_in_whole_rows(H, norm):
     assert rel_err(Fn.mhc_post(x, res, post, comb), R.mhc_post(x, res, pr, cr)) < 5e-3
 
 
+@pytest.mark.parametrize("T", [5, 70, 300])
+@pytest.mark.parametrize("iters", [0, 1, 2])
+@pytest.mark.parametrize("H", [1024, 4608])
+def test_mhc_pre_of_few_normalisations(T, iters, H):
+    """Columns are normalised once whatever the number, in every kernel that serves a step: clusters, row dots, products of many tokens."""
+    torch.manual_seed(2)
+    hc = 4
+    res = torch.randn(T, hc, H, device=dev()).to(BF16)
+    fn = torch.randn(24, hc * H, device=dev()) * 0.02
+    base, scale = torch.randn(24, device=dev()), torch.tensor([1.0, 0.7, 1.3], device=dev())
+    _, _, comb = Fn.mhc_pre(res, fn, base, scale, None, 1e-6, 1e-6, iters)
+    _, _, cr = R.mhc_pre(res, fn, base, scale, None, 1e-6, 1e-6, iters, round_bf16=True)
+    assert torch.allclose(comb.view(T, hc, hc), cr, atol=1e-4, rtol=1e-3)
+
+
 @pytest.mark.parametrize("n,e_local,start", [(2049, 300, 0), (5000, 37, 3), (24576, 256, 0)])
 def test_moe_align_many_pairs(n, e_local, start):
     """Chunks and experts that fill neither a batch of counts nor a warp; pairs of other ranks' experts."""
