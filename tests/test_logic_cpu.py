@@ -379,9 +379,13 @@ def test_scratch_views_follow_mode_graph_growth_and_branch(monkeypatch):
     get = lambda *shape, dtype=torch.float32: S.scratch("t.views", shape, dtype, "cpu")
     with torch.inference_mode():
         a = get(2, 3)
+        a.fill_(1.0)
     b = get(2, 3)
     b.zero_()                                          # not an inference tensor, which refuses this
     assert a.data_ptr() == b.data_ptr() and get(2, 3) is b
+    with torch.inference_mode():
+        get(2, 3).fill_(2.0)
+    assert bool((b == 2.0).all())
     b.copy_(torch.ones(2, 3, requires_grad=True))      # b is part of a graph now
     assert not get(2, 3).requires_grad
     for shape in ((3, 2), (2, 3), (6,), (2, 3)):       # two shapes in turn
