@@ -76,7 +76,8 @@ def _kv_slots(text: str) -> Tuple[bool, str]:
 
 
 def _attn_slots(text: str) -> Tuple[bool, str]:
-    lo = _count(text, r"slot\s*(>=|<)\s*0")
+    # where a slot is followed, and where its row (listed as kNoRow if there is none) is given a weight
+    lo = _count(text, r"slot\s*(>=|<)\s*0|!=\s*kNoRow\b")
     return lo >= 2, f"gathered-row validity checks: {lo}/2"
 
 
