@@ -1853,7 +1853,8 @@ static int fp8_tokens_split(int T, int N, int K, int sm_count) {
 // rounds of single CTAs in 1.62 to 1.92 times the time of one, so they are taken where they need no more than half the rounds.
 // Measured, us, single / pair (rounds): 512 tokens x 16384 x 4096: 59 / 50 (4 / 2);  3000 x 4096 x 4096: 84 / 70 (6 / 3);
 //   4096 x 1024 x 8192: 55 / 46 (2 / 1);  4096 x 40960 x 1536: 456 / 424 (70 / 35);  1500 x 4096 x 8192: 79 / 86 (3 / 2);
-//   4096 x 4096 x 8192: 176 / 192 (7 / 4): at K = 8192 both run into the power limit (1.3 to 1.5 GHz).
+//   4096 x 4096 x 8192: 176 / 192 (7 / 4): at K = 8192 both run into the power limit (single CTAs: 1.66 to 1.70 GHz
+//   sampled at 1000 W).
 static bool fp8_pair_serves(int T, int N, int sm_count) {
   const int pairs = sm_count / 2;
   if (pairs < 1) return false;

@@ -259,8 +259,9 @@ def sparse_mla(q: torch.Tensor, swa_cache: PagedCache, swa_slots: torch.Tensor, 
     """q [T, nh, D] bf16 -> out [T, nh, D] bf16 attending to the SWA rows then the top-k rows.
 
     Only the first swa_lens[t] / topk_lens[t] entries of each list are read; -1 entries inside that
-    range are masked.  Finite values of any size are served; from nine tokens on (fp8 rows) what lies more than 2^17 below the
-    largest of its row, or of its head's queries, may be dropped.  inv_rope = (positions, inv_freq): also apply the inverse RoPE to the output's
+    range are masked.  From nine tokens on, finite queries and rows of any size are served; on the tensor-core
+    path (fp8 rows) what lies more than 2^17 below the largest of its row, or of its head's queries, may be dropped.  Up to eight
+    tokens the decode kernel multiplies in fp16, which normed queries and rows fit.  inv_rope = (positions, inv_freq): also apply the inverse RoPE to the output's
     rope dims (fused into the split-merge kernel on the tensor-core path).
     q_prep = (positions, inv_freq, eps): q is the raw projection output; its per-head weightless RMSNorm and RoPE are
     applied here (inside the decode kernel when it serves the step, else by the stand-alone op first).

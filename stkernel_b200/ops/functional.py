@@ -233,7 +233,7 @@ def linear(x, lw: LinearWeight, out: Optional[torch.Tensor] = None, out_dtype=BF
     if out is None:
         out = torch.empty(t, n, dtype=out_dtype, device=dev)
     if xa is None and ar_ctx is None and _skinny_ok(x, t, k, lw.is_fp8, n // max(groups, 1), n):
-        # one to four tokens: weight-streaming kernel, activations unquantised
+        # up to eight tokens: weight-streaming kernels (fp8 weights: activations unquantised up to four tokens, quantised inside above)
         _lib.call("stk_skinny_linear", lw.w, lw.w.stride(0), 1 if lw.is_fp8 else 0, lw.scale,
                   lw.scale.stride(0) if lw.is_fp8 else 0, x, x.stride(0), out, out.stride(0), t, n, k,
                   1 if out.dtype == F32 else 0, _lib.sm_count(), groups, 0, 0.0, _lib.stream())
