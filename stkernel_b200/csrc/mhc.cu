@@ -353,7 +353,7 @@ mhc_finalize_rows_kernel(const __nv_bfloat16* __restrict__ x, const float* __res
       if (act) rs += other;
     }
     c = act ? e / rs + hc_eps : 0.f;
-    for (int it = 0; it < max(2 * sinkhorn_iters - 1, 1); ++it) {
+    for (int it = 0; it < 2 * sinkhorn_iters - 1; ++it) {
       // even steps normalise columns, odd steps rows
       const bool col = (it & 1) == 0;
       float s = c;
@@ -498,6 +498,7 @@ STK_API int stk_mhc_finalize_rows(const void* x, const float* prod, int prod_ld,
                                   float hc_eps, int sinkhorn_iters, float post_mult, void* stream) {
   if (T <= 0) return 0;
   if (hc != 4 || H % 8 || H > 4 * 2048 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(norm_w)) & 15)) return -5;
+  if (sinkhorn_iters < 1) sinkhorn_iters = 1;             // columns are normalised once in any case
   cudaStream_t st = (cudaStream_t)stream;
 #define STK_FR(P_) mhc_finalize_rows_kernel<P_><<<T, 256, 0, st>>>((const __nv_bfloat16*)x, prod, prod_ld, lo_at, base, scale,     (const __nv_bfloat16*)norm_w, post, comb, (__nv_bfloat16*)y, H, rms_eps, hc_eps, sinkhorn_iters, post_mult)
   if (H <= 2048) STK_FR(1); else if (H <= 4096) STK_FR(2); else STK_FR(4);
@@ -700,7 +701,7 @@ mhc_cluster_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
         row_src[o] = j * hc + ((k + o) % hc);
         col_src[o] = ((j + o) % hc) * hc + k;
       }
-      for (int it = 0; it < max(2 * sinkhorn_iters - 1, 1); ++it) {
+      for (int it = 0; it < 2 * sinkhorn_iters - 1; ++it) {
         // even steps normalise columns, odd steps rows
         const bool col = (it & 1) == 0;
         float s = c;
@@ -814,6 +815,7 @@ static int mhc_cluster_launch(const void* x, const float* fn, const float* base,
                               float* post, float* comb, void* y, int T, int H, int hc, int n_mix, float rms_eps,
                               float hc_eps, int sinkhorn_iters, float post_mult, int mode, const MhcFuse& fz, void* stream) {
   if (T <= 0) return 0;
+  if (sinkhorn_iters < 1) sinkhorn_iters = 1;             // columns are normalised once in any case
   if (fz.fa != nullptr && (hc > 4 || H % 4 || ((H * hc / kClusterSize + 1) & ~1) % 4)) return -3;
   if (hc * hc > 32 || H % 2 || H > kClusterSize * kClusterThreads * 2 * 2 || (H * hc) % 2) return -1;
   cudaLaunchConfig_t cfg = {};

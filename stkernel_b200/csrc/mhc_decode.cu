@@ -292,7 +292,7 @@ mhc_decode_kernel(const MhcDecodeArgs a) {
 #pragma unroll
     for (int o = 1; o < 4; ++o) rs += __shfl_sync(0xffffffffu, e, row_src[o]);
     c = act ? e / rs + a.hc_eps : 0.f;
-    for (int it = 0; it < max(2 * a.sinkhorn_iters - 1, 1); ++it) {
+    for (int it = 0; it < 2 * a.sinkhorn_iters - 1; ++it) {
       const bool col = (it & 1) == 0;                 // even steps normalise columns, odd steps rows
       const float a1 = __shfl_sync(0xffffffffu, c, col ? col_src[1] : row_src[1]);
       const float a2 = __shfl_sync(0xffffffffu, c, col ? col_src[2] : row_src[2]);
@@ -416,7 +416,9 @@ STK_API int stk_mhc_decode(const void* x, const void* fa, const void* res_old, c
   a.norm_w = (const __nv_bfloat16*)norm_w;
   a.post = post; a.comb = comb;
   a.y = (__nv_bfloat16*)y;
-  a.H = H; a.rms_eps = rms_eps; a.hc_eps = hc_eps; a.sinkhorn_iters = sinkhorn_iters; a.post_mult = post_mult;
+  a.H = H; a.rms_eps = rms_eps; a.hc_eps = hc_eps;
+  a.sinkhorn_iters = sinkhorn_iters < 1 ? 1 : sinkhorn_iters;      // columns are normalised once in any case
+  a.post_mult = post_mult;
   a.status = status;
   if (x == nullptr) {
     if (res_old == nullptr || post_old == nullptr || comb_old == nullptr || x_out == nullptr || x_out == res_old) return -2;
