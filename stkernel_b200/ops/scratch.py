@@ -53,8 +53,10 @@ def scratch(name: str, shape: Sequence[int], dtype: torch.dtype, device, zero: b
     last = _views.get(place)
     if last is not None and last[0] == shape and last[1] is dtype and _pool.get(last[4]) is last[2] and not last[3].requires_grad:
         return last[3]
-    with torch.inference_mode(False):
-        return _cut(name, shape, dtype, device, zero, place)
+    if torch.is_inference_mode_enabled():
+        with torch.inference_mode(False):
+            return _cut(name, shape, dtype, device, zero, place)
+    return _cut(name, shape, dtype, device, zero, place)
 
 
 def _cut(name: str, shape: tuple, dtype: torch.dtype, device, zero: bool, place: tuple) -> torch.Tensor:
